@@ -171,6 +171,24 @@ int gather_clauses(const GatherArgs &a, cudaStream_t stream, int sm_count);
 // or, with cell_words > 0, 8-byte {clause * cell_words + word, mask} records.
 int launch_pack_reports(const gss_report *parts, const uint32_t *counts, uint32_t n_parts, uint32_t cap,
                         uint32_t cell_words, uint32_t *packed, cudaStream_t stream, int sm_count);
+// What a pass's counters buffer holds: the n_parts report counters, then the
+// kernel's error flag and the work counter of the persistent kernels. One
+// memset clears them all.
+constexpr uint32_t kExtraCounters = 2;
+__host__ __device__ __forceinline__ uint32_t *err_counter(uint32_t *counts, uint32_t n_parts) {
+    return counts + n_parts;
+}
+__host__ __device__ __forceinline__ uint32_t *work_counter(uint32_t *counts, uint32_t n_parts) {
+    return counts + n_parts + 1;
+}
+// Hands a pass's outcome to the host: writes the n_parts counters and the
+// error flag to `host` (pinned), and, when the pass has at most max_inline
+// records and no partition overflowed, the records too, partition after
+// partition from byte kInlineOffset on. With d_args the queues are those of
+// the arguments in device memory (a captured graph outlives a queue's growth).
+constexpr size_t kInlineOffset = 256;
+int launch_deliver(const CheckArgs *d_args, const gss_report *parts, const uint32_t *counts, uint32_t n_parts,
+                   uint32_t cap, void *host, uint32_t max_inline, cudaStream_t stream);
 // Synchronizes `stream`; returns the live clause and literal counts.
 int compact_by_id(const CompactArgs &a, cudaStream_t stream, int sm_count, uint32_t *n_out, int64_t *lits_out);
 

@@ -168,8 +168,8 @@ int ensure_queues(gss_engine *eng) {
         GSS_TRY(eng->reports.reserve((size_t) per * eng->n_parts * sizeof(gss_report)));
         eng->cap_per_part = (uint32_t) per;
     }
-    GSS_TRY(eng->counts.reserve(sizeof(uint32_t) * eng->n_parts));
-    GSS_TRY(eng->h_counts.reserve(sizeof(uint32_t) * (eng->n_parts + 1)));
+    GSS_TRY(eng->counts.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
+    GSS_TRY(eng->h_counts.reserve(kInlineOffset + (size_t) kEngineInline * sizeof(gss_report)));
     return GSS_OK;
 }
 
@@ -739,10 +739,11 @@ int gss_check_set_capacity(gss_engine *eng, int64_t records) {
 namespace {
 
 // Launches one check pass of the engine's database against `state` (laid out
-// as the engine's current state), into `reports`/`counts`, then copies the
-// counts and the error flag into `h_counts` (pinned), all on the engine's
-// stream.
-int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf &counts, PinnedBuf &h_counts);
+// as the engine's current state), into `reports`/`counts`, then hands the
+// counts, the error flag and up to max_inline records to `h_counts` (pinned),
+// all on the engine's stream.
+int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf &counts, PinnedBuf &h_counts,
+                     uint32_t max_inline);
 
 }  // namespace
 
@@ -750,9 +751,10 @@ int gss_check_launch(gss_engine *eng) {
     if (!eng) return set_error(GSS_ERR_INVALID, "engine is NULL");
     GSS_TRY(ensure_device(eng));
     GSS_TRY(ensure_queues(eng));
-    GSS_TRY(launch_pass_into(eng, eng->state.ptr, eng->reports, eng->counts, eng->h_counts));
+    GSS_TRY(launch_pass_into(eng, eng->state.ptr, eng->reports, eng->counts, eng->h_counts, kEngineInline));
     eng->launches++;
     eng->pass_pending = true;
+    eng->inline_ok = true;
     return GSS_OK;
 }
 
@@ -807,7 +809,8 @@ int build_plan(gss_engine *eng) {
     return GSS_OK;
 }
 
-int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf &counts, PinnedBuf &h_counts) {
+int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf &counts, PinnedBuf &h_counts,
+                     uint32_t max_inline) {
     order_quiesce(eng);  // a scoring in flight reads the buffers this pass may reallocate
     if (eng->n_clauses > 0 && eng->max_var >= eng->n_vars)
         return set_error(GSS_ERR_INVALID, "database uses variable %lld but the state has %lld variables",
@@ -851,14 +854,15 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
         }
         a.alive = (const uint32_t *) eng->alive.ptr;
     }
-    GSS_TRY(eng->err.reserve(sizeof(uint32_t)));
-    a.err = (uint32_t *) eng->err.ptr;
     a.start = (const uint32_t *) eng->start.ptr;
     a.solver_of_word = (const int32_t *) eng->solver_of_word.ptr;
     a.out = (gss_report *) reports.ptr;
     a.counts = (uint32_t *) counts.ptr;
     a.n_parts = eng->n_parts;
     a.cap_per_part = eng->cap_per_part;
+    a.err = err_counter(a.counts, a.n_parts);
+    uint32_t *const work = work_counter(a.counts, a.n_parts);
+    const size_t counter_bytes = sizeof(uint32_t) * (a.n_parts + kExtraCounters);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (eng->timing) {
         for (cudaEvent_t *ev : {&ev0, &ev1}) {
@@ -894,34 +898,28 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
         // arguments through device memory, so the same graph serves every pass
         if (bucketed) GSS_TRY(build_plan(eng));
         GSS_TRY(eng->d_args.reserve(sizeof(CheckArgs)));
-        GSS_TRY(eng->work.reserve(sizeof(uint32_t)));
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->d_args.ptr, &a, sizeof a, cudaMemcpyHostToDevice, eng->stream));
         if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
         auto body = [&]() -> int {
-            GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, sizeof(uint32_t) * a.n_parts, eng->stream));
-            GSS_CUDA_TRY(cudaMemsetAsync(a.err, 0, sizeof(uint32_t), eng->stream));
-            GSS_CUDA_TRY(cudaMemsetAsync(eng->work.ptr, 0, sizeof(uint32_t), eng->stream));
+            GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes, eng->stream));
             if (a.n_clauses > 0 && a.n_blocks > 0) {
                 if (bucketed) {
                     if (eng->plan_ranges > 0)
                         GSS_TRY(launch_check_bucketed((const CheckArgs *) eng->d_args.ptr,
-                                                      (const BucketPlan *) eng->d_plan.ptr, (uint32_t *) eng->work.ptr,
-                                                      eng->stream, eng->sm_count));
+                                                      (const BucketPlan *) eng->d_plan.ptr, work, eng->stream,
+                                                      eng->sm_count));
                 } else {
                     GSS_TRY(launch_check_wide_persist((const CheckArgs *) eng->d_args.ptr, a,
                                                       words_per_lane(eng->state_kind), eng->state_lpc, eng->state_g,
-                                                      (uint32_t *) eng->work.ptr, eng->stream, eng->sm_count));
+                                                      work, eng->stream, eng->sm_count));
                 }
             }
-            GSS_CUDA_TRY(cudaMemcpyAsync(h_counts.ptr, counts.ptr, sizeof(uint32_t) * eng->n_parts,
-                                         cudaMemcpyDeviceToHost, eng->stream));
-            GSS_CUDA_TRY(cudaMemcpyAsync((uint32_t *) h_counts.ptr + eng->n_parts, a.err, sizeof(uint32_t),
-                                         cudaMemcpyDeviceToHost, eng->stream));
-            return GSS_OK;
+            return launch_deliver((const CheckArgs *) eng->d_args.ptr, a.out, a.counts, a.n_parts, a.cap_per_part,
+                                  h_counts.ptr, max_inline, eng->stream);
         };
         if (eng->use_graph) {
             const std::vector<uintptr_t> key = {
-                (uintptr_t) a.counts, (uintptr_t) h_counts.ptr, (uintptr_t) a.err, (uintptr_t) eng->work.ptr,
+                (uintptr_t) a.counts, (uintptr_t) h_counts.ptr, (uintptr_t) max_inline,
                 (uintptr_t) eng->d_args.ptr, (uintptr_t) eng->state_kind, (uintptr_t) eng->state_lpc,
                 (uintptr_t) eng->state_g, (uintptr_t) eng->n_parts, (uintptr_t) (a.n_clauses > 0 && a.n_blocks > 0),
                 (uintptr_t) bucketed, (uintptr_t) eng->d_plan.ptr, (uintptr_t) (eng->plan_ranges > 0)};
@@ -951,18 +949,18 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
         }
         return GSS_OK;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, sizeof(uint32_t) * a.n_parts, eng->stream));
-    GSS_CUDA_TRY(cudaMemsetAsync(a.err, 0, sizeof(uint32_t), eng->stream));
+    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes, eng->stream));
     if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
-    if (persistent) GSS_TRY(eng->work.reserve(sizeof(uint32_t)));
+    bool work_used = false;  // the memset above cleared the work counter for the first launch
     auto launch = [&](const CheckArgs &args) -> int {
         if (eng->state_kind == GSS_KERNEL_TILED) return launch_check_tiled(args, eng->stream, eng->sm_count);
         if (persistent) {
             // arguments by value; the work counter restarts for each launch
-            GSS_CUDA_TRY(cudaMemsetAsync(eng->work.ptr, 0, sizeof(uint32_t), eng->stream));
+            if (work_used) GSS_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(uint32_t), eng->stream));
+            work_used = true;
             if (args.n_clauses == 0 || args.n_blocks == 0 || scan_count(args) == 0) return GSS_OK;
             return launch_check_wide_persist(nullptr, args, words_per_lane(eng->state_kind), eng->state_lpc,
-                                             eng->state_g, (uint32_t *) eng->work.ptr, eng->stream, eng->sm_count);
+                                             eng->state_g, work, eng->stream, eng->sm_count);
         }
         const int occ = (eng->flags & GSS_VARIANT_OCCUPANCY) ? 1 : 0;
         if (wide && (eng->flags & GSS_VARIANT_PIPELINED))
@@ -993,11 +991,7 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
         GSS_CUDA_TRY(cudaEventRecord(ev1, eng->stream));
         eng->ev_pending.emplace_back(ev0, ev1);
     }
-    GSS_CUDA_TRY(cudaMemcpyAsync(h_counts.ptr, counts.ptr, sizeof(uint32_t) * eng->n_parts, cudaMemcpyDeviceToHost,
-                                 eng->stream));
-    GSS_CUDA_TRY(cudaMemcpyAsync((uint32_t *) h_counts.ptr + eng->n_parts, a.err, sizeof(uint32_t),
-                                 cudaMemcpyDeviceToHost, eng->stream));
-    return GSS_OK;
+    return launch_deliver(nullptr, a.out, a.counts, a.n_parts, a.cap_per_part, h_counts.ptr, max_inline, eng->stream);
 }
 
 }  // namespace
@@ -1041,6 +1035,10 @@ int gss_check_copy_reports(gss_engine *eng, gss_report *out, int64_t cap, int64_
                                       (long long) total);
     if (total == 0) return GSS_OK;
     const uint32_t *hc = (const uint32_t *) eng->h_counts.ptr;
+    if (eng->inline_ok && total <= (int64_t) kEngineInline) {
+        memcpy(out, (const char *) eng->h_counts.ptr + kInlineOffset, (size_t) total * sizeof(gss_report));
+        return GSS_OK;
+    }
     int64_t pos = 0;
     for (uint32_t p = 0; p < eng->n_parts; p++) {
         if (hc[p] == 0) continue;
@@ -1096,6 +1094,7 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
     // layout, start and solver words from the first pass (copies its state too)
     GSS_TRY(gss_state_set(eng, states[0], n_vars, n_words, start, solver_of_word, 0));
     GSS_TRY(ensure_queues(eng));
+    eng->inline_ok = false;  // the slots' records stay on the device until they are copied
     const bool direct = eng->n_blocks == 1 && eng->n_words == eng->state_bw;
     const size_t sbytes = (size_t) n_vars * n_words * 2 * sizeof(uint32_t);
     const size_t bbytes = (size_t) eng->n_blocks * n_vars * eng->state_bw * sizeof(uint2);
@@ -1120,8 +1119,8 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         return GSS_OK;
     };
     GSS_TRY(reserve_reports());
-    GSS_TRY(eng->counts2.reserve(sizeof(uint32_t) * eng->n_parts));
-    GSS_TRY(eng->counts3.reserve(sizeof(uint32_t) * eng->n_parts));
+    GSS_TRY(eng->counts2.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
+    GSS_TRY(eng->counts3.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
     auto reserve_packed = [&]() -> int {
         for (int b = 0; b < NB && packed; b++)
             GSS_TRY(eng->packed[b].reserve((size_t) eng->cap_per_part * eng->n_parts * rec_words * sizeof(uint32_t)));
@@ -1168,13 +1167,13 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
             GSS_TRY(ensure_queues(eng));
             GSS_TRY(reserve_reports());
             GSS_TRY(reserve_packed());
-            GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b]));
+            GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
             GSS_TRY(pack(b, *rep_buf[b], *cnt_buf[b]));
             eng->launches++;
             GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[b], eng->stream));
             if (j + 1 < launched) {
                 const int nb = (j + 1) % NB;
-                GSS_TRY(launch_pass_into(eng, state_buf[nb]->ptr, *rep_buf[nb], *cnt_buf[nb], *hcnt_buf[nb]));
+                GSS_TRY(launch_pass_into(eng, state_buf[nb]->ptr, *rep_buf[nb], *cnt_buf[nb], *hcnt_buf[nb], 0));
                 GSS_TRY(pack(nb, *rep_buf[nb], *cnt_buf[nb]));
                 eng->launches++;
                 GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[nb], eng->stream));
@@ -1224,7 +1223,7 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         }
         // report set b is free once pass i-3's reports are back
         if (i >= NB) GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_d2h[b], 0));
-        GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b]));
+        GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
         GSS_TRY(pack(b, *rep_buf[b], *cnt_buf[b]));
         eng->launches++;
         launched = i + 1;

@@ -48,7 +48,6 @@ struct gss_engine {
     // kernel variant: kind (GSS_KERNEL_*), lanes (words) per clause (0 = pick
     // from the word count), loads in flight / clause slots, cache hints
     int kind = GSS_KERNEL_AUTO, lpc = 0, g = 2, flags = 0;
-    DevBuf err;
 
     // assignment state, block-major [n_blocks][n_vars][state_bw words]
     DevBuf state, state_raw, start, solver_of_word;
@@ -67,7 +66,10 @@ struct gss_engine {
     uint32_t n_parts = 16;
     uint32_t cap_per_part = 0;
     int64_t requested_cap = 0;
+    // counters, error flag and, up to kEngineInline records, the pass's
+    // reports (launch_deliver); inline_ok: of the pass launched last
     PinnedBuf h_counts;
+    bool inline_ok = false;
     bool pass_pending = false;
 
     // pipelined passes through host buffers (gss_check_passes_host): second
@@ -80,10 +82,10 @@ struct gss_engine {
     cudaStream_t h2d = nullptr, d2h = nullptr;
     cudaEvent_t ev_h2d[3] = {}, ev_kernel[3] = {}, ev_d2h[3] = {};
 
-    // persistent kernel: arguments in device memory, task counter; optional
+    // persistent kernel: arguments in device memory; optional
     // CUDA graph of a pass (memsets, kernel, count readback), recaptured when
     // a buffer it names changes
-    DevBuf d_args, work;
+    DevBuf d_args;
     // length plan of the bucketed kernel (gss_engine_set_length_plan): class
     // bounds and lane layouts; the position ranges are rebuilt on the device
     // when plan_built differs from db_version
@@ -112,6 +114,11 @@ struct gss_engine {
 
 
 namespace gss {
+// Records that come back with the counters (1 MB of pinned memory); a pass
+// with more is fetched with a copy per partition, whose fixed cost is then
+// below the copies' own time.
+constexpr uint32_t kEngineInline = 65536;
+
 // Learned scan order hooks, called by the engine's pass (order.cu).
 // Before the scan: the scan permutation of this pass (computed while the
 // previous pass ran, or now on the engine's stream). It covers positions

@@ -1133,9 +1133,10 @@ int order_prepare(gss_engine *eng, const uint32_t **perm, uint32_t *head, uint32
 int order_after_head(gss_engine *eng, const DevBuf &counts) {
     OrderState &o = *eng->order;
     GSS_CUDA_TRY(cudaEventRecord(o.ev[2], eng->stream));
-    GSS_TRY(o.h_head_counts.reserve(sizeof(uint32_t) * (eng->n_parts + 1)));
-    GSS_CUDA_TRY(cudaMemcpyAsync(o.h_head_counts.ptr, counts.ptr, sizeof(uint32_t) * eng->n_parts,
-                                 cudaMemcpyDeviceToHost, eng->stream));
+    // the head's counts and records, on their way while the tail runs
+    GSS_TRY(o.h_head_counts.reserve(kInlineOffset + (size_t) kEngineInline * sizeof(gss_report)));
+    GSS_TRY(launch_deliver(nullptr, (const gss_report *) eng->reports.ptr, (const uint32_t *) counts.ptr, eng->n_parts,
+                           eng->cap_per_part, o.h_head_counts.ptr, kEngineInline, eng->stream));
     GSS_CUDA_TRY(cudaEventRecord(o.ev[4], eng->stream));
     o.pending = true;
     return GSS_OK;
@@ -1300,6 +1301,10 @@ int gss_check_wait_head(gss_engine *eng, gss_report *out, int64_t cap, int64_t *
     if (n_reports) *n_reports = total;
     if (total > cap) return set_error(GSS_ERR_OVERFLOW, "output holds %lld records, the head has %lld",
                                       (long long) cap, (long long) total);
+    if (total <= (int64_t) kEngineInline) {
+        memcpy(out, (const char *) o.h_head_counts.ptr + kInlineOffset, (size_t) total * sizeof(gss_report));
+        return GSS_OK;
+    }
     if (!eng->d2h) GSS_CUDA_TRY(cudaStreamCreateWithFlags(&eng->d2h, cudaStreamNonBlocking));
     int64_t pos = 0;
     for (uint32_t q = 0; q < eng->n_parts; q++) {
@@ -1327,6 +1332,16 @@ int gss_check_copy_tail(gss_engine *eng, gss_report *out, int64_t cap, int64_t *
     if (n > cap) return set_error(GSS_ERR_OVERFLOW, "output holds %lld records, the tail has %lld", (long long) cap,
                                   (long long) n);
     int64_t pos = 0;
+    if (eng->inline_ok && total <= (int64_t) kEngineInline) {
+        // the pass's records came with its counters: each partition's tail
+        const gss_report *all = (const gss_report *) ((const char *) eng->h_counts.ptr + kInlineOffset);
+        for (uint32_t q = 0; q < eng->n_parts; q++) {
+            memcpy(out + pos, all + hc[q], (size_t) (ac[q] - hc[q]) * sizeof(gss_report));
+            pos += ac[q] - hc[q];
+            all += ac[q];
+        }
+        return GSS_OK;
+    }
     for (uint32_t q = 0; q < eng->n_parts; q++) {
         if (ac[q] == hc[q]) continue;
         GSS_CUDA_TRY(cudaMemcpyAsync(out + pos,

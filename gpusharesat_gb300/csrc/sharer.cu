@@ -229,12 +229,11 @@ int Sharer::init(int device) {
     for (Pass &p : pass_) {
         GSS_CUDA_TRY(cudaEventCreateWithFlags(&p.counted, cudaEventDisableTiming));
         GSS_CUDA_TRY(cudaEventCreateWithFlags(&p.copied, cudaEventDisableTiming));
-        GSS_TRY(p.d_counts.reserve(sizeof(uint32_t) * n_parts_));
-        GSS_TRY(p.h_counts.reserve(sizeof(uint32_t) * (n_parts_ + 1)));
+        GSS_TRY(p.d_counts.reserve(sizeof(uint32_t) * (n_parts_ + kExtraCounters)));
+        GSS_TRY(p.h_counts.reserve(kInlineOffset + (size_t) kSharerInline * sizeof(gss_report)));
     }
     GSS_CUDA_TRY(cudaEventCreateWithFlags(&alive_staged_, cudaEventDisableTiming));
     GSS_CUDA_TRY(cudaEventCreateWithFlags(&append_staged_, cudaEventDisableTiming));
-    GSS_TRY(d_err_.reserve(sizeof(uint32_t)));
     // one solver until told otherwise (HostAssigs constructor, Assigs.cu:311)
     return set_solver_count(1);
 }
@@ -891,7 +890,7 @@ int Sharer::run_check(Pass &p) {
     a.lpc = eff_lpc_;
     a.g = eff_depth_;
     a.cache_hints = (flags_ & GSS_VARIANT_L2_HINT) ? 1 : 0;
-    a.err = (uint32_t *) d_err_.ptr;
+    a.err = err_counter(a.counts, n_parts_);
     a.alive = nullptr;
     if (dev_dead_ > 0) {
         // evicted clauses still on the device: skipped through the bitmap
@@ -899,28 +898,22 @@ int Sharer::run_check(Pass &p) {
         a.alive = (const uint32_t *) d_alive_.ptr;
         a.alive_by_id = 1;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, sizeof(uint32_t) * n_parts_, stream_));
-    GSS_CUDA_TRY(cudaMemsetAsync(a.err, 0, sizeof(uint32_t), stream_));
+    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, sizeof(uint32_t) * (n_parts_ + kExtraCounters), stream_));
     if (p.active_words > 0 && p.n_clauses > 0) {
         const int wpl = eff_kind_ == GSS_KERNEL_WIDE4 ? 4 : 2;
         const bool wide = eff_kind_ == GSS_KERNEL_WIDE4 || eff_kind_ == GSS_KERNEL_WIDE2;
         if (wide && ((flags_ & GSS_VARIANT_PERSISTENT) ||
                      (kind_ == GSS_KERNEL_AUTO && valid_wide_persist_variant(wpl, eff_lpc_, eff_depth_)))) {
             // the persistent form, as the engine's automatic variant
-            GSS_TRY(d_work_.reserve(sizeof(uint32_t)));
-            GSS_CUDA_TRY(cudaMemsetAsync(d_work_.ptr, 0, sizeof(uint32_t), stream_));
-            GSS_TRY(launch_check_wide_persist(nullptr, a, wpl, eff_lpc_, eff_depth_, (uint32_t *) d_work_.ptr, stream_,
-                                              sm_count_));
+            GSS_TRY(launch_check_wide_persist(nullptr, a, wpl, eff_lpc_, eff_depth_, work_counter(a.counts, n_parts_),
+                                              stream_, sm_count_));
         } else if (wide) {
             GSS_TRY(launch_check_wide(a, wpl, (flags_ & GSS_VARIANT_OCCUPANCY) ? 1 : 0, stream_, sm_count_));
         } else {
             GSS_TRY(launch_check(a, stream_, sm_count_));
         }
     }
-    GSS_CUDA_TRY(cudaMemcpyAsync(p.h_counts.ptr, p.d_counts.ptr, sizeof(uint32_t) * n_parts_, cudaMemcpyDeviceToHost,
-                                 stream_));
-    GSS_CUDA_TRY(cudaMemcpyAsync((uint32_t *) p.h_counts.ptr + n_parts_, d_err_.ptr, sizeof(uint32_t),
-                                 cudaMemcpyDeviceToHost, stream_));
+    GSS_TRY(launch_deliver(nullptr, a.out, a.counts, n_parts_, p.cap_per_part, p.h_counts.ptr, kSharerInline, stream_));
     GSS_CUDA_TRY(cudaEventRecord(p.counted, stream_));
     return GSS_OK;
 }
@@ -946,6 +939,10 @@ int Sharer::collect(Pass &p) {
         }
         if (!overflow) {
             p.n_reports = total;
+            if (total <= (int64_t) kSharerInline) {  // already here, with the counters
+                p.reports = (const gss_report *) ((const char *) p.h_counts.ptr + kInlineOffset);
+                break;
+            }
             GSS_TRY(p.h_reports.reserve(std::max<size_t>((size_t) total, 1) * sizeof(gss_report)));
             int64_t pos = 0;
             for (uint32_t q = 0; q < n_parts_; q++) {
@@ -955,6 +952,7 @@ int Sharer::collect(Pass &p) {
                                              hc[q] * sizeof(gss_report), cudaMemcpyDeviceToHost, stream_));
                 pos += hc[q];
             }
+            p.reports = (const gss_report *) p.h_reports.ptr;
             break;
         }
         if (attempt >= 3) return set_error(GSS_ERR_OVERFLOW, "report queues kept overflowing");
@@ -987,7 +985,7 @@ int Sharer::note_reports(Pass &p) {
     // (GpuRunner::gatherGpuRunResults, gpuShareLib/GpuRunner.cu:360-378).
     if (!p.collected || p.noted) return GSS_OK;
     GSS_CUDA_TRY(cudaEventSynchronize(p.copied));
-    const gss_report *rep = (const gss_report *) p.h_reports.ptr;
+    const gss_report *rep = p.reports;
     stats_[kGpuRuns]++;
     stats_[kTotalAssigClauseTested] += (int64_t) p.n_clauses * p.assig_total;
     stats_[kClauseTestsOnGroups] += p.n_clauses;
@@ -1007,7 +1005,7 @@ int Sharer::deliver(Pass &p) {
     if (!p.collected) return GSS_OK;
     GSS_TRY(note_reports(p));
     const int64_t t1 = now_us();
-    const gss_report *rep = (const gss_report *) p.h_reports.ptr;
+    const gss_report *rep = p.reports;
     std::vector<ClauseBatch *> batch(reported_.size(), nullptr);
     for (size_t s = 0; s < p.assig.size() && s < reported_.size(); s++) {
         if (p.assig[s].count > 0) {

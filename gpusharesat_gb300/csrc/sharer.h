@@ -19,6 +19,8 @@ namespace gss {
 // Values as the reference's lbool: 0 true, 1 false, 2 undefined
 // (gpuShareLib/SolverTypes.h:81-83).
 constexpr uint8_t kTrue = 0, kFalse = 1, kUndef = 2;
+// records that come back with a pass's counters (256 KB of pinned memory)
+constexpr uint32_t kSharerInline = 16384;
 constexpr int kSlots = 32;  // assignments per solver per pass (Assigs.cuh:37-39)
 
 // Statistics, in the reference's order and with its names
@@ -185,9 +187,11 @@ private:
         // counters (+ error flag), the start and last-slot masks and the reports
         DevBuf d_reports, d_counts;
         uint32_t cap_per_part = 0;
+        // (+ up to kSharerInline reports, launch_deliver)
         PinnedBuf h_counts, h_start, h_last, h_reports;
-        cudaEvent_t counted = nullptr;  // counts copied to h_counts
-        cudaEvent_t copied = nullptr;   // reports copied to h_reports
+        const gss_report *reports = nullptr;  // the collected reports: in h_counts or h_reports
+        cudaEvent_t counted = nullptr;  // counts in h_counts
+        cudaEvent_t copied = nullptr;   // reports in place
     };
 
     int collect(Pass &p);
@@ -278,7 +282,6 @@ private:
     int eff_kind_ = GSS_KERNEL_DIRECT, eff_lpc_ = 1, eff_depth_ = 2, bw_ = 1, n_blocks_ = 0;
 
     // reports: two passes, alternating (the one launched last is pass_[cur_])
-    DevBuf d_err_, d_work_;  // kernel error flag, persistent kernel's task counter
     uint32_t n_parts_ = 16;
     uint32_t report_cap_ = 0;  // records per partition that earlier passes needed
     Pass pass_[2];
