@@ -36,22 +36,11 @@
 // partition keeps counting, so the host sees the overflow and runs again.
 #include <string.h>
 
-
-#include "common.h"
+#include "check_rows.cuh"
 
 namespace gss {
 
 namespace {
-
-constexpr int kWarps = 8;     // warps per block
-constexpr int kStage = 128;   // staged records per warp
-constexpr unsigned kFull = 0xFFFFFFFFu;
-
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
 
 // L2 eviction-priority policies (createpolicy): the slot block's state is
 // kept (evict-last), the clause literals stream past it (evict-first).
@@ -88,27 +77,6 @@ __device__ __forceinline__ int32_t ld_lit(const int32_t *p, bool hint, uint64_t 
         asm("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
     }
     return v;
-}
-
-// Writes a warp's staged records: one atomic reservation, then the records.
-// streaming = cache-streaming stores (the records are read back by the host,
-// not by the kernel: they need not displace state rows from L2).
-__device__ __forceinline__ void flush_stage(gss_report *stage, uint32_t n, gss_report *out, uint32_t *counter,
-                                            uint32_t cap, int lane, bool streaming = false) {
-    __syncwarp();
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(counter, n);
-    base = __shfl_sync(kFull, base, 0);
-    for (uint32_t i = lane; i < n; i += 32) {
-        uint32_t idx = base + i;
-        if (idx < cap) {
-            if (streaming)
-                __stcs(reinterpret_cast<int4 *>(out + idx), *reinterpret_cast<const int4 *>(stage + i));
-            else
-                out[idx] = stage[i];
-        }
-    }
-    __syncwarp();
 }
 
 template <int LPC, int G>
@@ -213,40 +181,6 @@ __global__ void __launch_bounds__(kWarps * 32) check_kernel(CheckArgs a) {
 // a clause, and the slot block is LPC * WPL words. With WPL = 4 and LPC = 8 a
 // warp checks 4 clauses against all 1024 slots of a 32-word pass with one
 // load instruction per literal step: 4 rows of 256 contiguous bytes.
-template <int WPL>
-struct Row;
-template <>
-struct Row<1> {
-    uint32_t v[2];
-};
-template <>
-struct Row<2> {
-    uint32_t v[4];
-};
-template <>
-struct Row<4> {
-    uint32_t v[8];
-};
-
-template <int WPL>
-__device__ __forceinline__ void ld_row(const uint2 *p, Row<WPL> &r);
-template <>
-__device__ __forceinline__ void ld_row<1>(const uint2 *p, Row<1> &r) {
-    asm("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(r.v[0]), "=r"(r.v[1]) : "l"(p));
-}
-template <>
-__device__ __forceinline__ void ld_row<2>(const uint2 *p, Row<2> &r) {
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-        : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "l"(p));
-}
-template <>
-__device__ __forceinline__ void ld_row<4>(const uint2 *p, Row<4> &r) {
-    asm("ld.global.nc.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
-          "=r"(r.v[7])
-        : "l"(p));
-}
-
 // The same gathers with an L2 eviction policy (cache_hints on).
 template <int WPL>
 __device__ __forceinline__ void ld_row_hint(const uint2 *p, Row<WPL> &r, uint64_t pol);
@@ -704,22 +638,6 @@ int launch_wide_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
     return GSS_OK;
 }
 
-// Host layout [n_vars][n_words]{isDef,isTrue} -> block-major
-// [n_blocks][n_vars][lpc]{isDef,isTrue}, words past n_words zero.
-__global__ void relayout_kernel(const uint2 *__restrict__ src, uint2 *__restrict__ dst, uint32_t n_vars,
-                                uint32_t n_words, uint32_t lpc, uint32_t n_blocks) {
-    const uint64_t total = (uint64_t) n_blocks * n_vars * lpc;
-    for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (uint64_t) gridDim.x * blockDim.x) {
-        const uint32_t s = (uint32_t) (i % lpc);
-        const uint64_t r = i / lpc;
-        const uint32_t v = (uint32_t) (r % n_vars);
-        const uint32_t b = (uint32_t) (r / n_vars);
-        const uint32_t w = b * lpc + s;
-        dst[i] = (w < n_words) ? src[(uint64_t) v * n_words + w] : make_uint2(0u, 0u);
-    }
-}
-
 template <int LPC, int G>
 int launch_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
     int per_sm = 0;
@@ -838,18 +756,6 @@ int launch_check(const CheckArgs &a, cudaStream_t stream, int sm_count) {
     GSS_VARIANT(32, 1) GSS_VARIANT(32, 2) GSS_VARIANT(32, 4) GSS_VARIANT(32, 8)
 #undef GSS_VARIANT
     return set_error(GSS_ERR_INVALID, "no kernel variant for %d lanes per clause, depth %d", a.lpc, a.g);
-}
-
-int launch_relayout(const uint2 *src, uint2 *dst, uint32_t n_vars, uint32_t n_words, uint32_t lpc,
-                    uint32_t n_blocks, cudaStream_t stream, int sm_count) {
-    const uint64_t total = (uint64_t) n_blocks * n_vars * lpc;
-    if (total == 0) return GSS_OK;
-    uint64_t blocks = (total + 255) / 256;
-    const uint64_t cap = (uint64_t) sm_count * 8;
-    if (blocks > cap) blocks = cap;
-    relayout_kernel<<<(unsigned) blocks, 256, 0, stream>>>(src, dst, n_vars, n_words, lpc, n_blocks);
-    GSS_CUDA_TRY(cudaGetLastError());
-    return GSS_OK;
 }
 
 }  // namespace gss

@@ -104,6 +104,10 @@ struct CheckArgs {
     const uint32_t *perm;
     uint32_t scan_begin, scan_end;
     uint32_t perm_end;
+    // filtered kernel only: the word-level table [n_blocks][2 * n_vars] of the
+    // state, and the counter of (clause, block) pairs it kept
+    const uint2 *agg;
+    uint32_t *kept;
 };
 
 __host__ __device__ __forceinline__ uint32_t scan_count(const CheckArgs &a) {
@@ -171,18 +175,26 @@ int gather_clauses(const GatherArgs &a, cudaStream_t stream, int sm_count);
 // or, with cell_words > 0, 8-byte {clause * cell_words + word, mask} records.
 int launch_pack_reports(const gss_report *parts, const uint32_t *counts, uint32_t n_parts, uint32_t cap,
                         uint32_t cell_words, uint32_t *packed, cudaStream_t stream, int sm_count);
-// What a pass's counters buffer holds: the n_parts report counters, then the
-// kernel's error flag and the work counter of the persistent kernels. One
+// What a pass's counters buffer holds: the n_parts report counters, the
+// kernel's error flag and the filter's counter of kept clauses, and, from
+// word kWorkOffset on, the work counters of the persistent kernels. One
 // memset clears them all.
 constexpr uint32_t kExtraCounters = 2;
+constexpr uint32_t kWorkOffset = 64;
+// One address takes an atomic every 1.5 ns or so: 62500 tasks from a single
+// counter are 100 us, whatever the tasks do. The filtered kernel's tasks are
+// that short, so they come from kWorkCounters counters (256 bytes apart).
+constexpr uint32_t kWorkCounters = 16, kWorkStride = 64;
+constexpr size_t kWorkBytes = sizeof(uint32_t) * kWorkCounters * kWorkStride;
+constexpr size_t kCounterBytes = sizeof(uint32_t) * kWorkOffset + kWorkBytes;
 __host__ __device__ __forceinline__ uint32_t *err_counter(uint32_t *counts, uint32_t n_parts) {
     return counts + n_parts;
 }
-__host__ __device__ __forceinline__ uint32_t *work_counter(uint32_t *counts, uint32_t n_parts) {
+__host__ __device__ __forceinline__ uint32_t *kept_counter(uint32_t *counts, uint32_t n_parts) {
     return counts + n_parts + 1;
 }
-// Hands a pass's outcome to the host: writes the n_parts counters and the
-// error flag to `host` (pinned), and, when the pass has at most max_inline
+__host__ __device__ __forceinline__ uint32_t *work_counter(uint32_t *counts) { return counts + kWorkOffset; }
+// Hands a pass's outcome to the host: writes the counters buffer to `host` (pinned), and, when the pass has at most max_inline
 // records and no partition overflowed, the records too, partition after
 // partition from byte kInlineOffset on. With d_args the queues are those of
 // the arguments in device memory (a captured graph outlives a queue's growth).
@@ -211,8 +223,34 @@ bool valid_wide_persist_variant(int wpl, int lpc, int g);
 bool valid_wide_variant(int wpl, int lpc, int g, int occ);
 bool valid_tiled_variant(int lpc, int k);
 
-// [n_vars][n_words] -> [n_blocks][n_vars][lpc], zero-padded words.
-int launch_relayout(const uint2 *src, uint2 *dst, uint32_t n_vars, uint32_t n_words, uint32_t lpc,
-                    uint32_t n_blocks, cudaStream_t stream, int sm_count);
+// The persistent wide kernel behind the word-level filter (h_args.agg, or
+// that of d_args).
+int launch_check_filtered(const CheckArgs *d_args, const CheckArgs &h_args, int wpl, int lpc, uint32_t *work,
+                          cudaStream_t stream, int sm_count);
+bool valid_filtered_variant(int wpl, int lpc);
+// Its tasks are counted in 32 bits (with room for what the warps take past the end).
+constexpr uint64_t kMaxFilterTasks = 1ull << 31;
+inline uint64_t filter_tasks(const CheckArgs &a) { return ((uint64_t) scan_count(a) + 31) / 32 * a.n_blocks; }
+// [n_vars][n_words] -> [n_blocks][n_vars][bw], zero-padded words (in_place:
+// src is laid out already), and the filter's table `agg` (NULL: none), 16
+// bytes a variable and block. `density` (NULL: none; added to) gets the
+// number of the table's "false" bits, over both literals.
+int launch_load_state(const uint2 *src, uint2 *dst, uint2 *agg, unsigned long long *density, uint32_t n_vars,
+                      uint32_t n_words, uint32_t bw, uint32_t n_blocks, bool in_place, cudaStream_t stream,
+                      int sm_count);
+// A word of a variable's state that a pass changes.
+struct StateUpdate {
+    uint32_t var;
+    uint32_t word;
+    uint32_t is_def;
+    uint32_t is_true;
+};
+// The table's entries of the rows that n updates changed, from the state.
+int launch_refresh_agg(const StateUpdate *u, uint32_t n, const uint2 *state, uint2 *agg, uint32_t n_vars,
+                       uint32_t n_words, uint32_t bw, cudaStream_t stream, int sm_count);
+// start and solver_of_word of a pass from device memory, padded with zeros to
+// `padded` words; solver_of_word NULL: the word's own number.
+int launch_load_masks(const uint32_t *start, const int32_t *solver_of_word, uint32_t n_words, uint32_t padded,
+                      uint32_t *start_out, int32_t *sow_out, cudaStream_t stream);
 
 }  // namespace gss

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256) deliver_kernel(const CheckArgs *__restric
         cap = pa->cap_per_part;
     }
     const uint32_t p = blockIdx.x / kStripes, stripe = blockIdx.x % kStripes;
-    if (blockIdx.x == 0 && threadIdx.x <= n_parts) host[threadIdx.x] = counts[threadIdx.x];  // the error flag follows
+    if (blockIdx.x == 0 && threadIdx.x < n_parts + kExtraCounters) host[threadIdx.x] = counts[threadIdx.x];
     if (max_inline == 0) return;
     uint64_t total = 0, base = 0;
     bool over = false;

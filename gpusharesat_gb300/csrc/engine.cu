@@ -150,6 +150,15 @@ namespace {
 
 int words_per_lane(int kind) { return kind == GSS_KERNEL_WIDE4 ? 4 : kind == GSS_KERNEL_WIDE2 ? 2 : 1; }
 
+// Whether the word-level filter pays for a state whose table has so many
+// bits set, of `pairs` (variable, word) pairs: F is the share of (literal,
+// word) pairs where some slot makes the literal false; a word outlives k
+// literals with a probability near F^k + k F^(k-1). Measured on 500k clauses x
+// 1024 slots over states of rising mixture, filtered against plain: F = 0.25
+// 28 to 45 against 58 to 67 us, 0.48 64 to 76 against 83 to 88; even at 0.70
+// (lengths 2-100), 0.67 (Zipf lengths) and 0.55 (lengths 2-30).
+bool use_filter(uint64_t n_false, double pairs) { return pairs > 0 && (double) n_false < 0.55 * 2.0 * pairs; }
+
 int ensure_device(gss_engine *eng) {
     GSS_CUDA_TRY(cudaSetDevice(eng->device));
     return GSS_OK;
@@ -168,8 +177,8 @@ int ensure_queues(gss_engine *eng) {
         GSS_TRY(eng->reports.reserve((size_t) per * eng->n_parts * sizeof(gss_report)));
         eng->cap_per_part = (uint32_t) per;
     }
-    GSS_TRY(eng->counts.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
-    GSS_TRY(eng->h_counts.reserve(kInlineOffset + (size_t) kEngineInline * sizeof(gss_report)));
+    GSS_TRY(eng->counts.reserve(kCounterBytes));
+    GSS_TRY(eng->h_counts.reserve(kInlineOffset));
     return GSS_OK;
 }
 
@@ -226,6 +235,7 @@ int gss_engine_destroy(gss_engine *eng) {
     if (eng->own_stream) cudaStreamDestroy(eng->own_stream);
     if (eng->graph_exec) cudaGraphExecDestroy(eng->graph_exec);
     if (eng->graph) cudaGraphDestroy(eng->graph);
+    if (eng->ev_caller) cudaEventDestroy(eng->ev_caller);
     if (eng->h2d) cudaStreamDestroy(eng->h2d);
     if (eng->d2h) cudaStreamDestroy(eng->d2h);
     for (int b = 0; b < 3; b++) {
@@ -635,45 +645,73 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     GSS_TRY(eng->state.reserve(std::max<size_t>(bbytes, 8)));
     GSS_TRY(eng->start.reserve(std::max<size_t>(padded * sizeof(uint32_t), 4)));
     GSS_TRY(eng->solver_of_word.reserve(std::max<size_t>(padded * sizeof(int32_t), 4)));
-    // start and solver_of_word, padded with zero words
-    std::vector<uint32_t> st(padded, 0u);
-    std::vector<int32_t> sw(padded, 0);
-    if (n_words) {
-        if (on_device) {
-            GSS_CUDA_TRY(cudaMemcpy(st.data(), start, n_words * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-            if (solver_of_word)
-                GSS_CUDA_TRY(cudaMemcpy(sw.data(), solver_of_word, n_words * sizeof(int32_t), cudaMemcpyDeviceToHost));
-        } else {
-            memcpy(st.data(), start, n_words * sizeof(uint32_t));
-            if (solver_of_word) memcpy(sw.data(), solver_of_word, n_words * sizeof(int32_t));
-        }
-        if (!solver_of_word)
-            for (int w = 0; w < n_words; w++) sw[w] = w;
+    // the filter's table: only the automatic variant runs behind it; without
+    // room for it the passes run without
+    const bool want_agg = eng->kind == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && sbytes > 0;
+    eng->filter = false;
+    const size_t abytes = (size_t) n_blocks * n_vars * 2 * sizeof(uint2);
+    const bool filtered = want_agg && eng->agg.reserve(abytes + sizeof(unsigned long long)) == GSS_OK;
+    uint2 *const agg = filtered ? (uint2 *) eng->agg.ptr : nullptr;
+    // the count of its bits: behind the table, and on the host in a corner of
+    // the counters' pinned buffer
+    unsigned long long *const density = filtered ? (unsigned long long *) ((char *) agg + abytes) : nullptr;
+    if (filtered) {
+        GSS_TRY(eng->h_counts.reserve(kInlineOffset));
+        GSS_CUDA_TRY(cudaMemsetAsync(density, 0, sizeof(unsigned long long), eng->stream));
     }
-    if (padded) {
+    unsigned long long *const h_density = (unsigned long long *) ((char *) eng->h_counts.ptr + kDensityOffset);
+    // start and solver_of_word, padded with zero words
+    std::vector<uint32_t> st;
+    std::vector<int32_t> sw;
+    if (on_device) {
+        // in order behind what the caller queued on the default stream
+        for (const void *p : {(const void *) start, (const void *) solver_of_word}) {
+            cudaPointerAttributes at;
+            if (p == nullptr || n_words == 0) continue;
+            GSS_CUDA_TRY(cudaPointerGetAttributes(&at, p));
+            if (at.devicePointer == nullptr)
+                return set_error(GSS_ERR_CUDA, "gss_state_set: a mask pointer that the device cannot read");
+        }
+        if (n_words) {
+            if (!eng->ev_caller) GSS_CUDA_TRY(cudaEventCreateWithFlags(&eng->ev_caller, cudaEventDisableTiming));
+            GSS_CUDA_TRY(cudaEventRecord(eng->ev_caller, cudaStreamLegacy));
+            GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_caller, 0));
+        }
+        GSS_TRY(launch_load_masks(start, solver_of_word, (uint32_t) n_words, (uint32_t) padded,
+                                  (uint32_t *) eng->start.ptr, (int32_t *) eng->solver_of_word.ptr, eng->stream));
+    } else if (padded) {
+        st.assign(padded, 0u);
+        sw.assign(padded, 0);
+        memcpy(st.data(), start, n_words * sizeof(uint32_t));
+        for (int w = 0; w < n_words; w++) sw[w] = solver_of_word ? solver_of_word[w] : w;
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->start.ptr, st.data(), padded * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                      eng->stream));
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->solver_of_word.ptr, sw.data(), padded * sizeof(int32_t),
                                      cudaMemcpyHostToDevice, eng->stream));
     }
     if (sbytes) {
-        if (n_blocks == 1 && n_words == bw) {
-            // block-major and host layouts coincide
-            GSS_CUDA_TRY(cudaMemcpyAsync(eng->state.ptr, state, sbytes,
-                                         on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, eng->stream));
-        } else {
-            const uint2 *src = (const uint2 *) state;
-            if (!on_device) {
-                GSS_TRY(eng->state_raw.reserve(sbytes));
-                GSS_CUDA_TRY(cudaMemcpyAsync(eng->state_raw.ptr, state, sbytes, cudaMemcpyHostToDevice, eng->stream));
-                src = (const uint2 *) eng->state_raw.ptr;
-            }
-            GSS_TRY(launch_relayout(src, (uint2 *) eng->state.ptr, (uint32_t) n_vars, (uint32_t) n_words,
-                                    (uint32_t) bw, (uint32_t) n_blocks, eng->stream, eng->sm_count));
+        const bool laid_out = n_blocks == 1 && n_words == bw;  // block-major and host layouts coincide
+        const cudaMemcpyKind dir = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        const uint2 *src = (const uint2 *) state;
+        const bool aligned = on_device && ((uintptr_t) state & 7) == 0;  // the kernel reads it as it is
+        if (laid_out && !(aligned && filtered)) {
+            GSS_CUDA_TRY(cudaMemcpyAsync(eng->state.ptr, state, sbytes, dir, eng->stream));
+            src = (const uint2 *) eng->state.ptr;
+        } else if (!aligned) {
+            GSS_TRY(eng->state_raw.reserve(sbytes));
+            GSS_CUDA_TRY(cudaMemcpyAsync(eng->state_raw.ptr, state, sbytes, dir, eng->stream));
+            src = (const uint2 *) eng->state_raw.ptr;
         }
+        GSS_TRY(launch_load_state(src, (uint2 *) eng->state.ptr, agg, density, (uint32_t) n_vars, (uint32_t) n_words,
+                                  (uint32_t) bw, (uint32_t) n_blocks, src == (const uint2 *) eng->state.ptr,
+                                  eng->stream, eng->sm_count));
     }
-    // the host vectors above are pageable: the async copies from them complete before return
+    if (filtered)
+        GSS_CUDA_TRY(cudaMemcpyAsync(h_density, density, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                     eng->stream));
+    // the caller's buffers are free (and the host vectors above too) when this returns
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
+    if (filtered) eng->filter = use_filter(*h_density, (double) n_vars * n_words);
     eng->n_vars = n_vars;
     eng->n_words = n_words;
     eng->n_blocks = n_blocks;
@@ -739,11 +777,11 @@ int gss_check_set_capacity(gss_engine *eng, int64_t records) {
 namespace {
 
 // Launches one check pass of the engine's database against `state` (laid out
-// as the engine's current state), into `reports`/`counts`, then hands the
+// as the engine's current state; `agg`: its filter table), into `reports`/`counts`, then hands the
 // counts, the error flag and up to max_inline records to `h_counts` (pinned),
 // all on the engine's stream.
-int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf &counts, PinnedBuf &h_counts,
-                     uint32_t max_inline);
+int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf &reports, DevBuf &counts,
+                     PinnedBuf &h_counts, uint32_t max_inline);
 
 }  // namespace
 
@@ -751,7 +789,8 @@ int gss_check_launch(gss_engine *eng) {
     if (!eng) return set_error(GSS_ERR_INVALID, "engine is NULL");
     GSS_TRY(ensure_device(eng));
     GSS_TRY(ensure_queues(eng));
-    GSS_TRY(launch_pass_into(eng, eng->state.ptr, eng->reports, eng->counts, eng->h_counts, kEngineInline));
+    GSS_TRY(eng->h_counts.reserve(kHostCounterBytes));
+    GSS_TRY(launch_pass_into(eng, eng->state.ptr, eng->agg.ptr, eng->reports, eng->counts, eng->h_counts, kEngineInline));
     eng->launches++;
     eng->pass_pending = true;
     eng->inline_ok = true;
@@ -809,8 +848,8 @@ int build_plan(gss_engine *eng) {
     return GSS_OK;
 }
 
-int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf &counts, PinnedBuf &h_counts,
-                     uint32_t max_inline) {
+int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf &reports, DevBuf &counts,
+                     PinnedBuf &h_counts, uint32_t max_inline) {
     order_quiesce(eng);  // a scoring in flight reads the buffers this pass may reallocate
     if (eng->n_clauses > 0 && eng->max_var >= eng->n_vars)
         return set_error(GSS_ERR_INVALID, "database uses variable %lld but the state has %lld variables",
@@ -861,8 +900,9 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
     a.n_parts = eng->n_parts;
     a.cap_per_part = eng->cap_per_part;
     a.err = err_counter(a.counts, a.n_parts);
-    uint32_t *const work = work_counter(a.counts, a.n_parts);
-    const size_t counter_bytes = sizeof(uint32_t) * (a.n_parts + kExtraCounters);
+    a.agg = (const uint2 *) agg;
+    a.kept = kept_counter(a.counts, a.n_parts);
+    uint32_t *const work = work_counter(a.counts);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (eng->timing) {
         for (cudaEvent_t *ev : {&ev0, &ev1}) {
@@ -886,6 +926,16 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
         wide && ((eng->flags & GSS_VARIANT_PERSISTENT) ||
                  (eng->kind == GSS_KERNEL_AUTO &&
                   valid_wide_persist_variant(words_per_lane(eng->state_kind), eng->state_lpc, eng->state_g)));
+    // behind the word-level filter where the state's table says that it pays
+    const bool filtered = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
+                          filter_tasks(a) < kMaxFilterTasks;
+    auto launch_persistent = [&](const CheckArgs *d_args, const CheckArgs &args) -> int {
+        if (filtered)
+            return launch_check_filtered(d_args, args, words_per_lane(eng->state_kind), eng->state_lpc, work,
+                                         eng->stream, eng->sm_count);
+        return launch_check_wide_persist(d_args, args, words_per_lane(eng->state_kind), eng->state_lpc, eng->state_g,
+                                         work, eng->stream, eng->sm_count);
+    };
     if (ordered && (eng->state_kind == GSS_KERNEL_TILED || bucketed))
         return set_error(GSS_ERR_STATE, "the learned scan order runs the direct, wide and persistent kernels (not the "
                          "tiled or bucketed ones)");
@@ -901,7 +951,7 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->d_args.ptr, &a, sizeof a, cudaMemcpyHostToDevice, eng->stream));
         if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
         auto body = [&]() -> int {
-            GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes, eng->stream));
+            GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, kCounterBytes, eng->stream));
             if (a.n_clauses > 0 && a.n_blocks > 0) {
                 if (bucketed) {
                     if (eng->plan_ranges > 0)
@@ -909,9 +959,7 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
                                                       (const BucketPlan *) eng->d_plan.ptr, work, eng->stream,
                                                       eng->sm_count));
                 } else {
-                    GSS_TRY(launch_check_wide_persist((const CheckArgs *) eng->d_args.ptr, a,
-                                                      words_per_lane(eng->state_kind), eng->state_lpc, eng->state_g,
-                                                      work, eng->stream, eng->sm_count));
+                    GSS_TRY(launch_persistent((const CheckArgs *) eng->d_args.ptr, a));
                 }
             }
             return launch_deliver((const CheckArgs *) eng->d_args.ptr, a.out, a.counts, a.n_parts, a.cap_per_part,
@@ -922,7 +970,7 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
                 (uintptr_t) a.counts, (uintptr_t) h_counts.ptr, (uintptr_t) max_inline,
                 (uintptr_t) eng->d_args.ptr, (uintptr_t) eng->state_kind, (uintptr_t) eng->state_lpc,
                 (uintptr_t) eng->state_g, (uintptr_t) eng->n_parts, (uintptr_t) (a.n_clauses > 0 && a.n_blocks > 0),
-                (uintptr_t) bucketed, (uintptr_t) eng->d_plan.ptr, (uintptr_t) (eng->plan_ranges > 0)};
+                (uintptr_t) bucketed, (uintptr_t) filtered, (uintptr_t) eng->d_plan.ptr, (uintptr_t) (eng->plan_ranges > 0)};
             if (key != eng->graph_key || !eng->graph_exec) {
                 if (eng->graph_exec) cudaGraphExecDestroy(eng->graph_exec);
                 if (eng->graph) cudaGraphDestroy(eng->graph);
@@ -949,18 +997,17 @@ int launch_pass_into(gss_engine *eng, const void *state, DevBuf &reports, DevBuf
         }
         return GSS_OK;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes, eng->stream));
+    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, kCounterBytes, eng->stream));
     if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
     bool work_used = false;  // the memset above cleared the work counter for the first launch
     auto launch = [&](const CheckArgs &args) -> int {
         if (eng->state_kind == GSS_KERNEL_TILED) return launch_check_tiled(args, eng->stream, eng->sm_count);
         if (persistent) {
             // arguments by value; the work counter restarts for each launch
-            if (work_used) GSS_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(uint32_t), eng->stream));
+            if (work_used) GSS_CUDA_TRY(cudaMemsetAsync(work, 0, kWorkBytes, eng->stream));
             work_used = true;
             if (args.n_clauses == 0 || args.n_blocks == 0 || scan_count(args) == 0) return GSS_OK;
-            return launch_check_wide_persist(nullptr, args, words_per_lane(eng->state_kind), eng->state_lpc,
-                                             eng->state_g, work, eng->stream, eng->sm_count);
+            return launch_persistent(nullptr, args);
         }
         const int occ = (eng->flags & GSS_VARIANT_OCCUPANCY) ? 1 : 0;
         if (wide && (eng->flags & GSS_VARIANT_PIPELINED))
@@ -1113,14 +1160,20 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         GSS_TRY(eng->state_raw2.reserve(std::max<size_t>(sbytes, 8)));
         GSS_TRY(eng->state_raw3.reserve(std::max<size_t>(sbytes, 8)));
     }
+    // The first state decides for all of them: a later one whose table keeps
+    // more costs time, not reports.
+    if (eng->filter) {
+        const size_t abytes = (size_t) eng->n_blocks * n_vars * 2 * sizeof(uint2);
+        if (eng->agg2.reserve(abytes) != GSS_OK || eng->agg3.reserve(abytes) != GSS_OK) eng->filter = false;
+    }
     auto reserve_reports = [&]() -> int {
         GSS_TRY(eng->reports2.reserve((size_t) eng->cap_per_part * eng->n_parts * sizeof(gss_report)));
         GSS_TRY(eng->reports3.reserve((size_t) eng->cap_per_part * eng->n_parts * sizeof(gss_report)));
         return GSS_OK;
     };
     GSS_TRY(reserve_reports());
-    GSS_TRY(eng->counts2.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
-    GSS_TRY(eng->counts3.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
+    GSS_TRY(eng->counts2.reserve(kCounterBytes));
+    GSS_TRY(eng->counts3.reserve(kCounterBytes));
     auto reserve_packed = [&]() -> int {
         for (int b = 0; b < NB && packed; b++)
             GSS_TRY(eng->packed[b].reserve((size_t) eng->cap_per_part * eng->n_parts * rec_words * sizeof(uint32_t)));
@@ -1137,6 +1190,7 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
     GSS_TRY(eng->h_counts2.reserve(sizeof(uint32_t) * (eng->n_parts + 1)));
     GSS_TRY(eng->h_counts3.reserve(sizeof(uint32_t) * (eng->n_parts + 1)));
     DevBuf *state_buf[NB] = {&eng->state, &eng->state2, &eng->state3};
+    DevBuf *agg_buf[NB] = {&eng->agg, &eng->agg2, &eng->agg3};
     DevBuf *raw_buf[NB] = {&eng->state_raw, &eng->state_raw2, &eng->state_raw3};
     DevBuf *rep_buf[NB] = {&eng->reports, &eng->reports2, &eng->reports3};
     DevBuf *cnt_buf[NB] = {&eng->counts, &eng->counts2, &eng->counts3};
@@ -1167,13 +1221,13 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
             GSS_TRY(ensure_queues(eng));
             GSS_TRY(reserve_reports());
             GSS_TRY(reserve_packed());
-            GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
+            GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, agg_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
             GSS_TRY(pack(b, *rep_buf[b], *cnt_buf[b]));
             eng->launches++;
             GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[b], eng->stream));
             if (j + 1 < launched) {
                 const int nb = (j + 1) % NB;
-                GSS_TRY(launch_pass_into(eng, state_buf[nb]->ptr, *rep_buf[nb], *cnt_buf[nb], *hcnt_buf[nb], 0));
+                GSS_TRY(launch_pass_into(eng, state_buf[nb]->ptr, agg_buf[nb]->ptr, *rep_buf[nb], *cnt_buf[nb], *hcnt_buf[nb], 0));
                 GSS_TRY(pack(nb, *rep_buf[nb], *cnt_buf[nb]));
                 eng->launches++;
                 GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[nb], eng->stream));
@@ -1216,14 +1270,15 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
             GSS_CUDA_TRY(cudaMemcpyAsync(dst, states[i], sbytes, cudaMemcpyHostToDevice, eng->h2d));
             GSS_CUDA_TRY(cudaEventRecord(eng->ev_h2d[b], eng->h2d));
             GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_h2d[b], 0));
-            if (!direct)
-                GSS_TRY(launch_relayout((const uint2 *) raw_buf[b]->ptr, (uint2 *) state_buf[b]->ptr, (uint32_t) n_vars,
-                                        (uint32_t) n_words, (uint32_t) eng->state_bw, (uint32_t) eng->n_blocks,
-                                        eng->stream, eng->sm_count));
+            if (!direct || eng->filter)
+                GSS_TRY(launch_load_state((const uint2 *) dst, (uint2 *) state_buf[b]->ptr,
+                                          eng->filter ? (uint2 *) agg_buf[b]->ptr : nullptr, nullptr,
+                                          (uint32_t) n_vars, (uint32_t) n_words, (uint32_t) eng->state_bw,
+                                          (uint32_t) eng->n_blocks, direct, eng->stream, eng->sm_count));
         }
         // report set b is free once pass i-3's reports are back
         if (i >= NB) GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_d2h[b], 0));
-        GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
+        GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, agg_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
         GSS_TRY(pack(b, *rep_buf[b], *cnt_buf[b]));
         eng->launches++;
         launched = i + 1;

@@ -51,6 +51,11 @@ struct gss_engine {
 
     // assignment state, block-major [n_blocks][n_vars][state_bw words]
     DevBuf state, state_raw, start, solver_of_word;
+    // the filter's table of the state (and the count of its bits), and whether
+    // passes run behind it (use_filter)
+    DevBuf agg;
+    bool filter = false;
+    cudaEvent_t ev_caller = nullptr;  // the caller's work on the default stream (gss_state_set, on_device)
     int64_t n_vars = 0;
     int n_words = 0;
     int n_blocks = 0;
@@ -75,8 +80,8 @@ struct gss_engine {
     // pipelined passes through host buffers (gss_check_passes_host): second
     // state and report buffers, copy streams and events
     // slots 1 and 2 of the three-slot pipeline (slot 0 is the engine's own)
-    DevBuf state2, state_raw2, reports2, counts2;
-    DevBuf state3, state_raw3, reports3, counts3;
+    DevBuf state2, state_raw2, agg2, reports2, counts2;
+    DevBuf state3, state_raw3, agg3, reports3, counts3;
     DevBuf packed[3];  // 12-byte records of gss_check_passes_host_packed
     PinnedBuf h_counts2, h_counts3;
     cudaStream_t h2d = nullptr, d2h = nullptr;
@@ -117,7 +122,10 @@ namespace gss {
 // Records that come back with the counters (1 MB of pinned memory); a pass
 // with more is fetched with a copy per partition, whose fixed cost is then
 // below the copies' own time.
-constexpr uint32_t kEngineInline = 65536;
+constexpr uint32_t kEngineInline = 65536 - kInlineOffset / sizeof(gss_report);
+constexpr size_t kHostCounterBytes = kInlineOffset + (size_t) kEngineInline * sizeof(gss_report);
+// where gss_state_set's count of the filter's bits comes back, past the counters
+constexpr size_t kDensityOffset = 192;
 
 // Learned scan order hooks, called by the engine's pass (order.cu).
 // Before the scan: the scan permutation of this pass (computed while the

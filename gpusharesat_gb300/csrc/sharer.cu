@@ -52,18 +52,11 @@ int64_t now_us() {
         .count();
 }
 
-struct DevUpdate {
-    uint32_t var;
-    uint32_t word;
-    uint32_t is_def;
-    uint32_t is_true;
-};
-
 // state[(word / bw) * n_vars + var][word % bw] = update
-__global__ void scatter_updates_kernel(const DevUpdate *__restrict__ u, uint32_t n, uint2 *__restrict__ state,
+__global__ void scatter_updates_kernel(const StateUpdate *__restrict__ u, uint32_t n, uint2 *__restrict__ state,
                                        uint32_t n_vars, uint32_t bw) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const DevUpdate x = u[i];
+        const StateUpdate x = u[i];
         const size_t idx = ((size_t) (x.word / bw) * n_vars + x.var) * bw + x.word % bw;
         state[idx] = make_uint2(x.is_def, x.is_true);
     }
@@ -71,10 +64,10 @@ __global__ void scatter_updates_kernel(const DevUpdate *__restrict__ u, uint32_t
 
 // After the check: every slot of an updated variable takes the value of the
 // solver's last slot (dSetAllAssigsToLast, gpuShareLib/Assigs.cu:118-141).
-__global__ void set_to_last_kernel(const DevUpdate *__restrict__ u, uint32_t n, const uint32_t *__restrict__ last,
+__global__ void set_to_last_kernel(const StateUpdate *__restrict__ u, uint32_t n, const uint32_t *__restrict__ last,
                                    uint2 *__restrict__ state, uint32_t n_vars, uint32_t bw) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const DevUpdate x = u[i];
+        const StateUpdate x = u[i];
         const uint32_t m = last[x.word];
         const size_t idx = ((size_t) (x.word / bw) * n_vars + x.var) * bw + x.word % bw;
         state[idx] = make_uint2((x.is_def & m) ? ~0u : 0u, (x.is_true & m) ? ~0u : 0u);
@@ -102,6 +95,11 @@ unsigned grid_for(uint64_t n, int sm_count) {
 }
 
 }  // namespace
+
+// The filter's use (Sharer::collect). Its own pass is about a quarter of the
+// plain check's time, and what it keeps costs the plain check's share again.
+constexpr double kFilterKeepMost = 0.5;
+constexpr int kFilterPause = 64;
 
 // ---- one solver's ring ----
 
@@ -229,7 +227,7 @@ int Sharer::init(int device) {
     for (Pass &p : pass_) {
         GSS_CUDA_TRY(cudaEventCreateWithFlags(&p.counted, cudaEventDisableTiming));
         GSS_CUDA_TRY(cudaEventCreateWithFlags(&p.copied, cudaEventDisableTiming));
-        GSS_TRY(p.d_counts.reserve(sizeof(uint32_t) * (n_parts_ + kExtraCounters)));
+        GSS_TRY(p.d_counts.reserve(kCounterBytes));
         GSS_TRY(p.h_counts.reserve(kInlineOffset + (size_t) kSharerInline * sizeof(gss_report)));
     }
     GSS_CUDA_TRY(cudaEventCreateWithFlags(&alive_staged_, cudaEventDisableTiming));
@@ -515,7 +513,29 @@ int Sharer::ensure_state() {
     std::vector<int32_t> sow(n_blocks * bw);
     for (int w = 0; w < n_blocks * bw; w++) sow[w] = w < n_words ? w : 0;
     GSS_CUDA_TRY(cudaMemcpy(d_sow_.ptr, sow.data(), sow.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    // the filter's table; without room for it the passes run without
+    agg_ok_ = kind_ == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && need_vars > 0 && n_words > 0 &&
+              d_agg_.reserve((size_t) n_blocks * need_vars * 2 * sizeof(uint2)) == GSS_OK;
+    filter_pause_ = 0;
+    if (agg_ok_)
+        GSS_TRY(launch_load_state((const uint2 *) d_state_.ptr, nullptr, (uint2 *) d_agg_.ptr, nullptr,
+                                  (uint32_t) dev_vars_, (uint32_t) dev_words_, (uint32_t) bw_, (uint32_t) n_blocks_,
+                                  true, stream_, sm_count_));
     return GSS_OK;
+}
+
+int Sharer::refresh_agg(int64_t n_updates) {
+    // The filter's table after n_updates words of the state (d_updates_)
+    // changed: their rows again, or all of them when that is less to read (an
+    // update's row is 8 * bw_ bytes; several updates may share one).
+    if (!agg_ok_ || n_updates == 0) return GSS_OK;
+    if (n_updates >= (int64_t) dev_vars_ * n_blocks_)
+        return launch_load_state((const uint2 *) d_state_.ptr, nullptr, (uint2 *) d_agg_.ptr, nullptr,
+                                 (uint32_t) dev_vars_, (uint32_t) dev_words_, (uint32_t) bw_, (uint32_t) n_blocks_,
+                                 true, stream_, sm_count_);
+    return launch_refresh_agg((const StateUpdate *) d_updates_.ptr, (uint32_t) n_updates,
+                              (const uint2 *) d_state_.ptr, (uint2 *) d_agg_.ptr, (uint32_t) dev_vars_,
+                              (uint32_t) dev_words_, (uint32_t) bw_, stream_, sm_count_);
 }
 
 int Sharer::upload_db() {
@@ -891,6 +911,9 @@ int Sharer::run_check(Pass &p) {
     a.g = eff_depth_;
     a.cache_hints = (flags_ & GSS_VARIANT_L2_HINT) ? 1 : 0;
     a.err = err_counter(a.counts, n_parts_);
+    a.agg = (const uint2 *) d_agg_.ptr;
+    a.kept = kept_counter(a.counts, n_parts_);
+    p.filtered = false;
     a.alive = nullptr;
     if (dev_dead_ > 0) {
         // evicted clauses still on the device: skipped through the bitmap
@@ -898,15 +921,19 @@ int Sharer::run_check(Pass &p) {
         a.alive = (const uint32_t *) d_alive_.ptr;
         a.alive_by_id = 1;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, sizeof(uint32_t) * (n_parts_ + kExtraCounters), stream_));
+    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, kCounterBytes, stream_));
     if (p.active_words > 0 && p.n_clauses > 0) {
         const int wpl = eff_kind_ == GSS_KERNEL_WIDE4 ? 4 : 2;
         const bool wide = eff_kind_ == GSS_KERNEL_WIDE4 || eff_kind_ == GSS_KERNEL_WIDE2;
         if (wide && ((flags_ & GSS_VARIANT_PERSISTENT) ||
                      (kind_ == GSS_KERNEL_AUTO && valid_wide_persist_variant(wpl, eff_lpc_, eff_depth_)))) {
             // the persistent form, as the engine's automatic variant
-            GSS_TRY(launch_check_wide_persist(nullptr, a, wpl, eff_lpc_, eff_depth_, work_counter(a.counts, n_parts_),
-                                              stream_, sm_count_));
+            uint32_t *const work = work_counter(a.counts);
+            p.filtered = agg_ok_ && filter_pause_ == 0 && filter_tasks(a) < kMaxFilterTasks;
+            if (p.filtered)
+                GSS_TRY(launch_check_filtered(nullptr, a, wpl, eff_lpc_, work, stream_, sm_count_));
+            else
+                GSS_TRY(launch_check_wide_persist(nullptr, a, wpl, eff_lpc_, eff_depth_, work, stream_, sm_count_));
         } else if (wide) {
             GSS_TRY(launch_check_wide(a, wpl, (flags_ & GSS_VARIANT_OCCUPANCY) ? 1 : 0, stream_, sm_count_));
         } else {
@@ -968,10 +995,17 @@ int Sharer::collect(Pass &p) {
         GSS_CUDA_TRY(cudaMemcpyAsync(d_last_mask_.ptr, p.h_last.ptr, (size_t) n_blocks_ * bw_ * sizeof(uint32_t),
                                      cudaMemcpyHostToDevice, stream_));
         set_to_last_kernel<<<grid_for(p.n_updates, sm_count_), 256, 0, stream_>>>(
-            (const DevUpdate *) d_updates_.ptr, (uint32_t) p.n_updates, (const uint32_t *) d_last_mask_.ptr,
+            (const StateUpdate *) d_updates_.ptr, (uint32_t) p.n_updates, (const uint32_t *) d_last_mask_.ptr,
             (uint2 *) d_state_.ptr, (uint32_t) dev_vars_, (uint32_t) bw_);
         GSS_CUDA_TRY(cudaGetLastError());
+        GSS_TRY(refresh_agg(p.n_updates));
     }
+    // a filter that keeps most clauses costs more than it saves: leave it out
+    // for some passes, then look again
+    if (filter_pause_ > 0) filter_pause_--;
+    if (p.filtered && (double) ((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1] >
+                          kFilterKeepMost * (double) p.n_clauses * n_blocks_)
+        filter_pause_ = kFilterPause;
     GSS_CUDA_TRY(cudaEventRecord(p.copied, stream_));
     p.pending = false;
     p.collected = true;
@@ -1094,7 +1128,7 @@ int Sharer::launch_pass() {
     p.assig.assign(n_solvers, AssigIds());
     p.assig_total = 0;
     p.active_words = 0;
-    std::vector<DevUpdate> ups;
+    std::vector<StateUpdate> ups;
     for (int s = 0; s < n_solvers; s++) {
         SolverAssigs &sa = *solvers_[s];
         // HostAssigs::fillAssigsAsync (Assigs.cu:347-357): a solver whose lock
@@ -1113,7 +1147,7 @@ int Sharer::launch_pass() {
         start[s] = ~sa.not_completed;
         last[s] = 1u << (uint32_t) (last_id % kSlots);
         for (const VarUpdate &u : sa.updates)
-            if ((int) u.var < dev_vars_) ups.push_back(DevUpdate{u.var, (uint32_t) s, u.is_def, u.is_true});
+            if ((int) u.var < dev_vars_) ups.push_back(StateUpdate{u.var, (uint32_t) s, u.is_def, u.is_true});
         sa.updates.clear();
         sa.first_id_used = sa.current_id;
         sa.not_completed = ~0u;
@@ -1129,15 +1163,16 @@ int Sharer::launch_pass() {
         if (!ups.empty()) {
             // h_updates_ is free: the previous pass's copy from it ran before
             // that pass's check, which has finished
-            const size_t bytes = ups.size() * sizeof(DevUpdate);
+            const size_t bytes = ups.size() * sizeof(StateUpdate);
             GSS_TRY(d_updates_.reserve(bytes));
             GSS_TRY(h_updates_.reserve(bytes));
             memcpy(h_updates_.ptr, ups.data(), bytes);
             GSS_CUDA_TRY(cudaMemcpyAsync(d_updates_.ptr, h_updates_.ptr, bytes, cudaMemcpyHostToDevice, stream_));
             scatter_updates_kernel<<<grid_for(ups.size(), sm_count_), 256, 0, stream_>>>(
-                (const DevUpdate *) d_updates_.ptr, (uint32_t) ups.size(), (uint2 *) d_state_.ptr,
+                (const StateUpdate *) d_updates_.ptr, (uint32_t) ups.size(), (uint2 *) d_state_.ptr,
                 (uint32_t) dev_vars_, (uint32_t) bw_);
             GSS_CUDA_TRY(cudaGetLastError());
+            GSS_TRY(refresh_agg((int64_t) ups.size()));
         }
         p.n_clauses = dev_clauses_;
         return run_check(p);

@@ -20,7 +20,7 @@ namespace gss {
 // (gpuShareLib/SolverTypes.h:81-83).
 constexpr uint8_t kTrue = 0, kFalse = 1, kUndef = 2;
 // records that come back with a pass's counters (256 KB of pinned memory)
-constexpr uint32_t kSharerInline = 16384;
+constexpr uint32_t kSharerInline = 16384 - kInlineOffset / sizeof(gss_report);
 constexpr int kSlots = 32;  // assignments per solver per pass (Assigs.cuh:37-39)
 
 // Statistics, in the reference's order and with its names
@@ -183,6 +183,7 @@ private:
         int active_words = 0;
         int64_t n_reports = 0;
         int32_t number = 0;      // pass_no_ at its launch
+        bool filtered = false;   // checked behind the word-level filter
         // device report queues and their counters, pinned host copies of the
         // counters (+ error flag), the start and last-slot masks and the reports
         DevBuf d_reports, d_counts;
@@ -203,6 +204,7 @@ private:
     int recover_from_oom();
     int launch_pass();
     int run_check(Pass &p);
+    int refresh_agg(int64_t n_updates);
     int ensure_state();
     int append_clauses(std::vector<int64_t> &ids, std::vector<int32_t> &lits, std::vector<uint32_t> &lens);
     void reserve_for_budget(size_t n_new, size_t n_new_lits);
@@ -274,6 +276,9 @@ private:
     std::vector<std::unique_ptr<SolverAssigs>> solvers_;
     std::vector<std::unique_ptr<SolverReported>> reported_;
     DevBuf d_state_, d_start_, d_sow_, d_updates_, d_last_mask_;
+    DevBuf d_agg_;              // the filter's table of d_state_, kept as variables change
+    bool agg_ok_ = false;       // d_agg_ follows the state
+    int filter_pause_ = 0;      // passes to run without the filter (it kept too much)
     PinnedBuf h_updates_;
     PinnedBuf h_append_;             // staging of appended clauses (literals, offsets, ids)
     cudaEvent_t append_staged_ = nullptr;

@@ -6,7 +6,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-INLINE = 65536  # kEngineInline
+INLINE = 65520  # kEngineInline
 
 
 def _unit_clauses(eng, n, n_words):
