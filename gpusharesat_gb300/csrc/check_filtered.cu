@@ -28,50 +28,12 @@ namespace {
 
 // The filter's table of a literal: words with a slot where it is false (x)
 // and where it is undefined (y).
-__device__ __forceinline__ uint64_t policy_keep() {
-    uint64_t p;
-    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
 __device__ __forceinline__ uint2 ld_agg(const uint2 *p) {
     uint2 v;
     asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;"
         : "=r"(v.x), "=r"(v.y)
         : "l"(p), "l"(policy_keep()));
     return v;
-}
-
-// The 16-byte chunk of literals that holds position `pos` (kClausePad literals
-// after the last clause keep it inside the buffer).
-__device__ __forceinline__ uint4 ld_chunk(const int32_t *lits, uint32_t pos) {
-    uint4 v;
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-        : "l"(lits + (pos & ~3u)));
-    return v;
-}
-
-__device__ __forceinline__ int lane_id() {
-    int l;
-    asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
-    return l;
-}
-
-// Combines two runs of literals: f = every literal false, o = one undefined
-// and the rest false; the order does not matter.
-__device__ __forceinline__ void merge_runs(uint32_t &f, uint32_t &o, uint32_t f2, uint32_t o2) {
-    o = (f & o2) | (o & f2);
-    f &= f2;
-}
-
-// A run of up to 32 literals, one per lane, over the whole warp; every lane
-// gets the result.
-__device__ __forceinline__ void warp_runs(uint32_t &f, uint32_t &o) {
-#pragma unroll
-    for (int d = 16; d; d >>= 1) {
-        const uint32_t f2 = __shfl_xor_sync(kFull, f, d), o2 = __shfl_xor_sync(kFull, o, d);
-        merge_runs(f, o, f2, o2);
-    }
 }
 
 constexpr int kPair = 2;        // table entries a lane reads at a time
@@ -83,11 +45,6 @@ constexpr uint32_t kFewChunks = 3;
 constexpr int kFewWords = 4;    // words left for which a survivor is checked literal-parallel
 constexpr int kFewSurvivors = 8;
 constexpr int kFilterStage = 64;  // staged records per warp: few are found
-
-__device__ __forceinline__ void flush_block_part(const CheckArgs &a, gss_report *stage, uint32_t n) {
-    const uint32_t part = blockIdx.x % a.n_parts;
-    flush_stage(stage, n, a.out + (size_t) part * a.cap_per_part, a.counts + part, a.cap_per_part, lane_id());
-}
 
 // The rest of the filter for the clauses of the lanes in `open`, one by one
 // with 32 literals a step; returns the lane's words left.
@@ -261,23 +218,15 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_filtered_kernel(const
     const uint32_t n_groups = (n_scan + 31) / 32;
     const uint32_t n_tasks = n_groups * a.n_blocks;  // below 2^32 (launch_check_filtered)
     // A task's clauses and their offsets are loaded during the task before it,
-    // its number (a work counter's) two tasks before.
-    // Every warp starts with the task of its own number; the rest come from
-    // its block's counter, of kWorkCounters that share the tasks in turn, so
-    // that warps side by side in time stay side by side in the database.
-    const uint32_t n_warps = gridDim.x * kWarps;
-    const uint32_t n_counters = gridDim.x < 4 * kWorkCounters ? 1u : kWorkCounters;
-    const uint32_t mine = blockIdx.x % n_counters;
-    auto take = [&]() -> uint32_t {
-        return lane == 0 ? n_warps + mine + n_counters * atomicAdd(work + mine * kWorkStride, 1u) : 0u;
-    };
+    // its number two tasks before.
+    const TaskCounter counter(work);
     auto clause_at = [&](uint32_t task) -> uint32_t {
         if (task >= n_tasks) return 0xFFFFFFFFu;
         const uint32_t i = task % n_groups * 32 + lane;
         return i < n_scan ? scan_clause(a, i) : 0xFFFFFFFFu;
     };
-    uint32_t task = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    uint32_t next = __shfl_sync(kFull, take(), 0);
+    uint32_t task = counter.first();
+    uint32_t next = __shfl_sync(kFull, counter.take(lane), 0);
     uint32_t c = clause_at(task), pos = 0, end = 0;
     if (c < a.n_clauses) {
         pos = (uint32_t) __ldg(a.offsets + c);
@@ -286,7 +235,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_filtered_kernel(const
     uint4 chunk = make_uint4(0u, 0u, 0u, 0u);  // the literals around pos
     if (pos < end) chunk = ld_chunk(a.lits, pos);
     while (task < n_tasks) {
-        const uint32_t after = take();
+        const uint32_t after = counter.take(lane);
         const uint32_t c1 = clause_at(next);
         uint32_t pos1 = 0, end1 = 0;
         if (c1 < a.n_clauses) {

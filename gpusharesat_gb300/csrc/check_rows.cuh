@@ -38,6 +38,72 @@ __device__ __forceinline__ void flush_stage(gss_report *stage, uint32_t n, gss_r
     __syncwarp();
 }
 
+__device__ __forceinline__ int lane_id() {
+    int l;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
+    return l;
+}
+
+// Flushes a warp's stage into its block's partition.
+__device__ __forceinline__ void flush_block_part(const CheckArgs &a, gss_report *stage, uint32_t n) {
+    const uint32_t part = blockIdx.x % a.n_parts;
+    flush_stage(stage, n, a.out + (size_t) part * a.cap_per_part, a.counts + part, a.cap_per_part, lane_id());
+}
+
+// L2 policy of small tables that every warp gathers from: they keep their
+// place. (L1::no_allocate without a policy marks a load evict-first in L2.)
+__device__ __forceinline__ uint64_t policy_keep() {
+    uint64_t p;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+// The 16-byte chunk of literals that holds position `pos` (kClausePad literals
+// after the last clause keep it inside the buffer).
+__device__ __forceinline__ uint4 ld_chunk(const int32_t *lits, uint32_t pos) {
+    uint4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+        : "l"(lits + (pos & ~3u)));
+    return v;
+}
+
+// Combines two runs of literals: f = every literal false, o = one undefined
+// and the rest false; the order does not matter.
+__device__ __forceinline__ void merge_runs(uint32_t &f, uint32_t &o, uint32_t f2, uint32_t o2) {
+    o = (f & o2) | (o & f2);
+    f &= f2;
+}
+
+// A run of up to 32 literals, one per lane, over the whole warp; every lane
+// gets the result.
+__device__ __forceinline__ void warp_runs(uint32_t &f, uint32_t &o) {
+#pragma unroll
+    for (int d = 16; d; d >>= 1) {
+        const uint32_t f2 = __shfl_xor_sync(kFull, f, d), o2 = __shfl_xor_sync(kFull, o, d);
+        merge_runs(f, o, f2, o2);
+    }
+}
+
+// Tasks of a persistent kernel: every warp starts with the task of its own
+// number; the rest come from its block's counter, of kWorkCounters that share
+// the tasks in turn, so that warps side by side in time stay side by side in
+// the database.
+struct TaskCounter {
+    uint32_t *counter;
+    uint32_t base, step;
+    __device__ __forceinline__ explicit TaskCounter(uint32_t *work) {
+        step = gridDim.x < 4 * kWorkCounters ? 1u : kWorkCounters;
+        const uint32_t mine = blockIdx.x % step;
+        counter = work + mine * kWorkStride;
+        base = gridDim.x * kWarps + mine;
+    }
+    __device__ __forceinline__ uint32_t first() const { return blockIdx.x * kWarps + (threadIdx.x >> 5); }
+    // lane 0 gets a task's number (to be broadcast), the others 0
+    __device__ __forceinline__ uint32_t take(int lane) const {
+        return lane == 0 ? base + step * atomicAdd(counter, 1u) : 0u;
+    }
+};
+
 // {isDef, isTrue} of WPL consecutive words
 template <int WPL>
 struct Row {

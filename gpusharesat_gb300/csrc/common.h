@@ -223,6 +223,10 @@ bool valid_wide_persist_variant(int wpl, int lpc, int g);
 bool valid_wide_variant(int wpl, int lpc, int g, int occ);
 bool valid_tiled_variant(int lpc, int k);
 
+// A pass of one slot block of 1, 2 or 4 words (a.lpc), a lane per clause;
+// tasks from the counters at `work`.
+int launch_check_narrow(const CheckArgs &a, uint32_t *work, cudaStream_t stream, int sm_count);
+bool valid_narrow_variant(int words);
 // The persistent wide kernel behind the word-level filter (h_args.agg, or
 // that of d_args).
 int launch_check_filtered(const CheckArgs *d_args, const CheckArgs &h_args, int wpl, int lpc, uint32_t *work,

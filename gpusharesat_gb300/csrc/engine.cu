@@ -926,6 +926,9 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         wide && ((eng->flags & GSS_VARIANT_PERSISTENT) ||
                  (eng->kind == GSS_KERNEL_AUTO &&
                   valid_wide_persist_variant(words_per_lane(eng->state_kind), eng->state_lpc, eng->state_g)));
+    // up to four words: a lane takes a clause with all of them
+    const bool narrow = eng->kind == GSS_KERNEL_AUTO && eng->state_kind == GSS_KERNEL_DIRECT && eng->n_blocks == 1 &&
+                        valid_narrow_variant(eng->state_lpc);
     // behind the word-level filter where the state's table says that it pays
     const bool filtered = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
                           filter_tasks(a) < kMaxFilterTasks;
@@ -1002,6 +1005,11 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     bool work_used = false;  // the memset above cleared the work counter for the first launch
     auto launch = [&](const CheckArgs &args) -> int {
         if (eng->state_kind == GSS_KERNEL_TILED) return launch_check_tiled(args, eng->stream, eng->sm_count);
+        if (narrow) {
+            if (work_used) GSS_CUDA_TRY(cudaMemsetAsync(work, 0, kWorkBytes, eng->stream));
+            work_used = true;
+            return launch_check_narrow(args, work, eng->stream, eng->sm_count);
+        }
         if (persistent) {
             // arguments by value; the work counter restarts for each launch
             if (work_used) GSS_CUDA_TRY(cudaMemsetAsync(work, 0, kWorkBytes, eng->stream));

@@ -936,6 +936,8 @@ int Sharer::run_check(Pass &p) {
                 GSS_TRY(launch_check_wide_persist(nullptr, a, wpl, eff_lpc_, eff_depth_, work, stream_, sm_count_));
         } else if (wide) {
             GSS_TRY(launch_check_wide(a, wpl, (flags_ & GSS_VARIANT_OCCUPANCY) ? 1 : 0, stream_, sm_count_));
+        } else if (kind_ == GSS_KERNEL_AUTO && n_blocks_ == 1 && valid_narrow_variant(eff_lpc_)) {
+            GSS_TRY(launch_check_narrow(a, work_counter(a.counts), stream_, sm_count_));
         } else {
             GSS_TRY(launch_check(a, stream_, sm_count_));
         }
