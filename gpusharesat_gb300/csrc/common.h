@@ -204,6 +204,24 @@ int launch_deliver(const CheckArgs *d_args, const gss_report *parts, const uint3
 // Synchronizes `stream`; returns the live clause and literal counts.
 int compact_by_id(const CompactArgs &a, cudaStream_t stream, int sm_count, uint32_t *n_out, int64_t *lits_out);
 
+// The automatic variant for a pass of n_words words: kind, lanes per clause,
+// loads in flight. Up to four words a lane takes the whole clause (narrow
+// kernel). From five on, four words a lane with 256-bit loads, and the
+// narrowest row that holds all words (32 at most): one scan of the database
+// where two blocks of half the width read every clause twice. Measured, one
+// wide block against the narrower kind or two blocks (600k clauses, lengths
+// 2-100), on fair-coin slots: 6 words 51 against 79 us, 11 words 73 against
+// 84, 24 words 120 against 129, 17 words 114 against 110; on trails, behind
+// the filter: 6 words 25 against 61, 11 and 17 words 28 against 37.
+inline void auto_layout(int n_words, int &kind, int &lpc, int &depth) {
+    kind = n_words > 4 ? GSS_KERNEL_WIDE4 : GSS_KERNEL_DIRECT;
+    if (n_words > 4)
+        lpc = n_words > 16 ? 8 : n_words > 8 ? 4 : 2;
+    else
+        lpc = n_words > 2 ? 4 : n_words > 1 ? 2 : 1;
+    depth = lpc == 1 ? 1 : 2;
+}
+
 // Launches the check kernel on `stream` (the counters must already be zero).
 // Returns a GSS status.
 int launch_check(const CheckArgs &a, cudaStream_t stream, int sm_count);

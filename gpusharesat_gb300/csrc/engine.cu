@@ -610,21 +610,7 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     if (n_vars > 0x7FFFFFFF) return set_error(GSS_ERR_INVALID, "too many variables");
     GSS_TRY(ensure_device(eng));
     int kind = eng->kind, lpc = eng->lpc, depth = eng->g;
-    if (kind == GSS_KERNEL_AUTO) {
-        // Measured on GB300 for the at-scale workload: four words per lane with
-        // 256-bit loads, two loads in flight, is fastest once a clause spans
-        // eight or more words; below that one word per lane.
-        depth = 2;
-        if (n_words >= 8) {
-            kind = GSS_KERNEL_WIDE4;
-            lpc = n_words >= 32 ? 8 : n_words >= 16 ? 4 : 2;
-        } else {
-            kind = GSS_KERNEL_DIRECT;
-            lpc = 1;
-            while (lpc < n_words) lpc *= 2;
-            if (lpc == 1) depth = 1;
-        }
-    }
+    if (kind == GSS_KERNEL_AUTO) auto_layout(n_words, kind, lpc, depth);
     const int wpl = words_per_lane(kind);
     if (lpc == 0) {
         // one word per lane up to a full warp (wide kinds: 32 words per block)

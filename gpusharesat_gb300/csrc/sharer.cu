@@ -99,6 +99,10 @@ unsigned grid_for(uint64_t n, int sm_count) {
 // The filter's use (Sharer::collect). Its own pass is about a quarter of the
 // plain check's time, and what it keeps costs the plain check's share again.
 constexpr double kFilterKeepMost = 0.5;
+// (clauses x slot blocks) from which the filter pays for its table's upkeep,
+// two launches a pass (7 solvers, 50k clauses: 120 us a pass without, 126
+// with; 64 solvers, 1.2e6 clauses: 220 us of check without, 85 with).
+constexpr int64_t kFilterMinPairs = 150000;
 constexpr int kFilterPause = 64;
 
 // ---- one solver's ring ----
@@ -457,18 +461,7 @@ int Sharer::ensure_state() {
     const int need_vars = (int) std::max<int64_t>(n_vars_, max_var_ + 1);
     // resolve the kernel variant for this word count (as gss_state_set)
     int kind = kind_, lpc = lpc_req_, depth = depth_req_;
-    if (kind == GSS_KERNEL_AUTO) {
-        depth = 2;
-        if (n_words >= 8) {
-            kind = GSS_KERNEL_WIDE4;
-            lpc = n_words >= 32 ? 8 : n_words >= 16 ? 4 : 2;
-        } else {
-            kind = GSS_KERNEL_DIRECT;
-            lpc = 1;
-            while (lpc < n_words) lpc *= 2;
-            if (lpc == 1) depth = 1;
-        }
-    }
+    if (kind == GSS_KERNEL_AUTO) auto_layout(n_words, kind, lpc, depth);
     const int wpl = kind == GSS_KERNEL_WIDE4 ? 4 : kind == GSS_KERNEL_WIDE2 ? 2 : 1;
     if (lpc == 0) {
         lpc = 1;
@@ -513,26 +506,27 @@ int Sharer::ensure_state() {
     std::vector<int32_t> sow(n_blocks * bw);
     for (int w = 0; w < n_blocks * bw; w++) sow[w] = w < n_words ? w : 0;
     GSS_CUDA_TRY(cudaMemcpy(d_sow_.ptr, sow.data(), sow.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    // the filter's table; without room for it the passes run without
-    agg_ok_ = kind_ == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && need_vars > 0 && n_words > 0 &&
-              d_agg_.reserve((size_t) n_blocks * need_vars * 2 * sizeof(uint2)) == GSS_OK;
+    agg_possible_ = kind_ == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && need_vars > 0 && n_words > 0;
+    agg_ok_ = false;
     filter_pause_ = 0;
-    if (agg_ok_)
-        GSS_TRY(launch_load_state((const uint2 *) d_state_.ptr, nullptr, (uint2 *) d_agg_.ptr, nullptr,
-                                  (uint32_t) dev_vars_, (uint32_t) dev_words_, (uint32_t) bw_, (uint32_t) n_blocks_,
-                                  true, stream_, sm_count_));
     return GSS_OK;
+}
+
+int Sharer::rebuild_agg() {
+    // without room for the table the passes run without it
+    agg_ok_ = d_agg_.reserve((size_t) n_blocks_ * dev_vars_ * 2 * sizeof(uint2)) == GSS_OK;
+    if (!agg_ok_) return GSS_OK;
+    return launch_load_state((const uint2 *) d_state_.ptr, nullptr, (uint2 *) d_agg_.ptr, nullptr,
+                             (uint32_t) dev_vars_, (uint32_t) dev_words_, (uint32_t) bw_, (uint32_t) n_blocks_, true,
+                             stream_, sm_count_);
 }
 
 int Sharer::refresh_agg(int64_t n_updates) {
     // The filter's table after n_updates words of the state (d_updates_)
     // changed: their rows again, or all of them when that is less to read (an
     // update's row is 8 * bw_ bytes; several updates may share one).
-    if (!agg_ok_ || n_updates == 0) return GSS_OK;
-    if (n_updates >= (int64_t) dev_vars_ * n_blocks_)
-        return launch_load_state((const uint2 *) d_state_.ptr, nullptr, (uint2 *) d_agg_.ptr, nullptr,
-                                 (uint32_t) dev_vars_, (uint32_t) dev_words_, (uint32_t) bw_, (uint32_t) n_blocks_,
-                                 true, stream_, sm_count_);
+    if (n_updates == 0) return GSS_OK;
+    if (n_updates >= (int64_t) dev_vars_ * n_blocks_) return rebuild_agg();
     return launch_refresh_agg((const StateUpdate *) d_updates_.ptr, (uint32_t) n_updates,
                               (const uint2 *) d_state_.ptr, (uint2 *) d_agg_.ptr, (uint32_t) dev_vars_,
                               (uint32_t) dev_words_, (uint32_t) bw_, stream_, sm_count_);
@@ -1000,7 +994,7 @@ int Sharer::collect(Pass &p) {
             (const StateUpdate *) d_updates_.ptr, (uint32_t) p.n_updates, (const uint32_t *) d_last_mask_.ptr,
             (uint2 *) d_state_.ptr, (uint32_t) dev_vars_, (uint32_t) bw_);
         GSS_CUDA_TRY(cudaGetLastError());
-        GSS_TRY(refresh_agg(p.n_updates));
+        if (agg_ok_) GSS_TRY(refresh_agg(p.n_updates));
     }
     // a filter that keeps most clauses costs more than it saves: leave it out
     // for some passes, then look again
@@ -1174,8 +1168,14 @@ int Sharer::launch_pass() {
                 (const StateUpdate *) d_updates_.ptr, (uint32_t) ups.size(), (uint2 *) d_state_.ptr,
                 (uint32_t) dev_vars_, (uint32_t) bw_);
             GSS_CUDA_TRY(cudaGetLastError());
-            GSS_TRY(refresh_agg((int64_t) ups.size()));
         }
+        // the filter's table follows while the database is large enough for it
+        if (!agg_possible_ || (int64_t) dev_clauses_ * n_blocks_ < kFilterMinPairs)
+            agg_ok_ = false;
+        else if (!agg_ok_)
+            GSS_TRY(rebuild_agg());
+        else
+            GSS_TRY(refresh_agg((int64_t) ups.size()));
         p.n_clauses = dev_clauses_;
         return run_check(p);
     };

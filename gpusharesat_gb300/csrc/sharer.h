@@ -204,6 +204,7 @@ private:
     int recover_from_oom();
     int launch_pass();
     int run_check(Pass &p);
+    int rebuild_agg();
     int refresh_agg(int64_t n_updates);
     int ensure_state();
     int append_clauses(std::vector<int64_t> &ids, std::vector<int32_t> &lits, std::vector<uint32_t> &lens);
@@ -277,6 +278,7 @@ private:
     std::vector<std::unique_ptr<SolverReported>> reported_;
     DevBuf d_state_, d_start_, d_sow_, d_updates_, d_last_mask_;
     DevBuf d_agg_;              // the filter's table of d_state_, kept as variables change
+    bool agg_possible_ = false; // the layout has a filtered kernel
     bool agg_ok_ = false;       // d_agg_ follows the state
     int filter_pause_ = 0;      // passes to run without the filter (it kept too much)
     PinnedBuf h_updates_;

@@ -51,7 +51,7 @@ def _same(eng, lits, offsets, state, start, alive=None):
     return len(got)
 
 
-@pytest.mark.parametrize("n_words", [8, 9, 11, 15, 16, 17, 31, 32, 33, 45, 96])
+@pytest.mark.parametrize("n_words", [5, 7, 8, 9, 11, 15, 16, 17, 31, 32, 33, 45, 96])
 @pytest.mark.parametrize("n", [1, 31, 33, 3000])
 def test_filtered_pass_equals_oracle(lib, n_words, n):
     import gpusharesat_gb300 as g
