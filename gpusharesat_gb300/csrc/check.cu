@@ -36,6 +36,8 @@
 // partition keeps counting, so the host sees the overflow and runs again.
 #include <string.h>
 
+#include <algorithm>
+
 #include "check_rows.cuh"
 
 namespace gss {
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(kWarps * 32) check_kernel(CheckArgs a) {
     gss_report *stage = stage_all[wib];
     const uint32_t part = blockIdx.x % a.n_parts;
     gss_report *out = a.out + (size_t) part * a.cap_per_part;
-    uint32_t *counter = a.counts + part;
+    uint32_t *counter = a.counts + (size_t) part * a.count_stride;
     uint32_t nstaged = 0;
     const bool hint = a.cache_hints != 0;
     const uint64_t pol_keep = policy_evict_last();
@@ -210,10 +212,9 @@ __device__ __forceinline__ void ld_row_hint<4>(const uint2 *p, Row<4> &r, uint64
 // variants need their registers for the rows in flight and stay uncapped.
 constexpr int default_min_blocks(int wpl, int g) { return (wpl == 4 && g <= 2) ? 6 : 1; }
 
-// MAP_IDS = false: reports carry the clause's CSR index itself (a.orig unused).
 // With cache_hints: state rows evict-last in L2, clause literals evict-first,
 // report records streamed.
-template <int WPL, int LPC, int G, int MINB, bool MAP_IDS = true, bool HINT = false>
+template <int WPL, int LPC, int G, int MINB, bool HINT = false>
 __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_kernel(CheckArgs a) {
     constexpr int CPW = 32 / LPC;
     constexpr int BW = WPL * LPC;
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_kernel(CheckArgs
     gss_report *stage = stage_all[wib];
     const uint32_t part = blockIdx.x % a.n_parts;
     gss_report *out = a.out + (size_t) part * a.cap_per_part;
-    uint32_t *counter = a.counts + part;
+    uint32_t *counter = a.counts + (size_t) part * a.count_stride;
     uint32_t nstaged = 0;
     constexpr bool hint = HINT;
     const uint64_t pol_keep = hint ? policy_evict_last() : 0ull;
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_kernel(CheckArgs
                 }
                 if (rep) {
                     gss_report r;
-                    r.clause = MAP_IDS ? __ldg(a.orig + c) : c;
+                    r.clause = __ldg(a.orig + c);
                     r.word = w0 + j;
                     r.mask = rep;
                     r.solver = (uint32_t) __ldg(a.solver_of_word + w0 + j);
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_pf_kernel(CheckA
     gss_report *stage = stage_all[wib];
     const uint32_t part = blockIdx.x % a.n_parts;
     gss_report *out = a.out + (size_t) part * a.cap_per_part;
-    uint32_t *counter = a.counts + part;
+    uint32_t *counter = a.counts + (size_t) part * a.count_stride;
     uint32_t nstaged = 0;
 
     const uint32_t n_scan = scan_count(a);
@@ -467,33 +468,41 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_pf_kernel(CheckA
     if (nstaged) flush_stage(stage, nstaged, out, counter, a.cap_per_part, lane);
 }
 
-// Persistent wide variant: as check_wide_kernel, with (1) its arguments read
-// from device memory, so a captured CUDA graph can run it pass after pass
-// while the database and the assignment state change, and (2) tasks taken in
-// chunks from a device work counter (zeroed before the launch) instead of a
-// fixed stride, so clauses of very different lengths balance across warps.
+// Persistent wide variant: as check_wide_kernel, with (1) its arguments by
+// value or, for a captured CUDA graph that runs pass after pass while the
+// database and the assignment state change, from device memory (DEV), and (2)
+// tasks of kTaskChunk clause groups from work counters (zeroed before the
+// launch) instead of a fixed stride, so clauses of very different lengths
+// balance across warps that stay side by side in the database.
+//
+// Bound by instruction issue while the state fits L2 (2e6 clauses x 1024
+// fair-coin slots over 2^17 variables: 356 -> 315 us) and by the random
+// row gathers beyond it (2^20: 474 -> 457 us). Hence a division per task of
+// four groups, not per group, three logic operations a word and literal
+// (apply_literal), and records that get their clause id and solver where they
+// are flushed, 32 at a time (a stage of 192 records: 315 against 327 us with
+// 128, over 2^17 variables). The arguments are read from shared memory: kept
+// in the constant bank, their loads are hoisted into registers that spill
+// (401 us).
 constexpr uint32_t kTaskChunk = 4;
+constexpr int kPersistStage = 192;
 
-template <int WPL, int LPC, int G, int MINB>
+template <int WPL, int LPC, int G, int MINB, bool DEV>
 __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(const CheckArgs *__restrict__ pa,
-                                                                                const CheckArgs av,
+                                                                                const __grid_constant__ CheckArgs av,
                                                                                 uint32_t *__restrict__ work) {
     constexpr int CPW = 32 / LPC;
     constexpr int BW = WPL * LPC;
     __shared__ CheckArgs sa;
-    __shared__ gss_report stage_all[kWarps][kStage];
-    if (threadIdx.x == 0) sa = pa ? *pa : av;
+    __shared__ gss_report stage_all[kWarps][kPersistStage];
+    if (threadIdx.x == 0) sa = DEV ? *pa : av;
     __syncthreads();
     const CheckArgs &a = sa;
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
     const int sub = lane % LPC;
     const int grp = lane / LPC;
     const int gbase = grp * LPC;
-    gss_report *stage = stage_all[wib];
-    const uint32_t part = blockIdx.x % a.n_parts;
-    gss_report *out = a.out + (size_t) part * a.cap_per_part;
-    uint32_t *counter = a.counts + part;
+    gss_report *stage = stage_all[threadIdx.x >> 5];
     uint32_t nstaged = 0;
 
     const uint32_t n_scan = scan_count(a);
@@ -505,24 +514,26 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
 #pragma unroll
         for (int q = 0; q < 2 * WPL; q++) st[i].v[q] = 0u;
     while (true) {
-        uint32_t first = 0;
-        if (lane == 0) first = atomicAdd(work, kTaskChunk);
-        first = __shfl_sync(kFull, first, 0);
-        if ((uint64_t) first >= n_tasks) break;
-        const uint64_t last = min((uint64_t) first + kTaskChunk, n_tasks);
-        for (uint64_t task = first; task < last; task++) {
-            const uint32_t blk = (uint32_t) (task / n_groups);
-            const uint32_t g = (uint32_t) (task - (uint64_t) blk * n_groups);
+        uint32_t unit = 0;
+        if (lane == 0) unit = task_from(work);
+        unit = __shfl_sync(kFull, unit, 0);
+        const uint64_t first = (uint64_t) unit * kTaskChunk;
+        if (first >= n_tasks) break;
+        uint32_t blk, g;
+        if (n_tasks <= 0xFFFFFFFFull) {
+            blk = (uint32_t) first / n_groups;
+            g = (uint32_t) first - blk * n_groups;
+        } else {
+            blk = (uint32_t) (first / n_groups);
+            g = (uint32_t) (first - (uint64_t) blk * n_groups);
+        }
+        for (uint32_t left = (uint32_t) min((uint64_t) kTaskChunk, n_tasks - first); left; left--) {
             const uint32_t i = g * CPW + grp;
             const uint32_t c = i < n_scan ? scan_clause(a, i) : 0xFFFFFFFFu;
             const bool valid = c < a.n_clauses && clause_live(a, c);
-            const uint32_t w0 = blk * BW + sub * WPL;
-            uint32_t af[WPL], ou[WPL];
+            uint32_t af[WPL], live[WPL];
 #pragma unroll
-            for (int j = 0; j < WPL; j++) {
-                af[j] = valid ? __ldg(a.start + w0 + j) : 0u;
-                ou[j] = 0u;
-            }
+            for (int j = 0; j < WPL; j++) af[j] = live[j] = valid ? __ldg(a.start + blk * BW + sub * WPL + j) : 0u;
             uint32_t pos = 0, end = 0;
             if (valid) {
                 pos = (uint32_t) __ldg(a.offsets + c);
@@ -532,7 +543,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
             while (true) {
                 bool alive = false;
 #pragma unroll
-                for (int j = 0; j < WPL; j++) alive |= (af[j] | ou[j]) != 0u;
+                for (int j = 0; j < WPL; j++) alive |= live[j] != 0u;
                 if (!__any_sync(kFull, alive && pos < end)) break;
                 const int32_t chunk = (pos + sub < end) ? __ldg(a.lits + pos + sub) : 0;
                 const int navail = (int) min((uint32_t) LPC, end > pos ? end - pos : 0u);
@@ -540,7 +551,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
                 for (int k0 = 0; k0 < LPC; k0 += G) {
                     alive = false;
 #pragma unroll
-                    for (int j = 0; j < WPL; j++) alive |= (af[j] | ou[j]) != 0u;
+                    for (int j = 0; j < WPL; j++) alive |= live[j] != 0u;
                     if (!__any_sync(kFull, alive && k0 < navail)) break;
                     uint32_t lit[G];
 #pragma unroll
@@ -552,14 +563,10 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
 #pragma unroll
                     for (int i = 0; i < G; i++) {
                         if (k0 + i < navail) {
-                            const bool neg = (lit[i] & 1u) != 0u;
+                            const uint32_t neg = (lit[i] & 1u) - 1u;
 #pragma unroll
-                            for (int j = 0; j < WPL; j++) {
-                                const uint32_t d = st[i].v[2 * j], t = st[i].v[2 * j + 1];
-                                const uint32_t f = (neg ? t : ~t) & d;
-                                ou[j] = (af[j] & ~d) | (ou[j] & f);
-                                af[j] &= f;
-                            }
+                            for (int j = 0; j < WPL; j++)
+                                apply_literal(st[i].v[2 * j], st[i].v[2 * j + 1], neg, af[j], live[j]);
                         }
                     }
                 }
@@ -567,27 +574,24 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
             }
 #pragma unroll
             for (int j = 0; j < WPL; j++) {
-                const uint32_t rep = af[j] | ou[j];
-                const unsigned bal = __ballot_sync(kFull, rep != 0u);
+                const unsigned bal = __ballot_sync(kFull, live[j] != 0u);
                 if (bal) {
-                    if (nstaged + 32 > (uint32_t) kStage) {
-                        flush_stage(stage, nstaged, out, counter, a.cap_per_part, lane);
+                    if (nstaged + 32 > (uint32_t) kPersistStage) {
+                        flush_mapped(a, stage, nstaged);
                         nstaged = 0;
                     }
-                    if (rep) {
-                        gss_report r;
-                        r.clause = __ldg(a.orig + c);
-                        r.word = w0 + j;
-                        r.mask = rep;
-                        r.solver = (uint32_t) __ldg(a.solver_of_word + w0 + j);
-                        stage[nstaged + __popc(bal & lanemask_lt())] = r;
-                    }
+                    if (live[j])
+                        stage_record(stage + nstaged + __popc(bal & lanemask_lt()), c, blk * BW + sub * WPL + j, live[j]);
                     nstaged += __popc(bal);
                 }
             }
+            if (++g == n_groups) {
+                g = 0;
+                blk++;
+            }
         }
     }
-    if (nstaged) flush_stage(stage, nstaged, out, counter, a.cap_per_part, lane);
+    if (nstaged) flush_mapped(a, stage, nstaged);
 }
 
 template <int WPL, int LPC, int G>
@@ -595,11 +599,21 @@ int launch_wide_persist_variant(const CheckArgs *d_args, const CheckArgs &h_args
                                 int sm_count) {
     constexpr int MINB = default_min_blocks(WPL, G);
     int per_sm = 0;
-    GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, check_wide_persist_kernel<WPL, LPC, G, MINB>,
-                                                               kWarps * 32, 0));
+    GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, check_wide_persist_kernel<WPL, LPC, G, MINB, false>, kWarps * 32, 0));
     if (per_sm < 1) per_sm = 1;
-    check_wide_persist_kernel<WPL, LPC, G, MINB><<<(unsigned) (sm_count * per_sm), kWarps * 32, 0, stream>>>(
-        d_args, h_args, work);
+    uint64_t blocks = (uint64_t) sm_count * per_sm;
+    if (d_args) {  // a captured graph serves databases of other sizes too: the full grid
+        check_wide_persist_kernel<WPL, LPC, G, MINB, true><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
+            d_args, h_args, work);
+    } else {
+        constexpr int CPW = 32 / LPC;
+        const uint64_t n_tasks = (uint64_t) ((scan_count(h_args) + CPW - 1) / CPW) * h_args.n_blocks;
+        const uint64_t units = (n_tasks + kTaskChunk - 1) / kTaskChunk;
+        blocks = std::min<uint64_t>(blocks, std::max<uint64_t>((units + kWarps - 1) / kWarps, 1));
+        check_wide_persist_kernel<WPL, LPC, G, MINB, false><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
+            nullptr, h_args, work);
+    }
     GSS_CUDA_TRY(cudaGetLastError());
     return GSS_OK;
 }
@@ -621,11 +635,11 @@ int launch_wide_pf_variant(const CheckArgs &a, cudaStream_t stream, int sm_count
     return GSS_OK;
 }
 
-template <int WPL, int LPC, int G, int MINB, bool MAP_IDS = true, bool HINT = false>
+template <int WPL, int LPC, int G, int MINB, bool HINT = false>
 int launch_wide_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
     int per_sm = 0;
     GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, check_wide_kernel<WPL, LPC, G, MINB, MAP_IDS, HINT>, kWarps * 32, 0));
+        &per_sm, check_wide_kernel<WPL, LPC, G, MINB, HINT>, kWarps * 32, 0));
     if (per_sm < 1) per_sm = 1;
     constexpr int CPW = 32 / LPC;
     const uint64_t n_tasks = (uint64_t) ((scan_count(a) + CPW - 1) / CPW) * a.n_blocks;
@@ -633,7 +647,7 @@ int launch_wide_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
     const uint64_t need = (n_tasks + kWarps - 1) / kWarps;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
-    check_wide_kernel<WPL, LPC, G, MINB, MAP_IDS, HINT><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(a);
+    check_wide_kernel<WPL, LPC, G, MINB, HINT><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(a);
     GSS_CUDA_TRY(cudaGetLastError());
     return GSS_OK;
 }
@@ -713,9 +727,9 @@ int launch_check_wide(const CheckArgs &a, int wpl, int occ, cudaStream_t stream,
     if (a.n_clauses == 0 || a.n_blocks == 0 || scan_count(a) == 0) return GSS_OK;
     // L2 policies (cache_hints) for the 4-words-per-lane, 8-lane kinds
     if (wpl == 4 && a.lpc == 8 && !occ && a.cache_hints) {
-        if (a.g == 1) return launch_wide_variant<4, 8, 1, 1, true, true>(a, stream, sm_count);
-        if (a.g == 2) return launch_wide_variant<4, 8, 2, 1, true, true>(a, stream, sm_count);
-        if (a.g == 4) return launch_wide_variant<4, 8, 4, 1, true, true>(a, stream, sm_count);
+        if (a.g == 1) return launch_wide_variant<4, 8, 1, 1, true>(a, stream, sm_count);
+        if (a.g == 2) return launch_wide_variant<4, 8, 2, 1, true>(a, stream, sm_count);
+        if (a.g == 4) return launch_wide_variant<4, 8, 4, 1, true>(a, stream, sm_count);
     }
 #define GSS_WV(W, L, GG)                                                                      \
     if (wpl == W && a.lpc == L && a.g == GG)                                                  \
@@ -762,19 +776,20 @@ int launch_check(const CheckArgs &a, cudaStream_t stream, int sm_count) {
 
 // ------------------------------------------------ allocation-free pass ----
 //
-// gss_check_noalloc: the wide check kernel for callers that cannot allocate
-// device memory. The kernel's only working memory is its report reservation
-// counters (one per output partition); here they live in a fixed,
-// file-scope device array instead of a cudaMalloc'ed buffer, so the call
-// allocates nothing. Every GPU that loads this library holds the array
-// (256 bytes) until the process exits.
+// gss_check_noalloc: the persistent wide kernel for callers that cannot
+// allocate device memory. The kernel's only working memory is its counters
+// (report reservations and tasks, 256 bytes each, see counter_bytes); here
+// they live in a fixed, file-scope device array instead of a cudaMalloc'ed
+// buffer, so the call allocates nothing. Every GPU that loads this library
+// holds the array (20 KB) until the process exits.
 
 namespace {
 
 constexpr uint32_t kNoAllocMaxParts = 64;
 
-// Report reservation counters of gss_check_noalloc, shared by all its calls.
-static __device__ __align__(256) uint32_t g_noalloc_counters[kNoAllocMaxParts];
+// Counters of gss_check_noalloc, shared by all its calls.
+static __device__ __align__(256) uint32_t
+    g_noalloc_counters[(kNoAllocMaxParts + 1 + gss::kWorkCounters) * gss::kCountStride];
 
 // The counters' device address on the current device. In host code the
 // array's name is only a host-side stand-in, so every call asks the runtime
@@ -785,6 +800,11 @@ int noalloc_counters(uint32_t **out) {
     GSS_CUDA_TRY(cudaGetSymbolAddress(&p, g_noalloc_counters));
     *out = (uint32_t *) p;
     return GSS_OK;
+}
+
+__global__ void noalloc_counts_kernel(const uint32_t *__restrict__ counters, uint32_t n_parts,
+                                      uint32_t *__restrict__ out) {
+    if (threadIdx.x < n_parts) out[threadIdx.x] = counters[threadIdx.x * gss::kCountStride];
 }
 
 }  // namespace
@@ -811,7 +831,7 @@ extern "C" int gss_check_noalloc(const int32_t *lits, const int64_t *offsets, ui
     uint32_t *counters = nullptr;
     GSS_TRY(noalloc_counters(&counters));
     // every call starts from zeroed counters: they keep the previous call's values
-    GSS_CUDA_TRY(cudaMemsetAsync(counters, 0, n_parts * sizeof(uint32_t), st));
+    GSS_CUDA_TRY(cudaMemsetAsync(counters, 0, counter_bytes(n_parts), st));
     if (n_clauses > 0 && n_blocks > 0) {
         int dev = 0, sms = 0;
         GSS_CUDA_TRY(cudaGetDevice(&dev));
@@ -831,12 +851,14 @@ extern "C" int gss_check_noalloc(const int32_t *lits, const int64_t *offsets, ui
         a.solver_of_word = solver_of_word;
         a.out = out;
         a.counts = counters;
+        a.count_stride = kCountStride;
         a.n_parts = n_parts;
         a.cap_per_part = cap_per_part;
         a.lpc = 8;
         a.g = 2;
-        GSS_TRY((launch_wide_variant<4, 8, 2, default_min_blocks(4, 2), false>(a, st, sms)));
+        GSS_TRY((launch_wide_persist_variant<4, 8, 2>(nullptr, a, work_counter(counters, n_parts), st, sms)));
     }
-    GSS_CUDA_TRY(cudaMemcpyAsync(counts_out, counters, n_parts * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+    noalloc_counts_kernel<<<1, kNoAllocMaxParts, 0, st>>>(counters, n_parts, counts_out);
+    GSS_CUDA_TRY(cudaGetLastError());
     return GSS_OK;
 }

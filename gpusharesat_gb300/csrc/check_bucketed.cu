@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) check_bucketed_kernel(const Ch
     wo.stage = stage_all[threadIdx.x >> 5];
     const uint32_t part = blockIdx.x % a.n_parts;
     wo.out = a.out + (size_t) part * a.cap_per_part;
-    wo.counter = a.counts + part;
+    wo.counter = a.counts + (size_t) part * a.count_stride;
     wo.nstaged = 0;
     const uint32_t n_ranges = plan->n_ranges;
     const uint32_t groups = plan->group_base[n_ranges];  // clause groups over all ranges

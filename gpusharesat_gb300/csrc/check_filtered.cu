@@ -154,7 +154,7 @@ __device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, gss_repo
 #pragma unroll
         for (int j = 0; j < WPL; j++)
             al[j] = lv[j] = (words >> (sub * WPL + j)) & 1u ? __ldg(start + sub * WPL + j) : 0u;
-        scan_rows<WPL, LPC, G>(a.lits, rows + sub * WPL, p, e, sub, gbase, al, lv, st);
+        scan_rows<WPL, LPC, G>(a, rows + sub * WPL, p, e, sub, gbase, al, lv, st);
 #pragma unroll
         for (int j = 0; j < WPL; j++) {
             const unsigned bal = __ballot_sync(kFull, lv[j] != 0u);

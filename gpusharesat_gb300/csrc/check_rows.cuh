@@ -47,7 +47,31 @@ __device__ __forceinline__ int lane_id() {
 // Flushes a warp's stage into its block's partition.
 __device__ __forceinline__ void flush_block_part(const CheckArgs &a, gss_report *stage, uint32_t n) {
     const uint32_t part = blockIdx.x % a.n_parts;
-    flush_stage(stage, n, a.out + (size_t) part * a.cap_per_part, a.counts + part, a.cap_per_part, lane_id());
+    flush_stage(stage, n, a.out + (size_t) part * a.cap_per_part, a.counts + (size_t) part * a.count_stride,
+                a.cap_per_part, lane_id());
+}
+
+// A record as the kernels stage it: the clause's position; flush_mapped turns
+// it into the clause's id (or leaves it, without an id map) and adds the
+// solver, 32 records at a time.
+__device__ __forceinline__ void stage_record(gss_report *to, uint32_t c, uint32_t word, uint32_t mask) {
+    *reinterpret_cast<uint4 *>(to) = make_uint4(c, word, mask, 0u);
+}
+__device__ __forceinline__ void flush_mapped(const CheckArgs &a, const gss_report *stage, uint32_t n) {
+    const int lane = lane_id();
+    const uint32_t part = blockIdx.x % a.n_parts;
+    __syncwarp();
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(a.counts + (size_t) part * a.count_stride, n);
+    base = __shfl_sync(kFull, base, 0);
+    gss_report *out = a.out + (size_t) part * a.cap_per_part;
+    for (uint32_t i = lane; i < n; i += 32) {
+        uint4 r = reinterpret_cast<const uint4 *>(stage)[i];  // {clause, word, mask, solver}
+        if (a.orig) r.x = __ldg(a.orig + r.x);
+        r.w = (uint32_t) __ldg(a.solver_of_word + r.y);
+        if (base + i < a.cap_per_part) reinterpret_cast<uint4 *>(out)[base + i] = r;
+    }
+    __syncwarp();
 }
 
 // L2 policy of small tables that every warp gathers from: they keep their
@@ -84,6 +108,17 @@ __device__ __forceinline__ void warp_runs(uint32_t &f, uint32_t &o) {
     }
 }
 
+// A persistent kernel's next task, from its block's counter: kWorkCounters
+// of them share the tasks in turn, so that warps side by side in time stay
+// side by side in the database. (The block number is read where it is needed:
+// kept from the start it would cost a register.)
+__device__ __forceinline__ uint32_t task_from(uint32_t *work) {
+    uint32_t b;
+    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(b));
+    const uint32_t n = min(gridDim.x, kWorkCounters), mine = b % n;
+    return n * atomicAdd(work + mine * kCountStride, 1u) + mine;
+}
+
 // Tasks of a persistent kernel: every warp starts with the task of its own
 // number; the rest come from its block's counter, of kWorkCounters that share
 // the tasks in turn, so that warps side by side in time stay side by side in
@@ -94,7 +129,7 @@ struct TaskCounter {
     __device__ __forceinline__ explicit TaskCounter(uint32_t *work) {
         step = gridDim.x < 4 * kWorkCounters ? 1u : kWorkCounters;
         const uint32_t mine = blockIdx.x % step;
-        counter = work + mine * kWorkStride;
+        counter = work + mine * kCountStride;
         base = gridDim.x * kWarps + mine;
     }
     __device__ __forceinline__ uint32_t first() const { return blockIdx.x * kWarps + (threadIdx.x >> 5); }
@@ -146,7 +181,7 @@ __device__ __forceinline__ void apply_literal(uint32_t d, uint32_t t, uint32_t n
 // no group has a slot left. `st` may hold anything a lane read before (a lane
 // that is done loads nothing, and its zero masks ignore the rows).
 template <int WPL, int LPC, int G>
-__device__ __forceinline__ void scan_rows(const int32_t *__restrict__ lits, const uint2 *__restrict__ rows, uint32_t pos,
+__device__ __forceinline__ void scan_rows(const CheckArgs &a, const uint2 *__restrict__ rows, uint32_t pos,
                                           uint32_t end, int sub, int gbase, uint32_t (&all)[WPL],
                                           uint32_t (&live)[WPL], Row<WPL> (&st)[G]) {
     constexpr int BW = WPL * LPC;
@@ -155,7 +190,7 @@ __device__ __forceinline__ void scan_rows(const int32_t *__restrict__ lits, cons
 #pragma unroll
         for (int j = 1; j < WPL; j++) some |= live[j];
         if (!__any_sync(kFull, some != 0u && pos < end)) break;
-        const int32_t chunk = (pos + sub < end) ? __ldg(lits + pos + sub) : 0;
+        const int32_t chunk = (pos + sub < end) ? __ldg(a.lits + pos + sub) : 0;
         const int navail = (int) min((uint32_t) LPC, end > pos ? end - pos : 0u);
 #pragma unroll 1
         for (int k0 = 0; k0 < LPC; k0 += G) {

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kTWarps * 32) check_tiled_kernel(CheckArgs a) 
     WarpSmem &sm = smem_all[wib];
     const uint32_t part = blockIdx.x % a.n_parts;
     gss_report *out = a.out + (size_t) part * a.cap_per_part;
-    uint32_t *counter = a.counts + part;
+    uint32_t *counter = a.counts + (size_t) part * a.count_stride;
     uint32_t nstaged = 0;
     const bool hint = a.cache_hints != 0;
     const uint64_t pol_keep = policy_evict_last();

@@ -86,6 +86,7 @@ struct CheckArgs {
     const int32_t *solver_of_word;  // device, [n_blocks * lpc]
     gss_report *out;            // device, n_parts * cap_per_part records
     uint32_t *counts;           // device, n_parts counters (zeroed by the caller)
+    uint32_t count_stride;      // words from one counter to the next
     uint32_t n_parts;
     uint32_t cap_per_part;
     int lpc;                    // lanes (32-slot words) per clause
@@ -175,26 +176,32 @@ int gather_clauses(const GatherArgs &a, cudaStream_t stream, int sm_count);
 // or, with cell_words > 0, 8-byte {clause * cell_words + word, mask} records.
 int launch_pack_reports(const gss_report *parts, const uint32_t *counts, uint32_t n_parts, uint32_t cap,
                         uint32_t cell_words, uint32_t *packed, cudaStream_t stream, int sm_count);
-// What a pass's counters buffer holds: the n_parts report counters, the
-// kernel's error flag and the filter's counter of kept clauses, and, from
-// word kWorkOffset on, the work counters of the persistent kernels. One
-// memset clears them all.
+// A pass's counters buffer: the n_parts report counters, the kernel's error
+// flag and the filter's counter of kept clauses, and the work counters of the
+// persistent kernels. One memset clears them all. An address takes an atomic
+// every 1.5 ns or so, and neighbours in a line share that rate, so every
+// counter has 256 bytes to itself (500k clauses x 96 words of fair-coin slots,
+// eight reports a clause: 311 us, 559 with all counters side by side), and
+// the tasks come from kWorkCounters (62500 tasks from one counter took 100 us
+// whatever they did).
+constexpr uint32_t kCountStride = 64;
 constexpr uint32_t kExtraCounters = 2;
-constexpr uint32_t kWorkOffset = 64;
-// One address takes an atomic every 1.5 ns or so: 62500 tasks from a single
-// counter are 100 us, whatever the tasks do. The filtered kernel's tasks are
-// that short, so they come from kWorkCounters counters (256 bytes apart).
-constexpr uint32_t kWorkCounters = 16, kWorkStride = 64;
-constexpr size_t kWorkBytes = sizeof(uint32_t) * kWorkCounters * kWorkStride;
-constexpr size_t kCounterBytes = sizeof(uint32_t) * kWorkOffset + kWorkBytes;
+constexpr uint32_t kWorkCounters = 16;
+constexpr size_t kWorkBytes = sizeof(uint32_t) * kWorkCounters * kCountStride;
 __host__ __device__ __forceinline__ uint32_t *err_counter(uint32_t *counts, uint32_t n_parts) {
-    return counts + n_parts;
+    return counts + n_parts * kCountStride;
 }
 __host__ __device__ __forceinline__ uint32_t *kept_counter(uint32_t *counts, uint32_t n_parts) {
-    return counts + n_parts + 1;
+    return counts + n_parts * kCountStride + 1;
 }
-__host__ __device__ __forceinline__ uint32_t *work_counter(uint32_t *counts) { return counts + kWorkOffset; }
-// Hands a pass's outcome to the host: writes the counters buffer to `host` (pinned), and, when the pass has at most max_inline
+__host__ __device__ __forceinline__ uint32_t *work_counter(uint32_t *counts, uint32_t n_parts) {
+    return counts + (n_parts + 1) * kCountStride;
+}
+inline size_t counter_bytes(uint32_t n_parts) {
+    return sizeof(uint32_t) * (n_parts + 1) * kCountStride + kWorkBytes;
+}
+// Hands a pass's outcome to the host: writes the report counters, the error
+// flag and the filter's count, side by side, to `host` (pinned), and, when the pass has at most max_inline
 // records and no partition overflowed, the records too, partition after
 // partition from byte kInlineOffset on. With d_args the queues are those of
 // the arguments in device memory (a captured graph outlives a queue's growth).

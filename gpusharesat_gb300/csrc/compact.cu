@@ -202,9 +202,9 @@ __global__ void pack_reports_kernel(const gss_report *__restrict__ parts, const 
     for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (uint64_t) gridDim.x * blockDim.x) {
         const uint32_t p = (uint32_t) (i / cap), k = (uint32_t) (i - (uint64_t) p * cap);
-        if (k >= min(__ldg(counts + p), cap)) continue;
+        if (k >= min(__ldg(counts + p * kCountStride), cap)) continue;
         uint64_t base = 0;
-        for (uint32_t q = 0; q < p; q++) base += min(__ldg(counts + q), cap);
+        for (uint32_t q = 0; q < p; q++) base += min(__ldg(counts + q * kCountStride), cap);
         const gss_report r = parts[i];
         if (cell_words) {
             reinterpret_cast<uint2 *>(packed)[base + k] = make_uint2(r.clause * cell_words + r.word, r.mask);
@@ -235,18 +235,21 @@ __global__ void __launch_bounds__(256) deliver_kernel(const CheckArgs *__restric
         cap = pa->cap_per_part;
     }
     const uint32_t p = blockIdx.x / kStripes, stripe = blockIdx.x % kStripes;
-    if (blockIdx.x == 0 && threadIdx.x < n_parts + kExtraCounters) host[threadIdx.x] = counts[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x < n_parts + kExtraCounters) {
+        const uint32_t t = threadIdx.x;
+        host[t] = t < n_parts ? counts[t * kCountStride] : counts[n_parts * kCountStride + (t - n_parts)];
+    }
     if (max_inline == 0) return;
     uint64_t total = 0, base = 0;
     bool over = false;
     for (uint32_t q = 0; q < n_parts; q++) {
-        const uint32_t m = __ldg(counts + q);
+        const uint32_t m = __ldg(counts + q * kCountStride);
         over |= m > cap;
         if (q == p) base = total;
         total += m;
     }
     if (over || total > max_inline) return;
-    const uint32_t n = __ldg(counts + p);
+    const uint32_t n = __ldg(counts + p * kCountStride);
     const int4 *from = reinterpret_cast<const int4 *>(parts + (size_t) p * cap);
     int4 *to = reinterpret_cast<int4 *>(reinterpret_cast<char *>(host) + kInlineOffset) + base;
     for (uint32_t i = stripe * blockDim.x + threadIdx.x; i < n; i += kStripes * blockDim.x) to[i] = from[i];

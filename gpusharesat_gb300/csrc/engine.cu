@@ -177,7 +177,7 @@ int ensure_queues(gss_engine *eng) {
         GSS_TRY(eng->reports.reserve((size_t) per * eng->n_parts * sizeof(gss_report)));
         eng->cap_per_part = (uint32_t) per;
     }
-    GSS_TRY(eng->counts.reserve(kCounterBytes));
+    GSS_TRY(eng->counts.reserve(counter_bytes(eng->n_parts)));
     GSS_TRY(eng->h_counts.reserve(kInlineOffset));
     return GSS_OK;
 }
@@ -883,12 +883,13 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     a.solver_of_word = (const int32_t *) eng->solver_of_word.ptr;
     a.out = (gss_report *) reports.ptr;
     a.counts = (uint32_t *) counts.ptr;
+    a.count_stride = kCountStride;
     a.n_parts = eng->n_parts;
     a.cap_per_part = eng->cap_per_part;
     a.err = err_counter(a.counts, a.n_parts);
     a.agg = (const uint2 *) agg;
     a.kept = kept_counter(a.counts, a.n_parts);
-    uint32_t *const work = work_counter(a.counts);
+    uint32_t *const work = work_counter(a.counts, a.n_parts);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (eng->timing) {
         for (cudaEvent_t *ev : {&ev0, &ev1}) {
@@ -940,7 +941,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->d_args.ptr, &a, sizeof a, cudaMemcpyHostToDevice, eng->stream));
         if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
         auto body = [&]() -> int {
-            GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, kCounterBytes, eng->stream));
+            GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(a.n_parts), eng->stream));
             if (a.n_clauses > 0 && a.n_blocks > 0) {
                 if (bucketed) {
                     if (eng->plan_ranges > 0)
@@ -986,7 +987,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         }
         return GSS_OK;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, kCounterBytes, eng->stream));
+    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(a.n_parts), eng->stream));
     if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
     bool work_used = false;  // the memset above cleared the work counter for the first launch
     auto launch = [&](const CheckArgs &args) -> int {
@@ -1166,8 +1167,8 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         return GSS_OK;
     };
     GSS_TRY(reserve_reports());
-    GSS_TRY(eng->counts2.reserve(kCounterBytes));
-    GSS_TRY(eng->counts3.reserve(kCounterBytes));
+    GSS_TRY(eng->counts2.reserve(counter_bytes(eng->n_parts)));
+    GSS_TRY(eng->counts3.reserve(counter_bytes(eng->n_parts)));
     auto reserve_packed = [&]() -> int {
         for (int b = 0; b < NB && packed; b++)
             GSS_TRY(eng->packed[b].reserve((size_t) eng->cap_per_part * eng->n_parts * rec_words * sizeof(uint32_t)));

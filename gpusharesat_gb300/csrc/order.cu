@@ -836,7 +836,7 @@ __global__ void history_kernel(const gss_report *__restrict__ reports, const uin
     const uint32_t stripes = max(gridDim.x / n_parts, 1u);
     const uint32_t q = blockIdx.x % n_parts, stripe = blockIdx.x / n_parts;
     if (stripe >= stripes) return;
-    const uint32_t m = min(counts[q], cap_per_part);
+    const uint32_t m = min(counts[q * kCountStride], cap_per_part);
     const gss_report *r = reports + (size_t) q * cap_per_part;
     for (uint32_t i = stripe * blockDim.x + threadIdx.x; i < m; i += stripes * blockDim.x) {
         const uint32_t id = r[i].clause;

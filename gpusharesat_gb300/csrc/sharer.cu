@@ -231,7 +231,7 @@ int Sharer::init(int device) {
     for (Pass &p : pass_) {
         GSS_CUDA_TRY(cudaEventCreateWithFlags(&p.counted, cudaEventDisableTiming));
         GSS_CUDA_TRY(cudaEventCreateWithFlags(&p.copied, cudaEventDisableTiming));
-        GSS_TRY(p.d_counts.reserve(kCounterBytes));
+        GSS_TRY(p.d_counts.reserve(counter_bytes(n_parts_)));
         GSS_TRY(p.h_counts.reserve(kInlineOffset + (size_t) kSharerInline * sizeof(gss_report)));
     }
     GSS_CUDA_TRY(cudaEventCreateWithFlags(&alive_staged_, cudaEventDisableTiming));
@@ -899,6 +899,7 @@ int Sharer::run_check(Pass &p) {
     a.solver_of_word = (const int32_t *) d_sow_.ptr;
     a.out = (gss_report *) p.d_reports.ptr;
     a.counts = (uint32_t *) p.d_counts.ptr;
+    a.count_stride = kCountStride;
     a.n_parts = n_parts_;
     a.cap_per_part = p.cap_per_part;
     a.lpc = eff_lpc_;
@@ -915,14 +916,14 @@ int Sharer::run_check(Pass &p) {
         a.alive = (const uint32_t *) d_alive_.ptr;
         a.alive_by_id = 1;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, kCounterBytes, stream_));
+    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(n_parts_), stream_));
     if (p.active_words > 0 && p.n_clauses > 0) {
         const int wpl = eff_kind_ == GSS_KERNEL_WIDE4 ? 4 : 2;
         const bool wide = eff_kind_ == GSS_KERNEL_WIDE4 || eff_kind_ == GSS_KERNEL_WIDE2;
         if (wide && ((flags_ & GSS_VARIANT_PERSISTENT) ||
                      (kind_ == GSS_KERNEL_AUTO && valid_wide_persist_variant(wpl, eff_lpc_, eff_depth_)))) {
             // the persistent form, as the engine's automatic variant
-            uint32_t *const work = work_counter(a.counts);
+            uint32_t *const work = work_counter(a.counts, n_parts_);
             p.filtered = agg_ok_ && filter_pause_ == 0 && filter_tasks(a) < kMaxFilterTasks;
             if (p.filtered)
                 GSS_TRY(launch_check_filtered(nullptr, a, wpl, eff_lpc_, work, stream_, sm_count_));
@@ -931,7 +932,7 @@ int Sharer::run_check(Pass &p) {
         } else if (wide) {
             GSS_TRY(launch_check_wide(a, wpl, (flags_ & GSS_VARIANT_OCCUPANCY) ? 1 : 0, stream_, sm_count_));
         } else if (kind_ == GSS_KERNEL_AUTO && n_blocks_ == 1 && valid_narrow_variant(eff_lpc_)) {
-            GSS_TRY(launch_check_narrow(a, work_counter(a.counts), stream_, sm_count_));
+            GSS_TRY(launch_check_narrow(a, work_counter(a.counts, n_parts_), stream_, sm_count_));
         } else {
             GSS_TRY(launch_check(a, stream_, sm_count_));
         }

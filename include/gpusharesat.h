@@ -298,9 +298,9 @@ int gss_probe_gather(int device, uint64_t buffer_bytes, int depth, int blocks_pe
  * min(counts_out[p], cap_per_part) records from out + p * cap_per_part, with
  * `clause` the CSR index; counts_out[n_parts]. A count above cap_per_part
  * means that partition overflowed: run again with more room.
- * Limit: n_parts <= 64. The kernel's reservation counters live in one fixed
- * 256-byte device array, which every GPU that loads this library keeps until
- * the process exits, and which all calls share: overlapping calls on the GPU
+ * Limit: n_parts <= 64. The kernel's counters live in one fixed 20 KB device
+ * array, which every GPU that loads this library keeps until the process
+ * exits, and which all calls share: overlapping calls on the GPU
  * race and give wrong counts. Each call clears the counters first (they keep
  * the previous call's values). Each call looks up the array's device address
  * on the current device (a host-side lookup that allocates nothing, so the
