@@ -34,9 +34,9 @@
 // change the engine's buffers wait for it first (order_quiesce).
 //
 // Training (every retrain_interval passes, on a stream of its own, over a
-// snapshot of the log; and gss_scorer_train_step): FP32 forward and backward
-// kernels over a minibatch, per-32-row partial gradients reduced in a fixed
-// order (no atomics), and Adam. The passes take the new weights once the
+// snapshot of the log; and gss_scorer_train_step): one FP32 kernel from the
+// forward pass of a minibatch to its blocks' partial gradients, and one that
+// adds them in a fixed order (no atomics) and takes the Adam step. The passes take the new weights once the
 // training is done.
 #include <cuda_bf16.h>
 #include <math.h>
@@ -164,7 +164,8 @@ struct Scorer {
     DevBuf frag;           // BF16 mma fragments of W1 and W2
     bool frag_stale = true;
     int64_t adam_steps = 0;
-    DevBuf act;            // training activations
+    DevBuf act;            // the training blocks' partial gradients
+    int sm_count = 1;
     DevBuf io_x, io_y, io_out, loss;
 };
 
@@ -264,26 +265,14 @@ __device__ __forceinline__ void mlp16v(const float (&v)[8], const MlpShared &sm,
     out1 = s1 + sm.b3;
 }
 
-__device__ __forceinline__ void mlp16(const float (&x0)[kF], const float (&x1)[kF], const MlpShared &sm,
-                                      float &out0, float &out1) {
-    const int t = threadIdx.x & 3;
-    float v[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) v[q] = 0.0f;
-#pragma unroll
-    for (int c = 0; c < kF; c++) {
-        if (c == 2 * t) v[0] = x0[c], v[4] = x1[c];
-        if (c == 2 * t + 1) v[1] = x0[c], v[5] = x1[c];
-        if (c == 2 * t + 8) v[2] = x0[c], v[6] = x1[c];
-        if (c == 2 * t + 9) v[3] = x0[c], v[7] = x1[c];
-    }
-    mlp16v(v, sm, out0, out1);
-}
-
-
 constexpr int kMlpThreads = 256;
+constexpr int kInferBlocks = 3;  // of infer_rows_kernel, per multiprocessor
 
-// Logits of rows of features given in memory (x[n][kF]).
+// Logits of rows of features given in memory (x[n][kF]), a warp per 16 rows.
+// Each lane loads the columns of its fragment, 8 bytes at a time (every lane
+// of a row had loaded the whole row, 24 loads for 4), one tile ahead. The
+// blocks are few, because each first loads 11 KB of weights: 200k rows 20 us
+// with 8 blocks a multiprocessor and scalar loads, 12.5 us now.
 __global__ void __launch_bounds__(kMlpThreads) infer_rows_kernel(const float *__restrict__ w,
                                                                   const uint32_t *__restrict__ frag,
                                                                   const float *__restrict__ x, uint32_t n,
@@ -293,160 +282,253 @@ __global__ void __launch_bounds__(kMlpThreads) infer_rows_kernel(const float *__
     __syncthreads();
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile * 16 < n; tile += warps) {
-        const uint32_t r0 = tile * 16 + g, r1 = r0 + 8;
-        float x0[kF], x1[kF];
+    const uint32_t tiles = (n + 15) / 16;
+    auto load = [&](uint32_t tile, float (&v)[8]) {
 #pragma unroll
-        for (int c = 0; c < kF; c++) {
-            x0[c] = r0 < n ? x[(size_t) r0 * kF + c] : 0.0f;
-            x1[c] = r1 < n ? x[(size_t) r1 * kF + c] : 0.0f;
+        for (int q = 0; q < 2; q++) {
+            const uint64_t r = (uint64_t) tile * 16 + g + 8 * q;
+            float2 lo = make_float2(0.0f, 0.0f), hi = lo;
+            if (r < n) {
+                lo = __ldg(reinterpret_cast<const float2 *>(x + r * kF + 2 * t));
+                if (2 * t + 8 < kF) hi = __ldg(reinterpret_cast<const float2 *>(x + r * kF + 2 * t + 8));
+            }
+            v[4 * q] = lo.x, v[4 * q + 1] = lo.y, v[4 * q + 2] = hi.x, v[4 * q + 3] = hi.y;
         }
+    };
+    uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    float v[8];
+    if (tile < tiles) load(tile, v);
+    for (; tile < tiles; tile += warps) {
+        float next[8];
+        if (tile + warps < tiles) load(tile + warps, next);
         float o0, o1;
-        mlp16(x0, x1, sm, o0, o1);
+        mlp16v(v, sm, o0, o1);
         if (t == 0) {
-            if (r0 < n) out[r0] = o0;
-            if (r1 < n) out[r1] = o1;
+            const uint64_t r = (uint64_t) tile * 16 + g;
+            if (r < n) out[r] = o0;
+            if (r + 8 < n) out[r + 8] = o1;
         }
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = next[k];
     }
 }
 
 // ------------------------------------------------------------ training
 
-// Activations of a minibatch of B rows, unit-major so that threads (rows)
-// access them coalesced: h1, h2, d1, d2 [kH][B], dz[B], loss[B].
-__global__ void train_fwd_bwd_kernel(const float *__restrict__ w, const float *__restrict__ x,
-                                     const float *__restrict__ y, uint32_t start, uint32_t n_rows, uint32_t B,
-                                     float *__restrict__ act) {
-    __shared__ float sw[kP];
-    for (int i = threadIdx.x; i < kP; i += blockDim.x) sw[i] = w[i];
-    __syncthreads();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B) return;
-    const uint32_t r = (uint32_t) (((uint64_t) start + i) % n_rows);
-    float xr[kF];
-    for (int k = 0; k < kF; k++) xr[k] = x[(size_t) r * kF + k];
-    float *h1 = act + i;
-    float *h2 = act + (size_t) kH * B + i;
-    float *d1 = act + (size_t) 2 * kH * B + i;
-    float *d2 = act + (size_t) 3 * kH * B + i;
-    float *dz = act + (size_t) 4 * kH * B;
-    float *loss = dz + B;
-    for (int j = 0; j < kH; j++) {
-        float z = sw[oB1 + j];
-        for (int k = 0; k < kF; k++) z = fmaf(sw[oW1 + j * kF + k], xr[k], z);
-        h1[(size_t) j * B] = fmaxf(z, 0.0f);
-    }
-    float z3 = sw[oB3];
-    for (int j = 0; j < kH; j++) {
-        float z = sw[oB2 + j];
-        for (int k = 0; k < kH; k++) z = fmaf(sw[oW2 + j * kH + k], h1[(size_t) k * B], z);
-        const float hj = fmaxf(z, 0.0f);
-        h2[(size_t) j * B] = hj;
-        z3 = fmaf(sw[oW3 + j], hj, z3);
-    }
-    const float yr = y[r];
-    // logistic loss with logits: max(z,0) - z*y + log(1 + exp(-|z|))
-    loss[i] = fmaxf(z3, 0.0f) - z3 * yr + log1pf(expf(-fabsf(z3)));
-    const float p = 1.0f / (1.0f + expf(-z3));
-    const float g = (p - yr) / (float) B;
-    dz[i] = g;
-    for (int j = 0; j < kH; j++) d2[(size_t) j * B] = h2[(size_t) j * B] > 0.0f ? g * sw[oW3 + j] : 0.0f;
-    for (int k = 0; k < kH; k++) {
-        float s = 0.0f;
-        for (int j = 0; j < kH; j++) s = fmaf(sw[oW2 + j * kH + k], d2[(size_t) j * B], s);
-        d1[(size_t) k * B] = h1[(size_t) k * B] > 0.0f ? s : 0.0f;
-    }
-}
+// One minibatch of B rows starting at `start` (wrapping) of x/y: loss and
+// gradient, FP32. A block takes tiles of kTrainRows rows from the first layer
+// to the gradient without leaving the multiprocessor: weights and the tile's
+// activations are in shared memory (48 KB), a warp owns 4 units of all 32 rows
+// (lane = row: activations as 16-byte loads down its row, weights as
+// broadcasts), and for the gradient a thread owns 4 x 2 weights of the second
+// layer, summed over the rows in registers across all its tiles. One partial
+// gradient per block goes to global memory; train_reduce_kernel adds them in
+// block order (no atomics: the same bits every time). The former forward and
+// backward kernel (a thread per row, activations through global memory) took
+// 60 us for 4096 rows and the gradient of them another 17; this one 12.
+constexpr int kTrainRows = 32;
+constexpr int kTrainThreads = 512;
+constexpr int kTrainPad = kH + 4;  // 16-byte rows, conflict-free down a column of rows
 
-// Rows per gradient chunk: each block sums its chunk into one partial
-// gradient; grad_reduce_kernel adds the partials in chunk order.
-constexpr int kGradRows = 32;
-
-__global__ void __launch_bounds__(256) train_grad_kernel(const float *__restrict__ x, uint32_t start,
-                                                         uint32_t n_rows, uint32_t B,
-                                                         const float *__restrict__ act,
-                                                         float *__restrict__ partial) {
-    __shared__ float xs[kGradRows][kF];
-    __shared__ float h1s[kGradRows][kH + 1], h2s[kGradRows][kH + 1], d1s[kGradRows][kH + 1],
-        d2s[kGradRows][kH + 1];
-    __shared__ float dzs[kGradRows];
-    const uint32_t r0 = blockIdx.x * kGradRows;
-    const uint32_t rows = min((uint32_t) kGradRows, B - r0);
-    for (int e = threadIdx.x; e < kH * kGradRows; e += blockDim.x) {
-        const int j = e / kGradRows, rr = e % kGradRows;
-        const bool in = (uint32_t) rr < rows;
-        const size_t g = (size_t) j * B + r0 + rr;
-        h1s[rr][j] = in ? act[g] : 0.0f;
-        h2s[rr][j] = in ? act[(size_t) kH * B + g] : 0.0f;
-        d1s[rr][j] = in ? act[(size_t) 2 * kH * B + g] : 0.0f;
-        d2s[rr][j] = in ? act[(size_t) 3 * kH * B + g] : 0.0f;
-    }
-    for (int e = threadIdx.x; e < kF * kGradRows; e += blockDim.x) {
-        const int rr = e / kF, k = e % kF;
-        const uint32_t r = (uint32_t) (((uint64_t) start + r0 + rr) % n_rows);
-        xs[rr][k] = (uint32_t) rr < rows ? x[(size_t) r * kF + k] : 0.0f;
-    }
-    if (threadIdx.x < kGradRows)
-        dzs[threadIdx.x] = threadIdx.x < rows ? act[(size_t) 4 * kH * B + r0 + threadIdx.x] : 0.0f;
-    __syncthreads();
-    for (int p = threadIdx.x; p < kP; p += blockDim.x) {
-        float s = 0.0f;
-        if (p < oB1) {
-            const int j = p / kF, k = p % kF;
-            for (int rr = 0; rr < kGradRows; rr++) s = fmaf(d1s[rr][j], xs[rr][k], s);
-        } else if (p < oW2) {
-            for (int rr = 0; rr < kGradRows; rr++) s += d1s[rr][p - oB1];
-        } else if (p < oB2) {
-            const int j = (p - oW2) / kH, k = (p - oW2) % kH;
-            for (int rr = 0; rr < kGradRows; rr++) s = fmaf(d2s[rr][j], h1s[rr][k], s);
-        } else if (p < oW3) {
-            for (int rr = 0; rr < kGradRows; rr++) s += d2s[rr][p - oB2];
-        } else if (p < oB3) {
-            for (int rr = 0; rr < kGradRows; rr++) s = fmaf(dzs[rr], h2s[rr][p - oW3], s);
-        } else {
-            for (int rr = 0; rr < kGradRows; rr++) s += dzs[rr];
+__global__ void __launch_bounds__(kTrainThreads) train_tiles_kernel(const float *__restrict__ w,
+                                                                    const float *__restrict__ x,
+                                                                    const float *__restrict__ y, uint32_t start,
+                                                                    uint32_t n_rows, uint32_t B,
+                                                                    float *__restrict__ partial) {
+    __shared__ alignas(16) float sw[kP + 3];
+    __shared__ alignas(16) float h1s[kTrainRows][kTrainPad], h2s[kTrainRows][kTrainPad], d2s[kTrainRows][kTrainPad];
+    __shared__ alignas(16) float xs[kTrainRows][kF];
+    __shared__ float dzs[kTrainRows];
+    float(*const d1s)[kTrainPad] = h2s;  // the second layer's output is done with by then
+    const int tid = threadIdx.x, lane = tid & 31, u0 = (tid >> 5) * 4;  // this thread: row `lane`, units u0..u0+3
+    for (int i = tid; i < kP / 4; i += kTrainThreads)
+        *reinterpret_cast<float4 *>(sw + 4 * i) = *reinterpret_cast<const float4 *>(w + 4 * i);
+    if (tid < kP % 4) sw[kP / 4 * 4 + tid] = w[kP / 4 * 4 + tid];
+    // gradients of this thread's parameters: W2[4][2], W1[2] (three quarters
+    // of the threads), and one of b1, b2, w3, b3
+    const int gj = tid / 32 * 4, gk = tid % 32 * 2;
+    const int fj = tid / 6, fk = tid % 6 * 2;
+    float g2[4][2] = {}, g1[2] = {}, gb = 0.0f, loss = 0.0f;
+    for (uint32_t r0 = blockIdx.x * kTrainRows; r0 < B; r0 += gridDim.x * kTrainRows) {
+        __syncthreads();  // the last tile's reads are done
+        for (int e = tid; e < kTrainRows * kF; e += kTrainThreads) {
+            const uint32_t i = r0 + e / kF;
+            uint64_t r = (uint64_t) start + i;
+            if (r >= n_rows) r -= n_rows;
+            xs[e / kF][e % kF] = i < B ? x[r * kF + e % kF] : 0.0f;
         }
-        partial[(size_t) blockIdx.x * kP + p] = s;
+        __syncthreads();
+        const bool in = r0 + lane < B;  // rows past the end count for nothing
+        float h[4];
+        {
+            float xr[kF];
+#pragma unroll
+            for (int k = 0; k < kF; k++) xr[k] = xs[lane][k];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                float z = sw[oB1 + u0 + u];
+#pragma unroll
+                for (int k = 0; k < kF; k++) z = fmaf(sw[oW1 + (u0 + u) * kF + k], xr[k], z);
+                h[u] = in ? fmaxf(z, 0.0f) : 0.0f;
+            }
+        }
+        *reinterpret_cast<float4 *>(&h1s[lane][u0]) = make_float4(h[0], h[1], h[2], h[3]);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; u++) h[u] = sw[oB2 + u0 + u];
+#pragma unroll 4
+        for (int k = 0; k < kH; k += 4) {
+            const float4 a = *reinterpret_cast<const float4 *>(&h1s[lane][k]);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float4 b = *reinterpret_cast<const float4 *>(&sw[oW2 + (u0 + u) * kH + k]);
+                h[u] = fmaf(b.w, a.w, fmaf(b.z, a.z, fmaf(b.y, a.y, fmaf(b.x, a.x, h[u]))));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) h[u] = in ? fmaxf(h[u], 0.0f) : 0.0f;
+        *reinterpret_cast<float4 *>(&h2s[lane][u0]) = make_float4(h[0], h[1], h[2], h[3]);
+        __syncthreads();
+        if (tid < kTrainRows) {
+            float z3 = sw[oB3];
+#pragma unroll 4
+            for (int j = 0; j < kH; j += 4) {
+                const float4 a = *reinterpret_cast<const float4 *>(&h2s[lane][j]);
+                z3 = fmaf(sw[oW3 + j], a.x, z3);
+                z3 = fmaf(sw[oW3 + j + 1], a.y, z3);
+                z3 = fmaf(sw[oW3 + j + 2], a.z, z3);
+                z3 = fmaf(sw[oW3 + j + 3], a.w, z3);
+            }
+            float g = 0.0f;
+            if (in) {
+                uint64_t r = (uint64_t) start + r0 + lane;
+                if (r >= n_rows) r -= n_rows;
+                const float yr = y[r];
+                // logistic loss with logits: max(z,0) - z*y + log(1 + exp(-|z|))
+                loss += fmaxf(z3, 0.0f) - z3 * yr + log1pf(expf(-fabsf(z3)));
+                const float p = 1.0f / (1.0f + expf(-z3));
+                g = (p - yr) / (float) B;
+            }
+            dzs[lane] = g;
+        }
+        __syncthreads();
+        {
+            const float g = dzs[lane];
+            float d[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) d[u] = h[u] > 0.0f ? g * sw[oW3 + u0 + u] : 0.0f;
+            *reinterpret_cast<float4 *>(&d2s[lane][u0]) = make_float4(d[0], d[1], d[2], d[3]);
+        }
+        // the third layer's gradient, while the second layer's output is still there
+        if (tid >= 2 * kH && tid < 3 * kH) {
+            for (int r = 0; r < kTrainRows; r++) gb = fmaf(dzs[r], h2s[r][tid - 2 * kH], gb);
+        } else if (tid == 3 * kH) {
+            for (int r = 0; r < kTrainRows; r++) gb += dzs[r];
+        }
+        __syncthreads();
+        {
+            float d[4] = {};
+#pragma unroll 4
+            for (int j = 0; j < kH; j += 4) {
+                const float4 a = *reinterpret_cast<const float4 *>(&d2s[lane][j]);
+                const float aj[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const float4 b0 = *reinterpret_cast<const float4 *>(&sw[oW2 + (j + q) * kH + u0]);
+                    d[0] = fmaf(b0.x, aj[q], d[0]), d[1] = fmaf(b0.y, aj[q], d[1]);
+                    d[2] = fmaf(b0.z, aj[q], d[2]), d[3] = fmaf(b0.w, aj[q], d[3]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) d[u] = h1s[lane][u0 + u] > 0.0f ? d[u] : 0.0f;
+            *reinterpret_cast<float4 *>(&d1s[lane][u0]) = make_float4(d[0], d[1], d[2], d[3]);
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int r = 0; r < kTrainRows; r++) {
+            const float4 d = *reinterpret_cast<const float4 *>(&d2s[r][gj]);
+            const float2 a = *reinterpret_cast<const float2 *>(&h1s[r][gk]);
+            const float dj[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                g2[q][0] = fmaf(dj[q], a.x, g2[q][0]), g2[q][1] = fmaf(dj[q], a.y, g2[q][1]);
+            }
+            if (tid < kH * kF / 2) {
+                const float d1 = d1s[r][fj];
+                const float2 c = *reinterpret_cast<const float2 *>(&xs[r][fk]);
+                g1[0] = fmaf(d1, c.x, g1[0]), g1[1] = fmaf(d1, c.y, g1[1]);
+            }
+        }
+        if (tid < 2 * kH) {
+            float(*const d)[kTrainPad] = tid < kH ? d1s : d2s;
+            for (int r = 0; r < kTrainRows; r++) gb += d[r][tid % kH];
+        }
+    }
+    float *out = partial + (size_t) blockIdx.x * (kP + 1);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int k = 0; k < 2; k++) out[oW2 + (gj + q) * kH + gk + k] = g2[q][k];
+    if (tid < kH * kF / 2) {
+        out[oW1 + fj * kF + fk] = g1[0];
+        out[oW1 + fj * kF + fk + 1] = g1[1];
+    }
+    if (tid < kH)
+        out[oB1 + tid] = gb;
+    else if (tid < 2 * kH)
+        out[oB2 + tid - kH] = gb;
+    else if (tid < 3 * kH)
+        out[oW3 + tid - 2 * kH] = gb;
+    else if (tid == 3 * kH)
+        out[oB3] = gb;
+    if (tid < 32) {
+        for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(kFullMask, loss, o);
+        if (tid == 0) out[kP] = loss;
     }
 }
 
-__global__ void grad_reduce_kernel(const float *__restrict__ partial, uint32_t n_chunks, float *__restrict__ grad) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kP) return;
+// Adds the blocks' partial gradients, writes the gradient and the mean loss,
+// and (ADAM) takes the Adam step with it. Four threads a parameter, each over
+// a quarter of the blocks in block order, their sums added in a fixed order: a
+// chain of 128 dependent adds behind four rounds of loads took 9.7 us, this
+// 5.5.
+constexpr int kReduceParams = 64;  // per block of 4 * kReduceParams threads
+template <bool ADAM>
+__global__ void __launch_bounds__(4 * kReduceParams)
+    train_reduce_kernel(const float *__restrict__ partial, uint32_t n_blocks, uint32_t B, float *__restrict__ grad,
+                        float *__restrict__ loss, float *__restrict__ w, float *__restrict__ m,
+                        float *__restrict__ v, float lr, float c1, float c2) {
+    __shared__ float sums[4][kReduceParams];
+    const int lp = threadIdx.x % kReduceParams, quarter = threadIdx.x / kReduceParams;
+    const int p = blockIdx.x * kReduceParams + lp;
+    const uint32_t per = (n_blocks + 3) / 4, from = min(quarter * per, n_blocks), to = min(from + per, n_blocks);
     float s = 0.0f;
-    for (uint32_t c = 0; c < n_chunks; c++) s += partial[(size_t) c * kP + p];
-    grad[p] = s;
-}
-
-__global__ void mean_kernel(const float *__restrict__ v, uint32_t n, float *__restrict__ out) {
-    __shared__ float part[32];
-    float s = 0.0f;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFullMask, s, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    if (p <= kP) {
+#pragma unroll 32
+        for (uint32_t c = from; c < to; c++) s += __ldg(partial + (size_t) c * (kP + 1) + p);
+    }
+    sums[quarter][lp] = s;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.0f;
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFullMask, s, o);
-        if (threadIdx.x == 0) *out = s / (float) (n ? n : 1);
+    if (quarter != 0 || p > kP) return;
+    s = (sums[0][lp] + sums[1][lp]) + (sums[2][lp] + sums[3][lp]);
+    if (p == kP) {
+        *loss = s / (float) B;
+        return;
     }
-}
-
-__global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, float lr, float c1, float c2) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kP) return;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float gp = g[p];
-    const float mp = b1 * m[p] + (1.0f - b1) * gp;
-    const float vp = b2 * v[p] + (1.0f - b2) * gp * gp;
-    m[p] = mp;
-    v[p] = vp;
-    w[p] -= lr * (mp / c1) / (sqrtf(vp / c2) + eps);
+    grad[p] = s;
+    if (ADAM) {
+        const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+        const float mp = b1 * m[p] + (1.0f - b1) * s;
+        const float vp = b2 * v[p] + (1.0f - b2) * s * s;
+        m[p] = mp;
+        v[p] = vp;
+        w[p] -= lr * (mp / c1) / (sqrtf(vp / c2) + eps);
+    }
 }
 
 int scorer_init(Scorer *s, int device, uint64_t seed, cudaStream_t stream) {
     s->device = device;
+    GSS_CUDA_TRY(cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, device));
     GSS_TRY(s->w.reserve(kP * sizeof(float)));
     GSS_TRY(s->m.reserve(kP * sizeof(float)));
     GSS_TRY(s->v.reserve(kP * sizeof(float)));
@@ -481,33 +563,30 @@ int scorer_frags(Scorer *s, cudaStream_t stream) {
     return GSS_OK;
 }
 
-// Gradient (and mean loss, left in s->loss) of B rows starting at `start`
-// (wrapping) of x/y with n_rows rows, all on the device.
-int scorer_grad_dev(Scorer *s, const float *x, const float *y, uint32_t n_rows, uint32_t start, uint32_t B,
+// Gradient and mean loss (left in s->grad and s->loss) of B rows starting at
+// `start` (wrapping) of x/y with n_rows >= B rows, all on the device; lr > 0
+// also takes an Adam step with it.
+int scorer_grad_dev(Scorer *s, const float *x, const float *y, uint32_t n_rows, uint32_t start, uint32_t B, float lr,
                     cudaStream_t stream) {
-    const uint32_t n_chunks = (B + kGradRows - 1) / kGradRows;
-    const size_t act_floats = (size_t) 4 * B * kH + 2 * (size_t) B;
-    GSS_TRY(s->act.reserve((act_floats + (size_t) n_chunks * kP) * sizeof(float)));
-    float *act = (float *) s->act.ptr;
-    float *partial = act + act_floats;
-    train_fwd_bwd_kernel<<<(B + 63) / 64, 64, 0, stream>>>((const float *) s->w.ptr, x, y, start, n_rows, B, act);
+    const uint32_t tiles = (B + kTrainRows - 1) / kTrainRows;
+    // a block per multiprocessor at most: the partials stay few and their sum short
+    const uint32_t blocks = std::min<uint32_t>(tiles, (uint32_t) std::max(s->sm_count, 1));
+    GSS_TRY(s->act.reserve((size_t) blocks * (kP + 1) * sizeof(float)));
+    float *partial = (float *) s->act.ptr;
+    train_tiles_kernel<<<blocks, kTrainThreads, 0, stream>>>((const float *) s->w.ptr, x, y, start, n_rows, B, partial);
     GSS_CUDA_TRY(cudaGetLastError());
-    train_grad_kernel<<<n_chunks, 256, 0, stream>>>(x, start, n_rows, B, act, partial);
+    float c1 = 1.0f, c2 = 1.0f;
+    if (lr > 0.0f) {
+        s->adam_steps++;
+        c1 = 1.0f - powf(0.9f, (float) s->adam_steps);
+        c2 = 1.0f - powf(0.999f, (float) s->adam_steps);
+        s->frag_stale = true;
+    }
+    constexpr unsigned reduce_blocks = (kP + kReduceParams) / kReduceParams;  // kP parameters and the loss
+    (lr > 0.0f ? train_reduce_kernel<true> : train_reduce_kernel<false>)<<<reduce_blocks, 4 * kReduceParams, 0, stream>>>(
+        partial, blocks, B, (float *) s->grad.ptr, (float *) s->loss.ptr, (float *) s->w.ptr, (float *) s->m.ptr,
+        (float *) s->v.ptr, lr, c1, c2);
     GSS_CUDA_TRY(cudaGetLastError());
-    grad_reduce_kernel<<<(kP + 127) / 128, 128, 0, stream>>>(partial, n_chunks, (float *) s->grad.ptr);
-    GSS_CUDA_TRY(cudaGetLastError());
-    mean_kernel<<<1, 1024, 0, stream>>>(act + (size_t) 4 * B * kH + B, B, (float *) s->loss.ptr);
-    GSS_CUDA_TRY(cudaGetLastError());
-    return GSS_OK;
-}
-
-int scorer_adam_dev(Scorer *s, float lr, cudaStream_t stream) {
-    s->adam_steps++;
-    const float c1 = 1.0f - powf(0.9f, (float) s->adam_steps), c2 = 1.0f - powf(0.999f, (float) s->adam_steps);
-    adam_kernel<<<(kP + 127) / 128, 128, 0, stream>>>((float *) s->w.ptr, (const float *) s->grad.ptr,
-                                                       (float *) s->m.ptr, (float *) s->v.ptr, lr, c1, c2);
-    GSS_CUDA_TRY(cudaGetLastError());
-    s->frag_stale = true;
     return GSS_OK;
 }
 
@@ -912,8 +991,7 @@ int train_start(gss_engine *eng) {
     for (uint64_t st = 0; st < steps; st++) {
         const uint32_t start = (uint32_t) (o.rng() % logged);
         GSS_TRY(scorer_grad_dev(&o.trainer, (const float *) o.snap_x.ptr, (const float *) o.snap_y.ptr,
-                                (uint32_t) logged, start, B, o.train_stream));
-        GSS_TRY(scorer_adam_dev(&o.trainer, o.prm.learning_rate, o.train_stream));
+                                (uint32_t) logged, start, B, o.prm.learning_rate, o.train_stream));
     }
     GSS_CUDA_TRY(cudaEventRecord(o.ev_train_done, o.train_stream));
     o.training = true;
@@ -1561,9 +1639,10 @@ int gss_scorer_infer(gss_scorer *s, const float *x, int64_t n, float *logits) {
     GSS_TRY(upload_rows(s, x, nullptr, n));
     GSS_TRY(s->s.io_out.reserve((size_t) n * sizeof(float)));
     GSS_TRY(scorer_frags(&s->s, s->stream));
-    int sm = 0;
-    GSS_CUDA_TRY(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, s->s.device));
-    infer_rows_kernel<<<grid_for_n((uint64_t) (n + 15) / 16 * 32, sm, kMlpThreads), kMlpThreads, 0, s->stream>>>(
+    const uint64_t tiles = ((uint64_t) n + 15) / 16;
+    const unsigned blocks = (unsigned) std::min<uint64_t>((tiles + kMlpThreads / 32 - 1) / (kMlpThreads / 32),
+                                                          (uint64_t) s->s.sm_count * kInferBlocks);
+    infer_rows_kernel<<<blocks, kMlpThreads, 0, s->stream>>>(
         (const float *) s->s.w.ptr, (const uint32_t *) s->s.frag.ptr, (const float *) s->s.io_x.ptr, (uint32_t) n,
         (float *) s->s.io_out.ptr);
     GSS_CUDA_TRY(cudaGetLastError());
@@ -1579,7 +1658,7 @@ int gss_scorer_gradient(gss_scorer *s, const float *x, const float *y, int64_t n
     GSS_CUDA_TRY(cudaSetDevice(s->s.device));
     GSS_TRY(upload_rows(s, x, y, n));
     GSS_TRY(scorer_grad_dev(&s->s, (const float *) s->s.io_x.ptr, (const float *) s->s.io_y.ptr, (uint32_t) n, 0,
-                            (uint32_t) n, s->stream));
+                            (uint32_t) n, 0.0f, s->stream));
     GSS_CUDA_TRY(cudaMemcpyAsync(grad, s->s.grad.ptr, kP * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
     float l = 0.0f;
     GSS_CUDA_TRY(cudaMemcpyAsync(&l, s->s.loss.ptr, sizeof l, cudaMemcpyDeviceToHost, s->stream));
@@ -1594,8 +1673,7 @@ int gss_scorer_train_step(gss_scorer *s, const float *x, const float *y, int64_t
     GSS_CUDA_TRY(cudaSetDevice(s->s.device));
     GSS_TRY(upload_rows(s, x, y, n));
     GSS_TRY(scorer_grad_dev(&s->s, (const float *) s->s.io_x.ptr, (const float *) s->s.io_y.ptr, (uint32_t) n, 0,
-                            (uint32_t) n, s->stream));
-    GSS_TRY(scorer_adam_dev(&s->s, lr, s->stream));
+                            (uint32_t) n, lr, s->stream));
     float l = 0.0f;
     GSS_CUDA_TRY(cudaMemcpyAsync(&l, s->s.loss.ptr, sizeof l, cudaMemcpyDeviceToHost, s->stream));
     GSS_CUDA_TRY(cudaStreamSynchronize(s->stream));
