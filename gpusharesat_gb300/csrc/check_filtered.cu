@@ -43,7 +43,7 @@ constexpr int kPair = 2;        // table entries a lane reads at a time
 constexpr int kFewLanes = 2;
 constexpr uint32_t kFewChunks = 3;
 constexpr int kFewWords = 4;    // words left for which a survivor is checked literal-parallel
-constexpr int kFewSurvivors = 8;
+constexpr int kFewSurvivors = 16;
 constexpr int kFilterStage = 64;  // staged records per warp: few are found
 
 // The rest of the filter for the clauses of the lanes in `open`, one by one
@@ -76,9 +76,9 @@ __device__ __forceinline__ uint32_t finish_clauses(const int32_t *__restrict__ l
 
 // The exact check of the clauses (c of each lane) that the filter kept, on
 // the words `live` it left; records go to the warp's stage, whose new fill is
-// returned. Few survivors with few words each (the rule: reports) are checked
-// literal-parallel, a word at a time; otherwise groups of LPC lanes scan them
-// as the plain wide kernel does.
+// returned. Few survivors with few words each (reports, and clauses that the
+// word-level bits could not tell from them) are checked literal-parallel;
+// otherwise groups of LPC lanes scan them as the plain wide kernel does.
 template <int WPL, int LPC, int G>
 __device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, gss_report *stage, uint32_t nstaged, uint32_t blk,
                                                  uint32_t c, uint32_t live) {
@@ -91,44 +91,63 @@ __device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, gss_repo
     if (__popc(left) <= kFewSurvivors) {
         unsigned by_literal = __ballot_sync(kFull, live != 0u && __popc(live) <= kFewWords);
         left &= ~by_literal;
-        while (by_literal) {
-            const int src = __ffs(by_literal) - 1;
-            by_literal &= by_literal - 1;
-            const uint32_t cc = __shfl_sync(kFull, c, src);
-            const uint32_t b = (uint32_t) __ldg(a.offsets + cc), e = (uint32_t) __ldg(a.offsets + cc + 1);
-            uint32_t words = __shfl_sync(kFull, live, src);
-            while (words) {
-                const int w = __ffs(words) - 1;
-                words &= words - 1;
-                uint32_t fa = __ldg(start + w), fl = fa;
-                for (uint32_t p = b; p < e && fl; p += 32) {
-                    uint32_t f = ~0u, o = 0u;
-                    if (p + lane < e) {
-                        const uint32_t lit = (uint32_t) __ldg(a.lits + p + lane);
-                        Row<1> v;
-                        ld_row<1>(rows + (size_t) (lit >> 1) * BW + w, v);
-                        f = (v.v[1] ^ ((lit & 1u) - 1u)) & v.v[0];
-                        o = ~v.v[0];
-                    }
-                    warp_runs(f, o);
-                    fl = (fa & o) | (fl & f);
-                    fa &= f;
+        // up to four (clause, word) pairs at a time, eight lanes each; a pair
+        // on its own gets the whole warp
+        uint32_t words = 0;
+        int src = 0;
+        while (by_literal || words) {
+            int n_pairs = 0, my_src = 0, my_word = 0;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (!words && by_literal) {
+                    src = __ffs(by_literal) - 1;
+                    by_literal &= by_literal - 1;
+                    words = __shfl_sync(kFull, live, src);
                 }
-                if (fl) {
-                    if (nstaged + 1 > (uint32_t) kFilterStage) {
-                        flush_block_part(a, stage, nstaged);
-                        nstaged = 0;
-                    }
-                    if (lane == 0) {
-                        gss_report rep;
-                        rep.clause = __ldg(a.orig + cc);
-                        rep.word = blk * BW + w;
-                        rep.mask = fl;
-                        rep.solver = (uint32_t) __ldg(a.solver_of_word + blk * BW + w);
-                        stage[nstaged] = rep;
-                    }
-                    nstaged++;
+                if (words) {
+                    if (lane / 8 == q || q == 0) my_src = src, my_word = __ffs(words) - 1;
+                    words &= words - 1;
+                    n_pairs++;
                 }
+            }
+            const bool alone = n_pairs == 1;
+            const uint32_t cc = __shfl_sync(kFull, c, my_src);
+            const bool on = alone || lane / 8 < n_pairs;
+            const uint32_t step = alone ? 32u : 8u;
+            uint32_t fa = 0, fl = 0, p = 0, e = 0;
+            if (on) {
+                p = (uint32_t) __ldg(a.offsets + cc) + (alone ? lane : lane % 8);
+                e = (uint32_t) __ldg(a.offsets + cc + 1);
+                fa = fl = __ldg(start + my_word);
+            }
+            while (__any_sync(kFull, p < e && fl)) {
+                uint32_t f = ~0u, o = 0u;
+                if (p < e && fl) {
+                    const uint32_t lit = (uint32_t) __ldg(a.lits + p);
+                    Row<1> v;
+                    ld_row<1>(rows + (size_t) (lit >> 1) * BW + my_word, v);
+                    f = (v.v[1] ^ ((lit & 1u) - 1u)) & v.v[0];
+                    o = ~v.v[0];
+                }
+#pragma unroll
+                for (int d = 1; d < 32; d *= 2) {
+                    if (d >= 8 && !alone) break;
+                    const uint32_t f2 = __shfl_xor_sync(kFull, f, d), o2 = __shfl_xor_sync(kFull, o, d);
+                    merge_runs(f, o, f2, o2);
+                }
+                fl = (fa & o) | (fl & f);
+                fa &= f;
+                p += step;
+            }
+            const bool writes = alone ? lane == 0 : lane % 8 == 0;
+            const unsigned bal = __ballot_sync(kFull, writes && fl != 0u);
+            if (bal) {
+                if (nstaged + 4 > (uint32_t) kFilterStage) {
+                    flush_mapped(a, stage, nstaged);
+                    nstaged = 0;
+                }
+                if (writes && fl) stage_record(stage + nstaged + __popc(bal & lanemask_lt()), cc, blk * BW + my_word, fl);
+                nstaged += __popc(bal);
             }
         }
     }
@@ -160,17 +179,11 @@ __device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, gss_repo
             const unsigned bal = __ballot_sync(kFull, lv[j] != 0u);
             if (bal) {
                 if (nstaged + 32 > (uint32_t) kFilterStage) {
-                    flush_block_part(a, stage, nstaged);
+                    flush_mapped(a, stage, nstaged);
                     nstaged = 0;
                 }
-                if (lv[j]) {
-                    gss_report rep;
-                    rep.clause = __ldg(a.orig + cc);
-                    rep.word = blk * BW + sub * WPL + j;
-                    rep.mask = lv[j];
-                    rep.solver = (uint32_t) __ldg(a.solver_of_word + rep.word);
-                    stage[nstaged + __popc(bal & lanemask_lt())] = rep;
-                }
+                if (lv[j])
+                    stage_record(stage + nstaged + __popc(bal & lanemask_lt()), cc, blk * BW + sub * WPL + j, lv[j]);
                 nstaged += __popc(bal);
             }
         }
@@ -294,7 +307,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_filtered_kernel(const
         pos = pos1;
         end = end1;
     }
-    if (nstaged) flush_block_part(a, stage, nstaged);
+    if (nstaged) flush_mapped(a, stage, nstaged);
     // how many (clause, block) pairs the filter kept: tells whether it pays
     if (lane == 0 && kept) atomicAdd(&survivors, kept);
     __syncthreads();
@@ -320,8 +333,9 @@ __device__ __forceinline__ void row_entries(uint2 v, uint32_t real_words, int la
 // [n_blocks][n_vars][BW] (zero past the last word) and fills the filter's
 // table on the way; src == dst leaves the state in place (it is laid out
 // already). HBM-bound: a warp moves 256 bytes a step, kUnroll steps in
-// flight; the row index is per warp, not per word (one 64-bit division per 8
-// bytes had made the copy alone 160 us at 402 MB, 5.0 TB/s).
+// flight, with a 32-bit division a row at most, and streaming stores (402 MB
+// in three blocks, a whole gss_state_set: 201 us with plain stores, 193 so; a
+// plain copy of it alone 123).
 template <int BW>
 __global__ void __launch_bounds__(256) load_state_kernel(const uint2 *__restrict__ src, uint2 *__restrict__ dst,
                                                          uint2 *__restrict__ agg, unsigned long long *__restrict__ density,
@@ -342,8 +356,11 @@ __global__ void __launch_bounds__(256) load_state_kernel(const uint2 *__restrict
 #pragma unroll
         for (int q = 0; q < kUnroll; q++) {
             const uint64_t r = (s * kUnroll + q) * RPW + lane / BW;
-            const uint32_t var = n_blocks == 1 ? (uint32_t) r : (uint32_t) (r / n_blocks);
-            const uint32_t blk = n_blocks == 1 ? 0u : (uint32_t) (r - (uint64_t) var * n_blocks);
+            uint32_t var = (uint32_t) r, blk = 0u;
+            if (n_blocks != 1) {
+                var = n_rows <= 0xFFFFFFFFull ? (uint32_t) r / n_blocks : (uint32_t) (r / n_blocks);
+                blk = (uint32_t) (r - (uint64_t) var * n_blocks);
+            }
             const uint32_t word = blk * BW + w;
             const bool in = r < n_rows;
             to[q] = in ? ((size_t) blk * n_vars + var) : ~(size_t) 0;
@@ -354,7 +371,7 @@ __global__ void __launch_bounds__(256) load_state_kernel(const uint2 *__restrict
 #pragma unroll
         for (int q = 0; q < kUnroll; q++) {
             const bool in = to[q] != ~(size_t) 0;
-            if (in && !in_place) dst[to[q] * BW + w] = v[q];
+            if (in && !in_place) __stcs(dst + to[q] * BW + w, v[q]);  // read rarely behind the filter
             if (agg) {
                 uint2 p, n;
                 row_entries<BW>(v[q], real[q], lane, p, n);

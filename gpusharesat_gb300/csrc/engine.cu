@@ -155,8 +155,9 @@ int words_per_lane(int kind) { return kind == GSS_KERNEL_WIDE4 ? 4 : kind == GSS
 // word) pairs where some slot makes the literal false; a word outlives k
 // literals with a probability near F^k + k F^(k-1). Measured on 500k clauses x
 // 1024 slots over states of rising mixture, filtered against plain: F = 0.25
-// 28 to 45 against 58 to 67 us, 0.48 64 to 76 against 83 to 88; even at 0.70
-// (lengths 2-100), 0.67 (Zipf lengths) and 0.55 (lengths 2-30).
+// 28 to 49 against 58 to 67 us, 0.33 43 to 62 against 69 to 72; past 0.6 the
+// filter alone costs what it saves. In between it depends on how many clauses
+// report, which the pass itself tells (kFilterKeepMost).
 bool use_filter(uint64_t n_false, double pairs) { return pairs > 0 && (double) n_false < 0.55 * 2.0 * pairs; }
 
 int ensure_device(gss_engine *eng) {
@@ -917,8 +918,11 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     const bool narrow = eng->kind == GSS_KERNEL_AUTO && eng->state_kind == GSS_KERNEL_DIRECT && eng->n_blocks == 1 &&
                         valid_narrow_variant(eng->state_lpc);
     // behind the word-level filter where the state's table says that it pays
-    const bool filtered = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
-                          filter_tasks(a) < kMaxFilterTasks;
+    const bool may_filter = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
+                            filter_tasks(a) < kMaxFilterTasks;
+    const bool filtered = may_filter && eng->filter_pause == 0;
+    if (may_filter && eng->filter_pause > 0) eng->filter_pause--;
+    eng->pass_filtered = filtered;
     auto launch_persistent = [&](const CheckArgs *d_args, const CheckArgs &args) -> int {
         if (filtered)
             return launch_check_filtered(d_args, args, words_per_lane(eng->state_kind), eng->state_lpc, work,
@@ -1039,6 +1043,14 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
 }  // namespace
 
 
+namespace {
+// After a pass: what its filter kept (hc: the counters on the host).
+void note_kept(gss_engine *eng, const uint32_t *hc, bool filtered) {
+    if (filtered && filter_keeps_too_much(hc[eng->n_parts + 1], eng->n_clauses, eng->n_blocks))
+        eng->filter_pause = kFilterPause;
+}
+}  // namespace
+
 int gss_check_wait(gss_engine *eng, int64_t *n_reports) {
     if (!eng) return set_error(GSS_ERR_INVALID, "engine is NULL");
     GSS_TRY(ensure_device(eng));
@@ -1056,6 +1068,8 @@ int gss_check_wait(gss_engine *eng, int64_t *n_reports) {
         if (hc[p] > eng->cap_per_part) overflow = true;
     }
     if (n_reports) *n_reports = total;
+    note_kept(eng, hc, eng->pass_filtered);
+    eng->pass_filtered = false;
     if (hc[eng->n_parts] != 0)
         return set_error(GSS_ERR_CUDA, "a bounded wait in the check kernel gave up (flag %u); the pass is incomplete",
                          hc[eng->n_parts]);
@@ -1193,11 +1207,13 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));  // pass 0's state is in buffer 0
 
     int launched = 0;
+    bool slot_filtered[NB] = {false, false, false};
     // copies the reports of pass j back (the host waits for its kernel)
     auto finish = [&](int j) -> int {
         const int b = j % NB;
         GSS_CUDA_TRY(cudaEventSynchronize(eng->ev_kernel[b]));
         const uint32_t *hc = (const uint32_t *) hcnt_buf[b]->ptr;
+        note_kept(eng, hc, slot_filtered[b]);
         if (hc[eng->n_parts] != 0)
             return set_error(GSS_ERR_CUDA, "a bounded wait in the check kernel gave up (pass %d)", j);
         int64_t total = 0;
@@ -1276,6 +1292,7 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, agg_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
         GSS_TRY(pack(b, *rep_buf[b], *cnt_buf[b]));
         eng->launches++;
+        slot_filtered[b] = eng->pass_filtered;
         launched = i + 1;
         GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[b], eng->stream));
         if (i > 0) GSS_TRY(finish(i - 1));

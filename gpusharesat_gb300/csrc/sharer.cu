@@ -96,14 +96,10 @@ unsigned grid_for(uint64_t n, int sm_count) {
 
 }  // namespace
 
-// The filter's use (Sharer::collect). Its own pass is about a quarter of the
-// plain check's time, and what it keeps costs the plain check's share again.
-constexpr double kFilterKeepMost = 0.5;
 // (clauses x slot blocks) from which the filter pays for its table's upkeep,
 // two launches a pass (7 solvers, 50k clauses: 120 us a pass without, 126
 // with; 64 solvers, 1.2e6 clauses: 220 us of check without, 85 with).
 constexpr int64_t kFilterMinPairs = 150000;
-constexpr int kFilterPause = 64;
 
 // ---- one solver's ring ----
 
@@ -1000,8 +996,7 @@ int Sharer::collect(Pass &p) {
     // a filter that keeps most clauses costs more than it saves: leave it out
     // for some passes, then look again
     if (filter_pause_ > 0) filter_pause_--;
-    if (p.filtered && (double) ((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1] >
-                          kFilterKeepMost * (double) p.n_clauses * n_blocks_)
+    if (p.filtered && filter_keeps_too_much(((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1], p.n_clauses, n_blocks_))
         filter_pause_ = kFilterPause;
     GSS_CUDA_TRY(cudaEventRecord(p.copied, stream_));
     p.pending = false;

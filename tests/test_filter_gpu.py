@@ -135,3 +135,29 @@ def test_filter_through_learned_order_and_host_passes(lib):
         for f in ("clause", "word", "mask"):
             np.testing.assert_array_equal(rep[f], ref[f], err_msg=f)
     eng.close()
+
+
+def test_reports_do_not_depend_on_the_pause(lib):
+    """A state whose filter keeps most clauses (every clause reports) turns it
+    off for some passes; the reports are the same with it, without, and after
+    it is tried again."""
+    import gpusharesat_gb300 as g
+    rng = np.random.default_rng(8)
+    n_vars, n, n_words = 600, 3000, 32
+    model = rng.integers(0, 2, n_vars).astype(np.uint8)
+    var = rng.integers(0, n_vars, 2 * n)
+    lits = (2 * var + model[var]).astype(np.int32)  # false under the model
+    offsets = np.arange(0, 2 * n + 1, 2, dtype=np.int64)
+    state = _trail_state(rng, n_vars, n_words, model, flips=3)
+    start = np.full(n_words, 0xFFFFFFFF, np.uint32)
+    ref = oracle.check(lits, offsets, state, start)
+    assert len(ref) > n * n_words // 4
+    eng = g.Engine(0)
+    eng.set_db(lits, offsets)
+    eng.set_state(state, start)
+    for _ in range(70):
+        got = g.sort_reports(eng.check())
+        assert len(got) == len(ref)
+        for f in ("clause", "word", "mask"):
+            np.testing.assert_array_equal(got[f], ref[f], err_msg=f)
+    eng.close()
