@@ -796,6 +796,9 @@ static __device__ __align__(256) uint32_t
 // for the real address (a host-side lookup: it allocates nothing, and it
 // stays right if the device's context is torn down and created again).
 int noalloc_counters(uint32_t **out) {
+    static_assert(sizeof g_noalloc_counters ==
+                      sizeof(uint32_t) * (kNoAllocMaxParts + 1) * gss::kCountStride + gss::kWorkBytes,
+                  "counter_bytes(kNoAllocMaxParts, 1)");
     void *p = nullptr;
     GSS_CUDA_TRY(cudaGetSymbolAddress(&p, g_noalloc_counters));
     *out = (uint32_t *) p;
@@ -831,7 +834,7 @@ extern "C" int gss_check_noalloc(const int32_t *lits, const int64_t *offsets, ui
     uint32_t *counters = nullptr;
     GSS_TRY(noalloc_counters(&counters));
     // every call starts from zeroed counters: they keep the previous call's values
-    GSS_CUDA_TRY(cudaMemsetAsync(counters, 0, counter_bytes(n_parts), st));
+    GSS_CUDA_TRY(cudaMemsetAsync(counters, 0, counter_bytes(n_parts, 1), st));
     if (n_clauses > 0 && n_blocks > 0) {
         int dev = 0, sms = 0;
         GSS_CUDA_TRY(cudaGetDevice(&dev));

@@ -44,10 +44,14 @@ constexpr int kFewLanes = 2;
 constexpr uint32_t kFewChunks = 3;
 constexpr int kFewWords = 4;    // words left for which a survivor is checked literal-parallel
 constexpr int kFewSurvivors = 16;
+// Literals a lane has in flight in both: a long clause that reports is the
+// last thing a pass waits for (400k Zipf clauses x 11 words: 26 us with one,
+// 24 with two; four spill, 59 against 57 us on 2e6 clauses x 1024 slots).
+constexpr int kLong = 2;
 constexpr int kFilterStage = 64;  // staged records per warp: few are found
 
 // The rest of the filter for the clauses of the lanes in `open`, one by one
-// with 32 literals a step; returns the lane's words left.
+// with 32 * kLong literals a step; returns the lane's words left.
 __device__ __forceinline__ uint32_t finish_clauses(const int32_t *__restrict__ lits, const uint2 *__restrict__ agg,
                                                 unsigned open, uint32_t pos, uint32_t end, uint32_t all,
                                                 uint32_t live) {
@@ -58,12 +62,17 @@ __device__ __forceinline__ uint32_t finish_clauses(const int32_t *__restrict__ l
         uint32_t p = __shfl_sync(kFull, pos, src), fa = __shfl_sync(kFull, all, src),
                  fl = __shfl_sync(kFull, live, src);
         const uint32_t e = __shfl_sync(kFull, end, src);
-        for (; p < e && fl; p += 32) {
-            uint32_t f = ~0u, o = 0u;
-            if (p + lane < e) {
-                const uint2 v = ld_agg(agg + (uint32_t) __ldg(lits + p + lane));
-                f = v.x;
-                o = v.y;
+        for (; p < e && fl; p += 32 * kLong) {
+            uint32_t lit[kLong], f = ~0u, o = 0u;
+#pragma unroll
+            for (int k = 0; k < kLong; k++) {
+                const uint32_t at = p + 32 * k + lane;
+                lit[k] = at < e ? (uint32_t) __ldg(lits + at) : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < kLong; k++) {
+                const uint2 v = p + 32 * k + lane < e ? ld_agg(agg + lit[k]) : make_uint2(~0u, 0u);
+                merge_runs(f, o, v.x, v.y);
             }
             warp_runs(f, o);
             fl = (fa & o) | (fl & f);
@@ -121,14 +130,18 @@ __device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, gss_repo
                 fa = fl = __ldg(start + my_word);
             }
             while (__any_sync(kFull, p < e && fl)) {
-                uint32_t f = ~0u, o = 0u;
-                if (p < e && fl) {
-                    const uint32_t lit = (uint32_t) __ldg(a.lits + p);
-                    Row<1> v;
-                    ld_row<1>(rows + (size_t) (lit >> 1) * BW + my_word, v);
-                    f = (v.v[1] ^ ((lit & 1u) - 1u)) & v.v[0];
-                    o = ~v.v[0];
-                }
+                uint32_t lit[kLong], f = ~0u, o = 0u;
+                Row<1> v[kLong];
+#pragma unroll
+                for (int k = 0; k < kLong; k++)
+                    lit[k] = p + k * step < e && fl ? (uint32_t) __ldg(a.lits + p + k * step) : 0u;
+#pragma unroll
+                for (int k = 0; k < kLong; k++)
+                    if (p + k * step < e && fl) ld_row<1>(rows + (size_t) (lit[k] >> 1) * BW + my_word, v[k]);
+#pragma unroll
+                for (int k = 0; k < kLong; k++)
+                    if (p + k * step < e && fl)
+                        merge_runs(f, o, (v[k].v[1] ^ ((lit[k] & 1u) - 1u)) & v[k].v[0], ~v[k].v[0]);
 #pragma unroll
                 for (int d = 1; d < 32; d *= 2) {
                     if (d >= 8 && !alone) break;
@@ -137,7 +150,7 @@ __device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, gss_repo
                 }
                 fl = (fa & o) | (fl & f);
                 fa &= f;
-                p += step;
+                p += kLong * step;
             }
             const bool writes = alone ? lane == 0 : lane % 8 == 0;
             const unsigned bal = __ballot_sync(kFull, writes && fl != 0u);

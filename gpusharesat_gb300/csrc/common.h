@@ -197,8 +197,10 @@ __host__ __device__ __forceinline__ uint32_t *kept_counter(uint32_t *counts, uin
 __host__ __device__ __forceinline__ uint32_t *work_counter(uint32_t *counts, uint32_t n_parts) {
     return counts + (n_parts + 1) * kCountStride;
 }
-inline size_t counter_bytes(uint32_t n_parts) {
-    return sizeof(uint32_t) * (n_parts + 1) * kCountStride + kWorkBytes;
+// Bytes of the buffer with `sets` sets of work counters: the head and the tail
+// of an ordered pass have one each.
+inline size_t counter_bytes(uint32_t n_parts, uint32_t sets = 2) {
+    return sizeof(uint32_t) * (n_parts + 1) * kCountStride + sets * kWorkBytes;
 }
 // Hands a pass's outcome to the host: writes the report counters, the error
 // flag and the filter's count, side by side, to `host` (pinned), and, when the pass has at most max_inline

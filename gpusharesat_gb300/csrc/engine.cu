@@ -890,7 +890,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     a.err = err_counter(a.counts, a.n_parts);
     a.agg = (const uint2 *) agg;
     a.kept = kept_counter(a.counts, a.n_parts);
-    uint32_t *const work = work_counter(a.counts, a.n_parts);
+    uint32_t *work = work_counter(a.counts, a.n_parts);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (eng->timing) {
         for (cudaEvent_t *ev : {&ev0, &ev1}) {
@@ -993,18 +993,13 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     }
     GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(a.n_parts), eng->stream));
     if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
-    bool work_used = false;  // the memset above cleared the work counter for the first launch
     auto launch = [&](const CheckArgs &args) -> int {
         if (eng->state_kind == GSS_KERNEL_TILED) return launch_check_tiled(args, eng->stream, eng->sm_count);
         if (narrow) {
-            if (work_used) GSS_CUDA_TRY(cudaMemsetAsync(work, 0, kWorkBytes, eng->stream));
-            work_used = true;
             return launch_check_narrow(args, work, eng->stream, eng->sm_count);
         }
         if (persistent) {
-            // arguments by value; the work counter restarts for each launch
-            if (work_used) GSS_CUDA_TRY(cudaMemsetAsync(work, 0, kWorkBytes, eng->stream));
-            work_used = true;
+            // arguments by value
             if (args.n_clauses == 0 || args.n_blocks == 0 || scan_count(args) == 0) return GSS_OK;
             return launch_persistent(nullptr, args);
         }
@@ -1028,6 +1023,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         GSS_TRY(order_after_head(eng, counts));
         a.scan_begin = head;
         a.scan_end = a.n_clauses;
+        work += kWorkCounters * kCountStride;  // the tail's own counters
         if (head < a.n_clauses) GSS_TRY(launch(a));
         GSS_TRY(order_after_pass(eng, reports, counts));
     } else {

@@ -15,10 +15,10 @@
 //   2. score_kernel, a lane per clause position (a warp per 32): computes
 //      the features; the warp runs the MLP on tensor cores (mma.sync
 //      m16n8k16, BF16 operands, FP32 accumulation) over its 32 clauses as two
-//      m16 tiles, and each lane writes its clause's score bucket
-//   3. bucket_hist_kernel, bucket_scan_kernel, head_key_kernel, then a
-//      stable one-digit radix sort of positions (bucket_hist, bucket_scan,
-//      bucket_base, bucket_scatter) by key: the octave of predicted
+//      m16 tiles, each lane writes its clause's score bucket, and the blocks
+//      count the clauses per bucket
+//   3. a stable one-digit radix sort of positions (key_hist_kernel,
+//      key_scan_kernel, key_scatter_kernel) by key: the octave of predicted
 //      probability for the clauses of the head (the best buckets up to
 //      head_fraction of the clauses), one key for the tail. Inside a key the
 //      plain database order holds (variable ranges, then length), so the
@@ -65,15 +65,22 @@ static_assert(kF <= 16 && kH == 64, "the tensor-core MLP is written for K1 <= 16
 constexpr int kFrag1 = 8 * 32;
 constexpr int kFrag2 = 32 * 32;
 
-// Sort key: the score bucket, 16 per octave of the predicted report
-// probability (0 = most likely); the last bucket holds deleted clauses.
+// Score bucket: 16 per octave of the predicted report probability (0 = most
+// likely); the last bucket holds deleted clauses.
 constexpr int kBucketsPerOctave = 16;
 constexpr int kBuckets = 256;
-// radix sort tiles: kSortThreads threads x kSortRounds positions
-constexpr int kSortThreads = 256;
-constexpr int kSortRounds = 16;
+constexpr uint32_t kTotalStride = 32;  // words between the buckets' totals (a line each: see counter_bytes)
+// Sort key of the scan: the octave of a clause of the head, then one key for
+// the tail and one for deleted clauses.
+constexpr int kOctaves = kBuckets / kBucketsPerOctave;
+constexpr int kTailKey = kOctaves, kDeadKey = kOctaves + 1, kKeys = kOctaves + 2;
+// sort tiles: kSortWarps warps x kSortRounds x 32 positions
+constexpr int kSortWarps = 8;
+constexpr int kSortThreads = kSortWarps * 32;
+constexpr int kSortRounds = 8;
 constexpr uint32_t kSortTile = kSortThreads * kSortRounds;
 static_assert(kSortThreads == kBuckets, "one sort thread per bucket");
+static_assert(kKeys <= 32, "a lane per key");
 
 constexpr unsigned kFullMask = 0xFFFFFFFFu;
 
@@ -204,7 +211,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 struct MlpShared {
     uint2 w1[8][32];   // layer-1 fragments [tile][lane]
     uint2 w2[32][32];  // layer-2 fragments [tile][lane]
-    float b1[kH], b2[kH], w3[kH];
+    alignas(8) float b1[kH], b2[kH], w3[kH];
     float b3;
 };
 
@@ -221,51 +228,78 @@ __device__ void load_mlp_shared(MlpShared &sm, const float *w, const uint32_t *f
     if (threadIdx.x == 0) sm.b3 = w[oB3];
 }
 
-// One warp, 16 rows: lane (g = lane/4, t = lane%4) brings the features of
-// rows g and g+8 and gets back both logits (every lane of the group).
-// v: columns 2t, 2t+1, 2t+8, 2t+9 of rows g (v[0..3]) and g+8 (v[4..7]).
-__device__ __forceinline__ void mlp16v(const float (&v)[8], const MlpShared &sm, float &out0, float &out1) {
+// One warp, T tiles of 16 rows: lane (g = lane/4, t = lane%4) brings of rows
+// g and g+8 of each tile the columns 2t, 2t+1, 2t+8, 2t+9 (v[0..3] and
+// v[4..7]) and gets back both logits (every lane of the group). Two tiles
+// share every fragment and bias read from shared memory.
+template <int T>
+__device__ __forceinline__ void mlp16(const float (&v)[T][8], const MlpShared &sm, float (&out0)[T], float (&out1)[T]) {
     const int lane = threadIdx.x & 31, t = lane & 3;
-    const uint32_t a0 = pack_bf16(v[0], v[1]), a1 = pack_bf16(v[4], v[5]);
-    const uint32_t a2 = pack_bf16(v[2], v[3]), a3 = pack_bf16(v[6], v[7]);
+    uint32_t a[T][4];
+#pragma unroll
+    for (int s = 0; s < T; s++) {
+        a[s][0] = pack_bf16(v[s][0], v[s][1]), a[s][1] = pack_bf16(v[s][4], v[s][5]);
+        a[s][2] = pack_bf16(v[s][2], v[s][3]), a[s][3] = pack_bf16(v[s][6], v[s][7]);
+    }
     // layer 1 one k-tile of layer 2 at a time (n-tiles 2kt and 2kt+1): bias
     // + ReLU, re-packed as the A operand of layer 2 (the accumulator layout
     // of n-tiles 2kt and 2kt+1 is the A layout of k-tile kt)
-    uint32_t h[4][4];
+    uint32_t h[T][4][4];
 #pragma unroll
     for (int kt = 0; kt < 4; kt++) {
-        float p0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, p1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         const uint2 b0 = sm.w1[2 * kt][lane], b1 = sm.w1[2 * kt + 1][lane];
-        mma_bf16(p0, a0, a1, a2, a3, b0.x, b0.y);
-        mma_bf16(p1, a0, a1, a2, a3, b1.x, b1.y);
         const int c0 = 16 * kt + 2 * t, c1 = c0 + 8;
-        h[kt][0] = pack_bf16(fmaxf(p0[0] + sm.b1[c0], 0.0f), fmaxf(p0[1] + sm.b1[c0 + 1], 0.0f));
-        h[kt][1] = pack_bf16(fmaxf(p0[2] + sm.b1[c0], 0.0f), fmaxf(p0[3] + sm.b1[c0 + 1], 0.0f));
-        h[kt][2] = pack_bf16(fmaxf(p1[0] + sm.b1[c1], 0.0f), fmaxf(p1[1] + sm.b1[c1 + 1], 0.0f));
-        h[kt][3] = pack_bf16(fmaxf(p1[2] + sm.b1[c1], 0.0f), fmaxf(p1[3] + sm.b1[c1 + 1], 0.0f));
+        const float2 e0 = *reinterpret_cast<const float2 *>(&sm.b1[c0]), e1 = *reinterpret_cast<const float2 *>(&sm.b1[c1]);
+#pragma unroll
+        for (int s = 0; s < T; s++) {
+            float p0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, p1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            mma_bf16(p0, a[s][0], a[s][1], a[s][2], a[s][3], b0.x, b0.y);
+            mma_bf16(p1, a[s][0], a[s][1], a[s][2], a[s][3], b1.x, b1.y);
+            h[s][kt][0] = pack_bf16(fmaxf(p0[0] + e0.x, 0.0f), fmaxf(p0[1] + e0.y, 0.0f));
+            h[s][kt][1] = pack_bf16(fmaxf(p0[2] + e0.x, 0.0f), fmaxf(p0[3] + e0.y, 0.0f));
+            h[s][kt][2] = pack_bf16(fmaxf(p1[0] + e1.x, 0.0f), fmaxf(p1[1] + e1.y, 0.0f));
+            h[s][kt][3] = pack_bf16(fmaxf(p1[2] + e1.x, 0.0f), fmaxf(p1[3] + e1.y, 0.0f));
+        }
     }
-    float s0 = 0.0f, s1 = 0.0f;
+    float s0[T], s1[T];
+#pragma unroll
+    for (int s = 0; s < T; s++) s0[s] = s1[s] = 0.0f;
 #pragma unroll
     for (int nt = 0; nt < 8; nt++) {
-        float d2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float d2[T][4];
+#pragma unroll
+        for (int s = 0; s < T; s++) d2[s][0] = d2[s][1] = d2[s][2] = d2[s][3] = 0.0f;
 #pragma unroll
         for (int kt = 0; kt < 4; kt++) {
             const uint2 b = sm.w2[kt * 8 + nt][lane];
-            mma_bf16(d2, h[kt][0], h[kt][1], h[kt][2], h[kt][3], b.x, b.y);
+#pragma unroll
+            for (int s = 0; s < T; s++) mma_bf16(d2[s], h[s][kt][0], h[s][kt][1], h[s][kt][2], h[s][kt][3], b.x, b.y);
         }
         const int c = nt * 8 + 2 * t;
-        s0 += fmaxf(d2[0] + sm.b2[c], 0.0f) * sm.w3[c] + fmaxf(d2[1] + sm.b2[c + 1], 0.0f) * sm.w3[c + 1];
-        s1 += fmaxf(d2[2] + sm.b2[c], 0.0f) * sm.w3[c] + fmaxf(d2[3] + sm.b2[c + 1], 0.0f) * sm.w3[c + 1];
+        const float2 e = *reinterpret_cast<const float2 *>(&sm.b2[c]), w3 = *reinterpret_cast<const float2 *>(&sm.w3[c]);
+#pragma unroll
+        for (int s = 0; s < T; s++) {
+            s0[s] += fmaxf(d2[s][0] + e.x, 0.0f) * w3.x + fmaxf(d2[s][1] + e.y, 0.0f) * w3.y;
+            s1[s] += fmaxf(d2[s][2] + e.x, 0.0f) * w3.x + fmaxf(d2[s][3] + e.y, 0.0f) * w3.y;
+        }
     }
-    s0 += __shfl_xor_sync(kFullMask, s0, 1);
-    s0 += __shfl_xor_sync(kFullMask, s0, 2);
-    s1 += __shfl_xor_sync(kFullMask, s1, 1);
-    s1 += __shfl_xor_sync(kFullMask, s1, 2);
-    out0 = s0 + sm.b3;
-    out1 = s1 + sm.b3;
+#pragma unroll
+    for (int s = 0; s < T; s++) {
+        s0[s] += __shfl_xor_sync(kFullMask, s0[s], 1);
+        s0[s] += __shfl_xor_sync(kFullMask, s0[s], 2);
+        s1[s] += __shfl_xor_sync(kFullMask, s1[s], 1);
+        s1[s] += __shfl_xor_sync(kFullMask, s1[s], 2);
+        out0[s] = s0[s] + sm.b3;
+        out1[s] = s1[s] + sm.b3;
+    }
 }
 
 constexpr int kMlpThreads = 256;
+// Blocks of score_kernel per multiprocessor: at once, and in the grid. Several
+// short rounds rather than one long: while the tail of a pass runs beside it,
+// its blocks (of a stream of higher priority) take the places that fall free.
+constexpr int kScoreBlocks = 3;
+constexpr int kScoreGrid = 8;
 constexpr int kInferBlocks = 3;  // of infer_rows_kernel, per multiprocessor
 
 // Logits of rows of features given in memory (x[n][kF]), a warp per 16 rows.
@@ -283,7 +317,7 @@ __global__ void __launch_bounds__(kMlpThreads) infer_rows_kernel(const float *__
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t tiles = (n + 15) / 16;
-    auto load = [&](uint32_t tile, float (&v)[8]) {
+    auto load = [&](uint32_t tile, float (&v)[1][8]) {
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             const uint64_t r = (uint64_t) tile * 16 + g + 8 * q;
@@ -292,24 +326,24 @@ __global__ void __launch_bounds__(kMlpThreads) infer_rows_kernel(const float *__
                 lo = __ldg(reinterpret_cast<const float2 *>(x + r * kF + 2 * t));
                 if (2 * t + 8 < kF) hi = __ldg(reinterpret_cast<const float2 *>(x + r * kF + 2 * t + 8));
             }
-            v[4 * q] = lo.x, v[4 * q + 1] = lo.y, v[4 * q + 2] = hi.x, v[4 * q + 3] = hi.y;
+            v[0][4 * q] = lo.x, v[0][4 * q + 1] = lo.y, v[0][4 * q + 2] = hi.x, v[0][4 * q + 3] = hi.y;
         }
     };
     uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    float v[8];
+    float v[1][8];
     if (tile < tiles) load(tile, v);
     for (; tile < tiles; tile += warps) {
-        float next[8];
+        float next[1][8];
         if (tile + warps < tiles) load(tile + warps, next);
-        float o0, o1;
-        mlp16v(v, sm, o0, o1);
+        float o0[1], o1[1];
+        mlp16(v, sm, o0, o1);
         if (t == 0) {
             const uint64_t r = (uint64_t) tile * 16 + g;
-            if (r < n) out[r] = o0;
-            if (r + 8 < n) out[r + 8] = o1;
+            if (r < n) out[r] = o0[0];
+            if (r + 8 < n) out[r + 8] = o1[0];
         }
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = next[k];
+        for (int k = 0; k < 8; k++) v[0][k] = next[0][k];
     }
 }
 
@@ -607,7 +641,7 @@ struct OrderState {
     int64_t cap_ids = 0;
     DevBuf rec;                                 // ClauseRecord per clause id
     DevBuf lbd_pairs;                           // staging of gss_db_set_lbd
-    DevBuf bucket, offs, totals, key_of;        // per position; per (bucket, sort tile); per bucket (x2)
+    DevBuf bucket, offs, totals;                // per position; per (key, sort tile); per bucket and per key
     DevBuf perm[2];                             // scan permutations: the current one and the next one
     // the scan permutation in force (rescored every rescore_interval passes):
     // its buffer, the positions it covers and the layout it was built for;
@@ -661,16 +695,22 @@ struct LogArgs {
 // One warp per 32 positions, a lane per position: the features of each live
 // clause from its history (through pass now - 1), then the lanes pass the
 // features to the MLP's fragment layout (two m16 tiles) and each lane writes
-// its clause's score bucket.
-__global__ void __launch_bounds__(kMlpThreads, 3) score_kernel(HistoryArgs h, const float *__restrict__ w,
+// its clause's score bucket. The blocks count their clauses per bucket on the
+// way (totals, zeroed before the launch). Bound by instruction issue: 1e6
+// clauses 57 us with one m16 tile at a time, 50 with both sharing each weight
+// read, the counting included (a launch of its own had taken 12).
+__global__ void __launch_bounds__(kMlpThreads, kScoreBlocks) score_kernel(HistoryArgs h, const float *__restrict__ w,
                                                                const uint32_t *__restrict__ frag,
                                                                const int64_t *__restrict__ offsets,
                                                                const uint32_t *__restrict__ orig,
                                                                const uint32_t *__restrict__ alive, uint32_t n,
-                                                               uint8_t *__restrict__ bucket) {
+                                                               uint8_t *__restrict__ bucket,
+                                                               uint32_t *__restrict__ totals) {
     __shared__ MlpShared sm;
+    __shared__ uint32_t hist[kBuckets];
     __shared__ float xs[kMlpThreads / 32][32][kF + 1];  // each warp's rows of features
     load_mlp_shared(sm, w, frag);
+    for (int b = threadIdx.x; b < kBuckets; b += blockDim.x) hist[b] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     float(*wx)[kF + 1] = xs[threadIdx.x >> 5];
@@ -697,31 +737,40 @@ __global__ void __launch_bounds__(kMlpThreads, 3) score_kernel(HistoryArgs h, co
 #pragma unroll
         for (int k = 0; k < kF; k++) wx[lane][k] = x[k];
         __syncwarp();
-        float logit = 0.0f;
-#pragma unroll 1
-        for (int sub = 0; sub < 2; sub++) {
-            const float *f0 = wx[sub * 16 + g], *f1 = wx[sub * 16 + g + 8];
+        float v[2][8], o0[2], o1[2];
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const float *f0 = wx[s * 16 + g], *f1 = wx[s * 16 + g + 8];
             const int c = 2 * t;
-            float v[8];
-            v[0] = f0[c];
-            v[1] = f0[c + 1];
-            v[2] = c + 8 < kF ? f0[c + 8] : 0.0f;
-            v[3] = c + 9 < kF ? f0[c + 9] : 0.0f;
-            v[4] = f1[c];
-            v[5] = f1[c + 1];
-            v[6] = c + 8 < kF ? f1[c + 8] : 0.0f;
-            v[7] = c + 9 < kF ? f1[c + 9] : 0.0f;
-            float o0, o1;
-            mlp16v(v, sm, o0, o1);
-            // back to the lane that owns the row: row i of the tile is in lanes 4(i%8)..
-            const int i = lane & 15;
-            const float a = __shfl_sync(kFullMask, o0, 4 * (i & 7));
-            const float b = __shfl_sync(kFullMask, o1, 4 * (i & 7));
-            if ((lane >> 4) == sub) logit = (i < 8) ? a : b;
+            v[s][0] = f0[c];
+            v[s][1] = f0[c + 1];
+            v[s][2] = c + 8 < kF ? f0[c + 8] : 0.0f;
+            v[s][3] = c + 9 < kF ? f0[c + 9] : 0.0f;
+            v[s][4] = f1[c];
+            v[s][5] = f1[c + 1];
+            v[s][6] = c + 8 < kF ? f1[c + 8] : 0.0f;
+            v[s][7] = c + 9 < kF ? f1[c + 9] : 0.0f;
         }
-        if (r < n) bucket[r] = (uint8_t) (live ? bucket_of(logit) : (uint32_t) (kBuckets - 1));
+        mlp16(v, sm, o0, o1);
+        // back to the lane that owns the row: row i of tile s is in lanes 4(i%8)..
+        const int i = lane & 15;
+        float logit = 0.0f;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const float a = __shfl_sync(kFullMask, o0[s], 4 * (i & 7));
+            const float b = __shfl_sync(kFullMask, o1[s], 4 * (i & 7));
+            if ((lane >> 4) == s) logit = (i < 8) ? a : b;
+        }
+        if (r < n) {
+            const uint32_t bk = live ? bucket_of(logit) : (uint32_t) (kBuckets - 1);
+            bucket[r] = (uint8_t) bk;
+            atomicAdd(&hist[bk], 1u);
+        }
         __syncwarp();  // wx is rewritten by the next tile
     }
+    __syncthreads();
+    for (int b = threadIdx.x; b < kBuckets; b += blockDim.x)
+        if (hist[b]) atomicAdd(totals + b * kTotalStride, hist[b]);
 }
 
 // Records of the ids first seen by the scoring step at `now` (ids in
@@ -811,98 +860,116 @@ __device__ uint32_t block_scan_inplace(uint32_t *__restrict__ a, uint32_t n) {
     return carry;
 }
 
-// The sort key of each score bucket for the final order: the bucket's octave
-// of predicted probability while the clauses of better buckets number fewer
-// than `cut` (the head, by octave, in database order inside an octave),
-// kBuckets - 2 for the rest (the tail, which then keeps the plain position
-// order and its memory locality), kBuckets - 1 for deleted clauses. totals
-// holds the clause count of each bucket. One block of kBuckets threads.
-__global__ void head_key_kernel(const uint32_t *__restrict__ totals, uint32_t cut, uint8_t *__restrict__ key_of) {
-    __shared__ uint32_t before[kBuckets];
-    const int b = threadIdx.x;
-    before[b] = totals[b];
-    __syncthreads();
-    if (b == 0) {
-        uint32_t acc = 0;
-        for (int k = 0; k < kBuckets; k++) {
-            const uint32_t c = before[k];
-            before[k] = acc;
-            acc += c;
-        }
+// The sort key of every score bucket, by a block of kBuckets threads: the
+// bucket's octave of predicted probability while the clauses of better buckets
+// number fewer than `cut` (the head, by octave, in database order inside an
+// octave: the head's reports are delivered when its launch ends, so its inner
+// order does not delay them, and the database order keeps its state-row
+// locality), kTailKey for the rest (the tail, in plain position order),
+// kDeadKey for deleted clauses. totals: the clauses of each bucket.
+__device__ void bucket_keys(const uint32_t *__restrict__ totals, uint32_t cut, uint8_t *key_of) {
+    __shared__ uint32_t warp_sum[kSortWarps];
+    const int b = threadIdx.x, lane = b & 31, wid = b >> 5;
+    const uint32_t c = __ldg(totals + b * kTotalStride);
+    uint32_t x = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFullMask, x, o);
+        if (lane >= o) x += y;
     }
+    if (lane == 31) warp_sum[wid] = x;
     __syncthreads();
-    // head buckets by octave of the predicted probability: within an octave
-    // the head keeps the database order (its state-row locality); the head's
-    // reports are delivered when the whole head launch ends, so the order
-    // inside it does not delay them
-    key_of[b] = (uint8_t) (b == kBuckets - 1 ? kBuckets - 1 : before[b] < cut ? b / kBucketsPerOctave : kBuckets - 2);
+    uint32_t before = x - c;
+    for (int w = 0; w < wid; w++) before += warp_sum[w];
+    key_of[b] = (uint8_t) (b == kBuckets - 1 ? kDeadKey : before < cut ? b / kBucketsPerOctave : kTailKey);
+    __syncthreads();
 }
 
-// Block b: exclusive scan of bucket b's per-tile counts; totals[b] = its sum.
-__global__ void bucket_scan_kernel(uint32_t *__restrict__ offs, uint32_t n_tiles, uint32_t *__restrict__ totals) {
+// Block k: exclusive scan of key k's per-tile counts; key_total[k] = its sum.
+__global__ void key_scan_kernel(uint32_t *__restrict__ offs, uint32_t n_tiles, uint32_t *__restrict__ key_total) {
     const uint32_t t = block_scan_inplace(offs + (size_t) blockIdx.x * n_tiles, n_tiles);
-    if (threadIdx.x == 0) totals[blockIdx.x] = t;
+    if (threadIdx.x == 0) key_total[blockIdx.x] = t;
 }
 
-// Exclusive scan of the bucket totals (one block): the first scan position of
-// each bucket.
-__global__ void bucket_base_kernel(uint32_t *__restrict__ totals, uint32_t n) { block_scan_inplace(totals, n); }
-
-// Per sort tile: how many positions fall in each bucket, stored bucket-major
-// (offs[b * n_tiles + tile]) for the scan.
-__global__ void __launch_bounds__(kSortThreads) bucket_hist_kernel(const uint8_t *__restrict__ bucket,
-                                                                   const uint8_t *__restrict__ key_of, uint32_t n,
-                                                                   uint32_t n_tiles, uint32_t *__restrict__ offs) {
-    __shared__ uint32_t hist[kBuckets];
-    hist[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t base = blockIdx.x * kSortTile;
+// The keys of a warp's part of a sort tile (kSortRounds x 32 consecutive
+// positions, a byte each, kKeys past the end), and how many there are of each
+// (counts[kKeys] of the warp).
+__device__ __forceinline__ void warp_keys(const uint8_t *__restrict__ bucket, const uint8_t *key_of, uint32_t base,
+                                          uint32_t n, uint8_t (&key)[kSortRounds], uint32_t *counts) {
+    const int lane = threadIdx.x & 31;
+    counts[lane] = 0;
+    __syncwarp();
+#pragma unroll
     for (int r = 0; r < kSortRounds; r++) {
-        const uint32_t pos = base + r * kSortThreads + threadIdx.x;
-        if (pos < n) atomicAdd(&hist[key_of ? key_of[bucket[pos]] : bucket[pos]], 1u);
+        const uint32_t pos = base + r * 32 + lane;
+        key[r] = pos < n ? key_of[bucket[pos]] : (uint8_t) kKeys;
+    }
+#pragma unroll
+    for (int r = 0; r < kSortRounds; r++) {
+        const unsigned peers = __match_any_sync(kFullMask, (unsigned) key[r]);
+        if (key[r] < kKeys && (peers & ((1u << lane) - 1u)) == 0) counts[key[r]] += (uint32_t) __popc(peers);
+        __syncwarp();
+    }
+}
+
+// Per sort tile: how many positions have each key, stored key-major
+// (offs[k * n_tiles + tile]) for the scan.
+__global__ void __launch_bounds__(kSortThreads) key_hist_kernel(const uint8_t *__restrict__ bucket,
+                                                                const uint32_t *__restrict__ totals, uint32_t cut,
+                                                                uint32_t n, uint32_t n_tiles,
+                                                                uint32_t *__restrict__ offs) {
+    __shared__ uint8_t key_of[kBuckets];
+    __shared__ uint32_t counts[kSortWarps][32];
+    bucket_keys(totals, cut, key_of);
+    const int wid = threadIdx.x >> 5;
+    uint8_t key[kSortRounds];
+    warp_keys(bucket, key_of, blockIdx.x * kSortTile + wid * kSortRounds * 32, n, key, counts[wid]);
+    __syncthreads();
+    if (threadIdx.x < kKeys) {
+        uint32_t s = 0;
+#pragma unroll
+        for (int w = 0; w < kSortWarps; w++) s += counts[w][threadIdx.x];
+        offs[(size_t) threadIdx.x * n_tiles + blockIdx.x] = s;
+    }
+}
+
+// Stable scatter: the positions of a key keep their order. Each warp ranks its
+// own run of consecutive positions (match in a round, a running count per key
+// over the rounds), after the earlier warps' and tiles' and smaller keys'.
+__global__ void __launch_bounds__(kSortThreads) key_scatter_kernel(const uint8_t *__restrict__ bucket,
+                                                                   const uint32_t *__restrict__ totals, uint32_t cut,
+                                                                   uint32_t n, uint32_t n_tiles,
+                                                                   const uint32_t *__restrict__ offs,
+                                                                   const uint32_t *__restrict__ key_total,
+                                                                   uint32_t *__restrict__ perm) {
+    __shared__ uint8_t key_of[kBuckets];
+    __shared__ uint32_t counts[kSortWarps][32];
+    bucket_keys(totals, cut, key_of);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t base = blockIdx.x * kSortTile + wid * kSortRounds * 32;
+    uint8_t key[kSortRounds];
+    warp_keys(bucket, key_of, base, n, key, counts[wid]);
+    __syncthreads();
+    if (threadIdx.x < kKeys) {
+        uint32_t at = offs[(size_t) threadIdx.x * n_tiles + blockIdx.x];
+        for (int k = 0; k < (int) threadIdx.x; k++) at += __ldg(key_total + k);
+#pragma unroll
+        for (int w = 0; w < kSortWarps; w++) {
+            const uint32_t c = counts[w][threadIdx.x];
+            counts[w][threadIdx.x] = at;
+            at += c;
+        }
     }
     __syncthreads();
-    offs[(size_t) threadIdx.x * n_tiles + blockIdx.x] = hist[threadIdx.x];
-}
-
-// Stable scatter: positions of a bucket keep their order. Each round takes
-// kSortThreads consecutive positions; a position's rank is its rank among the
-// equal buckets of its warp (match) plus the counts of the earlier warps.
-__global__ void __launch_bounds__(kSortThreads) bucket_scatter_kernel(const uint8_t *__restrict__ bucket,
-                                                                      const uint8_t *__restrict__ key_of, uint32_t n,
-                                                                      uint32_t n_tiles,
-                                                                      const uint32_t *__restrict__ offs,
-                                                                      const uint32_t *__restrict__ base_of,
-                                                                      uint32_t *__restrict__ perm) {
-    constexpr int kWarps = kSortThreads / 32;
-    __shared__ uint32_t run[kBuckets];
-    __shared__ uint16_t wcnt[kWarps][kBuckets];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    run[threadIdx.x] = base_of[threadIdx.x] + offs[(size_t) threadIdx.x * n_tiles + blockIdx.x];
-    const uint32_t base = blockIdx.x * kSortTile;
+    uint32_t *run = counts[wid];
+#pragma unroll
     for (int r = 0; r < kSortRounds; r++) {
-#pragma unroll
-        for (int w = 0; w < kWarps; w++) wcnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        const uint32_t pos = base + r * kSortThreads + threadIdx.x;
-        const bool valid = pos < n;
-        const uint32_t b = valid ? (key_of ? key_of[bucket[pos]] : bucket[pos]) : (uint32_t) kBuckets;  // kBuckets: none
-        const unsigned peers = __match_any_sync(kFullMask, b);
-        const unsigned lt = (1u << lane) - 1u;
-        const uint32_t rank = (uint32_t) __popc(peers & lt);
-        if (valid && rank == 0) wcnt[wid][b] = (uint16_t) __popc(peers);
-        __syncthreads();
-        if (valid) {
-            uint32_t dst = run[b] + rank;
-            for (int w = 0; w < wid; w++) dst += wcnt[w][b];
-            perm[dst] = pos;
-        }
-        __syncthreads();
-        uint32_t add = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; w++) add += wcnt[w][threadIdx.x];
-        run[threadIdx.x] += add;
-        __syncthreads();
+        const unsigned peers = __match_any_sync(kFullMask, (unsigned) key[r]);
+        const uint32_t rank = (uint32_t) __popc(peers & ((1u << lane) - 1u));
+        const bool valid = key[r] < kKeys;
+        if (valid) perm[run[key[r]] + rank] = base + r * 32 + lane;
+        __syncwarp();
+        if (valid && rank == 0) run[key[r]] += (uint32_t) __popc(peers);
+        __syncwarp();
     }
 }
 
@@ -1125,39 +1192,32 @@ int score_pass(gss_engine *eng, cudaStream_t st, int64_t q, uint32_t *covered, i
     const uint32_t n_tiles = (uint32_t) (((size_t) n + kSortTile - 1) / kSortTile);
     GSS_TRY(perm.reserve(std::max<size_t>(n, 1) * sizeof(uint32_t)));
     GSS_TRY(o.bucket.reserve(std::max<size_t>(n, 1)));
-    GSS_TRY(o.offs.reserve(std::max<size_t>((size_t) kBuckets * n_tiles, 1) * sizeof(uint32_t)));
-    GSS_TRY(o.totals.reserve(kBuckets * sizeof(uint32_t)));
-    GSS_TRY(o.key_of.reserve(kBuckets));
+    GSS_TRY(o.offs.reserve(std::max<size_t>((size_t) kKeys * n_tiles, 1) * sizeof(uint32_t)));
+    constexpr size_t total_bytes = kBuckets * kTotalStride * sizeof(uint32_t);
+    GSS_TRY(o.totals.reserve(total_bytes + kKeys * sizeof(uint32_t)));
     if (n) {
-        // features, MLP, score bucket
-        score_kernel<<<grid_for_n((uint64_t) (n + 31) / 32 * 32, eng->sm_count, kMlpThreads), kMlpThreads, 0, st>>>(
+        uint32_t *const totals = (uint32_t *) o.totals.ptr;
+        uint32_t *const key_total = totals + kBuckets * kTotalStride;
+        uint32_t *const offs = (uint32_t *) o.offs.ptr;
+        const uint8_t *const bucket = (const uint8_t *) o.bucket.ptr;
+        const uint32_t cut = head_cut(o, n);
+        // features, MLP, score bucket, clauses per bucket
+        GSS_CUDA_TRY(cudaMemsetAsync(totals, 0, total_bytes, st));
+        const unsigned blocks = (unsigned) std::min<uint64_t>(((uint64_t) n + kMlpThreads - 1) / kMlpThreads,
+                                                              (uint64_t) std::max(eng->sm_count, 1) * kScoreGrid);
+        score_kernel<<<blocks, kMlpThreads, 0, st>>>(
             h, (const float *) o.scorer.w.ptr, (const uint32_t *) o.scorer.frag.ptr,
-            (const int64_t *) eng->offsets.ptr, (const uint32_t *) eng->orig.ptr, alive, n, (uint8_t *) o.bucket.ptr);
+            (const int64_t *) eng->offsets.ptr, (const uint32_t *) eng->orig.ptr, alive, n, (uint8_t *) o.bucket.ptr,
+            totals);
         GSS_CUDA_TRY(cudaGetLastError());
-        // the clauses per score bucket, then the sort key of each bucket:
-        // score order in the head, plain order in the tail
-        bucket_hist_kernel<<<n_tiles, kSortThreads, 0, st>>>((const uint8_t *) o.bucket.ptr, nullptr, n, n_tiles,
-                                                              (uint32_t *) o.offs.ptr);
+        // stable sort of positions by key: score order in the head, plain
+        // order in the tail
+        key_hist_kernel<<<n_tiles, kSortThreads, 0, st>>>(bucket, totals, cut, n, n_tiles, offs);
         GSS_CUDA_TRY(cudaGetLastError());
-        bucket_scan_kernel<<<kBuckets, 1024, 0, st>>>((uint32_t *) o.offs.ptr, n_tiles, (uint32_t *) o.totals.ptr);
+        key_scan_kernel<<<kKeys, 1024, 0, st>>>(offs, n_tiles, key_total);
         GSS_CUDA_TRY(cudaGetLastError());
-        head_key_kernel<<<1, kBuckets, 0, st>>>((const uint32_t *) o.totals.ptr, head_cut(o, n),
-                                                (uint8_t *) o.key_of.ptr);
-        GSS_CUDA_TRY(cudaGetLastError());
-        // stable radix sort of positions by key
-        bucket_hist_kernel<<<n_tiles, kSortThreads, 0, st>>>((const uint8_t *) o.bucket.ptr,
-                                                              (const uint8_t *) o.key_of.ptr, n, n_tiles,
-                                                              (uint32_t *) o.offs.ptr);
-        GSS_CUDA_TRY(cudaGetLastError());
-        bucket_scan_kernel<<<kBuckets, 1024, 0, st>>>((uint32_t *) o.offs.ptr, n_tiles, (uint32_t *) o.totals.ptr);
-        GSS_CUDA_TRY(cudaGetLastError());
-        bucket_base_kernel<<<1, kBuckets, 0, st>>>((uint32_t *) o.totals.ptr, kBuckets);
-        GSS_CUDA_TRY(cudaGetLastError());
-        bucket_scatter_kernel<<<n_tiles, kSortThreads, 0, st>>>((const uint8_t *) o.bucket.ptr,
-                                                                 (const uint8_t *) o.key_of.ptr, n, n_tiles,
-                                                                 (const uint32_t *) o.offs.ptr,
-                                                                 (const uint32_t *) o.totals.ptr,
-                                                                 (uint32_t *) perm.ptr);
+        key_scatter_kernel<<<n_tiles, kSortThreads, 0, st>>>(bucket, totals, cut, n, n_tiles, offs, key_total,
+                                                             (uint32_t *) perm.ptr);
         GSS_CUDA_TRY(cudaGetLastError());
     }
     GSS_CUDA_TRY(cudaEventRecord(o.ev[1], st));
@@ -1233,8 +1293,9 @@ int order_after_pass(gss_engine *eng, const DevBuf &reports, const DevBuf &count
     GSS_CUDA_TRY(cudaGetLastError());
     o.have_times = true;
     // the order of pass q+1, on the scoring stream once the head of pass q is
-    // done (overlap) or pass q is: it folds the counts of pass q-1 (complete)
-    GSS_CUDA_TRY(cudaStreamWaitEvent(o.score_stream, o.prm.overlap ? o.ev[2] : o.ev[3], 0));
+    // done and its records are out, when the tail starts (overlap: earlier it
+    // would take the tail's places), or once pass q is: it folds the counts of pass q-1 (complete)
+    GSS_CUDA_TRY(cudaStreamWaitEvent(o.score_stream, o.prm.overlap ? o.ev[4] : o.ev[3], 0));
     uint32_t covered = 0;
     int buf = 0;
     GSS_TRY(score_pass(eng, o.score_stream, q + 1, &covered, &buf));
