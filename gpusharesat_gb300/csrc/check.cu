@@ -598,10 +598,7 @@ template <int WPL, int LPC, int G>
 int launch_wide_persist_variant(const CheckArgs *d_args, const CheckArgs &h_args, uint32_t *work, cudaStream_t stream,
                                 int sm_count) {
     constexpr int MINB = default_min_blocks(WPL, G);
-    int per_sm = 0;
-    GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, check_wide_persist_kernel<WPL, LPC, G, MINB, false>, kWarps * 32, 0));
-    if (per_sm < 1) per_sm = 1;
+    static const int per_sm = resident_blocks(check_wide_persist_kernel<WPL, LPC, G, MINB, false>);
     uint64_t blocks = (uint64_t) sm_count * per_sm;
     if (d_args) {  // a captured graph serves databases of other sizes too: the full grid
         check_wide_persist_kernel<WPL, LPC, G, MINB, true><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
@@ -620,10 +617,7 @@ int launch_wide_persist_variant(const CheckArgs *d_args, const CheckArgs &h_args
 
 template <int WPL, int LPC, int G, int MINB>
 int launch_wide_pf_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
-    int per_sm = 0;
-    GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, check_wide_pf_kernel<WPL, LPC, G, MINB>,
-                                                               kWarps * 32, 0));
-    if (per_sm < 1) per_sm = 1;
+    static const int per_sm = resident_blocks(check_wide_pf_kernel<WPL, LPC, G, MINB>);
     constexpr int CPW = 32 / LPC;
     const uint64_t n_tasks = (uint64_t) ((scan_count(a) + CPW - 1) / CPW) * a.n_blocks;
     uint64_t blocks = (uint64_t) sm_count * per_sm;
@@ -637,10 +631,7 @@ int launch_wide_pf_variant(const CheckArgs &a, cudaStream_t stream, int sm_count
 
 template <int WPL, int LPC, int G, int MINB, bool HINT = false>
 int launch_wide_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
-    int per_sm = 0;
-    GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, check_wide_kernel<WPL, LPC, G, MINB, HINT>, kWarps * 32, 0));
-    if (per_sm < 1) per_sm = 1;
+    static const int per_sm = resident_blocks(check_wide_kernel<WPL, LPC, G, MINB, HINT>);
     constexpr int CPW = 32 / LPC;
     const uint64_t n_tasks = (uint64_t) ((scan_count(a) + CPW - 1) / CPW) * a.n_blocks;
     uint64_t blocks = (uint64_t) sm_count * per_sm;
@@ -654,9 +645,7 @@ int launch_wide_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
 
 template <int LPC, int G>
 int launch_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
-    int per_sm = 0;
-    GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, check_kernel<LPC, G>, kWarps * 32, 0));
-    if (per_sm < 1) per_sm = 1;
+    static const int per_sm = resident_blocks(check_kernel<LPC, G>);
     constexpr int CPW = 32 / LPC;
     const uint64_t n_tasks = (uint64_t) ((scan_count(a) + CPW - 1) / CPW) * a.n_blocks;
     uint64_t blocks = (uint64_t) sm_count * per_sm;

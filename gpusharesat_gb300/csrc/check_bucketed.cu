@@ -228,9 +228,7 @@ int layout_lanes(int layout) {
 
 int launch_check_bucketed(const CheckArgs *d_args, const BucketPlan *d_plan, uint32_t *work, cudaStream_t stream,
                           int sm_count) {
-    int per_sm = 0;
-    GSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, check_bucketed_kernel, kWarps * 32, 0));
-    if (per_sm < 1) per_sm = 1;
+    static const int per_sm = resident_blocks(check_bucketed_kernel);
     check_bucketed_kernel<<<(unsigned) (sm_count * per_sm), kWarps * 32, 0, stream>>>(d_args, d_plan, work);
     GSS_CUDA_TRY(cudaGetLastError());
     return GSS_OK;

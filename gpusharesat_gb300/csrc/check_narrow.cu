@@ -187,10 +187,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_narrow_kernel(const C
 
 template <int NW, int MINB>
 int launch_narrow_variant(const CheckArgs &a, uint32_t *work, cudaStream_t stream, int sm_count) {
-    int per_sm = 0;
-    GSS_CUDA_TRY(
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, check_narrow_kernel<NW, MINB>, kWarps * 32, 0));
-    if (per_sm < 1) per_sm = 1;
+    static const int per_sm = resident_blocks(check_narrow_kernel<NW, MINB>);
     const uint64_t n_tasks = ((uint64_t) scan_count(a) + 31) / 32;
     const uint64_t blocks = std::min<uint64_t>((uint64_t) sm_count * per_sm, (n_tasks + kWarps - 1) / kWarps);
     check_narrow_kernel<NW, MINB><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(a, work);

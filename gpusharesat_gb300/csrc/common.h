@@ -13,6 +13,8 @@ namespace gss {
 // (MAX_CL_SIZE, gpuShareLib/BaseTypes.cuh:28); the sharer keeps that limit
 // by default, the engine itself takes clauses up to this length.
 constexpr int kMaxClauseLen = 4096;
+// Most 32-slot words of a pass.
+constexpr int kMaxWords = 4096;
 
 // Tiles of the tiled check kernel: consecutive length-sorted clauses with at
 // most kTileLits literals (a longer clause gets a tile of its own and is read
@@ -229,6 +231,18 @@ inline void auto_layout(int n_words, int &kind, int &lpc, int &depth) {
     else
         lpc = n_words > 2 ? 4 : n_words > 1 ? 2 : 1;
     depth = lpc == 1 ? 1 : 2;
+}
+
+// Resident blocks of 256 threads per multiprocessor of a kernel; for a static
+// in its launcher (asked of the runtime once, not at every launch).
+template <typename K>
+int resident_blocks(K kernel) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 256, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return n < 1 ? 1 : n;
 }
 
 // Launches the check kernel on `stream` (the counters must already be zero).

@@ -178,8 +178,6 @@ int ensure_queues(gss_engine *eng) {
         GSS_TRY(eng->reports.reserve((size_t) per * eng->n_parts * sizeof(gss_report)));
         eng->cap_per_part = (uint32_t) per;
     }
-    GSS_TRY(eng->counts.reserve(counter_bytes(eng->n_parts)));
-    GSS_TRY(eng->h_counts.reserve(kInlineOffset));
     return GSS_OK;
 }
 
@@ -220,6 +218,13 @@ int gss_engine_create(int device, gss_engine **out) {
             e = cudaStreamCreateWithPriority(&eng->own_stream, cudaStreamNonBlocking, greatest);
         if (e != cudaSuccess) rc = set_error(GSS_ERR_CUDA, "engine setup failed: %s", cudaGetErrorString(e));
     }
+    // the buffers whose size no pass changes, once, here: a pinned allocation
+    // takes 110 us (and 160 to free) whatever its size, a device one 35, and
+    // the first pass had waited for all of them
+    if (rc == GSS_OK) rc = eng->h_counts.reserve(kHostCounterBytes);
+    if (rc == GSS_OK) rc = eng->counts.reserve(counter_bytes(eng->n_parts));
+    if (rc == GSS_OK) rc = eng->start.reserve(kMaxWords * sizeof(uint32_t));
+    if (rc == GSS_OK) rc = eng->solver_of_word.reserve(kMaxWords * sizeof(int32_t));
     if (rc != GSS_OK) {
         delete eng;
         return rc;
@@ -607,7 +612,7 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
                   const int32_t *solver_of_word, int on_device) {
     if (!eng || n_vars < 0 || n_words < 0 || (n_vars > 0 && n_words > 0 && !state) || (n_words > 0 && !start))
         return set_error(GSS_ERR_INVALID, "bad arguments to gss_state_set");
-    if (n_words > 4096) return set_error(GSS_ERR_INVALID, "at most 4096 words (131072 slots) per pass");
+    if (n_words > kMaxWords) return set_error(GSS_ERR_INVALID, "at most 4096 words (131072 slots) per pass");
     if (n_vars > 0x7FFFFFFF) return set_error(GSS_ERR_INVALID, "too many variables");
     GSS_TRY(ensure_device(eng));
     int kind = eng->kind, lpc = eng->lpc, depth = eng->g;
@@ -643,7 +648,6 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     // the counters' pinned buffer
     unsigned long long *const density = filtered ? (unsigned long long *) ((char *) agg + abytes) : nullptr;
     if (filtered) {
-        GSS_TRY(eng->h_counts.reserve(kInlineOffset));
         GSS_CUDA_TRY(cudaMemsetAsync(density, 0, sizeof(unsigned long long), eng->stream));
     }
     unsigned long long *const h_density = (unsigned long long *) ((char *) eng->h_counts.ptr + kDensityOffset);
@@ -776,7 +780,6 @@ int gss_check_launch(gss_engine *eng) {
     if (!eng) return set_error(GSS_ERR_INVALID, "engine is NULL");
     GSS_TRY(ensure_device(eng));
     GSS_TRY(ensure_queues(eng));
-    GSS_TRY(eng->h_counts.reserve(kHostCounterBytes));
     GSS_TRY(launch_pass_into(eng, eng->state.ptr, eng->agg.ptr, eng->reports, eng->counts, eng->h_counts, kEngineInline));
     eng->launches++;
     eng->pass_pending = true;
@@ -1049,13 +1052,14 @@ void note_kept(gss_engine *eng, const uint32_t *hc, bool filtered) {
 
 int gss_check_wait(gss_engine *eng, int64_t *n_reports) {
     if (!eng) return set_error(GSS_ERR_INVALID, "engine is NULL");
-    GSS_TRY(ensure_device(eng));
-    GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
-    eng->pass_pending = false;
-    if (!eng->h_counts.ptr) {  // no pass launched yet: nothing to report
+    if (eng->launches == 0 && !eng->pass_pending) {  // no pass launched yet: nothing to report
         if (n_reports) *n_reports = 0;
         return GSS_OK;
     }
+    GSS_TRY(ensure_device(eng));
+    // (a pass that was waited for needs no second wait before its reports)
+    if (eng->pass_pending) GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
+    eng->pass_pending = false;
     const uint32_t *hc = (const uint32_t *) eng->h_counts.ptr;
     int64_t total = 0;
     bool overflow = false;

@@ -1272,7 +1272,6 @@ int order_after_head(gss_engine *eng, const DevBuf &counts) {
     OrderState &o = *eng->order;
     GSS_CUDA_TRY(cudaEventRecord(o.ev[2], eng->stream));
     // the head's counts and records, on their way while the tail runs
-    GSS_TRY(o.h_head_counts.reserve(kHostCounterBytes));
     GSS_TRY(launch_deliver(nullptr, (const gss_report *) eng->reports.ptr, (const uint32_t *) counts.ptr, eng->n_parts,
                            eng->cap_per_part, o.h_head_counts.ptr, kEngineInline, eng->stream));
     GSS_CUDA_TRY(cudaEventRecord(o.ev[4], eng->stream));
@@ -1367,6 +1366,7 @@ int gss_order_enable(gss_engine *eng, const gss_order_params *p) {
     }
     if (rc == GSS_OK) rc = o->log_count.reserve(sizeof(unsigned long long));
     if (rc == GSS_OK) rc = o->h_log_count.reserve(sizeof(unsigned long long));
+    if (rc == GSS_OK) rc = o->h_head_counts.reserve(kHostCounterBytes);
     if (rc == GSS_OK && cudaMemsetAsync(o->log_count.ptr, 0, sizeof(unsigned long long), eng->stream) != cudaSuccess)
         rc = set_error(GSS_ERR_CUDA, "cudaMemsetAsync failed");
     if (rc == GSS_OK) rc = ensure_ids(eng, std::max<int64_t>(eng->next_id, 1));
