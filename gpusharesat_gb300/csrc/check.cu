@@ -471,20 +471,22 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_pf_kernel(CheckA
 // Persistent wide variant: as check_wide_kernel, with (1) its arguments by
 // value or, for a captured CUDA graph that runs pass after pass while the
 // database and the assignment state change, from device memory (DEV), and (2)
-// tasks of kTaskChunk clause groups from work counters (zeroed before the
-// launch) instead of a fixed stride, so clauses of very different lengths
-// balance across warps that stay side by side in the database.
+// tasks of kUnit clauses from work counters (zeroed before the launch) instead
+// of a fixed stride, so clauses of very different lengths balance across warps
+// that stay side by side in the database.
 //
 // Bound by instruction issue while the state fits L2 (2e6 clauses x 1024
-// fair-coin slots over 2^17 variables: 356 -> 315 us) and by the random
-// row gathers beyond it (2^20: 474 -> 457 us). Hence a division per task of
-// four groups, not per group, three logic operations a word and literal
-// (apply_literal), and records that get their clause id and solver where they
-// are flushed, 32 at a time (a stage of 192 records: 315 against 327 us with
-// 128, over 2^17 variables). The arguments are read from shared memory: kept
-// in the constant bank, their loads are hoisted into registers that spill
-// (401 us).
-constexpr uint32_t kTaskChunk = 4;
+// fair-coin slots over 2^17 variables: 356 -> 307 us) and by the random row
+// gathers beyond it (2^20: 474 -> 446 us). Hence a task's clauses and offsets
+// loaded together, a lane each, and handed over in shared memory (a group of
+// four had loaded its own, one dependent step more: 315 and 458 us; tasks of
+// 32 clauses lose locality: 469), one division a task, three logic operations
+// a word and literal (apply_literal), and records that get their clause id and
+// solver where they are flushed, 32 at a time (a stage of 192 records; 128: 327
+// against 315 us, over 2^17 variables, 256: 329, of L1). The arguments are read
+// from shared memory: kept in the constant bank, their loads are hoisted into
+// registers that spill (401 us).
+constexpr uint32_t kUnit = 16;
 constexpr int kPersistStage = 192;
 
 template <int WPL, int LPC, int G, int MINB, bool DEV>
@@ -495,6 +497,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
     constexpr int BW = WPL * LPC;
     __shared__ CheckArgs sa;
     __shared__ gss_report stage_all[kWarps][kPersistStage];
+    __shared__ uint4 unit_all[kWarps][kUnit];
     if (threadIdx.x == 0) sa = DEV ? *pa : av;
     __syncthreads();
     const CheckArgs &a = sa;
@@ -503,11 +506,12 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
     const int grp = lane / LPC;
     const int gbase = grp * LPC;
     gss_report *stage = stage_all[threadIdx.x >> 5];
+    uint4 *const unit_clauses = unit_all[threadIdx.x >> 5];
     uint32_t nstaged = 0;
 
     const uint32_t n_scan = scan_count(a);
-    const uint32_t n_groups = (n_scan + CPW - 1) / CPW;
-    const uint64_t n_tasks = (uint64_t) n_groups * a.n_blocks;
+    const uint32_t per_block = (n_scan + kUnit - 1) / kUnit;  // tasks of a slot block
+    const uint64_t n_tasks = (uint64_t) per_block * a.n_blocks;
     Row<WPL> st[G];  // zeroed once, as in check_wide_kernel
 #pragma unroll
     for (int i = 0; i < G; i++)
@@ -517,28 +521,28 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
         uint32_t unit = 0;
         if (lane == 0) unit = task_from(work);
         unit = __shfl_sync(kFull, unit, 0);
-        const uint64_t first = (uint64_t) unit * kTaskChunk;
-        if (first >= n_tasks) break;
-        uint32_t blk, g;
-        if (n_tasks <= 0xFFFFFFFFull) {
-            blk = (uint32_t) first / n_groups;
-            g = (uint32_t) first - blk * n_groups;
-        } else {
-            blk = (uint32_t) (first / n_groups);
-            g = (uint32_t) (first - (uint64_t) blk * n_groups);
-        }
-        for (uint32_t left = (uint32_t) min((uint64_t) kTaskChunk, n_tasks - first); left; left--) {
-            const uint32_t i = g * CPW + grp;
-            const uint32_t c = i < n_scan ? scan_clause(a, i) : 0xFFFFFFFFu;
-            const bool valid = c < a.n_clauses && clause_live(a, c);
-            uint32_t af[WPL], live[WPL];
-#pragma unroll
-            for (int j = 0; j < WPL; j++) af[j] = live[j] = valid ? __ldg(a.start + blk * BW + sub * WPL + j) : 0u;
-            uint32_t pos = 0, end = 0;
-            if (valid) {
+        if (unit >= n_tasks) break;
+        const uint32_t blk = unit / per_block;
+        {  // the task's clauses and their offsets, a lane each
+            const uint32_t i = (unit - blk * per_block) * kUnit + lane;
+            const uint32_t c = lane < (int) kUnit && i < n_scan ? scan_clause(a, i) : 0xFFFFFFFFu;
+            uint32_t pos = 1, end = 0;  // no clause
+            if (c < a.n_clauses && clause_live(a, c)) {
                 pos = (uint32_t) __ldg(a.offsets + c);
                 end = (uint32_t) __ldg(a.offsets + c + 1);
             }
+            __syncwarp();
+            if (lane < (int) kUnit) unit_clauses[lane] = make_uint4(c, pos, end, 0u);
+            __syncwarp();
+        }
+        for (uint32_t g = 0; g < kUnit; g += CPW) {
+            const uint4 cl = unit_clauses[g + grp];
+            const uint32_t c = cl.x, end = cl.z;
+            uint32_t pos = cl.y;
+            uint32_t af[WPL], live[WPL];
+#pragma unroll
+            for (int j = 0; j < WPL; j++)
+                af[j] = live[j] = pos <= end ? __ldg(a.start + blk * BW + sub * WPL + j) : 0u;
             const uint2 *rows = a.state + (size_t) blk * a.n_vars * BW + sub * WPL;
             while (true) {
                 bool alive = false;
@@ -585,10 +589,6 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
                     nstaged += __popc(bal);
                 }
             }
-            if (++g == n_groups) {
-                g = 0;
-                blk++;
-            }
         }
     }
     if (nstaged) flush_mapped(a, stage, nstaged);
@@ -604,9 +604,7 @@ int launch_wide_persist_variant(const CheckArgs *d_args, const CheckArgs &h_args
         check_wide_persist_kernel<WPL, LPC, G, MINB, true><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
             d_args, h_args, work);
     } else {
-        constexpr int CPW = 32 / LPC;
-        const uint64_t n_tasks = (uint64_t) ((scan_count(h_args) + CPW - 1) / CPW) * h_args.n_blocks;
-        const uint64_t units = (n_tasks + kTaskChunk - 1) / kTaskChunk;
+        const uint64_t units = (uint64_t) ((scan_count(h_args) + kUnit - 1) / kUnit) * h_args.n_blocks;
         blocks = std::min<uint64_t>(blocks, std::max<uint64_t>((units + kWarps - 1) / kWarps, 1));
         check_wide_persist_kernel<WPL, LPC, G, MINB, false><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
             nullptr, h_args, work);
