@@ -201,7 +201,8 @@ __host__ __device__ __forceinline__ uint32_t *work_counter(uint32_t *counts, uin
 }
 // Bytes of the buffer with `sets` sets of work counters: the head and the tail
 // of an ordered pass have one each.
-inline size_t counter_bytes(uint32_t n_parts, uint32_t sets = 2) {
+constexpr uint32_t kWorkSets = 2;
+inline size_t counter_bytes(uint32_t n_parts, uint32_t sets = kWorkSets) {
     return sizeof(uint32_t) * (n_parts + 1) * kCountStride + sets * kWorkBytes;
 }
 // Hands a pass's outcome to the host: writes the report counters, the error
@@ -209,9 +210,11 @@ inline size_t counter_bytes(uint32_t n_parts, uint32_t sets = 2) {
 // records and no partition overflowed, the records too, partition after
 // partition from byte kInlineOffset on. With d_args the queues are those of
 // the arguments in device memory (a captured graph outlives a queue's growth).
+// clear: the counters are zero again when it is done (the last use of them in
+// the pass; it takes the place of the next pass's memset).
 constexpr size_t kInlineOffset = 256;
-int launch_deliver(const CheckArgs *d_args, const gss_report *parts, const uint32_t *counts, uint32_t n_parts,
-                   uint32_t cap, void *host, uint32_t max_inline, cudaStream_t stream);
+int launch_deliver(const CheckArgs *d_args, const gss_report *parts, uint32_t *counts, uint32_t n_parts,
+                   uint32_t cap, void *host, uint32_t max_inline, bool clear, cudaStream_t stream);
 // Synchronizes `stream`; returns the live clause and literal counts.
 int compact_by_id(const CompactArgs &a, cudaStream_t stream, int sm_count, uint32_t *n_out, int64_t *lits_out);
 

@@ -228,39 +228,51 @@ __global__ void pack_reports_kernel(const gss_report *__restrict__ parts, const 
 constexpr uint32_t kStripes = 4;
 __global__ void __launch_bounds__(256) deliver_kernel(const CheckArgs *__restrict__ pa,
                                                       const gss_report *__restrict__ parts,
-                                                      const uint32_t *__restrict__ counts, uint32_t n_parts,
-                                                      uint32_t cap, uint32_t *__restrict__ host, uint32_t max_inline) {
+                                                      uint32_t *__restrict__ counts, uint32_t n_parts, uint32_t cap,
+                                                      uint32_t *__restrict__ host, uint32_t max_inline, bool clear) {
     if (pa) {
         parts = pa->out;
         cap = pa->cap_per_part;
     }
-    const uint32_t p = blockIdx.x / kStripes, stripe = blockIdx.x % kStripes;
-    if (blockIdx.x == 0 && threadIdx.x < n_parts + kExtraCounters) {
-        const uint32_t t = threadIdx.x;
+    const uint32_t p = blockIdx.x / kStripes, stripe = blockIdx.x % kStripes, t = threadIdx.x;
+    if (blockIdx.x == 0 && t < n_parts + kExtraCounters)
         host[t] = t < n_parts ? counts[t * kCountStride] : counts[n_parts * kCountStride + (t - n_parts)];
-    }
-    if (max_inline == 0) return;
     uint64_t total = 0, base = 0;
+    uint32_t n = 0;
     bool over = false;
     for (uint32_t q = 0; q < n_parts; q++) {
-        const uint32_t m = __ldg(counts + q * kCountStride);
+        const uint32_t m = counts[q * kCountStride];
         over |= m > cap;
-        if (q == p) base = total;
+        if (q == p) base = total, n = m;
         total += m;
     }
+    if (clear) {
+        // once every block has read the counters, the last one zeroes them:
+        // the first word of each, the error flag's neighbours (the filter's
+        // count and this ticket)
+        __shared__ bool last;
+        __syncthreads();
+        uint32_t *const ticket = counts + n_parts * kCountStride + kExtraCounters;
+        if (t == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (last) {
+            for (uint32_t i = t; i < n_parts + 1 + kWorkSets * kWorkCounters; i += blockDim.x)
+                counts[i * kCountStride] = 0;
+            if (t < kExtraCounters) counts[n_parts * kCountStride + 1 + t] = 0;
+        }
+    }
     if (over || total > max_inline) return;
-    const uint32_t n = __ldg(counts + p * kCountStride);
     const int4 *from = reinterpret_cast<const int4 *>(parts + (size_t) p * cap);
     int4 *to = reinterpret_cast<int4 *>(reinterpret_cast<char *>(host) + kInlineOffset) + base;
-    for (uint32_t i = stripe * blockDim.x + threadIdx.x; i < n; i += kStripes * blockDim.x) to[i] = from[i];
+    for (uint32_t i = stripe * blockDim.x + t; i < n; i += kStripes * blockDim.x) to[i] = from[i];
 }
 
 }  // namespace
 
-int launch_deliver(const CheckArgs *d_args, const gss_report *parts, const uint32_t *counts, uint32_t n_parts,
-                   uint32_t cap, void *host, uint32_t max_inline, cudaStream_t stream) {
+int launch_deliver(const CheckArgs *d_args, const gss_report *parts, uint32_t *counts, uint32_t n_parts,
+                   uint32_t cap, void *host, uint32_t max_inline, bool clear, cudaStream_t stream) {
     deliver_kernel<<<max_inline ? n_parts * kStripes : 1, 256, 0, stream>>>(d_args, parts, counts, n_parts, cap,
-                                                                          (uint32_t *) host, max_inline);
+                                                                          (uint32_t *) host, max_inline, clear);
     GSS_CUDA_TRY(cudaGetLastError());
     return GSS_OK;
 }

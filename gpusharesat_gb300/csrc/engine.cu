@@ -894,6 +894,12 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     a.agg = (const uint2 *) agg;
     a.kept = kept_counter(a.counts, a.n_parts);
     uint32_t *work = work_counter(a.counts, a.n_parts);
+    // passes of the engine's own slot leave their counters zero; the slots of
+    // passes through host buffers are read again when they are packed
+    const bool clear = max_inline > 0;
+    if (!(clear && eng->counts_clean))
+        GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(a.n_parts), eng->stream));
+    eng->counts_clean = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (eng->timing) {
         for (cudaEvent_t *ev : {&ev0, &ev1}) {
@@ -948,7 +954,6 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->d_args.ptr, &a, sizeof a, cudaMemcpyHostToDevice, eng->stream));
         if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
         auto body = [&]() -> int {
-            GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(a.n_parts), eng->stream));
             if (a.n_clauses > 0 && a.n_blocks > 0) {
                 if (bucketed) {
                     if (eng->plan_ranges > 0)
@@ -960,7 +965,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
                 }
             }
             return launch_deliver((const CheckArgs *) eng->d_args.ptr, a.out, a.counts, a.n_parts, a.cap_per_part,
-                                  h_counts.ptr, max_inline, eng->stream);
+                                  h_counts.ptr, max_inline, clear, eng->stream);
         };
         if (eng->use_graph) {
             const std::vector<uintptr_t> key = {
@@ -992,9 +997,9 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
             GSS_CUDA_TRY(cudaEventRecord(ev1, eng->stream));
             eng->ev_pending.emplace_back(ev0, ev1);
         }
+        eng->counts_clean = clear;
         return GSS_OK;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(a.n_parts), eng->stream));
     if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
     auto launch = [&](const CheckArgs &args) -> int {
         if (eng->state_kind == GSS_KERNEL_TILED) return launch_check_tiled(args, eng->stream, eng->sm_count);
@@ -1036,7 +1041,10 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         GSS_CUDA_TRY(cudaEventRecord(ev1, eng->stream));
         eng->ev_pending.emplace_back(ev0, ev1);
     }
-    return launch_deliver(nullptr, a.out, a.counts, a.n_parts, a.cap_per_part, h_counts.ptr, max_inline, eng->stream);
+    GSS_TRY(launch_deliver(nullptr, a.out, a.counts, a.n_parts, a.cap_per_part, h_counts.ptr, max_inline, clear,
+                           eng->stream));
+    eng->counts_clean = clear;
+    return GSS_OK;
 }
 
 }  // namespace

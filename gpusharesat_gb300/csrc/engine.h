@@ -77,6 +77,7 @@ struct gss_engine {
     // reports (launch_deliver); inline_ok: of the pass launched last
     PinnedBuf h_counts;
     bool inline_ok = false;
+    bool counts_clean = false;  // `counts` is all zero (the last pass's delivery cleared it)
     bool pass_pending = false;
 
     // pipelined passes through host buffers (gss_check_passes_host): second

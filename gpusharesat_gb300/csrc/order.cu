@@ -1272,8 +1272,8 @@ int order_after_head(gss_engine *eng, const DevBuf &counts) {
     OrderState &o = *eng->order;
     GSS_CUDA_TRY(cudaEventRecord(o.ev[2], eng->stream));
     // the head's counts and records, on their way while the tail runs
-    GSS_TRY(launch_deliver(nullptr, (const gss_report *) eng->reports.ptr, (const uint32_t *) counts.ptr, eng->n_parts,
-                           eng->cap_per_part, o.h_head_counts.ptr, kEngineInline, eng->stream));
+    GSS_TRY(launch_deliver(nullptr, (const gss_report *) eng->reports.ptr, (uint32_t *) counts.ptr, eng->n_parts,
+                           eng->cap_per_part, o.h_head_counts.ptr, kEngineInline, false, eng->stream));
     GSS_CUDA_TRY(cudaEventRecord(o.ev[4], eng->stream));
     o.pending = true;
     return GSS_OK;

@@ -496,9 +496,7 @@ int Sharer::ensure_state() {
     eff_kind_ = kind;
     eff_lpc_ = lpc;
     eff_depth_ = depth;
-    GSS_TRY(d_start_.reserve(sizeof(uint32_t) * n_blocks * bw));
     GSS_TRY(d_sow_.reserve(sizeof(int32_t) * n_blocks * bw));
-    GSS_TRY(d_last_mask_.reserve(sizeof(uint32_t) * n_blocks * bw));
     std::vector<int32_t> sow(n_blocks * bw);
     for (int w = 0; w < n_blocks * bw; w++) sow[w] = w < n_words ? w : 0;
     GSS_CUDA_TRY(cudaMemcpy(d_sow_.ptr, sow.data(), sow.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -523,7 +521,7 @@ int Sharer::refresh_agg(int64_t n_updates) {
     // update's row is 8 * bw_ bytes; several updates may share one).
     if (n_updates == 0) return GSS_OK;
     if (n_updates >= (int64_t) dev_vars_ * n_blocks_) return rebuild_agg();
-    return launch_refresh_agg((const StateUpdate *) d_updates_.ptr, (uint32_t) n_updates,
+    return launch_refresh_agg(updates(), (uint32_t) n_updates,
                               (const uint2 *) d_state_.ptr, (uint2 *) d_agg_.ptr, (uint32_t) dev_vars_,
                               (uint32_t) dev_words_, (uint32_t) bw_, stream_, sm_count_);
 }
@@ -867,10 +865,7 @@ int Sharer::append_clauses(std::vector<int64_t> &ids, std::vector<int32_t> &lits
 }
 
 int Sharer::run_check(Pass &p) {
-    // start masks: p.h_start (pinned) holds n_blocks_ * bw_ words
-    const size_t padded = (size_t) n_blocks_ * bw_;
-    GSS_CUDA_TRY(cudaMemcpyAsync(d_start_.ptr, p.h_start.ptr, padded * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                                 stream_));
+    // (the start masks are at the head of d_updates_)
     // capacity: from the option (records per category x categories, as the
     // reference sizes its reporter) and what earlier passes needed
     const int64_t want = std::max<int64_t>((int64_t) opt_.init_report_count * opt_.block_count,
@@ -891,7 +886,7 @@ int Sharer::run_check(Pass &p) {
     a.state = (const uint2 *) d_state_.ptr;
     a.n_vars = (uint32_t) std::max(dev_vars_, 1);
     a.n_blocks = (uint32_t) n_blocks_;
-    a.start = (const uint32_t *) d_start_.ptr;
+    a.start = start_masks();
     a.solver_of_word = (const int32_t *) d_sow_.ptr;
     a.out = (gss_report *) p.d_reports.ptr;
     a.counts = (uint32_t *) p.d_counts.ptr;
@@ -912,7 +907,8 @@ int Sharer::run_check(Pass &p) {
         a.alive = (const uint32_t *) d_alive_.ptr;
         a.alive_by_id = 1;
     }
-    GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(n_parts_), stream_));
+    if (!p.counts_clean) GSS_CUDA_TRY(cudaMemsetAsync(a.counts, 0, counter_bytes(n_parts_), stream_));
+    p.counts_clean = false;
     if (p.active_words > 0 && p.n_clauses > 0) {
         const int wpl = eff_kind_ == GSS_KERNEL_WIDE4 ? 4 : 2;
         const bool wide = eff_kind_ == GSS_KERNEL_WIDE4 || eff_kind_ == GSS_KERNEL_WIDE2;
@@ -933,7 +929,9 @@ int Sharer::run_check(Pass &p) {
             GSS_TRY(launch_check(a, stream_, sm_count_));
         }
     }
-    GSS_TRY(launch_deliver(nullptr, a.out, a.counts, n_parts_, p.cap_per_part, p.h_counts.ptr, kSharerInline, stream_));
+    GSS_TRY(launch_deliver(nullptr, a.out, a.counts, n_parts_, p.cap_per_part, p.h_counts.ptr, kSharerInline, true,
+                           stream_));
+    p.counts_clean = true;
     GSS_CUDA_TRY(cudaEventRecord(p.counted, stream_));
     return GSS_OK;
 }
@@ -944,7 +942,8 @@ int Sharer::collect(Pass &p) {
     // copy of its reports (scheduleGpuToCpuCopyAsync, :325-328) behind the
     // set-to-last of its variables (launchGpu, :356-357).
     const int64_t t0 = now_us();
-    GSS_CUDA_TRY(cudaEventSynchronize(p.counted));
+    p.copying = false;
+    if (p.queued) GSS_CUDA_TRY(cudaEventSynchronize(p.counted));
     if (opt_.quick_prof) stats_[kTimeSpentTestingClauses] += now_us() - t0;
     for (int attempt = 0;; attempt++) {
         const uint32_t *hc = (const uint32_t *) p.h_counts.ptr;
@@ -973,6 +972,7 @@ int Sharer::collect(Pass &p) {
                 pos += hc[q];
             }
             p.reports = (const gss_report *) p.h_reports.ptr;
+            p.copying = true;
             break;
         }
         if (attempt >= 3) return set_error(GSS_ERR_OVERFLOW, "report queues kept overflowing");
@@ -985,11 +985,9 @@ int Sharer::collect(Pass &p) {
     // the pass's variables take their last slot's value in all 32 slots
     // (stream-ordered: the next pass's updates are scattered after this)
     if (p.n_updates > 0) {
-        GSS_CUDA_TRY(cudaMemcpyAsync(d_last_mask_.ptr, p.h_last.ptr, (size_t) n_blocks_ * bw_ * sizeof(uint32_t),
-                                     cudaMemcpyHostToDevice, stream_));
         set_to_last_kernel<<<grid_for(p.n_updates, sm_count_), 256, 0, stream_>>>(
-            (const StateUpdate *) d_updates_.ptr, (uint32_t) p.n_updates, (const uint32_t *) d_last_mask_.ptr,
-            (uint2 *) d_state_.ptr, (uint32_t) dev_vars_, (uint32_t) bw_);
+            updates(), (uint32_t) p.n_updates, last_masks(), (uint2 *) d_state_.ptr, (uint32_t) dev_vars_,
+            (uint32_t) bw_);
         GSS_CUDA_TRY(cudaGetLastError());
         if (agg_ok_) GSS_TRY(refresh_agg(p.n_updates));
     }
@@ -998,7 +996,7 @@ int Sharer::collect(Pass &p) {
     if (filter_pause_ > 0) filter_pause_--;
     if (p.filtered && filter_keeps_too_much(((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1], p.n_clauses, n_blocks_))
         filter_pause_ = kFilterPause;
-    GSS_CUDA_TRY(cudaEventRecord(p.copied, stream_));
+    if (p.copying) GSS_CUDA_TRY(cudaEventRecord(p.copied, stream_));
     p.pending = false;
     p.collected = true;
     p.noted = false;
@@ -1010,7 +1008,7 @@ int Sharer::note_reports(Pass &p) {
     // the next eviction: statistics, activity bumps and last-report passes
     // (GpuRunner::gatherGpuRunResults, gpuShareLib/GpuRunner.cu:360-378).
     if (!p.collected || p.noted) return GSS_OK;
-    GSS_CUDA_TRY(cudaEventSynchronize(p.copied));
+    if (p.copying) GSS_CUDA_TRY(cudaEventSynchronize(p.copied));
     const gss_report *rep = p.reports;
     stats_[kGpuRuns]++;
     stats_[kTotalAssigClauseTested] += (int64_t) p.n_clauses * p.assig_total;
@@ -1111,12 +1109,9 @@ int Sharer::launch_pass() {
     const int64_t t0 = now_us();
     const int n_solvers = (int) solvers_.size();
     const size_t padded = (size_t) n_blocks_ * bw_;
-    GSS_TRY(p.h_start.reserve(padded * sizeof(uint32_t)));
-    GSS_TRY(p.h_last.reserve(padded * sizeof(uint32_t)));
-    uint32_t *start = (uint32_t *) p.h_start.ptr;
-    uint32_t *last = (uint32_t *) p.h_last.ptr;
-    memset(start, 0, padded * sizeof(uint32_t));
-    memset(last, 0, padded * sizeof(uint32_t));
+    std::vector<uint32_t> masks(2 * padded, 0u);  // start, then last
+    uint32_t *start = masks.data();
+    uint32_t *last = start + padded;
     p.assig.assign(n_solvers, AssigIds());
     p.assig_total = 0;
     p.active_words = 0;
@@ -1152,17 +1147,17 @@ int Sharer::launch_pass() {
     // cannot grow, the database is reduced and the same updates are sent
     // again (GpuRunner::wholeRun, gpuShareLib/GpuRunner.cu:243-260).
     auto send_and_check = [&]() -> int {
+        // h_updates_ is free: the copy of the last pass that had one ran
+        // before that pass's check, which has finished
+        const size_t at = updates_offset(), bytes = at + ups.size() * sizeof(StateUpdate);
+        GSS_TRY(d_updates_.reserve(bytes));
+        GSS_TRY(h_updates_.reserve(bytes));
+        memcpy(h_updates_.ptr, masks.data(), masks.size() * sizeof(uint32_t));
+        if (!ups.empty()) memcpy((char *) h_updates_.ptr + at, ups.data(), ups.size() * sizeof(StateUpdate));
+        GSS_CUDA_TRY(cudaMemcpyAsync(d_updates_.ptr, h_updates_.ptr, bytes, cudaMemcpyHostToDevice, stream_));
         if (!ups.empty()) {
-            // h_updates_ is free: the previous pass's copy from it ran before
-            // that pass's check, which has finished
-            const size_t bytes = ups.size() * sizeof(StateUpdate);
-            GSS_TRY(d_updates_.reserve(bytes));
-            GSS_TRY(h_updates_.reserve(bytes));
-            memcpy(h_updates_.ptr, ups.data(), bytes);
-            GSS_CUDA_TRY(cudaMemcpyAsync(d_updates_.ptr, h_updates_.ptr, bytes, cudaMemcpyHostToDevice, stream_));
             scatter_updates_kernel<<<grid_for(ups.size(), sm_count_), 256, 0, stream_>>>(
-                (const StateUpdate *) d_updates_.ptr, (uint32_t) ups.size(), (uint2 *) d_state_.ptr,
-                (uint32_t) dev_vars_, (uint32_t) bw_);
+                updates(), (uint32_t) ups.size(), (uint2 *) d_state_.ptr, (uint32_t) dev_vars_, (uint32_t) bw_);
             GSS_CUDA_TRY(cudaGetLastError());
         }
         // the filter's table follows while the database is large enough for it
@@ -1175,12 +1170,21 @@ int Sharer::launch_pass() {
         p.n_clauses = dev_clauses_;
         return run_check(p);
     };
-    rc = send_and_check();
-    if (rc == GSS_ERR_NOMEM) {
-        GSS_TRY(recover_from_oom());
+    p.queued = !ups.empty() || (p.active_words > 0 && dev_clauses_ > 0);
+    if (p.queued) {
         rc = send_and_check();
+        if (rc == GSS_ERR_NOMEM) {
+            GSS_TRY(recover_from_oom());
+            rc = send_and_check();
+        }
+        GSS_TRY(rc);
+    } else {
+        // no assignment sent and no variable changed: nothing to check, send
+        // or wait for; the pass reports nothing when it is collected
+        p.n_clauses = dev_clauses_;
+        p.filtered = false;
+        memset(p.h_counts.ptr, 0, (n_parts_ + kExtraCounters) * sizeof(uint32_t));
     }
-    GSS_TRY(rc);
     if (opt_.quick_prof) stats_[kTimeSpentFillingAssigs] += now_us() - t0;
     p.pending = true;
     p.number = pass_no_++;

@@ -185,11 +185,14 @@ private:
         int32_t number = 0;      // pass_no_ at its launch
         bool filtered = false;   // checked behind the word-level filter
         // device report queues and their counters, pinned host copies of the
-        // counters (+ error flag), the start and last-slot masks and the reports
+        // counters (+ error flag) and the reports
         DevBuf d_reports, d_counts;
         uint32_t cap_per_part = 0;
         // (+ up to kSharerInline reports, launch_deliver)
-        PinnedBuf h_counts, h_start, h_last, h_reports;
+        PinnedBuf h_counts, h_reports;
+        bool counts_clean = false;      // d_counts is all zero (its last delivery cleared it)
+        bool queued = false;            // there was work for the GPU in it
+        bool copying = false;           // its reports are being copied to h_reports
         const gss_report *reports = nullptr;  // the collected reports: in h_counts or h_reports
         cudaEvent_t counted = nullptr;  // counts in h_counts
         cudaEvent_t copied = nullptr;   // reports in place
@@ -204,6 +207,12 @@ private:
     int recover_from_oom();
     int launch_pass();
     int run_check(Pass &p);
+    const uint32_t *start_masks() const { return (const uint32_t *) d_updates_.ptr; }
+    const uint32_t *last_masks() const { return start_masks() + (size_t) n_blocks_ * bw_; }
+    const StateUpdate *updates() const {
+        return (const StateUpdate *) ((const char *) d_updates_.ptr + updates_offset());
+    }
+    size_t updates_offset() const { return ((size_t) n_blocks_ * bw_ * 2 * sizeof(uint32_t) + 15) & ~(size_t) 15; }
     int rebuild_agg();
     int refresh_agg(int64_t n_updates);
     int ensure_state();
@@ -276,7 +285,9 @@ private:
     int n_vars_ = 0;
     std::vector<std::unique_ptr<SolverAssigs>> solvers_;
     std::vector<std::unique_ptr<SolverReported>> reported_;
-    DevBuf d_state_, d_start_, d_sow_, d_updates_, d_last_mask_;
+    // d_updates_: what a pass sends, in one copy: the start masks and the
+    // last-slot masks (n_blocks_ * bw_ words each), then the changed words
+    DevBuf d_state_, d_sow_, d_updates_;
     DevBuf d_agg_;              // the filter's table of d_state_, kept as variables change
     bool agg_possible_ = false; // the layout has a filtered kernel
     bool agg_ok_ = false;       // d_agg_ follows the state
