@@ -21,8 +21,9 @@
 // a variable's LPC words as one contiguous run of 8*LPC bytes, and the blocks
 // are scanned one after another so that the block being scanned can stay
 // resident in L2 while the clause literals stream past it (evict-first hint).
-// No prefilter is needed: a lane that has no slot left stops loading, and a
-// group stops reading literals once all its lanes are done.
+// Nothing is tested first here (check_filtered.cu does that): a lane that has
+// no slot left stops loading, and a group stops reading literals once all its
+// lanes are done.
 //
 // Memory-level parallelism: a group issues the state loads of G literals
 // before it consumes any of them (lanes that die inside the G are harmless: the

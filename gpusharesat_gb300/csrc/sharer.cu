@@ -14,7 +14,7 @@
 // per solver); each pass uploads only the changed variables, scatters them,
 // runs the check kernel, and broadcasts the last slot into all 32 after it
 // (dUpdateAssigs / dSetAllAssigsToLast, gpuShareLib/Assigs.cu:100-141, without
-// the reference's cross-solver aggregate, which the exact kernel does not need).
+// the reference's cross-solver aggregate; check_filtered.cu has a table instead).
 //
 // Pipeline: gpuRun() first collects the pass launched by the previous call,
 // then cuts and launches a new one, so the results of pass N are delivered at

@@ -100,8 +100,9 @@ int gss_engine_set_timing(gss_engine *eng, int on);
 int gss_engine_kernel_time(gss_engine *eng, double *total_ms, int64_t *n_launches);
 
 /* Check-kernel kinds. */
-#define GSS_KERNEL_AUTO -1   /* default: picked from the word count at gss_state_set (8 words or more: the
-                                wide kernel in its persistent form, 4 words per lane) */
+#define GSS_KERNEL_AUTO -1   /* default: picked from the word count at gss_state_set (up to 4 words: a lane
+                                per clause; more: the wide kernel in its persistent form, 4 words per
+                                lane, behind a word-level filter where the state makes that pay) */
 #define GSS_KERNEL_DIRECT 0  /* a lane group per clause, one 32-slot word per lane */
 #define GSS_KERNEL_TILED 1   /* clause tiles staged in shared memory by bulk copy, K clause slots */
 #define GSS_KERNEL_WIDE4 2   /* a lane group per clause, four words per lane (256-bit loads) */
