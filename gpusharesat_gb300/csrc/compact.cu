@@ -235,8 +235,10 @@ __global__ void __launch_bounds__(256) deliver_kernel(const CheckArgs *__restric
         cap = pa->cap_per_part;
     }
     const uint32_t p = blockIdx.x / kStripes, stripe = blockIdx.x % kStripes, t = threadIdx.x;
-    if (blockIdx.x == 0 && t < n_parts + kExtraCounters)
-        host[t] = t < n_parts ? counts[t * kCountStride] : counts[n_parts * kCountStride + (t - n_parts)];
+    const bool mine = blockIdx.x == 0 && t < n_parts + kExtraCounters;
+    const uint32_t counter = !mine         ? 0u
+                             : t < n_parts ? counts[t * kCountStride]
+                                           : counts[n_parts * kCountStride + (t - n_parts)];
     uint64_t total = 0, base = 0;
     uint32_t n = 0;
     bool over = false;
@@ -249,8 +251,11 @@ __global__ void __launch_bounds__(256) deliver_kernel(const CheckArgs *__restric
     if (clear) {
         // once every block has read the counters, the last one zeroes them:
         // the first word of each, the error flag's neighbours (the filter's
-        // count and this ticket)
+        // count and this ticket). The fence holds the ticket back until this
+        // thread's reads are done (its stores to the host come after it, so
+        // that it does not wait for them).
         __shared__ bool last;
+        __threadfence();
         __syncthreads();
         uint32_t *const ticket = counts + n_parts * kCountStride + kExtraCounters;
         if (t == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
@@ -261,6 +266,7 @@ __global__ void __launch_bounds__(256) deliver_kernel(const CheckArgs *__restric
             if (t < kExtraCounters) counts[n_parts * kCountStride + 1 + t] = 0;
         }
     }
+    if (mine) host[t] = counter;
     if (over || total > max_inline) return;
     const int4 *from = reinterpret_cast<const int4 *>(parts + (size_t) p * cap);
     int4 *to = reinterpret_cast<int4 *>(reinterpret_cast<char *>(host) + kInlineOffset) + base;

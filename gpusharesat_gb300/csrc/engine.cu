@@ -165,6 +165,17 @@ int ensure_device(gss_engine *eng) {
     return GSS_OK;
 }
 
+// A buffer that a pass cannot do without; the filter's tables, which it can,
+// make room for it where the device has no other.
+int reserve_over_table(gss_engine *eng, DevBuf &buf, size_t bytes) {
+    const int rc = buf.reserve(bytes);
+    if (rc != GSS_ERR_NOMEM || !(eng->agg.ptr || eng->agg2.ptr || eng->agg3.ptr)) return rc;
+    GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
+    eng->filter = false;
+    for (DevBuf *t : {&eng->agg, &eng->agg2, &eng->agg3}) t->release();
+    return buf.reserve(bytes);
+}
+
 int ensure_queues(gss_engine *eng) {
     int64_t want = eng->requested_cap;
     if (want <= 0) {
@@ -175,7 +186,7 @@ int ensure_queues(gss_engine *eng) {
     int64_t per = (want + eng->n_parts - 1) / eng->n_parts;
     if (per > 0x7FFFFFFF) per = 0x7FFFFFFF;
     if ((uint32_t) per > eng->cap_per_part || !eng->reports.ptr) {
-        GSS_TRY(eng->reports.reserve((size_t) per * eng->n_parts * sizeof(gss_report)));
+        GSS_TRY(reserve_over_table(eng, eng->reports, (size_t) per * eng->n_parts * sizeof(gss_report)));
         eng->cap_per_part = (uint32_t) per;
     }
     return GSS_OK;
@@ -634,9 +645,12 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     const size_t sbytes = (size_t) n_vars * n_words * 2 * sizeof(uint32_t);
     const size_t bbytes = (size_t) n_blocks * n_vars * bw * 2 * sizeof(uint32_t);
     if (eng->pass_pending) GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
-    GSS_TRY(eng->state.reserve(std::max<size_t>(bbytes, 8)));
+    GSS_TRY(reserve_over_table(eng, eng->state, std::max<size_t>(bbytes, 8)));
     GSS_TRY(eng->start.reserve(std::max<size_t>(padded * sizeof(uint32_t), 4)));
     GSS_TRY(eng->solver_of_word.reserve(std::max<size_t>(padded * sizeof(int32_t), 4)));
+    const bool laid_out = n_blocks == 1 && n_words == bw;  // block-major and host layouts coincide
+    const bool aligned = on_device && ((uintptr_t) state & 7) == 0;  // the copy kernel reads it as it is
+    if (sbytes && !laid_out && !aligned) GSS_TRY(reserve_over_table(eng, eng->state_raw, sbytes));
     // the filter's table: only the automatic variant runs behind it; without
     // room for it the passes run without
     const bool want_agg = eng->kind == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && sbytes > 0;
@@ -656,20 +670,33 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     std::vector<int32_t> sw;
     if (on_device) {
         // in order behind what the caller queued on the default stream
-        for (const void *p : {(const void *) start, (const void *) solver_of_word}) {
+        const void *read[3] = {start, solver_of_word, sbytes ? (const void *) state : nullptr};
+        for (const void *p : read) {
             cudaPointerAttributes at;
             if (p == nullptr || n_words == 0) continue;
             GSS_CUDA_TRY(cudaPointerGetAttributes(&at, p));
             if (at.devicePointer == nullptr)
-                return set_error(GSS_ERR_CUDA, "gss_state_set: a mask pointer that the device cannot read");
+                return set_error(GSS_ERR_CUDA, "gss_state_set: a pointer that the device cannot read");
         }
         if (n_words) {
             if (!eng->ev_caller) GSS_CUDA_TRY(cudaEventCreateWithFlags(&eng->ev_caller, cudaEventDisableTiming));
             GSS_CUDA_TRY(cudaEventRecord(eng->ev_caller, cudaStreamLegacy));
             GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_caller, 0));
         }
-        GSS_TRY(launch_load_masks(start, solver_of_word, (uint32_t) n_words, (uint32_t) padded,
-                                  (uint32_t *) eng->start.ptr, (int32_t *) eng->solver_of_word.ptr, eng->stream));
+        // masks that are no whole words in memory go through a copy
+        const uint32_t *m = start;
+        const int32_t *sow = solver_of_word;
+        if (n_words && ((uintptr_t) m & 3)) {
+            GSS_CUDA_TRY(cudaMemcpyAsync(eng->start.ptr, m, n_words * sizeof(uint32_t), cudaMemcpyDefault, eng->stream));
+            m = (const uint32_t *) eng->start.ptr;
+        }
+        if (n_words && ((uintptr_t) sow & 3)) {
+            GSS_CUDA_TRY(cudaMemcpyAsync(eng->solver_of_word.ptr, sow, n_words * sizeof(int32_t), cudaMemcpyDefault,
+                                         eng->stream));
+            sow = (const int32_t *) eng->solver_of_word.ptr;
+        }
+        GSS_TRY(launch_load_masks(m, sow, (uint32_t) n_words, (uint32_t) padded, (uint32_t *) eng->start.ptr,
+                                  (int32_t *) eng->solver_of_word.ptr, eng->stream));
     } else if (padded) {
         st.assign(padded, 0u);
         sw.assign(padded, 0);
@@ -681,15 +708,12 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
                                      cudaMemcpyHostToDevice, eng->stream));
     }
     if (sbytes) {
-        const bool laid_out = n_blocks == 1 && n_words == bw;  // block-major and host layouts coincide
         const cudaMemcpyKind dir = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         const uint2 *src = (const uint2 *) state;
-        const bool aligned = on_device && ((uintptr_t) state & 7) == 0;  // the kernel reads it as it is
         if (laid_out && !(aligned && filtered)) {
             GSS_CUDA_TRY(cudaMemcpyAsync(eng->state.ptr, state, sbytes, dir, eng->stream));
             src = (const uint2 *) eng->state.ptr;
         } else if (!aligned) {
-            GSS_TRY(eng->state_raw.reserve(sbytes));
             GSS_CUDA_TRY(cudaMemcpyAsync(eng->state_raw.ptr, state, sbytes, dir, eng->stream));
             src = (const uint2 *) eng->state_raw.ptr;
         }
@@ -710,6 +734,7 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     eng->state_lpc = lpc;
     eng->state_g = depth;
     eng->state_bw = bw;
+    eng->state_auto = eng->kind == GSS_KERNEL_AUTO;
     return GSS_OK;
 }
 
@@ -942,9 +967,11 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     if (ordered && (eng->state_kind == GSS_KERNEL_TILED || bucketed))
         return set_error(GSS_ERR_STATE, "the learned scan order runs the direct, wide and persistent kernels (not the "
                          "tiled or bucketed ones)");
-    if (bucketed && eng->n_words > 0 && eng->state_bw != 32)
+    // (an automatic layout of 17 to 31 words is one padded block of 32, whose
+    // empty words a plan's layouts would scan: refused like the narrower ones)
+    if (bucketed && eng->n_words > 0 && (eng->state_bw != 32 || (eng->state_auto && eng->n_words < 32)))
         return set_error(GSS_ERR_STATE, "the length plan needs a state laid out in 32-word blocks (%d here)",
-                         eng->state_bw);
+                         eng->state_bw != 32 ? eng->state_bw : eng->n_words);
     if (ordered && (&reports != &eng->reports || &counts != &eng->counts))
         return set_error(GSS_ERR_STATE, "the learned scan order runs through gss_check_launch");
     if (bucketed || (persistent && eng->use_graph && !ordered)) {
@@ -1170,22 +1197,17 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         if (!eng->ev_kernel[b]) GSS_CUDA_TRY(cudaEventCreateWithFlags(&eng->ev_kernel[b], cudaEventDisableTiming));
         if (!eng->ev_d2h[b]) GSS_CUDA_TRY(cudaEventCreateWithFlags(&eng->ev_d2h[b], cudaEventDisableTiming));
     }
-    GSS_TRY(eng->state2.reserve(std::max<size_t>(bbytes, 8)));
-    GSS_TRY(eng->state3.reserve(std::max<size_t>(bbytes, 8)));
+    auto reserve = [&](DevBuf &buf, size_t bytes) { return reserve_over_table(eng, buf, bytes); };
+    GSS_TRY(reserve(eng->state2, std::max<size_t>(bbytes, 8)));
+    GSS_TRY(reserve(eng->state3, std::max<size_t>(bbytes, 8)));
     if (!direct) {
-        GSS_TRY(eng->state_raw.reserve(std::max<size_t>(sbytes, 8)));
-        GSS_TRY(eng->state_raw2.reserve(std::max<size_t>(sbytes, 8)));
-        GSS_TRY(eng->state_raw3.reserve(std::max<size_t>(sbytes, 8)));
-    }
-    // The first state decides for all of them: a later one whose table keeps
-    // more costs time, not reports.
-    if (eng->filter) {
-        const size_t abytes = (size_t) eng->n_blocks * n_vars * 2 * sizeof(uint2);
-        if (eng->agg2.reserve(abytes) != GSS_OK || eng->agg3.reserve(abytes) != GSS_OK) eng->filter = false;
+        GSS_TRY(reserve(eng->state_raw, std::max<size_t>(sbytes, 8)));
+        GSS_TRY(reserve(eng->state_raw2, std::max<size_t>(sbytes, 8)));
+        GSS_TRY(reserve(eng->state_raw3, std::max<size_t>(sbytes, 8)));
     }
     auto reserve_reports = [&]() -> int {
-        GSS_TRY(eng->reports2.reserve((size_t) eng->cap_per_part * eng->n_parts * sizeof(gss_report)));
-        GSS_TRY(eng->reports3.reserve((size_t) eng->cap_per_part * eng->n_parts * sizeof(gss_report)));
+        GSS_TRY(reserve(eng->reports2, (size_t) eng->cap_per_part * eng->n_parts * sizeof(gss_report)));
+        GSS_TRY(reserve(eng->reports3, (size_t) eng->cap_per_part * eng->n_parts * sizeof(gss_report)));
         return GSS_OK;
     };
     GSS_TRY(reserve_reports());
@@ -1193,10 +1215,16 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
     GSS_TRY(eng->counts3.reserve(counter_bytes(eng->n_parts)));
     auto reserve_packed = [&]() -> int {
         for (int b = 0; b < NB && packed; b++)
-            GSS_TRY(eng->packed[b].reserve((size_t) eng->cap_per_part * eng->n_parts * rec_words * sizeof(uint32_t)));
+            GSS_TRY(reserve(eng->packed[b], (size_t) eng->cap_per_part * eng->n_parts * rec_words * sizeof(uint32_t)));
         return GSS_OK;
     };
     GSS_TRY(reserve_packed());
+    // The first state decides for all of them: a later one whose table keeps
+    // more costs time, not reports.
+    if (eng->filter) {
+        const size_t abytes = (size_t) eng->n_blocks * n_vars * 2 * sizeof(uint2);
+        if (eng->agg2.reserve(abytes) != GSS_OK || eng->agg3.reserve(abytes) != GSS_OK) eng->filter = false;
+    }
     // packs pass b's reports (after its check, on the engine stream)
     auto pack = [&](int b, const DevBuf &rep, const DevBuf &cnt) -> int {
         if (!packed) return GSS_OK;
@@ -1204,8 +1232,8 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
                                    eng->cap_per_part, format == kRecordsCells ? (uint32_t) n_words : 0u,
                                    (uint32_t *) eng->packed[b].ptr, eng->stream, eng->sm_count);
     };
-    GSS_TRY(eng->h_counts2.reserve(sizeof(uint32_t) * (eng->n_parts + 1)));
-    GSS_TRY(eng->h_counts3.reserve(sizeof(uint32_t) * (eng->n_parts + 1)));
+    GSS_TRY(eng->h_counts2.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
+    GSS_TRY(eng->h_counts3.reserve(sizeof(uint32_t) * (eng->n_parts + kExtraCounters)));
     DevBuf *state_buf[NB] = {&eng->state, &eng->state2, &eng->state3};
     DevBuf *agg_buf[NB] = {&eng->agg, &eng->agg2, &eng->agg3};
     DevBuf *raw_buf[NB] = {&eng->state_raw, &eng->state_raw2, &eng->state_raw3};

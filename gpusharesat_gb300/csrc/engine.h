@@ -67,6 +67,7 @@ struct gss_engine {
     int state_lpc = 0;  // lanes per clause
     int state_g = 2;
     int state_bw = 0;   // words per slot block
+    bool state_auto = false;  // the layout was chosen by the word count (GSS_KERNEL_AUTO)
 
     // report queues: n_parts partitions of cap_per_part records
     DevBuf reports, counts;

@@ -1202,6 +1202,10 @@ int Sharer::recover_from_oom() {
     out_of_memory_ = true;
     log(1, "c Ran out of GPU memory: reducing the GPU clause database\n");
     GSS_TRY(finish_pending());
+    // the filter's table goes too: passes run without it until the state's
+    // layout changes
+    agg_possible_ = agg_ok_ = false;
+    d_agg_.release();
     return reduce_now(false);  // an upload frees the old device buffers before allocating new ones
 }
 

@@ -161,3 +161,79 @@ def test_reports_do_not_depend_on_the_pause(lib):
         for f in ("clause", "word", "mask"):
             np.testing.assert_array_equal(got[f], ref[f], err_msg=f)
     eng.close()
+
+
+def test_masks_at_any_address(lib):
+    """Device masks that start between words are read as they are."""
+    import torch
+    import gpusharesat_gb300 as g
+    rng = np.random.default_rng(9)
+    n_vars, n_words = 400, 9
+    model = rng.integers(0, 2, n_vars).astype(np.uint8)
+    lits, offsets = _database(rng, 1500, n_vars, model)
+    state = _trail_state(rng, n_vars, n_words, model, flips=8)
+    start = rng.integers(0, 2 ** 32, n_words, dtype=np.uint32)
+    solver = rng.integers(0, 50, n_words).astype(np.int32)
+    ref = oracle.check(lits, offsets, state, start)
+    ds = torch.from_numpy(state.view(np.int32)).cuda()
+    for shift in (0, 1, 2, 3):
+        masks = [torch.zeros(4 * n_words + 4, dtype=torch.uint8, device="cuda") for _ in range(2)]
+        for m, src in zip(masks, (start, solver)):
+            m[shift:shift + 4 * n_words] = torch.from_numpy(src.view(np.uint8)).cuda()
+        eng = g.Engine(0)
+        eng.set_db(lits, offsets)
+        eng.set_state_device(ds.data_ptr(), n_vars, n_words, masks[0].data_ptr() + shift, masks[1].data_ptr() + shift)
+        got = g.sort_reports(eng.check())
+        assert len(got) == len(ref)
+        for f in ("clause", "word", "mask"):
+            np.testing.assert_array_equal(got[f], ref[f], err_msg=f)
+        np.testing.assert_array_equal(got["solver"], solver[got["word"]])
+        eng.close()
+
+
+def test_tables_make_room(lib):
+    """Without room for the queues the filter's table goes, not the pass."""
+    import gpusharesat_gb300 as g
+    rng = np.random.default_rng(10)
+    n_vars, n_words = 500, 40
+    model = rng.integers(0, 2, n_vars).astype(np.uint8)
+    lits, offsets = _database(rng, 2000, n_vars, model)
+    state = _trail_state(rng, n_vars, n_words, model, flips=8)
+    start = np.full(n_words, 0xFFFFFFFF, np.uint32)
+    eng = g.Engine(0)
+    eng.set_db(lits, offsets)
+    eng.set_state(state, start)
+    try:
+        g.debug_fail_device_alloc(1 << 23, 1)  # the queues, 16 MB
+        _same(eng, lits, offsets, state, start)
+        eng.set_state(state, start)
+        _same(eng, lits, offsets, state, start)
+        g.debug_fail_device_alloc(1 << 23, 2)  # with the table gone there is still no room
+        eng.set_capacity(1 << 22)
+        with pytest.raises(g.GssError):
+            eng.check()
+    finally:
+        g.debug_fail_device_alloc(0, 0)
+    _same(eng, lits, offsets, state, start)
+    eng.close()
+
+
+@pytest.mark.parametrize("n_words,ok", [(16, False), (17, False), (31, False), (32, True), (33, True)])
+def test_length_plan_wants_full_blocks(lib, n_words, ok):
+    import gpusharesat_gb300 as g
+    rng = np.random.default_rng(n_words)
+    n_vars = 300
+    model = rng.integers(0, 2, n_vars).astype(np.uint8)
+    lits, offsets = _database(rng, 500, n_vars, model)
+    state = _trail_state(rng, n_vars, n_words, model, flips=8)
+    start = np.full(n_words, 0xFFFFFFFF, np.uint32)
+    eng = g.Engine(0)
+    eng.set_db(lits, offsets)
+    eng.set_state(state, start)
+    eng.set_length_plan((4, 1 << 30), [g.LAYOUT_4x8_G2, g.LAYOUT_4x8_G1])
+    if ok:
+        _same(eng, lits, offsets, state, start)
+    else:
+        with pytest.raises(g.GssError):
+            eng.check()
+    eng.close()
