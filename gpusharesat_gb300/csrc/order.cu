@@ -533,22 +533,28 @@ __global__ void __launch_bounds__(4 * kReduceParams)
                         float *__restrict__ loss, float *__restrict__ w, float *__restrict__ m,
                         float *__restrict__ v, float lr, float c1, float c2) {
     __shared__ float sums[4][kReduceParams];
+    if (blockIdx.x == gridDim.x - 1) {
+        // the loss, thousands of rows' sum: a last bit in 32 bits is 1e-7 of it
+        // (one thread's 64-bit adds in the parameters' way took 3 us more)
+        if (threadIdx.x >= 32) return;
+        double l = 0.0;
+        for (uint32_t c = threadIdx.x; c < n_blocks; c += 32) l += (double) __ldg(partial + (size_t) c * (kP + 1) + kP);
+        for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(kFullMask, l, o);
+        if (threadIdx.x == 0) *loss = (float) (l / (double) B);
+        return;
+    }
     const int lp = threadIdx.x % kReduceParams, quarter = threadIdx.x / kReduceParams;
     const int p = blockIdx.x * kReduceParams + lp;
     const uint32_t per = (n_blocks + 3) / 4, from = min(quarter * per, n_blocks), to = min(from + per, n_blocks);
     float s = 0.0f;
-    if (p <= kP) {
+    if (p < kP) {
 #pragma unroll 32
         for (uint32_t c = from; c < to; c++) s += __ldg(partial + (size_t) c * (kP + 1) + p);
     }
     sums[quarter][lp] = s;
     __syncthreads();
-    if (quarter != 0 || p > kP) return;
+    if (quarter != 0 || p >= kP) return;
     s = (sums[0][lp] + sums[1][lp]) + (sums[2][lp] + sums[3][lp]);
-    if (p == kP) {
-        *loss = s / (float) B;
-        return;
-    }
     grad[p] = s;
     if (ADAM) {
         const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -616,7 +622,7 @@ int scorer_grad_dev(Scorer *s, const float *x, const float *y, uint32_t n_rows, 
         c2 = 1.0f - powf(0.999f, (float) s->adam_steps);
         s->frag_stale = true;
     }
-    constexpr unsigned reduce_blocks = (kP + kReduceParams) / kReduceParams;  // kP parameters and the loss
+    constexpr unsigned reduce_blocks = (kP + kReduceParams - 1) / kReduceParams + 1;  // the parameters', and the loss's
     (lr > 0.0f ? train_reduce_kernel<true> : train_reduce_kernel<false>)<<<reduce_blocks, 4 * kReduceParams, 0, stream>>>(
         partial, blocks, B, (float *) s->grad.ptr, (float *) s->loss.ptr, (float *) s->w.ptr, (float *) s->m.ptr,
         (float *) s->v.ptr, lr, c1, c2);
