@@ -237,7 +237,7 @@ int gss_engine_create(int device, gss_engine **out) {
     if (rc == GSS_OK) rc = eng->start.reserve(kMaxWords * sizeof(uint32_t));
     if (rc == GSS_OK) rc = eng->solver_of_word.reserve(kMaxWords * sizeof(int32_t));
     if (rc != GSS_OK) {
-        delete eng;
+        gss_engine_destroy(eng);
         return rc;
     }
     eng->stream = eng->own_stream;
