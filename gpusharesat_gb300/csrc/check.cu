@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_pf_kernel(CheckA
 constexpr uint32_t kUnit = 16;
 constexpr int kPersistStage = 192;
 
-template <int WPL, int LPC, int G, int MINB, bool DEV>
+template <int WPL, int LPC, int G, int MINB, bool DEV, bool WIDE_OUT = true>
 __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(const CheckArgs *__restrict__ pa,
                                                                                 const __grid_constant__ CheckArgs av,
                                                                                 uint32_t *__restrict__ work) {
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
                 const unsigned bal = __ballot_sync(kFull, live[j] != 0u);
                 if (bal) {
                     if (nstaged + 32 > (uint32_t) kPersistStage) {
-                        flush_mapped(a, stage, nstaged);
+                        flush_mapped<WIDE_OUT>(a, stage, nstaged);
                         nstaged = 0;
                     }
                     if (live[j])
@@ -592,22 +592,23 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
             }
         }
     }
-    if (nstaged) flush_mapped(a, stage, nstaged);
+    if (nstaged) flush_mapped<WIDE_OUT>(a, stage, nstaged);
 }
 
-template <int WPL, int LPC, int G>
+// WIDE_OUT: the queues lie on 16 bytes (see flush_mapped).
+template <int WPL, int LPC, int G, bool WIDE_OUT = true>
 int launch_wide_persist_variant(const CheckArgs *d_args, const CheckArgs &h_args, uint32_t *work, cudaStream_t stream,
                                 int sm_count) {
     constexpr int MINB = default_min_blocks(WPL, G);
-    static const int per_sm = resident_blocks(check_wide_persist_kernel<WPL, LPC, G, MINB, false>);
+    static const int per_sm = resident_blocks(check_wide_persist_kernel<WPL, LPC, G, MINB, false, WIDE_OUT>);
     uint64_t blocks = (uint64_t) sm_count * per_sm;
     if (d_args) {  // a captured graph serves databases of other sizes too: the full grid
-        check_wide_persist_kernel<WPL, LPC, G, MINB, true><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
+        check_wide_persist_kernel<WPL, LPC, G, MINB, true, WIDE_OUT><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
             d_args, h_args, work);
     } else {
         const uint64_t units = (uint64_t) ((scan_count(h_args) + kUnit - 1) / kUnit) * h_args.n_blocks;
         blocks = std::min<uint64_t>(blocks, std::max<uint64_t>((units + kWarps - 1) / kWarps, 1));
-        check_wide_persist_kernel<WPL, LPC, G, MINB, false><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
+        check_wide_persist_kernel<WPL, LPC, G, MINB, false, WIDE_OUT><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
             nullptr, h_args, work);
     }
     GSS_CUDA_TRY(cudaGetLastError());
@@ -818,12 +819,19 @@ extern "C" int gss_check_noalloc(const int32_t *lits, const int64_t *offsets, ui
         return set_error(GSS_ERR_INVALID, "gss_check_noalloc: %u clauses over 0 variables", n_clauses);
     if ((uint64_t) cap_per_part * n_parts > 0xFFFFFFFFull)
         return set_error(GSS_ERR_INVALID, "gss_check_noalloc: output capacity above 2^32 records");
+    // what the kernel reads and writes whole words of
+    const bool runs = n_clauses > 0 && n_blocks > 0;
+    const auto off = [](const void *p, uintptr_t align) { return ((uintptr_t) p & (align - 1)) != 0; };
+    if (runs && (off(lits, 4) || off(offsets, 8) || off(state, 32) || off(start, 4) || off(solver_of_word, 4) ||
+                 (cap_per_part > 0 && off(out, 4))))
+        return set_error(GSS_ERR_INVALID, "gss_check_noalloc: a misaligned buffer (offsets lie on 8 bytes, the state "
+                         "on 32, the others on 4)");
     cudaStream_t st = (cudaStream_t) stream;
     uint32_t *counters = nullptr;
     GSS_TRY(noalloc_counters(&counters));
     // every call starts from zeroed counters: they keep the previous call's values
     GSS_CUDA_TRY(cudaMemsetAsync(counters, 0, counter_bytes(n_parts, 1), st));
-    if (n_clauses > 0 && n_blocks > 0) {
+    if (runs) {
         int dev = 0, sms = 0;
         GSS_CUDA_TRY(cudaGetDevice(&dev));
         GSS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -847,7 +855,15 @@ extern "C" int gss_check_noalloc(const int32_t *lits, const int64_t *offsets, ui
         a.cap_per_part = cap_per_part;
         a.lpc = 8;
         a.g = 2;
-        GSS_TRY((launch_wide_persist_variant<4, 8, 2>(nullptr, a, work_counter(counters, n_parts), st, sms)));
+        // queues cut from the caller's pool may lie between 16-byte boundaries
+        uint32_t *const work = work_counter(counters, n_parts);
+        GSS_TRY(off(out, 16) ? (launch_wide_persist_variant<4, 8, 2, false>(nullptr, a, work, st, sms))
+                             : (launch_wide_persist_variant<4, 8, 2, true>(nullptr, a, work, st, sms)));
+    }
+    if (off(counts_out, 4)) {
+        GSS_CUDA_TRY(cudaMemcpy2DAsync(counts_out, sizeof(uint32_t), counters, kCountStride * sizeof(uint32_t),
+                                       sizeof(uint32_t), n_parts, cudaMemcpyDeviceToDevice, st));
+        return GSS_OK;
     }
     noalloc_counts_kernel<<<1, kNoAllocMaxParts, 0, st>>>(counters, n_parts, counts_out);
     GSS_CUDA_TRY(cudaGetLastError());

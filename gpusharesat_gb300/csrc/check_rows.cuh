@@ -53,10 +53,12 @@ __device__ __forceinline__ void flush_block_part(const CheckArgs &a, gss_report 
 
 // A record as the kernels stage it: the clause's position; flush_mapped turns
 // it into the clause's id (or leaves it, without an id map) and adds the
-// solver, 32 records at a time.
+// solver, 32 records at a time. WIDE: the queues lie on 16 bytes, as the
+// engine's do, and a record is one store; else it is four.
 __device__ __forceinline__ void stage_record(gss_report *to, uint32_t c, uint32_t word, uint32_t mask) {
     *reinterpret_cast<uint4 *>(to) = make_uint4(c, word, mask, 0u);
 }
+template <bool WIDE = true>
 __device__ __forceinline__ void flush_mapped(const CheckArgs &a, const gss_report *stage, uint32_t n) {
     const int lane = lane_id();
     const uint32_t part = blockIdx.x % a.n_parts;
@@ -69,7 +71,11 @@ __device__ __forceinline__ void flush_mapped(const CheckArgs &a, const gss_repor
         uint4 r = reinterpret_cast<const uint4 *>(stage)[i];  // {clause, word, mask, solver}
         if (a.orig) r.x = __ldg(a.orig + r.x);
         r.w = (uint32_t) __ldg(a.solver_of_word + r.y);
-        if (base + i < a.cap_per_part) reinterpret_cast<uint4 *>(out)[base + i] = r;
+        if (base + i >= a.cap_per_part) continue;
+        if (WIDE)
+            reinterpret_cast<uint4 *>(out)[base + i] = r;
+        else
+            out[base + i] = gss_report{r.x, r.y, r.z, r.w};
     }
     __syncwarp();
 }

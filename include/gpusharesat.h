@@ -294,7 +294,11 @@ int gss_probe_gather(int device, uint64_t buffer_bytes, int depth, int blocks_pe
  *   - start[] and solver_of_word[] hold n_blocks * 32 entries, start zero
  *     past the last real word (a padding word with start bits set reports).
  * The call itself refuses n_parts outside 1..64, n_clauses > 0 with
- * n_vars == 0, NULL pointers and an output capacity above 2^32 records.
+ * n_vars == 0, NULL pointers, an output capacity above 2^32 records and
+ * misaligned buffers: offsets lie on 8 bytes, state on 32 (a lane reads four
+ * words of a row at once), lits, start, solver_of_word and out on 4
+ * (counts_out may lie anywhere; records are written 16 bytes at a time where
+ * out lies on 16, 4 at a time elsewhere).
  * Outputs: out[n_parts * cap_per_part] report records, partition p holding
  * min(counts_out[p], cap_per_part) records from out + p * cap_per_part, with
  * `clause` the CSR index; counts_out[n_parts]. A count above cap_per_part

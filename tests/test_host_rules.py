@@ -1,8 +1,10 @@
 """What the library's host code decides, over a CUDA runtime without a GPU
 (fake_runtime.py)."""
+import ctypes
+
 import pytest
 
-from fake_runtime import Fake
+from fake_runtime import Fake, i64, vp
 
 
 @pytest.fixture(scope="module")
@@ -30,3 +32,35 @@ def test_engine_that_cannot_be_made_leaves_no_stream(fake, what):
         assert fake.lib.fake_streams() == before
     fake.fail(what)
     assert fake.engine()[0] != 0
+
+
+def _noalloc(fake, lits=0, offsets=0, state=0, start=0, sow=0, out=0, counts=0, n=100):
+    """One pass over buffers shifted by so many bytes; nothing is read."""
+    room = ctypes.create_string_buffer(1 << 16)
+    base = (ctypes.addressof(room) + 255) // 256 * 256
+    p = [vp(base + 4096 * k + s) for k, s in enumerate((lits, offsets, state, start, sow, out, counts))]
+    fake.reset()
+    rc = fake.lib.gss_check_noalloc(p[0], p[1], n, p[2], 10, 1, p[3], p[4], p[5], 4, 16, p[6], None)
+    return rc, [l.split()[1] for l in fake.log() if l.startswith("launch")], fake.log()
+
+
+def test_noalloc_queue_address_picks_the_stores(fake):
+    """A 16-byte store needs a queue on 16 bytes; a gss_report needs 4."""
+    rc, wide, _ = _noalloc(fake)
+    assert rc == 0 and len(wide) == 2 and "check_wide_persist" in wide[0]
+    assert _noalloc(fake, out=16)[1] == wide and _noalloc(fake, out=32)[1] == wide
+    by_word = set()
+    for shift in (4, 8, 12, 20):
+        rc, names, _ = _noalloc(fake, out=shift)
+        assert rc == 0 and "check_wide_persist" in names[0]
+        by_word.add(names[0])
+    assert len(by_word) == 1 and wide[0] not in by_word
+
+
+def test_noalloc_refuses_what_the_kernel_cannot_read(fake):
+    for kw in ({"state": 8}, {"state": 16}, {"lits": 2}, {"offsets": 4}, {"start": 1}, {"sow": 2}, {"out": 2}):
+        rc, names, _ = _noalloc(fake, **kw)
+        assert rc == -1 and not names, kw
+        assert _noalloc(fake, n=0, **kw)[0] == 0  # nothing to read
+    rc, names, log = _noalloc(fake, counts=1)  # copied, not stored by a kernel
+    assert rc == 0 and len(names) == 1 and any(l.startswith("copy2d") for l in log)
