@@ -87,13 +87,13 @@ __global__ void __launch_bounds__(kWarps * 32) check_kernel(CheckArgs a) {
     static_assert(LPC == 1 || LPC == 2 || LPC == 4 || LPC == 8 || LPC == 16 || LPC == 32, "lanes per clause");
     static_assert(G >= 1 && G <= LPC, "prefetch depth");
     constexpr int CPW = 32 / LPC;  // clauses per warp
-    __shared__ gss_report stage_all[kWarps][kStage];
+    __shared__ StagedReport stage_all[kWarps][kStage];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int sub = lane % LPC;     // word within the slot block
     const int grp = lane / LPC;     // clause within the warp
     const int gbase = grp * LPC;    // first lane of this clause group
-    gss_report *stage = stage_all[wib];
+    StagedReport *stage = stage_all[wib];
     const uint32_t part = blockIdx.x % a.n_parts;
     gss_report *out = a.out + (size_t) part * a.cap_per_part;
     uint32_t *counter = a.counts + (size_t) part * a.count_stride;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kWarps * 32) check_kernel(CheckArgs a) {
                 r.word = w;
                 r.mask = rep;
                 r.solver = (uint32_t) __ldg(a.solver_of_word + w);
-                stage[nstaged + __popc(bal & lanemask_lt())] = r;
+                stage[nstaged + __popc(bal & lanemask_lt())] = StagedReport{r};
             }
             nstaged += __popc(bal);
         }
@@ -220,13 +220,13 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_kernel(CheckArgs
     constexpr int CPW = 32 / LPC;
     constexpr int BW = WPL * LPC;
     static_assert(G >= 1 && G <= LPC, "depth");
-    __shared__ gss_report stage_all[kWarps][kStage];
+    __shared__ StagedReport stage_all[kWarps][kStage];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int sub = lane % LPC;
     const int grp = lane / LPC;
     const int gbase = grp * LPC;
-    gss_report *stage = stage_all[wib];
+    StagedReport *stage = stage_all[wib];
     const uint32_t part = blockIdx.x % a.n_parts;
     gss_report *out = a.out + (size_t) part * a.cap_per_part;
     uint32_t *counter = a.counts + (size_t) part * a.count_stride;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_kernel(CheckArgs
                     r.word = w0 + j;
                     r.mask = rep;
                     r.solver = (uint32_t) __ldg(a.solver_of_word + w0 + j);
-                    stage[nstaged + __popc(bal & lanemask_lt())] = r;
+                    stage[nstaged + __popc(bal & lanemask_lt())] = StagedReport{r};
                 }
                 nstaged += __popc(bal);
             }
@@ -342,13 +342,13 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_pf_kernel(CheckA
     constexpr int CPW = 32 / LPC;
     constexpr int BW = WPL * LPC;
     static_assert(G >= 1 && G <= LPC, "depth");
-    __shared__ gss_report stage_all[kWarps][kStage];
+    __shared__ StagedReport stage_all[kWarps][kStage];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int sub = lane % LPC;
     const int grp = lane / LPC;
     const int gbase = grp * LPC;
-    gss_report *stage = stage_all[wib];
+    StagedReport *stage = stage_all[wib];
     const uint32_t part = blockIdx.x % a.n_parts;
     gss_report *out = a.out + (size_t) part * a.cap_per_part;
     uint32_t *counter = a.counts + (size_t) part * a.count_stride;
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_pf_kernel(CheckA
                     r.word = w0 + j;
                     r.mask = rep;
                     r.solver = (uint32_t) __ldg(a.solver_of_word + w0 + j);
-                    stage[nstaged + __popc(bal & lanemask_lt())] = r;
+                    stage[nstaged + __popc(bal & lanemask_lt())] = StagedReport{r};
                 }
                 nstaged += __popc(bal);
             }
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
     constexpr int CPW = 32 / LPC;
     constexpr int BW = WPL * LPC;
     __shared__ CheckArgs sa;
-    __shared__ gss_report stage_all[kWarps][kPersistStage];
+    __shared__ StagedReport stage_all[kWarps][kPersistStage];
     __shared__ uint4 unit_all[kWarps][kUnit];
     if (threadIdx.x == 0) sa = DEV ? *pa : av;
     __syncthreads();
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_wide_persist_kernel(c
     const int sub = lane % LPC;
     const int grp = lane / LPC;
     const int gbase = grp * LPC;
-    gss_report *stage = stage_all[threadIdx.x >> 5];
+    StagedReport *stage = stage_all[threadIdx.x >> 5];
     uint4 *const unit_clauses = unit_all[threadIdx.x >> 5];
     uint32_t nstaged = 0;
 

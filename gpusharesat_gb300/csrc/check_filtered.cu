@@ -89,7 +89,7 @@ __device__ __forceinline__ uint32_t finish_clauses(const int32_t *__restrict__ l
 // word-level bits could not tell from them) are checked literal-parallel;
 // otherwise groups of LPC lanes scan them as the plain wide kernel does.
 template <int WPL, int LPC, int G>
-__device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, gss_report *stage, uint32_t nstaged, uint32_t blk,
+__device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, StagedReport *stage, uint32_t nstaged, uint32_t blk,
                                                  uint32_t c, uint32_t live) {
     constexpr int CPW = 32 / LPC;
     constexpr int BW = WPL * LPC;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_filtered_kernel(const
                                                                             uint32_t *__restrict__ work) {
     constexpr int BW = WPL * LPC;
     __shared__ CheckArgs sa;
-    __shared__ gss_report stage_all[kWarps][kFilterStage];
+    __shared__ StagedReport stage_all[kWarps][kFilterStage];
     __shared__ uint32_t survivors;
     if (threadIdx.x == 0) {
         sa = pa ? *pa : av;
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_filtered_kernel(const
     __syncthreads();
     const CheckArgs &a = sa;
     const int lane = threadIdx.x & 31;
-    gss_report *stage = stage_all[threadIdx.x >> 5];
+    StagedReport *stage = stage_all[threadIdx.x >> 5];
     uint32_t nstaged = 0, kept = 0;
 
     const uint32_t n_scan = scan_count(a);

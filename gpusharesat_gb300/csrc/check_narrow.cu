@@ -44,9 +44,9 @@ __device__ __forceinline__ void ld_narrow<4>(const uint2 *p, Row<4> &r) {
 template <int NW, int MINB>
 __global__ void __launch_bounds__(kWarps * 32, MINB) check_narrow_kernel(const CheckArgs a,
                                                                           uint32_t *__restrict__ work) {
-    __shared__ gss_report stage_all[kWarps][kStage];
+    __shared__ StagedReport stage_all[kWarps][kStage];
     const int lane = threadIdx.x & 31;
-    gss_report *stage = stage_all[threadIdx.x >> 5];
+    StagedReport *stage = stage_all[threadIdx.x >> 5];
     uint32_t nstaged = 0;
     const uint32_t n_scan = scan_count(a);
     const uint32_t n_tasks = (n_scan + 31) / 32;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_narrow_kernel(const C
                     rep.word = j;
                     rep.mask = live[j];
                     rep.solver = (uint32_t) __ldg(a.solver_of_word + j);
-                    stage[nstaged + __popc(bal & lanemask_lt())] = rep;
+                    stage[nstaged + __popc(bal & lanemask_lt())] = StagedReport{rep};
                 }
                 nstaged += __popc(bal);
             }

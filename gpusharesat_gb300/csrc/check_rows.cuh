@@ -17,10 +17,16 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
+// A report record in a warp's stage in shared memory: read and written 16
+// bytes at a time, so the type says where it lies (gss_report itself has the
+// alignment of its words).
+struct alignas(16) StagedReport : gss_report {};
+static_assert(sizeof(StagedReport) == sizeof(gss_report) && sizeof(gss_report) == sizeof(uint4), "a record is 16 bytes");
+
 // Writes a warp's staged records: one atomic reservation, then the records.
 // streaming = cache-streaming stores (the records are read back by the host,
 // not by the kernel: they need not displace state rows from L2).
-__device__ __forceinline__ void flush_stage(gss_report *stage, uint32_t n, gss_report *out, uint32_t *counter,
+__device__ __forceinline__ void flush_stage(const StagedReport *stage, uint32_t n, gss_report *out, uint32_t *counter,
                                             uint32_t cap, int lane, bool streaming = false) {
     __syncwarp();
     uint32_t base = 0;
@@ -45,7 +51,7 @@ __device__ __forceinline__ int lane_id() {
 }
 
 // Flushes a warp's stage into its block's partition.
-__device__ __forceinline__ void flush_block_part(const CheckArgs &a, gss_report *stage, uint32_t n) {
+__device__ __forceinline__ void flush_block_part(const CheckArgs &a, const StagedReport *stage, uint32_t n) {
     const uint32_t part = blockIdx.x % a.n_parts;
     flush_stage(stage, n, a.out + (size_t) part * a.cap_per_part, a.counts + (size_t) part * a.count_stride,
                 a.cap_per_part, lane_id());
@@ -55,11 +61,11 @@ __device__ __forceinline__ void flush_block_part(const CheckArgs &a, gss_report 
 // it into the clause's id (or leaves it, without an id map) and adds the
 // solver, 32 records at a time. WIDE: the queues lie on 16 bytes, as the
 // engine's do, and a record is one store; else it is four.
-__device__ __forceinline__ void stage_record(gss_report *to, uint32_t c, uint32_t word, uint32_t mask) {
+__device__ __forceinline__ void stage_record(StagedReport *to, uint32_t c, uint32_t word, uint32_t mask) {
     *reinterpret_cast<uint4 *>(to) = make_uint4(c, word, mask, 0u);
 }
 template <bool WIDE = true>
-__device__ __forceinline__ void flush_mapped(const CheckArgs &a, const gss_report *stage, uint32_t n) {
+__device__ __forceinline__ void flush_mapped(const CheckArgs &a, const StagedReport *stage, uint32_t n) {
     const int lane = lane_id();
     const uint32_t part = blockIdx.x % a.n_parts;
     __syncwarp();

@@ -1,8 +1,12 @@
 """What the library's host code decides, over a CUDA runtime without a GPU
 (fake_runtime.py)."""
 import ctypes
+import os
+import subprocess
 
 import pytest
+
+from gpusharesat_gb300 import build
 
 from fake_runtime import Fake, i64, vp
 
@@ -64,3 +68,10 @@ def test_noalloc_refuses_what_the_kernel_cannot_read(fake):
         assert _noalloc(fake, n=0, **kw)[0] == 0  # nothing to read
     rc, names, log = _noalloc(fake, counts=1)  # copied, not stored by a kernel
     assert rc == 0 and len(names) == 1 and any(l.startswith("copy2d") for l in log)
+
+
+def test_staged_records_lie_on_16_bytes_by_type(tmp_path):
+    here = os.path.dirname(os.path.abspath(__file__))
+    subprocess.run([build._nvcc(), *build.ARCH, "-std=c++17", "-I", os.path.join(build.ROOT, "include"), "-I",
+                    build.CSRC, "-c", os.path.join(here, "cpp", "stage_alignment.cu"), "-o",
+                    str(tmp_path / "stage_alignment.o")], check=True)
