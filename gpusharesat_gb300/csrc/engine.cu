@@ -644,13 +644,26 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     const int padded = n_blocks * bw;
     const size_t sbytes = (size_t) n_vars * n_words * 2 * sizeof(uint32_t);
     const size_t bbytes = (size_t) n_blocks * n_vars * bw * 2 * sizeof(uint32_t);
+    // Kernels read the caller's state and masks where they are whole words of
+    // this GPU's memory; what lies otherwise, or on another GPU, is copied
+    // (copies need no peer access).
+    bool read_state = on_device, read_masks = on_device;
+    const void *const given[3] = {state, start, solver_of_word};
+    for (int k = 0; k < 3 && on_device && n_words; k++) {
+        if (given[k] == nullptr || (k == 0 && sbytes == 0)) continue;
+        cudaPointerAttributes at;
+        GSS_CUDA_TRY(cudaPointerGetAttributes(&at, given[k]));
+        if (at.devicePointer == nullptr)
+            return set_error(GSS_ERR_CUDA, "gss_state_set: a pointer that the device cannot read");
+        if (at.device != eng->device || ((uintptr_t) given[k] & (k == 0 ? 7 : 3)) != 0)
+            (k == 0 ? read_state : read_masks) = false;
+    }
     if (eng->pass_pending) GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
     GSS_TRY(reserve_over_table(eng, eng->state, std::max<size_t>(bbytes, 8)));
     GSS_TRY(eng->start.reserve(std::max<size_t>(padded * sizeof(uint32_t), 4)));
     GSS_TRY(eng->solver_of_word.reserve(std::max<size_t>(padded * sizeof(int32_t), 4)));
     const bool laid_out = n_blocks == 1 && n_words == bw;  // block-major and host layouts coincide
-    const bool aligned = on_device && ((uintptr_t) state & 7) == 0;  // the copy kernel reads it as it is
-    if (sbytes && !laid_out && !aligned) GSS_TRY(reserve_over_table(eng, eng->state_raw, sbytes));
+    if (sbytes && !laid_out && !read_state) GSS_TRY(reserve_over_table(eng, eng->state_raw, sbytes));
     // the filter's table: only the automatic variant runs behind it; without
     // room for it the passes run without
     const bool want_agg = eng->kind == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && sbytes > 0;
@@ -668,40 +681,27 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     // start and solver_of_word, padded with zero words
     std::vector<uint32_t> st;
     std::vector<int32_t> sw;
-    if (on_device) {
+    if (on_device && n_words) {
         // in order behind what the caller queued on the default stream
-        const void *read[3] = {start, solver_of_word, sbytes ? (const void *) state : nullptr};
-        for (const void *p : read) {
-            cudaPointerAttributes at;
-            if (p == nullptr || n_words == 0) continue;
-            GSS_CUDA_TRY(cudaPointerGetAttributes(&at, p));
-            if (at.devicePointer == nullptr)
-                return set_error(GSS_ERR_CUDA, "gss_state_set: a pointer that the device cannot read");
-        }
-        if (n_words) {
-            if (!eng->ev_caller) GSS_CUDA_TRY(cudaEventCreateWithFlags(&eng->ev_caller, cudaEventDisableTiming));
-            GSS_CUDA_TRY(cudaEventRecord(eng->ev_caller, cudaStreamLegacy));
-            GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_caller, 0));
-        }
-        // masks that are no whole words in memory go through a copy
-        const uint32_t *m = start;
-        const int32_t *sow = solver_of_word;
-        if (n_words && ((uintptr_t) m & 3)) {
-            GSS_CUDA_TRY(cudaMemcpyAsync(eng->start.ptr, m, n_words * sizeof(uint32_t), cudaMemcpyDefault, eng->stream));
-            m = (const uint32_t *) eng->start.ptr;
-        }
-        if (n_words && ((uintptr_t) sow & 3)) {
-            GSS_CUDA_TRY(cudaMemcpyAsync(eng->solver_of_word.ptr, sow, n_words * sizeof(int32_t), cudaMemcpyDefault,
-                                         eng->stream));
-            sow = (const int32_t *) eng->solver_of_word.ptr;
-        }
-        GSS_TRY(launch_load_masks(m, sow, (uint32_t) n_words, (uint32_t) padded, (uint32_t *) eng->start.ptr,
-                                  (int32_t *) eng->solver_of_word.ptr, eng->stream));
+        if (!eng->ev_caller) GSS_CUDA_TRY(cudaEventCreateWithFlags(&eng->ev_caller, cudaEventDisableTiming));
+        GSS_CUDA_TRY(cudaEventRecord(eng->ev_caller, cudaStreamLegacy));
+        GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_caller, 0));
+    }
+    if (read_masks) {
+        GSS_TRY(launch_load_masks(start, solver_of_word, (uint32_t) n_words, (uint32_t) padded,
+                                  (uint32_t *) eng->start.ptr, (int32_t *) eng->solver_of_word.ptr, eng->stream));
     } else if (padded) {
         st.assign(padded, 0u);
         sw.assign(padded, 0);
-        memcpy(st.data(), start, n_words * sizeof(uint32_t));
-        for (int w = 0; w < n_words; w++) sw[w] = solver_of_word ? solver_of_word[w] : w;
+        for (int w = 0; w < n_words; w++) sw[w] = w;
+        for (const auto &m : {std::make_pair((void *) st.data(), (const void *) start),
+                              std::make_pair((void *) sw.data(), (const void *) solver_of_word)}) {
+            if (m.second == nullptr) continue;
+            if (on_device)
+                GSS_CUDA_TRY(cudaMemcpy(m.first, m.second, n_words * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+            else
+                memcpy(m.first, m.second, n_words * sizeof(uint32_t));
+        }
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->start.ptr, st.data(), padded * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                      eng->stream));
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->solver_of_word.ptr, sw.data(), padded * sizeof(int32_t),
@@ -710,10 +710,10 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     if (sbytes) {
         const cudaMemcpyKind dir = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         const uint2 *src = (const uint2 *) state;
-        if (laid_out && !(aligned && filtered)) {
+        if (laid_out && !(read_state && filtered)) {
             GSS_CUDA_TRY(cudaMemcpyAsync(eng->state.ptr, state, sbytes, dir, eng->stream));
             src = (const uint2 *) eng->state.ptr;
-        } else if (!aligned) {
+        } else if (!read_state) {
             GSS_CUDA_TRY(cudaMemcpyAsync(eng->state_raw.ptr, state, sbytes, dir, eng->stream));
             src = (const uint2 *) eng->state_raw.ptr;
         }

@@ -70,6 +70,41 @@ def test_noalloc_refuses_what_the_kernel_cannot_read(fake):
     assert rc == 0 and len(names) == 1 and any(l.startswith("copy2d") for l in log)
 
 
+def _read_by_kernels(fake):
+    """The first two addresses given to the kernels that load states and masks."""
+    return {int(a, 16) for l in fake.log() if l.startswith("launch") and "load_" in l for a in l.split()[2:4]}
+
+
+@pytest.mark.parametrize("n_words", [1, 3, 8, 32, 33, 64])
+def test_buffers_of_another_gpu_are_copied(fake, n_words):
+    """No kernel reads a buffer on another GPU, nor words that are none; the
+    copies take them. On the engine's own GPU the kernels read them."""
+    n_vars = 50
+    room = ctypes.create_string_buffer(1 << 16)
+    base = (ctypes.addressof(room) + 255) // 256 * 256
+    at = [base, base + (1 << 15), base + (1 << 15) + 1024]  # state, start, solver words
+    rc, eng = fake.engine()
+    assert rc == 0
+
+    def load(far=None, shift=(0, 0, 0)):
+        fake.reset()
+        p = [a + s for a, s in zip(at, shift)]
+        if far is not None:
+            fake.lib.fake_far(vp(p[far]), 512)
+        assert fake.lib.gss_state_set(eng, vp(p[0]), i64(n_vars), n_words, vp(p[1]), vp(p[2]), 1) == 0, fake.error()
+        copied = {int(l.split()[2], 16) for l in fake.log() if l.startswith("copy")}
+        return p, _read_by_kernels(fake), copied
+
+    for far, shift in ((0, (0, 0, 0)), (1, (0, 0, 0)), (2, (0, 0, 0)), (None, (4, 0, 0)), (None, (0, 1, 0)),
+                       (None, (0, 0, 2))):
+        k = far if far is not None else [i for i in range(3) if shift[i]][0]
+        p, read, copied = load(far, shift)
+        assert p[k] not in read and p[k] in copied, (far, shift)
+    p, read, copied = load()
+    assert p[1] in read and p[2] in read and (p[0] in read) != (p[0] in copied)
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
 def test_staged_records_lie_on_16_bytes_by_type(tmp_path):
     here = os.path.dirname(os.path.abspath(__file__))
     subprocess.run([build._nvcc(), *build.ARCH, "-std=c++17", "-I", os.path.join(build.ROOT, "include"), "-I",
