@@ -600,7 +600,9 @@ template <int WPL, int LPC, int G, bool WIDE_OUT = true>
 int launch_wide_persist_variant(const CheckArgs *d_args, const CheckArgs &h_args, uint32_t *work, cudaStream_t stream,
                                 int sm_count) {
     constexpr int MINB = default_min_blocks(WPL, G);
-    static const int per_sm = resident_blocks(check_wide_persist_kernel<WPL, LPC, G, MINB, false, WIDE_OUT>);
+    static std::atomic<int> known{0};
+    int per_sm = 0;
+    GSS_TRY((resident_blocks(check_wide_persist_kernel<WPL, LPC, G, MINB, false, WIDE_OUT>, known, per_sm)));
     uint64_t blocks = (uint64_t) sm_count * per_sm;
     if (d_args) {  // a captured graph serves databases of other sizes too: the full grid
         check_wide_persist_kernel<WPL, LPC, G, MINB, true, WIDE_OUT><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(
@@ -617,7 +619,9 @@ int launch_wide_persist_variant(const CheckArgs *d_args, const CheckArgs &h_args
 
 template <int WPL, int LPC, int G, int MINB>
 int launch_wide_pf_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
-    static const int per_sm = resident_blocks(check_wide_pf_kernel<WPL, LPC, G, MINB>);
+    static std::atomic<int> known{0};
+    int per_sm = 0;
+    GSS_TRY((resident_blocks(check_wide_pf_kernel<WPL, LPC, G, MINB>, known, per_sm)));
     constexpr int CPW = 32 / LPC;
     const uint64_t n_tasks = (uint64_t) ((scan_count(a) + CPW - 1) / CPW) * a.n_blocks;
     uint64_t blocks = (uint64_t) sm_count * per_sm;
@@ -631,7 +635,9 @@ int launch_wide_pf_variant(const CheckArgs &a, cudaStream_t stream, int sm_count
 
 template <int WPL, int LPC, int G, int MINB, bool HINT = false>
 int launch_wide_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
-    static const int per_sm = resident_blocks(check_wide_kernel<WPL, LPC, G, MINB, HINT>);
+    static std::atomic<int> known{0};
+    int per_sm = 0;
+    GSS_TRY((resident_blocks(check_wide_kernel<WPL, LPC, G, MINB, HINT>, known, per_sm)));
     constexpr int CPW = 32 / LPC;
     const uint64_t n_tasks = (uint64_t) ((scan_count(a) + CPW - 1) / CPW) * a.n_blocks;
     uint64_t blocks = (uint64_t) sm_count * per_sm;
@@ -645,7 +651,9 @@ int launch_wide_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
 
 template <int LPC, int G>
 int launch_variant(const CheckArgs &a, cudaStream_t stream, int sm_count) {
-    static const int per_sm = resident_blocks(check_kernel<LPC, G>);
+    static std::atomic<int> known{0};
+    int per_sm = 0;
+    GSS_TRY((resident_blocks(check_kernel<LPC, G>, known, per_sm)));
     constexpr int CPW = 32 / LPC;
     const uint64_t n_tasks = (uint64_t) ((scan_count(a) + CPW - 1) / CPW) * a.n_blocks;
     uint64_t blocks = (uint64_t) sm_count * per_sm;

@@ -228,7 +228,9 @@ int layout_lanes(int layout) {
 
 int launch_check_bucketed(const CheckArgs *d_args, const BucketPlan *d_plan, uint32_t *work, cudaStream_t stream,
                           int sm_count) {
-    static const int per_sm = resident_blocks(check_bucketed_kernel);
+    static std::atomic<int> known{0};
+    int per_sm = 0;
+    GSS_TRY((resident_blocks(check_bucketed_kernel, known, per_sm)));
     check_bucketed_kernel<<<(unsigned) (sm_count * per_sm), kWarps * 32, 0, stream>>>(d_args, d_plan, work);
     GSS_CUDA_TRY(cudaGetLastError());
     return GSS_OK;

@@ -440,7 +440,9 @@ template <int WPL, int LPC, int G>
 int launch_filtered_variant(const CheckArgs *d_args, const CheckArgs &h_args, uint32_t *work, cudaStream_t stream,
                             int sm_count) {
     constexpr int MINB = 4;
-    static const int per_sm = resident_blocks(check_filtered_kernel<WPL, LPC, G, MINB>);
+    static std::atomic<int> known{0};
+    int per_sm = 0;
+    GSS_TRY((resident_blocks(check_filtered_kernel<WPL, LPC, G, MINB>, known, per_sm)));
     // a captured graph serves databases of other sizes too: the full grid
     uint64_t blocks = (uint64_t) sm_count * per_sm;
     if (!d_args) {

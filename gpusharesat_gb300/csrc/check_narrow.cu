@@ -187,7 +187,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) check_narrow_kernel(const C
 
 template <int NW, int MINB>
 int launch_narrow_variant(const CheckArgs &a, uint32_t *work, cudaStream_t stream, int sm_count) {
-    static const int per_sm = resident_blocks(check_narrow_kernel<NW, MINB>);
+    static std::atomic<int> known{0};
+    int per_sm = 0;
+    GSS_TRY((resident_blocks(check_narrow_kernel<NW, MINB>, known, per_sm)));
     const uint64_t n_tasks = ((uint64_t) scan_count(a) + 31) / 32;
     const uint64_t blocks = std::min<uint64_t>((uint64_t) sm_count * per_sm, (n_tasks + kWarps - 1) / kWarps);
     check_narrow_kernel<NW, MINB><<<(unsigned) blocks, kWarps * 32, 0, stream>>>(a, work);

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <atomic>
 #include <string>
 
 #include "gpusharesat.h"
@@ -236,16 +238,22 @@ inline void auto_layout(int n_words, int &kind, int &lpc, int &depth) {
     depth = lpc == 1 ? 1 : 2;
 }
 
-// Resident blocks of 256 threads per multiprocessor of a kernel; for a static
-// in its launcher (asked of the runtime once, not at every launch).
+// Resident blocks of 256 threads per multiprocessor of a kernel; `known` is a
+// static of its launcher (asked of the runtime once, not at every launch; an
+// error is the call's, and the next one asks again).
 template <typename K>
-int resident_blocks(K kernel) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 256, 0) != cudaSuccess) {
-        cudaGetLastError();
-        return 1;
+int resident_blocks(K kernel, std::atomic<int> &known, int &n) {
+    n = known.load(std::memory_order_relaxed);
+    if (n > 0) return GSS_OK;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 256, 0);
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // said here; not to be met again after the next launch
+        return set_error(GSS_ERR_CUDA, "cudaOccupancyMaxActiveBlocksPerMultiprocessor failed: %s",
+                         cudaGetErrorString(e));
     }
-    return n < 1 ? 1 : n;
+    if (n < 1) n = 1;
+    known.store(n, std::memory_order_relaxed);
+    return GSS_OK;
 }
 
 // Launches the check kernel on `stream` (the counters must already be zero).

@@ -105,6 +105,36 @@ def test_buffers_of_another_gpu_are_copied(fake, n_words):
     assert fake.lib.gss_engine_destroy(eng) == 0
 
 
+def _database(fake, eng, n=100, n_vars=50):
+    lits = (ctypes.c_int32 * (2 * n))(*[2 * (k % n_vars) + k // n_vars % 2 for k in range(2 * n)])
+    offsets = (i64 * (n + 1))(*range(0, 2 * n + 1, 2))
+    assert fake.lib.gss_db_set(eng, lits, offsets, i64(n)) == 0, fake.error()
+
+
+def _state(fake, eng, n_words, n_vars=50):
+    state = (ctypes.c_uint32 * (2 * n_vars * n_words))()
+    start = (ctypes.c_uint32 * n_words)(*[0xFFFFFFFF] * n_words)
+    assert fake.lib.gss_state_set(eng, state, i64(n_vars), n_words, start, None, 0) == 0, fake.error()
+
+
+@pytest.mark.parametrize("n_words", [2, 20])
+def test_launcher_reports_the_runtime_error_and_asks_again(tmp_path, n_words):
+    """A library of its own: the launchers keep what they learned."""
+    fake = Fake(tmp_path)
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    _state(fake, eng, n_words)
+    fake.fail("occupancy")
+    assert fake.lib.gss_check_launch(eng) == -2 and "Occupancy" in fake.error()
+    for _ in range(2):
+        assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+        assert fake.lib.gss_check_wait(eng, None) == 0
+    assert fake.log().count("occupancy") == 2  # refused, answered; not asked a third time
+    checks = [l for l in fake.log() if "check_narrow_kernel" in l or "check_filtered_kernel" in l]
+    assert len(checks) == 2
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
 def test_staged_records_lie_on_16_bytes_by_type(tmp_path):
     here = os.path.dirname(os.path.abspath(__file__))
     subprocess.run([build._nvcc(), *build.ARCH, "-std=c++17", "-I", os.path.join(build.ROOT, "include"), "-I",
