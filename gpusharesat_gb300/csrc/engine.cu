@@ -141,6 +141,13 @@ int range_shift_for(int64_t max_var, int range_log2) {
     return shift;
 }
 
+bool release_tables(gss_engine *eng) {
+    if (!eng->agg.ptr && !eng->agg2.ptr && !eng->agg3.ptr) return false;
+    cudaStreamSynchronize(eng->stream);  // a pass in flight may be reading them
+    eng->filter = false;
+    for (DevBuf *t : {&eng->agg, &eng->agg2, &eng->agg3}) t->release();
+    return true;
+}
 
 }  // namespace gss
 
@@ -163,17 +170,6 @@ bool use_filter(uint64_t n_false, double pairs) { return pairs > 0 && (double) n
 int ensure_device(gss_engine *eng) {
     GSS_CUDA_TRY(cudaSetDevice(eng->device));
     return GSS_OK;
-}
-
-// A buffer that a pass cannot do without; the filter's tables, which it can,
-// make room for it where the device has no other.
-int reserve_over_table(gss_engine *eng, DevBuf &buf, size_t bytes) {
-    const int rc = buf.reserve(bytes);
-    if (rc != GSS_ERR_NOMEM || !(eng->agg.ptr || eng->agg2.ptr || eng->agg3.ptr)) return rc;
-    GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
-    eng->filter = false;
-    for (DevBuf *t : {&eng->agg, &eng->agg2, &eng->agg3}) t->release();
-    return buf.reserve(bytes);
 }
 
 int ensure_queues(gss_engine *eng) {
@@ -236,6 +232,7 @@ int gss_engine_create(int device, gss_engine **out) {
     if (rc == GSS_OK) rc = eng->counts.reserve(counter_bytes(eng->n_parts));
     if (rc == GSS_OK) rc = eng->start.reserve(kMaxWords * sizeof(uint32_t));
     if (rc == GSS_OK) rc = eng->solver_of_word.reserve(kMaxWords * sizeof(int32_t));
+    if (rc == GSS_OK) rc = eng->d_args.reserve(sizeof(CheckArgs));
     if (rc != GSS_OK) {
         gss_engine_destroy(eng);
         return rc;
@@ -359,8 +356,8 @@ int upload_tiles(gss_engine *eng) {
     }
     tclause.push_back((uint32_t) n);
     tlit.push_back((uint32_t) eng->h_off[n]);
-    GSS_TRY(eng->tile_clause.reserve(tclause.size() * sizeof(uint32_t)));
-    GSS_TRY(eng->tile_lit.reserve(tlit.size() * sizeof(uint32_t)));
+    GSS_TRY(reserve_over_table(eng, eng->tile_clause, tclause.size() * sizeof(uint32_t)));
+    GSS_TRY(reserve_over_table(eng, eng->tile_lit, tlit.size() * sizeof(uint32_t)));
     GSS_CUDA_TRY(cudaMemcpy(eng->tile_clause.ptr, tclause.data(), tclause.size() * sizeof(uint32_t),
                             cudaMemcpyHostToDevice));
     GSS_CUDA_TRY(cudaMemcpy(eng->tile_lit.ptr, tlit.data(), tlit.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -376,10 +373,10 @@ int upload_all(gss_engine *eng) {
     GSS_TRY(ensure_device(eng));
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
     // 8 literals of zero padding: tile copies round their end up to 16 bytes
-    GSS_TRY(eng->lits.reserve((n_lits + 8) * sizeof(int32_t)));
+    GSS_TRY(reserve_over_table(eng, eng->lits, (n_lits + 8) * sizeof(int32_t)));
     GSS_CUDA_TRY(cudaMemset(eng->lits.ptr, 0, (n_lits + 8) * sizeof(int32_t)));
-    GSS_TRY(eng->offsets.reserve((n + 1) * sizeof(int64_t)));
-    GSS_TRY(eng->orig.reserve(std::max<int64_t>(n, 1) * sizeof(uint32_t)));
+    GSS_TRY(reserve_over_table(eng, eng->offsets, (n + 1) * sizeof(int64_t)));
+    GSS_TRY(reserve_over_table(eng, eng->orig, std::max<int64_t>(n, 1) * sizeof(uint32_t)));
     if (n_lits)
         GSS_CUDA_TRY(cudaMemcpy(eng->lits.ptr, eng->h_lits.data(), n_lits * sizeof(int32_t), cudaMemcpyHostToDevice));
     GSS_CUDA_TRY(cudaMemcpy(eng->offsets.ptr, eng->h_off.data(), (n + 1) * sizeof(int64_t), cudaMemcpyHostToDevice));
@@ -507,9 +504,9 @@ int gss_db_append(gss_engine *eng, const int32_t *lits, const int64_t *offsets, 
     const int64_t n_lits = eng->h_off.back();
     GSS_TRY(ensure_device(eng));
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
-    GSS_TRY(eng->lits.grow_keep((n_lits + 8) * sizeof(int32_t), eng->stream, base * sizeof(int32_t)));
-    GSS_TRY(eng->offsets.grow_keep((n + 1) * sizeof(int64_t), eng->stream, (first + 1) * sizeof(int64_t)));
-    GSS_TRY(eng->orig.grow_keep(n * sizeof(uint32_t), eng->stream, first * sizeof(uint32_t)));
+    GSS_TRY(grow_over_table(eng, eng->lits, (n_lits + 8) * sizeof(int32_t), base * sizeof(int32_t)));
+    GSS_TRY(grow_over_table(eng, eng->offsets, (n + 1) * sizeof(int64_t), (first + 1) * sizeof(int64_t)));
+    GSS_TRY(grow_over_table(eng, eng->orig, n * sizeof(uint32_t), first * sizeof(uint32_t)));
     // new literals, then zero padding past the end
     std::vector<int32_t> tail(eng->h_lits.begin() + base, eng->h_lits.end());
     tail.resize(tail.size() + 8, 0);
@@ -855,7 +852,7 @@ int build_plan(gss_engine *eng) {
     }
     close_range();
     p.group_base[p.n_ranges] = groups;
-    GSS_TRY(eng->d_plan.reserve(sizeof(BucketPlan)));
+    GSS_TRY(reserve_over_table(eng, eng->d_plan, sizeof(BucketPlan)));
     GSS_CUDA_TRY(cudaMemcpyAsync(eng->d_plan.ptr, &p, sizeof(BucketPlan), cudaMemcpyHostToDevice, eng->stream));
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));  // pageable source
     eng->plan_ranges = p.n_ranges;
@@ -900,7 +897,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     a.alive = nullptr;
     if (eng->n_dead > 0) {
         if (eng->alive_dirty) {
-            GSS_TRY(eng->alive.reserve(std::max<size_t>(eng->h_alive.size(), 1) * sizeof(uint32_t)));
+            GSS_TRY(reserve_over_table(eng, eng->alive, std::max<size_t>(eng->h_alive.size(), 1) * sizeof(uint32_t)));
             GSS_CUDA_TRY(cudaMemcpyAsync(eng->alive.ptr, eng->h_alive.data(), eng->h_alive.size() * sizeof(uint32_t),
                                          cudaMemcpyHostToDevice, eng->stream));
             GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));  // pageable source
@@ -952,11 +949,16 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     const bool narrow = eng->kind == GSS_KERNEL_AUTO && eng->state_kind == GSS_KERNEL_DIRECT && eng->n_blocks == 1 &&
                         valid_narrow_variant(eng->state_lpc);
     // behind the word-level filter where the state's table says that it pays
-    const bool may_filter = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
-                            filter_tasks(a) < kMaxFilterTasks;
-    const bool filtered = may_filter && eng->filter_pause == 0;
-    if (may_filter && eng->filter_pause > 0) eng->filter_pause--;
-    eng->pass_filtered = filtered;
+    // (asked after the last reservation: that may have taken the table)
+    bool filtered = false;
+    eng->pass_filtered = false;
+    auto choose_filter = [&]() {
+        const bool may = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
+                         filter_tasks(a) < kMaxFilterTasks;
+        filtered = may && eng->filter_pause == 0;
+        if (may && eng->filter_pause > 0) eng->filter_pause--;
+        eng->pass_filtered = filtered;
+    };
     auto launch_persistent = [&](const CheckArgs *d_args, const CheckArgs &args) -> int {
         if (filtered)
             return launch_check_filtered(d_args, args, words_per_lane(eng->state_kind), eng->state_lpc, work,
@@ -977,7 +979,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     if (bucketed || (persistent && eng->use_graph && !ordered)) {
         // arguments through device memory, so the same graph serves every pass
         if (bucketed) GSS_TRY(build_plan(eng));
-        GSS_TRY(eng->d_args.reserve(sizeof(CheckArgs)));
+        choose_filter();
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->d_args.ptr, &a, sizeof a, cudaMemcpyHostToDevice, eng->stream));
         if (ev0) GSS_CUDA_TRY(cudaEventRecord(ev0, eng->stream));
         auto body = [&]() -> int {
@@ -1049,6 +1051,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         // counts for early delivery, the tail, and the history update
         uint32_t head = 0, covered = 0;
         GSS_TRY(order_prepare(eng, &a.perm, &head, &covered));
+        choose_filter();
         // positions appended since the order was computed (from `covered`
         // on) are scanned in place at the end of the tail
         a.perm_end = covered;
@@ -1062,6 +1065,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         if (head < a.n_clauses) GSS_TRY(launch(a));
         GSS_TRY(order_after_pass(eng, reports, counts));
     } else {
+        choose_filter();
         GSS_TRY(launch(a));
     }
     if (ev1) {
@@ -1211,8 +1215,8 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         return GSS_OK;
     };
     GSS_TRY(reserve_reports());
-    GSS_TRY(eng->counts2.reserve(counter_bytes(eng->n_parts)));
-    GSS_TRY(eng->counts3.reserve(counter_bytes(eng->n_parts)));
+    GSS_TRY(reserve(eng->counts2, counter_bytes(eng->n_parts)));
+    GSS_TRY(reserve(eng->counts3, counter_bytes(eng->n_parts)));
     auto reserve_packed = [&]() -> int {
         for (int b = 0; b < NB && packed; b++)
             GSS_TRY(reserve(eng->packed[b], (size_t) eng->cap_per_part * eng->n_parts * rec_words * sizeof(uint32_t)));

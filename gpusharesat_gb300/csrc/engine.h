@@ -131,6 +131,22 @@ constexpr size_t kHostCounterBytes = kInlineOffset + (size_t) kEngineInline * si
 // where gss_state_set's count of the filter's bits comes back, past the counters
 constexpr size_t kDensityOffset = 192;
 
+// The filter's tables, which a pass can do without, make room for what it
+// cannot: an allocation that fails is tried again once they are given back.
+// False: there are none.
+bool release_tables(gss_engine *eng);
+template <typename F>
+int over_table(gss_engine *eng, F allocate) {
+    const int rc = allocate();
+    return rc == GSS_ERR_NOMEM && release_tables(eng) ? allocate() : rc;
+}
+inline int reserve_over_table(gss_engine *eng, DevBuf &buf, size_t bytes) {
+    return over_table(eng, [&]() { return buf.reserve(bytes); });
+}
+inline int grow_over_table(gss_engine *eng, DevBuf &buf, size_t bytes, size_t keep_bytes) {
+    return over_table(eng, [&]() { return buf.grow_keep(bytes, eng->stream, keep_bytes); });
+}
+
 // Learned scan order hooks, called by the engine's pass (order.cu).
 // Before the scan: the scan permutation of this pass (computed while the
 // previous pass ran, or now on the engine's stream). It covers positions

@@ -1009,10 +1009,10 @@ unsigned grid_for_n(uint64_t n, int sm_count, int threads) {
 }
 
 template <typename T>
-int grow_ids(DevBuf &b, int64_t old_n, int64_t new_n, cudaStream_t stream, bool zero_tail) {
-    GSS_TRY(b.grow_keep((size_t) new_n * sizeof(T), stream, (size_t) old_n * sizeof(T)));
+int grow_ids(gss_engine *eng, DevBuf &b, int64_t old_n, int64_t new_n, bool zero_tail) {
+    GSS_TRY(grow_over_table(eng, b, (size_t) new_n * sizeof(T), (size_t) old_n * sizeof(T)));
     if (zero_tail && new_n > old_n)
-        GSS_CUDA_TRY(cudaMemsetAsync((T *) b.ptr + old_n, 0, (size_t) (new_n - old_n) * sizeof(T), stream));
+        GSS_CUDA_TRY(cudaMemsetAsync((T *) b.ptr + old_n, 0, (size_t) (new_n - old_n) * sizeof(T), eng->stream));
     return GSS_OK;
 }
 
@@ -1021,7 +1021,7 @@ int ensure_ids(gss_engine *eng, int64_t n_ids) {
     if (n_ids <= o.cap_ids) return GSS_OK;
     int64_t cap = std::max<int64_t>(o.cap_ids * 2, 1024);
     while (cap < n_ids) cap *= 2;
-    GSS_TRY(grow_ids<ClauseRecord>(o.rec, o.cap_ids, cap, eng->stream, true));
+    GSS_TRY(grow_ids<ClauseRecord>(eng, o.rec, o.cap_ids, cap, true));
     o.cap_ids = cap;
     return GSS_OK;
 }
@@ -1053,8 +1053,8 @@ int train_start(gss_engine *eng) {
     const uint32_t B = (uint32_t) std::min<uint64_t>((uint64_t) std::max(o.prm.batch, 1), logged);
     const uint64_t steps = std::min<uint64_t>(kMaxTrainSteps,
                                               (uint64_t) std::max(o.prm.train_epochs, 1) * ((logged + B - 1) / B));
-    GSS_TRY(o.snap_x.reserve((size_t) logged * kF * sizeof(float)));
-    GSS_TRY(o.snap_y.reserve((size_t) logged * sizeof(float)));
+    GSS_TRY(reserve_over_table(eng, o.snap_x, (size_t) logged * kF * sizeof(float)));
+    GSS_TRY(reserve_over_table(eng, o.snap_y, (size_t) logged * sizeof(float)));
     GSS_CUDA_TRY(cudaEventRecord(o.ev_train_start, eng->stream));
     GSS_CUDA_TRY(cudaStreamWaitEvent(o.train_stream, o.ev_train_start, 0));
     GSS_CUDA_TRY(cudaMemcpyAsync(o.snap_x.ptr, o.log_x.ptr, (size_t) logged * kF * sizeof(float),
@@ -1063,8 +1063,10 @@ int train_start(gss_engine *eng) {
                                  o.train_stream));
     for (uint64_t st = 0; st < steps; st++) {
         const uint32_t start = (uint32_t) (o.rng() % logged);
-        GSS_TRY(scorer_grad_dev(&o.trainer, (const float *) o.snap_x.ptr, (const float *) o.snap_y.ptr,
-                                (uint32_t) logged, start, B, o.prm.learning_rate, o.train_stream));
+        GSS_TRY(over_table(eng, [&]() {
+            return scorer_grad_dev(&o.trainer, (const float *) o.snap_x.ptr, (const float *) o.snap_y.ptr,
+                                   (uint32_t) logged, start, B, o.prm.learning_rate, o.train_stream);
+        }));
     }
     GSS_CUDA_TRY(cudaEventRecord(o.ev_train_done, o.train_stream));
     o.training = true;
@@ -1196,11 +1198,11 @@ int score_pass(gss_engine *eng, cudaStream_t st, int64_t q, uint32_t *covered, i
     const int b = 1 - o.inflight_buf;
     DevBuf &perm = o.perm[b];
     const uint32_t n_tiles = (uint32_t) (((size_t) n + kSortTile - 1) / kSortTile);
-    GSS_TRY(perm.reserve(std::max<size_t>(n, 1) * sizeof(uint32_t)));
-    GSS_TRY(o.bucket.reserve(std::max<size_t>(n, 1)));
-    GSS_TRY(o.offs.reserve(std::max<size_t>((size_t) kKeys * n_tiles, 1) * sizeof(uint32_t)));
+    GSS_TRY(reserve_over_table(eng, perm, std::max<size_t>(n, 1) * sizeof(uint32_t)));
+    GSS_TRY(reserve_over_table(eng, o.bucket, std::max<size_t>(n, 1)));
+    GSS_TRY(reserve_over_table(eng, o.offs, std::max<size_t>((size_t) kKeys * n_tiles, 1) * sizeof(uint32_t)));
     constexpr size_t total_bytes = kBuckets * kTotalStride * sizeof(uint32_t);
-    GSS_TRY(o.totals.reserve(total_bytes + kKeys * sizeof(uint32_t)));
+    GSS_TRY(reserve_over_table(eng, o.totals, total_bytes + kKeys * sizeof(uint32_t)));
     if (n) {
         uint32_t *const totals = (uint32_t *) o.totals.ptr;
         uint32_t *const key_total = totals + kBuckets * kTotalStride;
@@ -1355,8 +1357,9 @@ int gss_order_enable(gss_engine *eng, const gss_order_params *p) {
     o->rng.seed(prm.seed * 0x9E3779B97F4A7C15ull + 7);
     o->epoch = eng->db_epoch;
     eng->order = o;
-    int rc = scorer_init(&o->scorer, eng->device, prm.seed, eng->stream);
-    if (rc == GSS_OK) rc = scorer_init(&o->trainer, eng->device, prm.seed, eng->stream);  // the same weights
+    int rc = over_table(eng, [&]() { return scorer_init(&o->scorer, eng->device, prm.seed, eng->stream); });
+    if (rc == GSS_OK)  // the same weights
+        rc = over_table(eng, [&]() { return scorer_init(&o->trainer, eng->device, prm.seed, eng->stream); });
     for (int k = 0; rc == GSS_OK && k < 6; k++)
         if (cudaEventCreate(&o->ev[k]) != cudaSuccess) rc = set_error(GSS_ERR_CUDA, "cudaEventCreate failed");
     if (rc == GSS_OK && (cudaEventCreateWithFlags(&o->ev_score_done, cudaEventDisableTiming) != cudaSuccess ||
@@ -1367,10 +1370,10 @@ int gss_order_enable(gss_engine *eng, const gss_order_params *p) {
                          cudaStreamCreateWithFlags(&o->train_stream, cudaStreamNonBlocking) != cudaSuccess))
         rc = set_error(GSS_ERR_CUDA, "creating the training stream failed");
     if (rc == GSS_OK && prm.log_capacity > 0) {
-        rc = o->log_x.reserve((size_t) prm.log_capacity * kF * sizeof(float));
-        if (rc == GSS_OK) rc = o->log_y.reserve((size_t) prm.log_capacity * sizeof(float));
+        rc = reserve_over_table(eng, o->log_x, (size_t) prm.log_capacity * kF * sizeof(float));
+        if (rc == GSS_OK) rc = reserve_over_table(eng, o->log_y, (size_t) prm.log_capacity * sizeof(float));
     }
-    if (rc == GSS_OK) rc = o->log_count.reserve(sizeof(unsigned long long));
+    if (rc == GSS_OK) rc = reserve_over_table(eng, o->log_count, sizeof(unsigned long long));
     if (rc == GSS_OK) rc = o->h_log_count.reserve(sizeof(unsigned long long));
     if (rc == GSS_OK) rc = o->h_head_counts.reserve(kHostCounterBytes);
     if (rc == GSS_OK && cudaMemsetAsync(o->log_count.ptr, 0, sizeof(unsigned long long), eng->stream) != cudaSuccess)
@@ -1417,7 +1420,7 @@ int gss_db_set_lbd(gss_engine *eng, const uint32_t *ids, const uint16_t *lbd, in
         pairs[2 * i] = ids[i];
         pairs[2 * i + 1] = lbd[i];
     }
-    GSS_TRY(o.lbd_pairs.reserve(pairs.size() * sizeof(uint32_t)));
+    GSS_TRY(reserve_over_table(eng, o.lbd_pairs, pairs.size() * sizeof(uint32_t)));
     GSS_CUDA_TRY(cudaMemcpyAsync(o.lbd_pairs.ptr, pairs.data(), pairs.size() * sizeof(uint32_t),
                                  cudaMemcpyHostToDevice, eng->stream));
     set_lbd_kernel<<<grid_for_n((uint64_t) n, eng->sm_count, 256), 256, 0, eng->stream>>>(

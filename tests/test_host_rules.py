@@ -21,6 +21,7 @@ def clean(fake):
     fake.reset()
     yield
     fake.reset()
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 0)
 
 
 @pytest.mark.parametrize("what", ["malloc_host", "malloc"])
@@ -132,6 +133,66 @@ def test_launcher_reports_the_runtime_error_and_asks_again(tmp_path, n_words):
     assert fake.log().count("occupancy") == 2  # refused, answered; not asked a third time
     checks = [l for l in fake.log() if "check_narrow_kernel" in l or "check_filtered_kernel" in l]
     assert len(checks) == 2
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def _append(fake, eng):
+    n = 3000
+    lits = (ctypes.c_int32 * (2 * n))(*[2 * (k % 50) for k in range(2 * n)])
+    assert fake.lib.gss_db_append(eng, lits, (i64 * (n + 1))(*range(0, 2 * n + 1, 2)), i64(n), None) == 0, fake.error()
+
+
+def _delete(fake, eng):
+    ids = (ctypes.c_uint32 * 3)(5, 6, 7)
+    assert fake.lib.gss_db_delete(eng, ids, i64(3)) == 0
+    assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+
+
+def _launch(fake, eng):
+    assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+
+
+def _order(fake, eng):
+    assert fake.lib.gss_order_enable(eng, None) == 0, fake.error()
+
+
+@pytest.mark.parametrize("n_words", [20, 40])
+@pytest.mark.parametrize("grow", [lambda f, e: _database(f, e, 3000), _append, _delete, _launch, _order,
+                                  lambda f, e: _state(f, e, 64)],
+                         ids=["set", "append", "delete", "queues", "order", "state"])
+def test_filter_table_makes_room_for_what_a_pass_needs(fake, n_words, grow):
+    """Whatever the engine must have and cannot get, it gets once the filter's
+    table is given back, as if there had been no table."""
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    _state(fake, eng, n_words)
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 1)
+    grow(fake, eng)
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 0)
+    fake.reset()
+    assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+    assert fake.lib.gss_check_wait(eng, None) == 0
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def test_order_takes_the_table_before_the_pass_reads_it(fake):
+    """A pass whose own scoring makes the table go does not run behind it."""
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    assert fake.lib.gss_order_enable(eng, None) == 0
+    _state(fake, eng, 20)
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 1)  # the queues
+    fake.reset()
+    assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+    assert not any("check_filtered_kernel" in l for l in fake.log())
+    assert fake.lib.gss_check_wait(eng, None) == 0
+    _append(fake, eng)  # the scoring buffers have to grow
+    _state(fake, eng, 20)
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 1)
+    fake.reset()
+    assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+    assert not any("check_filtered_kernel" in l for l in fake.log())
+    assert any("check_wide_persist_kernel" in l for l in fake.log())
     assert fake.lib.gss_engine_destroy(eng) == 0
 
 
