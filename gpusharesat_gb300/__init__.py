@@ -84,6 +84,7 @@ def load():
     _sig(lib, "gss_engine_set_timing", c_int, vp, c_int)
     _sig(lib, "gss_engine_set_graph", c_int, vp, c_int)
     _sig(lib, "gss_engine_graph_captures", c_i64, vp)
+    _sig(lib, "gss_engine_filtered_passes", c_i64, vp)
     _sig(lib, "gss_engine_kernel_time", c_int, vp, vp, vp)
     _sig(lib, "gss_engine_set_variant", c_int, vp, c_int, c_int, c_int, c_int)
     _sig(lib, "gss_db_set", c_int, vp, vp, vp, c_i64)
@@ -189,6 +190,11 @@ class Engine:
     @property
     def graph_captures(self):
         return int(self.lib.gss_engine_graph_captures(self.h))
+
+    @property
+    def filtered_passes(self):
+        """Passes that ran behind the word-level filter."""
+        return int(self.lib.gss_engine_filtered_passes(self.h))
 
     def set_timing(self, on=True):
         _check(self.lib.gss_engine_set_timing(self.h, 1 if on else 0))
@@ -607,6 +613,8 @@ def _sharer_sigs(lib):
     _sig(lib, "gss_sharer_set_locality", c_int, vp, c_int)
     _sig(lib, "gss_sharer_evicted_count", c_i64, vp)
     _sig(lib, "gss_sharer_device_compactions", c_i64, vp)
+    _sig(lib, "gss_sharer_set_filter_from", c_int, vp, c_i64)
+    _sig(lib, "gss_sharer_filtered_passes", c_i64, vp)
     _sig(lib, "gss_serving_run", c_int, vp, vp)
     _sig(lib, "gss_activity_create", vp, ctypes.c_float)
     _sig(lib, "gss_activity_destroy", None, vp)
@@ -765,6 +773,14 @@ class ClauseSharer:
 
     def deviceCompactions(self):
         return int(self.lib.gss_sharer_device_compactions(self.h))
+
+    def setFilterFrom(self, pairs):
+        """(clauses x slot blocks) from which passes run behind the word-level
+        filter (-1: the measured default)."""
+        _check(self.lib.gss_sharer_set_filter_from(self.h, pairs))
+
+    def filteredPasses(self):
+        return int(self.lib.gss_sharer_filtered_passes(self.h))
 
 
 class ServingParams(ctypes.Structure):

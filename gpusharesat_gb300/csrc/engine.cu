@@ -283,6 +283,8 @@ int gss_engine_set_graph(gss_engine *eng, int on) {
 
 int64_t gss_engine_graph_captures(const gss_engine *eng) { return eng ? eng->graph_captures : -1; }
 
+int64_t gss_engine_filtered_passes(const gss_engine *eng) { return eng ? eng->filtered_passes : -1; }
+
 int gss_engine_set_timing(gss_engine *eng, int on) {
     if (!eng) return set_error(GSS_ERR_INVALID, "engine is NULL");
     eng->timing = on != 0;
@@ -958,6 +960,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
         filtered = may && eng->filter_pause == 0;
         if (may && eng->filter_pause > 0) eng->filter_pause--;
         eng->pass_filtered = filtered;
+        eng->filtered_passes += filtered;
     };
     auto launch_persistent = [&](const CheckArgs *d_args, const CheckArgs &args) -> int {
         if (filtered)

@@ -108,6 +108,7 @@ struct gss_engine {
     cudaGraphExec_t graph_exec = nullptr;
     std::vector<uintptr_t> graph_key;
     int64_t graph_captures = 0;
+    int64_t filtered_passes = 0;
 
     // optional CUDA-event timing of each check kernel (on the launch stream)
     bool timing = false;

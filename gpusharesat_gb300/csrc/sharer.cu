@@ -96,11 +96,6 @@ unsigned grid_for(uint64_t n, int sm_count) {
 
 }  // namespace
 
-// (clauses x slot blocks) from which the filter pays for its table's upkeep,
-// two launches a pass (7 solvers, 50k clauses: 120 us a pass without, 126
-// with; 64 solvers, 1.2e6 clauses: 220 us of check without, 85 with).
-constexpr int64_t kFilterMinPairs = 150000;
-
 // ---- one solver's ring ----
 
 void SolverAssigs::set_var_locked(uint32_t var, uint8_t val) {
@@ -503,6 +498,12 @@ int Sharer::ensure_state() {
     agg_possible_ = kind_ == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && need_vars > 0 && n_words > 0;
     agg_ok_ = false;
     filter_pause_ = 0;
+    return GSS_OK;
+}
+
+int Sharer::set_filter_from(int64_t pairs) {
+    if (pairs < -1) return set_error(GSS_ERR_INVALID, "pairs must be 0 or more, or -1 for the default");
+    filter_from_ = pairs < 0 ? kFilterMinPairs : pairs;
     return GSS_OK;
 }
 
@@ -917,6 +918,7 @@ int Sharer::run_check(Pass &p) {
             // the persistent form, as the engine's automatic variant
             uint32_t *const work = work_counter(a.counts, n_parts_);
             p.filtered = agg_ok_ && filter_pause_ == 0 && filter_tasks(a) < kMaxFilterTasks;
+            filtered_passes_ += p.filtered;
             if (p.filtered)
                 GSS_TRY(launch_check_filtered(nullptr, a, wpl, eff_lpc_, work, stream_, sm_count_));
             else
@@ -1161,7 +1163,7 @@ int Sharer::launch_pass() {
             GSS_CUDA_TRY(cudaGetLastError());
         }
         // the filter's table follows while the database is large enough for it
-        if (!agg_possible_ || (int64_t) dev_clauses_ * n_blocks_ < kFilterMinPairs)
+        if (!agg_possible_ || (int64_t) dev_clauses_ * n_blocks_ < filter_from_)
             agg_ok_ = false;
         else if (!agg_ok_)
             GSS_TRY(rebuild_agg());
@@ -1560,6 +1562,13 @@ int gss_sharer_set_clause_budget(gss_sharer *s, int64_t max_clauses) {
 
 int64_t gss_sharer_evicted_count(gss_sharer *s) { return s ? s->impl->evicted() : -1; }
 int64_t gss_sharer_device_compactions(gss_sharer *s) { return s ? s->impl->device_compactions() : -1; }
+
+int gss_sharer_set_filter_from(gss_sharer *s, int64_t pairs) {
+    if (!s) return gss::set_error(GSS_ERR_INVALID, "sharer is NULL");
+    return s->impl->set_filter_from(pairs);
+}
+
+int64_t gss_sharer_filtered_passes(gss_sharer *s) { return s ? s->impl->filtered_passes() : -1; }
 
 int gss_sharer_set_locality(gss_sharer *s, int range_log2) {
     if (!s) return gss::set_error(GSS_ERR_INVALID, "sharer is NULL");

@@ -21,6 +21,10 @@ namespace gss {
 constexpr uint8_t kTrue = 0, kFalse = 1, kUndef = 2;
 // records that come back with a pass's counters (256 KB of pinned memory)
 constexpr uint32_t kSharerInline = 16384 - kInlineOffset / sizeof(gss_report);
+// (clauses x slot blocks) from which the filter pays for its table's upkeep,
+// two launches a pass (7 solvers, 50k clauses: 120 us a pass without, 126
+// with; 64 solvers, 1.2e6 clauses: 220 us of check without, 85 with).
+constexpr int64_t kFilterMinPairs = 150000;
 constexpr int kSlots = 32;  // assignments per solver per pass (Assigs.cuh:37-39)
 
 // Statistics, in the reference's order and with its names
@@ -167,6 +171,8 @@ public:
     void set_locality(int r) { range_log2_ = r; }
     int64_t evicted() const { return evicted_; }
     int64_t device_compactions() const { return device_compactions_; }
+    int set_filter_from(int64_t pairs);
+    int64_t filtered_passes() const { return filtered_passes_; }
     int64_t live_clauses() const { return (int64_t) meta_.size() - n_dead_; }
 
 private:
@@ -292,6 +298,8 @@ private:
     bool agg_possible_ = false; // the layout has a filtered kernel
     bool agg_ok_ = false;       // d_agg_ follows the state
     int filter_pause_ = 0;      // passes to run without the filter (it kept too much)
+    int64_t filter_from_ = kFilterMinPairs;  // (clauses x slot blocks) from which passes run behind it
+    int64_t filtered_passes_ = 0;
     PinnedBuf h_updates_;
     PinnedBuf h_append_;             // staging of appended clauses (literals, offsets, ids)
     cudaEvent_t append_staged_ = nullptr;

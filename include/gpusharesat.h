@@ -93,6 +93,8 @@ int64_t gss_engine_launch_count(const gss_engine *eng);
 int gss_engine_set_graph(gss_engine *eng, int on);
 /* How many times a pass graph was captured (for tests and tuning). */
 int64_t gss_engine_graph_captures(const gss_engine *eng);
+/* How many passes ran behind the word-level filter (for tests and tuning). */
+int64_t gss_engine_filtered_passes(const gss_engine *eng);
 /* When on, each check kernel is bracketed by CUDA events on its stream. */
 int gss_engine_set_timing(gss_engine *eng, int on);
 /* Sum of the bracketed kernel durations since the last call (waits for
@@ -498,6 +500,11 @@ int gss_sharer_set_variant(gss_sharer *s, int kind, int lanes_per_clause, int de
  * automatic variable ranges, 0 length order, 11..31); applies to batches
  * appended from then on and to reduceDb. No counterpart in the reference. */
 int gss_sharer_set_locality(gss_sharer *s, int range_log2);
+/* (clauses x slot blocks) from which a pass of the automatic variant runs
+ * behind the word-level filter (0 or more; -1 = the measured default), and how
+ * many passes did (for tests and tuning). The reports do not depend on it. */
+int gss_sharer_set_filter_from(gss_sharer *s, int64_t pairs);
+int64_t gss_sharer_filtered_passes(gss_sharer *s);
 
 /* ---- serving load generator (no counterpart in the reference) ----
  * Simulated solver threads drive one sharer on the calling thread's current
