@@ -471,7 +471,7 @@ int Sharer::ensure_state() {
     }
     const size_t bytes = std::max<size_t>((size_t) n_blocks * std::max(need_vars, 1) * bw * sizeof(uint2), 8);
     DevBuf fresh;
-    GSS_TRY(fresh.reserve(bytes));
+    GSS_TRY(reserve(fresh, bytes));
     GSS_CUDA_TRY(cudaMemsetAsync(fresh.ptr, 0, bytes, stream_));
     if (d_state_.ptr && dev_vars_ > 0 && dev_words_ > 0) {
         const uint32_t nv = (uint32_t) std::min(dev_vars_, need_vars);
@@ -491,7 +491,7 @@ int Sharer::ensure_state() {
     eff_kind_ = kind;
     eff_lpc_ = lpc;
     eff_depth_ = depth;
-    GSS_TRY(d_sow_.reserve(sizeof(int32_t) * n_blocks * bw));
+    GSS_TRY(reserve(d_sow_, sizeof(int32_t) * n_blocks * bw));
     std::vector<int32_t> sow(n_blocks * bw);
     for (int w = 0; w < n_blocks * bw; w++) sow[w] = w < n_words ? w : 0;
     GSS_CUDA_TRY(cudaMemcpy(d_sow_.ptr, sow.data(), sow.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -505,6 +505,13 @@ int Sharer::set_filter_from(int64_t pairs) {
     if (pairs < -1) return set_error(GSS_ERR_INVALID, "pairs must be 0 or more, or -1 for the default");
     filter_from_ = pairs < 0 ? kFilterMinPairs : pairs;
     return GSS_OK;
+}
+
+void Sharer::give_table_back() {
+    // passes run without it until the state's layout changes
+    cudaStreamSynchronize(stream_);
+    agg_possible_ = agg_ok_ = false;
+    d_agg_.release();
 }
 
 int Sharer::rebuild_agg() {
@@ -540,9 +547,9 @@ int Sharer::upload_db() {
     for (uint32_t i = 0; i < n; i++) meta_[i].lit_off = (uint32_t) offsets[i];
     std::vector<uint32_t> orig(std::max<uint32_t>(n, 1));
     for (uint32_t i = 0; i < n; i++) orig[i] = i;
-    GSS_TRY(d_lits_.reserve(lits.size() * sizeof(int32_t)));
-    GSS_TRY(d_offsets_.reserve((n + 1) * sizeof(int64_t)));
-    GSS_TRY(d_orig_.reserve(orig.size() * sizeof(uint32_t)));
+    GSS_TRY(reserve(d_lits_, lits.size() * sizeof(int32_t)));
+    GSS_TRY(reserve(d_offsets_, (n + 1) * sizeof(int64_t)));
+    GSS_TRY(reserve(d_orig_, orig.size() * sizeof(uint32_t)));
     GSS_CUDA_TRY(cudaMemcpyAsync(d_lits_.ptr, lits.data(), lits.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                                  stream_));
     GSS_CUDA_TRY(cudaMemcpyAsync(d_offsets_.ptr, offsets.data(), (n + 1) * sizeof(int64_t),
@@ -579,8 +586,8 @@ int Sharer::sync_alive() {
         alive_hi_ = h_alive_.size();
     }
     if (d_alive_.bytes < words * sizeof(uint32_t)) {
-        GSS_TRY(d_alive_.grow_keep(words * sizeof(uint32_t), stream_,
-                                   alive_synced_ ? std::min(d_alive_.bytes, words * sizeof(uint32_t)) : 0));
+        GSS_TRY(grow(d_alive_, words * sizeof(uint32_t),
+                     alive_synced_ ? std::min(d_alive_.bytes, words * sizeof(uint32_t)) : 0));
     }
     alive_hi_ = std::min(alive_hi_, h_alive_.size());
     if (alive_lo_ < alive_hi_) {
@@ -605,10 +612,10 @@ int Sharer::compact_device() {
     GSS_TRY(sync_alive());
     const uint32_t n = dev_clauses_;
     const int64_t live_lits = dev_lits_;  // an upper bound on what stays
-    GSS_TRY(d_lits2_.reserve((size_t) (live_lits + kClausePad) * sizeof(int32_t)));
-    GSS_TRY(d_offsets2_.reserve(((size_t) n + 1) * sizeof(int64_t)));
-    GSS_TRY(d_orig2_.reserve(std::max<size_t>(n, 1) * sizeof(uint32_t)));
-    GSS_TRY(d_compact_.reserve(compact_scratch_bytes(n)));
+    GSS_TRY(reserve(d_lits2_, (size_t) (live_lits + kClausePad) * sizeof(int32_t)));
+    GSS_TRY(reserve(d_offsets2_, ((size_t) n + 1) * sizeof(int64_t)));
+    GSS_TRY(reserve(d_orig2_, std::max<size_t>(n, 1) * sizeof(uint32_t)));
+    GSS_TRY(reserve(d_compact_, compact_scratch_bytes(n)));
     CompactArgs c;
     c.lits = (const int32_t *) d_lits_.ptr;
     c.offsets = (const int64_t *) d_offsets_.ptr;
@@ -728,13 +735,12 @@ void Sharer::reserve_for_budget(size_t n_new, size_t n_new_lits) {
     h_lits_.reserve(h_lits_.size() + (size_t) (mean_len * (double) budget_) + n_new_lits);
     // best effort: without the device room, the arrays grow when needed (and
     // a failure there takes the out-of-memory path)
-    if (d_lits_.grow_keep(dev_lits * sizeof(int32_t), stream_, (size_t) dev_lits_ * sizeof(int32_t)) == GSS_OK &&
-        d_offsets_.grow_keep((dev_clauses + 1) * sizeof(int64_t), stream_,
-                             (size_t) (dev_clauses_ ? dev_clauses_ + 1 : 0) * sizeof(int64_t)) == GSS_OK &&
-        d_orig_.grow_keep(dev_clauses * sizeof(uint32_t), stream_, (size_t) dev_clauses_ * sizeof(uint32_t)) ==
-            GSS_OK) {
-        d_alive_.grow_keep((host_clauses + 31) / 32 * sizeof(uint32_t), stream_,
-                           alive_synced_ ? std::min(d_alive_.bytes, (host_clauses + 31) / 32 * sizeof(uint32_t)) : 0);
+    if (grow(d_lits_, dev_lits * sizeof(int32_t), (size_t) dev_lits_ * sizeof(int32_t)) == GSS_OK &&
+        grow(d_offsets_, (dev_clauses + 1) * sizeof(int64_t),
+             (size_t) (dev_clauses_ ? dev_clauses_ + 1 : 0) * sizeof(int64_t)) == GSS_OK &&
+        grow(d_orig_, dev_clauses * sizeof(uint32_t), (size_t) dev_clauses_ * sizeof(uint32_t)) == GSS_OK) {
+        grow(d_alive_, (host_clauses + 31) / 32 * sizeof(uint32_t),
+             alive_synced_ ? std::min(d_alive_.bytes, (host_clauses + 31) / 32 * sizeof(uint32_t)) : 0);
     }
     reserved_for_ = budget_;
 }
@@ -811,9 +817,9 @@ int Sharer::append_clauses(std::vector<int64_t> &ids, std::vector<int32_t> &lits
     mark_alive(first >> 5, h_alive_.size());
     if (end_off > 0x7FFFFF00LL) return set_error(GSS_ERR_NOMEM, "clause database exceeds 2^31 literals");
     // grow the device arrays, keeping their contents
-    GSS_TRY(d_lits_.grow_keep((end_off + kClausePad) * sizeof(int32_t), stream_, base_off * sizeof(int32_t)));
-    GSS_TRY(d_offsets_.grow_keep((n_dev + 1) * sizeof(int64_t), stream_, (dpos + 1) * sizeof(int64_t)));
-    GSS_TRY(d_orig_.grow_keep(n_dev * sizeof(uint32_t), stream_, dpos * sizeof(uint32_t)));
+    GSS_TRY(grow(d_lits_, (end_off + kClausePad) * sizeof(int32_t), base_off * sizeof(int32_t)));
+    GSS_TRY(grow(d_offsets_, (n_dev + 1) * sizeof(int64_t), (dpos + 1) * sizeof(int64_t)));
+    GSS_TRY(grow(d_orig_, n_dev * sizeof(uint32_t), dpos * sizeof(uint32_t)));
     // The batch goes up through one pinned stage (a copy from pageable
     // memory would first wait for the whole stream, the pass in flight
     // included): literals (+ zero padding), the offsets of the clause ends
@@ -873,7 +879,7 @@ int Sharer::run_check(Pass &p) {
                                            (int64_t) report_cap_ * n_parts_);
     const int64_t per = std::min<int64_t>((want + n_parts_ - 1) / n_parts_, 0x7FFFFFFF);
     if ((uint32_t) per > p.cap_per_part || !p.d_reports.ptr) {
-        GSS_TRY(p.d_reports.reserve((size_t) per * n_parts_ * sizeof(gss_report)));
+        GSS_TRY(reserve(p.d_reports, (size_t) per * n_parts_ * sizeof(gss_report)));
         p.cap_per_part = (uint32_t) per;
     }
     CheckArgs a;
@@ -1152,7 +1158,7 @@ int Sharer::launch_pass() {
         // h_updates_ is free: the copy of the last pass that had one ran
         // before that pass's check, which has finished
         const size_t at = updates_offset(), bytes = at + ups.size() * sizeof(StateUpdate);
-        GSS_TRY(d_updates_.reserve(bytes));
+        GSS_TRY(reserve(d_updates_, bytes));
         GSS_TRY(h_updates_.reserve(bytes));
         memcpy(h_updates_.ptr, masks.data(), masks.size() * sizeof(uint32_t));
         if (!ups.empty()) memcpy((char *) h_updates_.ptr + at, ups.data(), ups.size() * sizeof(StateUpdate));
@@ -1204,10 +1210,6 @@ int Sharer::recover_from_oom() {
     out_of_memory_ = true;
     log(1, "c Ran out of GPU memory: reducing the GPU clause database\n");
     GSS_TRY(finish_pending());
-    // the filter's table goes too: passes run without it until the state's
-    // layout changes
-    agg_possible_ = agg_ok_ = false;
-    d_agg_.release();
     return reduce_now(false);  // an upload frees the old device buffers before allocating new ones
 }
 
@@ -1325,10 +1327,10 @@ int Sharer::rebuild_on_device(const std::vector<uint32_t> &src) {
     std::vector<int64_t> offsets(n + 1, 0);
     for (uint32_t i = 0; i < n; i++) offsets[i + 1] = offsets[i] + meta_[i].len;
     const int64_t n_lits = offsets[n];
-    GSS_TRY(d_lits2_.reserve((size_t) (n_lits + kClausePad) * sizeof(int32_t)));
-    GSS_TRY(d_offsets2_.reserve(((size_t) n + 1) * sizeof(int64_t)));
-    GSS_TRY(d_orig2_.reserve(std::max<size_t>(n, 1) * sizeof(uint32_t)));
-    GSS_TRY(d_compact_.reserve(std::max<size_t>(n, 1) * sizeof(uint32_t)));
+    GSS_TRY(reserve(d_lits2_, (size_t) (n_lits + kClausePad) * sizeof(int32_t)));
+    GSS_TRY(reserve(d_offsets2_, ((size_t) n + 1) * sizeof(int64_t)));
+    GSS_TRY(reserve(d_orig2_, std::max<size_t>(n, 1) * sizeof(uint32_t)));
+    GSS_TRY(reserve(d_compact_, std::max<size_t>(n, 1) * sizeof(uint32_t)));
     GSS_CUDA_TRY(cudaMemcpy(d_offsets2_.ptr, offsets.data(), ((size_t) n + 1) * sizeof(int64_t),
                             cudaMemcpyHostToDevice));
     GSS_CUDA_TRY(cudaMemcpy(d_compact_.ptr, src.data(), std::max<size_t>(n, 1) * sizeof(uint32_t),

@@ -219,6 +219,22 @@ private:
         return (const StateUpdate *) ((const char *) d_updates_.ptr + updates_offset());
     }
     size_t updates_offset() const { return ((size_t) n_blocks_ * bw_ * 2 * sizeof(uint32_t) + 15) & ~(size_t) 15; }
+    // The filter's table, which a pass can do without, goes before clauses do:
+    // an allocation that fails is tried again once it is given back.
+    template <typename F>
+    int over_table(F allocate) {
+        const int rc = allocate();
+        if (rc != GSS_ERR_NOMEM || !d_agg_.ptr) return rc;
+        give_table_back();
+        return allocate();
+    }
+    int reserve(DevBuf &buf, size_t bytes) {
+        return over_table([&]() { return buf.reserve(bytes); });
+    }
+    int grow(DevBuf &buf, size_t bytes, size_t keep_bytes) {
+        return over_table([&]() { return buf.grow_keep(bytes, stream_, keep_bytes); });
+    }
+    void give_table_back();
     int rebuild_agg();
     int refresh_agg(int64_t n_updates);
     int ensure_state();

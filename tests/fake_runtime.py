@@ -15,12 +15,12 @@ class Fake:
     def __init__(self, folder):
         build.build()
         objs = [obj for _, obj, _ in build.compile_commands()]
-        fake, path = str(folder / "fake_cudart.o"), str(folder / "libfake.so")
+        fake, self.path = str(folder / "fake_cudart.o"), str(folder / "libfake.so")
         subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-I", build._cuda_include(), "-c",
                         os.path.join(HERE, "cpp", "fake_cudart.cpp"), "-o", fake], check=True)
         # (the library's own symbols first: a process may hold the real one too)
-        subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", path, *objs, fake, "-lpthread"], check=True)
-        self.lib = ctypes.CDLL(path)
+        subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", self.path, *objs, fake, "-lpthread"], check=True)
+        self.lib = ctypes.CDLL(self.path)
         self.lib.fake_log.restype = self.lib.gss_last_error.restype = ctypes.c_char_p
         self.lib.gss_engine_graph_captures.restype = i64
         self.lib.gss_sharer_add_clause.restype = i64

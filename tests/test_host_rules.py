@@ -196,6 +196,61 @@ def test_order_takes_the_table_before_the_pass_reads_it(fake):
     assert fake.lib.gss_engine_destroy(eng) == 0
 
 
+@pytest.fixture
+def sharer(fake, monkeypatch):
+    """The Python sharer over the library without a GPU: five solvers, every
+    pass behind the filter, one of them run."""
+    import gpusharesat_gb300 as g
+    monkeypatch.setattr(g, "_lib", None)
+    monkeypatch.setattr(g, "LIB_PATH", fake.path)
+    s = g.ClauseSharer(minGpuLatencyMicros=0, verbosity=0)
+    s.setFilterFrom(0)
+    s.setVarCount(60)
+    s.setCpuSolverCount(5)
+    _some_clauses(s, 50)
+    _some_passes(s)
+    assert s.filteredPasses() == 2
+    yield s
+    s.close()
+
+
+def _some_clauses(s, n):
+    for k in range(n):
+        assert s.addClause(-1, [2 * (k % 20), 2 * (20 + k % 20), 2 * (40 + k % 20)]) >= 0
+
+
+def _some_passes(s, n_vars=20):
+    for solver in range(5):
+        assert s.trySetSolverValues(solver, [2 * v for v in range(n_vars)])
+        s.trySendAssignment(solver)
+        s.unsetSolverValues(solver, [2 * v for v in range(n_vars)])
+    s.gpuRun()
+    for solver in range(5):
+        s.trySendAssignment(solver)
+    s.gpuRun()
+
+
+@pytest.mark.parametrize("grow", ["clauses", "updates", "variables", "solvers"])
+def test_sharer_drops_the_table_before_clauses(fake, sharer, grow):
+    """An allocation that fails takes the filter's table, not the clauses: the
+    database is not reduced and no out-of-memory is noted."""
+    before = sharer.getGlobalStat("gpuReduceDbs")
+    if grow == "clauses":
+        _some_clauses(sharer, 5000)
+    elif grow == "variables":
+        sharer.setVarCount(5000)
+    elif grow == "solvers":
+        sharer.setCpuSolverCount(40)
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 1)
+    if grow == "updates":
+        sharer.setVarCount(60)
+    for _ in range(3):
+        _some_passes(sharer, 60)
+    assert fake.lib.gss_debug_fail_device_alloc(i64(0), 0) == 0
+    assert not sharer.hasRunOutOfGpuMemoryOnce()
+    assert sharer.getGlobalStat("gpuReduceDbs") == before
+
+
 def test_staged_records_lie_on_16_bytes_by_type(tmp_path):
     here = os.path.dirname(os.path.abspath(__file__))
     subprocess.run([build._nvcc(), *build.ARCH, "-std=c++17", "-I", os.path.join(build.ROOT, "include"), "-I",
