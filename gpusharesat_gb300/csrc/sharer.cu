@@ -470,7 +470,9 @@ int Sharer::ensure_state() {
         return GSS_OK;
     }
     const size_t bytes = std::max<size_t>((size_t) n_blocks * std::max(need_vars, 1) * bw * sizeof(uint2), 8);
+    // (all the room first: a layout is taken whole or not at all)
     DevBuf fresh;
+    GSS_TRY(reserve(d_sow_, sizeof(int32_t) * n_blocks * bw));
     GSS_TRY(reserve(fresh, bytes));
     GSS_CUDA_TRY(cudaMemsetAsync(fresh.ptr, 0, bytes, stream_));
     if (d_state_.ptr && dev_vars_ > 0 && dev_words_ > 0) {
@@ -491,7 +493,6 @@ int Sharer::ensure_state() {
     eff_kind_ = kind;
     eff_lpc_ = lpc;
     eff_depth_ = depth;
-    GSS_TRY(reserve(d_sow_, sizeof(int32_t) * n_blocks * bw));
     std::vector<int32_t> sow(n_blocks * bw);
     for (int w = 0; w < n_blocks * bw; w++) sow[w] = w < n_words ? w : 0;
     GSS_CUDA_TRY(cudaMemcpy(d_sow_.ptr, sow.data(), sow.size() * sizeof(int32_t), cudaMemcpyHostToDevice));

@@ -197,21 +197,28 @@ def test_order_takes_the_table_before_the_pass_reads_it(fake):
 
 
 @pytest.fixture
-def sharer(fake, monkeypatch):
-    """The Python sharer over the library without a GPU: five solvers, every
-    pass behind the filter, one of them run."""
+def make_sharer(fake, monkeypatch):
+    """The Python sharer over the library without a GPU: five solvers, one
+    pass run with assignments and one without changes."""
     import gpusharesat_gb300 as g
     monkeypatch.setattr(g, "_lib", None)
     monkeypatch.setattr(g, "LIB_PATH", fake.path)
-    s = g.ClauseSharer(minGpuLatencyMicros=0, verbosity=0)
-    s.setFilterFrom(0)
-    s.setVarCount(60)
-    s.setCpuSolverCount(5)
-    _some_clauses(s, 50)
-    _some_passes(s)
-    assert s.filteredPasses() == 2
-    yield s
-    s.close()
+    made = []
+
+    def make(filter_from):
+        s = g.ClauseSharer(minGpuLatencyMicros=0, verbosity=0)
+        made.append(s)
+        s.setFilterFrom(filter_from)
+        s.setVarCount(60)
+        s.setCpuSolverCount(5)
+        _some_clauses(s, 50)
+        _some_passes(s)
+        assert s.filteredPasses() == (2 if filter_from == 0 else 0)
+        return s
+
+    yield make
+    for s in made:
+        s.close()
 
 
 def _some_clauses(s, n):
@@ -231,9 +238,10 @@ def _some_passes(s, n_vars=20):
 
 
 @pytest.mark.parametrize("grow", ["clauses", "updates", "variables", "solvers"])
-def test_sharer_drops_the_table_before_clauses(fake, sharer, grow):
+def test_sharer_drops_the_table_before_clauses(fake, make_sharer, grow):
     """An allocation that fails takes the filter's table, not the clauses: the
     database is not reduced and no out-of-memory is noted."""
+    sharer = make_sharer(0)
     before = sharer.getGlobalStat("gpuReduceDbs")
     if grow == "clauses":
         _some_clauses(sharer, 5000)
@@ -249,6 +257,18 @@ def test_sharer_drops_the_table_before_clauses(fake, sharer, grow):
     assert fake.lib.gss_debug_fail_device_alloc(i64(0), 0) == 0
     assert not sharer.hasRunOutOfGpuMemoryOnce()
     assert sharer.getGlobalStat("gpuReduceDbs") == before
+
+
+@pytest.mark.parametrize("after", [0, 1, 2])
+def test_sharer_layout_that_ran_out_of_memory_is_made_again(fake, make_sharer, after):
+    """The solvers' numbers of a new layout, 35 blocks of 32 words, reach the
+    device whichever of its allocations failed."""
+    sharer = make_sharer(1 << 60)  # (no table that could make room)
+    sharer.setCpuSolverCount(1100)
+    fake.reset()
+    fake.fail("malloc", after)
+    _some_passes(sharer)
+    assert any(l.startswith("copy") and l.split()[3] == str(4 * 32 * 35) for l in fake.log())
 
 
 def test_staged_records_lie_on_16_bytes_by_type(tmp_path):
