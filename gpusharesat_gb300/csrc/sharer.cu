@@ -292,7 +292,7 @@ int Sharer::set_variant(int kind, int lpc, int depth, int flags) {
     lpc_req_ = lpc;
     depth_req_ = depth;
     flags_ = flags;
-    dev_words_ = -1;  // force a re-layout at the next pass
+    relayout_ = true;
     return GSS_OK;
 }
 
@@ -463,7 +463,7 @@ int Sharer::ensure_state() {
     }
     const int bw = lpc * wpl;
     const int n_blocks = (n_words + bw - 1) / bw;
-    if (dev_vars_ == need_vars && dev_words_ == n_words && bw == bw_ && d_state_.ptr) {
+    if (dev_vars_ == need_vars && dev_words_ == n_words && bw == bw_ && d_state_.ptr && !relayout_) {
         eff_kind_ = kind;
         eff_lpc_ = lpc;
         eff_depth_ = depth;
@@ -499,6 +499,7 @@ int Sharer::ensure_state() {
     agg_possible_ = kind_ == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && need_vars > 0 && n_words > 0;
     agg_ok_ = false;
     filter_pause_ = 0;
+    relayout_ = false;
     return GSS_OK;
 }
 

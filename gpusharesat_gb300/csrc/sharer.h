@@ -311,6 +311,7 @@ private:
     // last-slot masks (n_blocks_ * bw_ words each), then the changed words
     DevBuf d_state_, d_sow_, d_updates_;
     DevBuf d_agg_;              // the filter's table of d_state_, kept as variables change
+    bool relayout_ = false;     // the variant changed: lay the state out at the next pass
     bool agg_possible_ = false; // the layout has a filtered kernel
     bool agg_ok_ = false;       // d_agg_ follows the state
     int filter_pause_ = 0;      // passes to run without the filter (it kept too much)

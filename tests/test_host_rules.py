@@ -271,6 +271,20 @@ def test_sharer_layout_that_ran_out_of_memory_is_made_again(fake, make_sharer, a
     assert any(l.startswith("copy") and l.split()[3] == str(4 * 32 * 35) for l in fake.log())
 
 
+def test_sharer_keeps_its_state_when_the_variant_changes(fake, make_sharer):
+    """The values that the solvers sent go over to the new layout, which runs
+    the kernel that was asked for."""
+    sharer = make_sharer(0)
+    for kind, lanes, kernel in ((3, 16, "check_wide_kernel"), (2, 8, "check_wide_kernel"), (0, 4, "check_kernel"),
+                                (-1, 0, "check_filtered_kernel")):
+        sharer.setVariant(kind, lanes, 2)
+        fake.reset()
+        _some_passes(sharer)
+        launched = [l.split()[1] for l in fake.log() if l.startswith("launch")]
+        assert sum("copy_layout_kernel" in l for l in launched) == 1, kind
+        assert sum(kernel in l for l in launched) == 2, (kind, launched)
+
+
 def test_staged_records_lie_on_16_bytes_by_type(tmp_path):
     here = os.path.dirname(os.path.abspath(__file__))
     subprocess.run([build._nvcc(), *build.ARCH, "-std=c++17", "-I", os.path.join(build.ROOT, "include"), "-I",

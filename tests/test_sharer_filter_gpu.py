@@ -152,6 +152,31 @@ def test_filter_switched_on_and_off(lib):
         plain.close()
 
 
+def test_variant_changed_between_passes(lib):
+    """The state that the solvers sent goes over to the layout of another
+    kernel, and back behind the filter."""
+    n_vars, n_solvers = 80, 12
+    rng = np.random.default_rng(4)
+    s, plain = _pair(n_vars, n_solvers)
+    try:
+        ses = _Session(rng, [s, plain], n_vars, n_solvers)
+        reports = 0
+        for step, variant in enumerate(((-1, 0, 2), (0, 4, 2), (2, 8, 2), (-1, 0, 2), (3, 16, 2), (-1, 0, 2))):
+            s.setVariant(*variant)
+            for _ in range(3):
+                ses.add(40, planted=8)
+                for solver in range(n_solvers):
+                    ses.move(solver, 30 if step == 0 else 4)
+                ses.run()
+                reports += ses.compare(step)
+        ses.run()
+        assert reports + ses.compare("end") > 50
+        assert s.filteredPasses() == 9  # (the last call's pass had nothing to do)
+    finally:
+        s.close()
+        plain.close()
+
+
 def test_evictions_and_reductions_behind_the_filter(lib):
     """Evicted clauses stay on the device as tombstones until a compaction;
     reduceDb moves the rest."""
