@@ -287,12 +287,31 @@ bool valid_filtered_variant(int wpl, int lpc);
 // A filtered pass that keeps more than this share of its (clause, block) pairs
 // costs more than the plain one (500k clauses x 1024 slots: 0.29 kept 51
 // against 62 us, 0.34 to 0.37 even, 0.40 73 against 67); the passes after it run
-// without, kFilterPause of them, before the next try.
+// without before the next try.
 constexpr double kFilterKeepMost = 1.0 / 3;
-constexpr int kFilterPause = 64;
 inline bool filter_keeps_too_much(uint32_t kept, int64_t n_clauses, int64_t n_blocks) {
     return (double) kept > kFilterKeepMost * (double) n_clauses * (double) n_blocks;
 }
+// How long: a state that comes and goes should not cost the ones after it the
+// filter, and one that stays should not be tried often. The pause doubles
+// with every try that fails, from 4 passes to 64 (a state that stays costs
+// five tries in its first 64 passes, one in 65 from then on), and starts
+// again where a try succeeds or the database or the layout is another.
+struct FilterPause {
+    static constexpr int kLeast = 4, kMost = 64;
+    int left = 0;  // passes to run without
+    int next = kLeast;
+    void note(bool kept_too_much) {  // of a pass that ran behind the filter
+        if (left > 0) return;        // (launched before the pause began)
+        if (kept_too_much) {
+            left = next;
+            next = next < kMost ? 2 * next : kMost;
+        } else {
+            next = kLeast;
+        }
+    }
+    void end() { left = 0, next = kLeast; }
+};
 // Its tasks are counted in 32 bits (with room for what the warps take past the end).
 constexpr uint64_t kMaxFilterTasks = 1ull << 31;
 inline uint64_t filter_tasks(const CheckArgs &a) { return ((uint64_t) scan_count(a) + 31) / 32 * a.n_blocks; }

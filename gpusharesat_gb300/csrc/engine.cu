@@ -479,6 +479,7 @@ int gss_db_set(gss_engine *eng, const int32_t *lits, const int64_t *offsets, int
     eng->next_id = 0;
     eng->db_epoch++;
     eng->layout_epoch++;
+    eng->filter_pause.end();
     mirror_append(eng, lits, offsets, n_clauses, nullptr, max_var);
     GSS_TRY(upload_all(eng));
     eng->max_var = max_var;
@@ -726,6 +727,7 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     // the caller's buffers are free (and the host vectors above too) when this returns
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
     if (filtered) eng->filter = use_filter(*h_density, (double) n_vars * n_words);
+    if (n_vars != eng->n_vars || n_words != eng->n_words) eng->filter_pause.end();
     eng->n_vars = n_vars;
     eng->n_words = n_words;
     eng->n_blocks = n_blocks;
@@ -957,8 +959,8 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     auto choose_filter = [&]() {
         const bool may = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
                          filter_tasks(a) < kMaxFilterTasks;
-        filtered = may && eng->filter_pause == 0;
-        if (may && eng->filter_pause > 0) eng->filter_pause--;
+        filtered = may && eng->filter_pause.left == 0;
+        if (may && !filtered) eng->filter_pause.left--;
         eng->pass_filtered = filtered;
         eng->filtered_passes += filtered;
     };
@@ -1087,8 +1089,7 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
 namespace {
 // After a pass: what its filter kept (hc: the counters on the host).
 void note_kept(gss_engine *eng, const uint32_t *hc, bool filtered) {
-    if (filtered && filter_keeps_too_much(hc[eng->n_parts + 1], eng->n_clauses, eng->n_blocks))
-        eng->filter_pause = kFilterPause;
+    if (filtered) eng->filter_pause.note(filter_keeps_too_much(hc[eng->n_parts + 1], eng->n_clauses, eng->n_blocks));
 }
 }  // namespace
 

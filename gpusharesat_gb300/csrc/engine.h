@@ -56,7 +56,7 @@ struct gss_engine {
     DevBuf agg;
     bool filter = false;
     bool pass_filtered = false;  // the pass launched last
-    int filter_pause = 0;        // passes to run without it: it kept too much
+    gss::FilterPause filter_pause;  // passes to run without it: it kept too much
     cudaEvent_t ev_caller = nullptr;  // the caller's work on the default stream (gss_state_set, on_device)
     int64_t n_vars = 0;
     int n_words = 0;

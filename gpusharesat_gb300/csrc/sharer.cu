@@ -498,7 +498,7 @@ int Sharer::ensure_state() {
     GSS_CUDA_TRY(cudaMemcpy(d_sow_.ptr, sow.data(), sow.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     agg_possible_ = kind_ == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && need_vars > 0 && n_words > 0;
     agg_ok_ = false;
-    filter_pause_ = 0;
+    filter_pause_.end();
     relayout_ = false;
     return GSS_OK;
 }
@@ -925,7 +925,7 @@ int Sharer::run_check(Pass &p) {
                      (kind_ == GSS_KERNEL_AUTO && valid_wide_persist_variant(wpl, eff_lpc_, eff_depth_)))) {
             // the persistent form, as the engine's automatic variant
             uint32_t *const work = work_counter(a.counts, n_parts_);
-            p.filtered = agg_ok_ && filter_pause_ == 0 && filter_tasks(a) < kMaxFilterTasks;
+            p.filtered = agg_ok_ && filter_pause_.left == 0 && filter_tasks(a) < kMaxFilterTasks;
             filtered_passes_ += p.filtered;
             if (p.filtered)
                 GSS_TRY(launch_check_filtered(nullptr, a, wpl, eff_lpc_, work, stream_, sm_count_));
@@ -1003,9 +1003,10 @@ int Sharer::collect(Pass &p) {
     }
     // a filter that keeps most clauses costs more than it saves: leave it out
     // for some passes, then look again
-    if (filter_pause_ > 0) filter_pause_--;
-    if (p.filtered && filter_keeps_too_much(((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1], p.n_clauses, n_blocks_))
-        filter_pause_ = kFilterPause;
+    if (filter_pause_.left > 0) filter_pause_.left--;
+    if (p.filtered)
+        filter_pause_.note(filter_keeps_too_much(((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1], p.n_clauses,
+                                                 n_blocks_));
     if (p.copying) GSS_CUDA_TRY(cudaEventRecord(p.copied, stream_));
     p.pending = false;
     p.collected = true;

@@ -314,7 +314,7 @@ private:
     bool relayout_ = false;     // the variant changed: lay the state out at the next pass
     bool agg_possible_ = false; // the layout has a filtered kernel
     bool agg_ok_ = false;       // d_agg_ follows the state
-    int filter_pause_ = 0;      // passes to run without the filter (it kept too much)
+    FilterPause filter_pause_;  // passes to run without the filter (it kept too much)
     int64_t filter_from_ = kFilterMinPairs;  // (clauses x slot blocks) from which passes run behind it
     int64_t filtered_passes_ = 0;
     PinnedBuf h_updates_;

@@ -22,7 +22,7 @@ class Fake:
         subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", self.path, *objs, fake, "-lpthread"], check=True)
         self.lib = ctypes.CDLL(self.path)
         self.lib.fake_log.restype = self.lib.gss_last_error.restype = ctypes.c_char_p
-        self.lib.gss_engine_graph_captures.restype = i64
+        self.lib.gss_engine_graph_captures.restype = self.lib.gss_engine_filtered_passes.restype = i64
         self.lib.gss_sharer_add_clause.restype = i64
 
     def log(self):

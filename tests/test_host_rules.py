@@ -196,6 +196,53 @@ def test_order_takes_the_table_before_the_pass_reads_it(fake):
     assert fake.lib.gss_engine_destroy(eng) == 0
 
 
+def _passes(fake, eng, n, kept=0, n_false=0):
+    """n passes; how many of them ran behind the filter."""
+    before = fake.lib.gss_engine_filtered_passes(eng)
+    fake.lib.fake_filter(ctypes.c_ulonglong(n_false), kept)
+    for _ in range(n):
+        assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+        assert fake.lib.gss_check_wait(eng, None) == 0, fake.error()
+    return fake.lib.gss_engine_filtered_passes(eng) - before
+
+
+@pytest.mark.parametrize("other", ["states", "database", "words", "variables"])
+def test_pause_of_the_filter_ends_with_what_caused_it(fake, other):
+    """One state of which the filter keeps too much: the states after it, or
+    another database or layout, do not wait 64 passes for the filter."""
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    _state(fake, eng, 20)
+    assert _passes(fake, eng, 1, kept=90) == 1
+    assert _passes(fake, eng, 3) == 0  # it pauses
+    if other == "states":
+        assert _passes(fake, eng, 1) == 0
+        for _ in range(10):
+            _state(fake, eng, 20)
+            assert _passes(fake, eng, 1) == 1
+    else:
+        if other == "database":
+            _database(fake, eng, 200)
+        elif other == "words":
+            _state(fake, eng, 21)
+        else:
+            _state(fake, eng, 20, 51)
+        assert _passes(fake, eng, 10) == 10
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def test_pause_of_the_filter_grows_while_it_keeps_too_much(fake):
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    _state(fake, eng, 20)
+    ran = [_passes(fake, eng, 1, kept=90) for _ in range(1 + 4 + 1 + 8 + 1 + 16 + 1 + 32 + 1 + 64 + 1 + 64 + 1)]
+    assert [k for k, r in enumerate(ran) if r] == [0, 5, 14, 31, 64, 129, 194]
+    # one success, and the next failure pauses for as long as the first
+    assert [_passes(fake, eng, 1) for _ in range(65)] == [0] * 64 + [1]
+    assert [_passes(fake, eng, 1, kept=90) for _ in range(6)] == [1, 0, 0, 0, 0, 1]
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
 @pytest.fixture
 def make_sharer(fake, monkeypatch):
     """The Python sharer over the library without a GPU: five solvers, one
