@@ -13,8 +13,8 @@
 // variables, and solvers of one formula agree on much, so on trails a clause
 // is dropped after 4 to 6 literals of 8 bytes, where the exact scan gathers 7
 // rows of 256 bytes. Independent fair-coin slots make every bit 1 and drop
-// nothing; the table's own density tells (use_filter), and such states keep
-// the plain kernel.
+// nothing; a sample of the state tells (use_filter), and such states keep
+// the plain kernel and get no table.
 //
 // (The reference tests a clause first against an aggregate over all solvers,
 // gpuShareLib/GpuRunner.cu:152-170; its aggregate is one bit per solver too,
@@ -351,16 +351,14 @@ __device__ __forceinline__ void row_entries(uint2 v, uint32_t real_words, int la
 // plain copy of it alone 123).
 template <int BW>
 __global__ void __launch_bounds__(256) load_state_kernel(const uint2 *__restrict__ src, uint2 *__restrict__ dst,
-                                                         uint2 *__restrict__ agg, unsigned long long *__restrict__ density,
-                                                         uint32_t n_vars, uint32_t n_words, uint32_t n_blocks,
-                                                         bool in_place) {
+                                                         uint2 *__restrict__ agg, uint32_t n_vars, uint32_t n_words,
+                                                         uint32_t n_blocks, bool in_place) {
     constexpr int RPW = 32 / BW;  // rows per warp step
     constexpr int kUnroll = 4;
     const int lane = threadIdx.x & 31;
     const uint32_t w = lane % BW;
     const uint64_t n_rows = (uint64_t) n_vars * n_blocks;  // row r: variable r / n_blocks, block r % n_blocks
     const uint64_t warps = (uint64_t) gridDim.x * (blockDim.x >> 5);
-    uint32_t n_false = 0;
     for (uint64_t s = (uint64_t) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s * kUnroll * RPW < n_rows;
          s += warps) {
         uint2 v[kUnroll];
@@ -388,21 +386,9 @@ __global__ void __launch_bounds__(256) load_state_kernel(const uint2 *__restrict
             if (agg) {
                 uint2 p, n;
                 row_entries<BW>(v[q], real[q], lane, p, n);
-                if (in && w == 0) {
-                    reinterpret_cast<uint4 *>(agg)[to[q]] = make_uint4(p.x, p.y, n.x, n.y);
-                    n_false += __popc(p.x) + __popc(n.x);
-                }
+                if (in && w == 0) reinterpret_cast<uint4 *>(agg)[to[q]] = make_uint4(p.x, p.y, n.x, n.y);
             }
         }
-    }
-    if (density) {
-        __shared__ uint32_t sum;
-        if (threadIdx.x == 0) sum = 0;
-        __syncthreads();
-        n_false = __reduce_add_sync(kFull, n_false);
-        if (lane == 0) atomicAdd(&sum, n_false);
-        __syncthreads();
-        if (threadIdx.x == 0) atomicAdd(density, (unsigned long long) sum);
     }
 }
 
@@ -427,9 +413,37 @@ __global__ void __launch_bounds__(256) refresh_agg_kernel(const StateUpdate *__r
     }
 }
 
-__global__ void load_masks_kernel(const uint32_t *__restrict__ start, const int32_t *__restrict__ sow,
-                                  uint32_t n_words, uint32_t padded, uint32_t *__restrict__ start_out,
-                                  int32_t *__restrict__ sow_out) {
+// Block 0 copies the masks; block 1 samples the state for the density of its
+// table, straight to the host: pairs spread over the state by a multiplicative
+// hash, 4 for a thread. 2^12 pairs tell the share of a bit to within 0.8%
+// (one standard deviation) in 2 us (2^14: 10), before a table is filled that
+// may not be wanted. (The kernel that fills the table had counted all its
+// bits, with a fill and a copy of their own: a whole gss_state_set of 8 words
+// and 2^18 variables 32 us; so 25 with the table and 22 without.)
+constexpr int kSampleThreads = 1024;
+__global__ void __launch_bounds__(kSampleThreads)
+    load_masks_kernel(const uint32_t *__restrict__ start, const int32_t *__restrict__ sow, uint32_t n_words,
+                      uint32_t padded, uint32_t *__restrict__ start_out, int32_t *__restrict__ sow_out,
+                      const uint2 *__restrict__ state, uint64_t n_pairs, uint32_t samples,
+                      uint32_t *__restrict__ n_false) {
+    if (blockIdx.x == 1) {
+        __shared__ uint32_t sum;
+        if (threadIdx.x == 0) sum = 0;
+        __syncthreads();
+        uint32_t n = 0;
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < samples; i += kSampleThreads) {
+            const uint64_t at = samples == n_pairs ? i : __umul64hi(((uint64_t) i + 1) * 0x9E3779B97F4A7C15ull, n_pairs);
+            const uint2 v = state[at];
+            n += ((v.x & ~v.y) != 0u) + ((v.x & v.y) != 0u);
+        }
+        n = __reduce_add_sync(kFull, n);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sum, n);
+        __syncthreads();
+        if (threadIdx.x == 0) *n_false = sum;
+        return;
+    }
+    if (start == nullptr) return;
     for (uint32_t w = threadIdx.x; w < padded; w += blockDim.x) {
         start_out[w] = w < n_words ? start[w] : 0u;
         sow_out[w] = w < n_words ? (sow ? sow[w] : (int32_t) w) : 0;
@@ -466,16 +480,15 @@ int launch_check_filtered(const CheckArgs *d_args, const CheckArgs &h_args, int 
     return set_error(GSS_ERR_INVALID, "no filtered kernel for %d words per lane, %d lanes", wpl, lpc);
 }
 
-int launch_load_state(const uint2 *src, uint2 *dst, uint2 *agg, unsigned long long *density, uint32_t n_vars,
-                      uint32_t n_words, uint32_t bw, uint32_t n_blocks, bool in_place, cudaStream_t stream,
-                      int sm_count) {
+int launch_load_state(const uint2 *src, uint2 *dst, uint2 *agg, uint32_t n_vars, uint32_t n_words, uint32_t bw,
+                      uint32_t n_blocks, bool in_place, cudaStream_t stream, int sm_count) {
     const uint64_t rows = (uint64_t) n_vars * n_blocks;
     if (rows == 0 || (in_place && !agg)) return GSS_OK;
     const uint64_t steps = (rows * bw + 127) / 128;  // 128 words a warp step
     const unsigned blocks = (unsigned) std::min<uint64_t>((steps + 7) / 8, (uint64_t) sm_count * 8);
 #define GSS_LOAD(B)                                                                                                  \
     if (bw == B) {                                                                                                   \
-        load_state_kernel<B><<<blocks, 256, 0, stream>>>(src, dst, agg, density, n_vars, n_words, n_blocks, in_place); \
+        load_state_kernel<B><<<blocks, 256, 0, stream>>>(src, dst, agg, n_vars, n_words, n_blocks, in_place);         \
         GSS_CUDA_TRY(cudaGetLastError());                                                                            \
         return GSS_OK;                                                                                               \
     }
@@ -485,9 +498,12 @@ int launch_load_state(const uint2 *src, uint2 *dst, uint2 *agg, unsigned long lo
 }
 
 int launch_load_masks(const uint32_t *start, const int32_t *solver_of_word, uint32_t n_words, uint32_t padded,
-                      uint32_t *start_out, int32_t *sow_out, cudaStream_t stream) {
-    if (padded == 0) return GSS_OK;
-    load_masks_kernel<<<1, 256, 0, stream>>>(start, solver_of_word, n_words, padded, start_out, sow_out);
+                      uint32_t *start_out, int32_t *sow_out, const uint2 *state, uint64_t n_pairs, uint32_t *n_false,
+                      cudaStream_t stream) {
+    if ((start == nullptr || padded == 0) && state == nullptr) return GSS_OK;
+    load_masks_kernel<<<state ? 2 : 1, kSampleThreads, 0, stream>>>(start, solver_of_word, n_words, padded, start_out,
+                                                                     sow_out, state, n_pairs,
+                                                                     (uint32_t) density_samples(n_pairs), n_false);
     GSS_CUDA_TRY(cudaGetLastError());
     return GSS_OK;
 }

@@ -317,11 +317,9 @@ constexpr uint64_t kMaxFilterTasks = 1ull << 31;
 inline uint64_t filter_tasks(const CheckArgs &a) { return ((uint64_t) scan_count(a) + 31) / 32 * a.n_blocks; }
 // [n_vars][n_words] -> [n_blocks][n_vars][bw], zero-padded words (in_place:
 // src is laid out already), and the filter's table `agg` (NULL: none), 16
-// bytes a variable and block. `density` (NULL: none; added to) gets the
-// number of the table's "false" bits, over both literals.
-int launch_load_state(const uint2 *src, uint2 *dst, uint2 *agg, unsigned long long *density, uint32_t n_vars,
-                      uint32_t n_words, uint32_t bw, uint32_t n_blocks, bool in_place, cudaStream_t stream,
-                      int sm_count);
+// bytes a variable and block.
+int launch_load_state(const uint2 *src, uint2 *dst, uint2 *agg, uint32_t n_vars, uint32_t n_words, uint32_t bw,
+                      uint32_t n_blocks, bool in_place, cudaStream_t stream, int sm_count);
 // A word of a variable's state that a pass changes.
 struct StateUpdate {
     uint32_t var;
@@ -333,8 +331,14 @@ struct StateUpdate {
 int launch_refresh_agg(const StateUpdate *u, uint32_t n, const uint2 *state, uint2 *agg, uint32_t n_vars,
                        uint32_t n_words, uint32_t bw, cudaStream_t stream, int sm_count);
 // start and solver_of_word of a pass from device memory, padded with zeros to
-// `padded` words; solver_of_word NULL: the word's own number.
+// `padded` words; solver_of_word NULL: the word's own number. With `state`,
+// n_pairs (variable, word) pairs in any order, also counts the "false" bits
+// that density_samples(n_pairs) of them give the filter's table, over both
+// literals, into *n_false (pinned). start NULL: the masks are there already.
 int launch_load_masks(const uint32_t *start, const int32_t *solver_of_word, uint32_t n_words, uint32_t padded,
-                      uint32_t *start_out, int32_t *sow_out, cudaStream_t stream);
+                      uint32_t *start_out, int32_t *sow_out, const uint2 *state, uint64_t n_pairs, uint32_t *n_false,
+                      cudaStream_t stream);
+constexpr uint64_t kDensitySamples = 1 << 12;
+inline uint64_t density_samples(uint64_t n_pairs) { return n_pairs < kDensitySamples ? n_pairs : kDensitySamples; }
 
 }  // namespace gss

@@ -144,7 +144,7 @@ int range_shift_for(int64_t max_var, int range_log2) {
 bool release_tables(gss_engine *eng) {
     if (!eng->agg.ptr && !eng->agg2.ptr && !eng->agg3.ptr) return false;
     cudaStreamSynchronize(eng->stream);  // a pass in flight may be reading them
-    eng->filter = false;
+    eng->filter = eng->table_ok = false;
     for (DevBuf *t : {&eng->agg, &eng->agg2, &eng->agg3}) t->release();
     return true;
 }
@@ -166,6 +166,48 @@ int words_per_lane(int kind) { return kind == GSS_KERNEL_WIDE4 ? 4 : kind == GSS
 // filter alone costs what it saves. In between it depends on how many clauses
 // report, which the pass itself tells (kFilterKeepMost).
 bool use_filter(uint64_t n_false, double pairs) { return pairs > 0 && (double) n_false < 0.55 * 2.0 * pairs; }
+
+// What a pass saves behind a table that pays, and what filling the table adds
+// to gss_state_set (in place: the state is read once more for it), in us. A
+// table is filled for the pass after it where it costs no more than that pass
+// saves. Measured on model and trail states, 2 to 100 literals a clause, pass
+// behind the table against plain, 5e3 / 2e5 / 4e5 clauses over 2^18 variables:
+// 8 words 21/23, 27/30, 32/37 us; 13 words 21/25, 27/31, 32/42; 32 words
+// 21/29, 27/42, 31/60; 64 words 21/28, 31/65, 39/96. gss_state_set with the
+// table against without, 2^18 / 2^20 variables: 8 words 25/22, 47/41; 13 words
+// 31/26, 70/61; 32 words 44/41, 114/99; 64 words 80/72, 240/224.
+double filter_gain(int64_t n_clauses, int n_words) {
+    return 0.25 * std::min(n_words, 32) + 2.0e-6 * (double) n_clauses * n_words;
+}
+double table_cost(int64_t n_vars, int n_blocks, int bw, bool in_place) {
+    const double rows = (double) n_vars * n_blocks, block_bytes = (double) n_vars * bw * sizeof(uint2);
+    return in_place ? 3.0 + 4.0e-6 * rows + block_bytes * n_blocks / 6.0e6 : 1.2 + 4.0e-6 * rows + block_bytes / 25.0e6;
+}
+
+// Whether the layout of the automatic variant has a filtered kernel.
+bool can_filter(const gss_engine *eng, int wpl, int lpc) {
+    return eng->kind == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc);
+}
+
+// Fills the engine's own table before a pass of its state where that pays.
+// (A state used once is not worth a table that costs more than one pass
+// saves; by the time its passes would have saved that much it is.)
+int ensure_table(gss_engine *eng) {
+    if (!eng->filter || eng->table_ok || eng->filter_pause.left > 0 ||
+        !can_filter(eng, words_per_lane(eng->state_kind), eng->state_lpc))
+        return GSS_OK;
+    eng->table_owed += filter_gain(eng->n_clauses, eng->n_words);
+    if (eng->table_owed < table_cost(eng->n_vars, eng->n_blocks, eng->state_bw, true)) return GSS_OK;
+    if (eng->agg.reserve((size_t) eng->n_blocks * eng->n_vars * 2 * sizeof(uint2)) != GSS_OK) {
+        eng->filter = false;  // no room: without
+        return GSS_OK;
+    }
+    GSS_TRY(launch_load_state((const uint2 *) eng->state.ptr, nullptr, (uint2 *) eng->agg.ptr, (uint32_t) eng->n_vars,
+                              (uint32_t) eng->n_words, (uint32_t) eng->state_bw, (uint32_t) eng->n_blocks, true,
+                              eng->stream, eng->sm_count));
+    eng->table_ok = true;
+    return GSS_OK;
+}
 
 int ensure_device(gss_engine *eng) {
     GSS_CUDA_TRY(cudaSetDevice(eng->device));
@@ -664,20 +706,20 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     GSS_TRY(eng->solver_of_word.reserve(std::max<size_t>(padded * sizeof(int32_t), 4)));
     const bool laid_out = n_blocks == 1 && n_words == bw;  // block-major and host layouts coincide
     if (sbytes && !laid_out && !read_state) GSS_TRY(reserve_over_table(eng, eng->state_raw, sbytes));
-    // the filter's table: only the automatic variant runs behind it; without
-    // room for it the passes run without
-    const bool want_agg = eng->kind == GSS_KERNEL_AUTO && valid_filtered_variant(wpl, lpc) && sbytes > 0;
-    eng->filter = false;
-    const size_t abytes = (size_t) n_blocks * n_vars * 2 * sizeof(uint2);
-    const bool filtered = want_agg && eng->agg.reserve(abytes + sizeof(unsigned long long)) == GSS_OK;
-    uint2 *const agg = filtered ? (uint2 *) eng->agg.ptr : nullptr;
-    // the count of its bits: behind the table, and on the host in a corner of
-    // the counters' pinned buffer
-    unsigned long long *const density = filtered ? (unsigned long long *) ((char *) agg + abytes) : nullptr;
-    if (filtered) {
-        GSS_CUDA_TRY(cudaMemsetAsync(density, 0, sizeof(unsigned long long), eng->stream));
-    }
-    unsigned long long *const h_density = (unsigned long long *) ((char *) eng->h_counts.ptr + kDensityOffset);
+    // The filter's table is filled on the way where the next pass is expected
+    // to run behind it and saves more than that; without room for it the
+    // passes run without.
+    const bool may_filter = can_filter(eng, wpl, lpc) && sbytes > 0;
+    if (n_vars != eng->n_vars || n_words != eng->n_words) eng->filter_pause.end();
+    eng->filter = eng->table_ok = false;
+    eng->table_owed = 0;
+    const bool fill = may_filter && !eng->dense_before && eng->filter_pause.left == 0 &&
+                      filter_gain(eng->n_clauses, n_words) >=
+                          table_cost(n_vars, n_blocks, bw, laid_out && !read_state) &&
+                      eng->agg.reserve((size_t) n_blocks * n_vars * 2 * sizeof(uint2)) == GSS_OK;
+    // the density's sample, in a corner of the counters' pinned buffer
+    uint32_t *const h_density = (uint32_t *) ((char *) eng->h_counts.ptr + kDensityOffset);
+    const uint64_t n_pairs = (uint64_t) n_vars * n_words;
     // start and solver_of_word, padded with zero words
     std::vector<uint32_t> st;
     std::vector<int32_t> sw;
@@ -687,10 +729,7 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
         GSS_CUDA_TRY(cudaEventRecord(eng->ev_caller, cudaStreamLegacy));
         GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_caller, 0));
     }
-    if (read_masks) {
-        GSS_TRY(launch_load_masks(start, solver_of_word, (uint32_t) n_words, (uint32_t) padded,
-                                  (uint32_t *) eng->start.ptr, (int32_t *) eng->solver_of_word.ptr, eng->stream));
-    } else if (padded) {
+    if (!read_masks && padded) {
         st.assign(padded, 0u);
         sw.assign(padded, 0);
         for (int w = 0; w < n_words; w++) sw[w] = w;
@@ -707,27 +746,29 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
         GSS_CUDA_TRY(cudaMemcpyAsync(eng->solver_of_word.ptr, sw.data(), padded * sizeof(int32_t),
                                      cudaMemcpyHostToDevice, eng->stream));
     }
-    if (sbytes) {
-        const cudaMemcpyKind dir = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-        const uint2 *src = (const uint2 *) state;
-        if (laid_out && !(read_state && filtered)) {
-            GSS_CUDA_TRY(cudaMemcpyAsync(eng->state.ptr, state, sbytes, dir, eng->stream));
-            src = (const uint2 *) eng->state.ptr;
-        } else if (!read_state) {
-            GSS_CUDA_TRY(cudaMemcpyAsync(eng->state_raw.ptr, state, sbytes, dir, eng->stream));
-            src = (const uint2 *) eng->state_raw.ptr;
-        }
-        GSS_TRY(launch_load_state(src, (uint2 *) eng->state.ptr, agg, density, (uint32_t) n_vars, (uint32_t) n_words,
-                                  (uint32_t) bw, (uint32_t) n_blocks, src == (const uint2 *) eng->state.ptr,
-                                  eng->stream, eng->sm_count));
+    const cudaMemcpyKind dir = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    const uint2 *src = (const uint2 *) state;
+    if (sbytes && laid_out && !(read_state && fill)) {
+        GSS_CUDA_TRY(cudaMemcpyAsync(eng->state.ptr, state, sbytes, dir, eng->stream));
+        src = (const uint2 *) eng->state.ptr;
+    } else if (sbytes && !read_state) {
+        GSS_CUDA_TRY(cudaMemcpyAsync(eng->state_raw.ptr, state, sbytes, dir, eng->stream));
+        src = (const uint2 *) eng->state_raw.ptr;
     }
-    if (filtered)
-        GSS_CUDA_TRY(cudaMemcpyAsync(h_density, density, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                     eng->stream));
+    GSS_TRY(launch_load_masks(read_masks ? start : nullptr, read_masks ? solver_of_word : nullptr, (uint32_t) n_words,
+                              (uint32_t) padded, (uint32_t *) eng->start.ptr, (int32_t *) eng->solver_of_word.ptr,
+                              may_filter ? src : nullptr, n_pairs, h_density, eng->stream));
+    if (sbytes)
+        GSS_TRY(launch_load_state(src, (uint2 *) eng->state.ptr, fill ? (uint2 *) eng->agg.ptr : nullptr,
+                                  (uint32_t) n_vars, (uint32_t) n_words, (uint32_t) bw, (uint32_t) n_blocks,
+                                  src == (const uint2 *) eng->state.ptr, eng->stream, eng->sm_count));
     // the caller's buffers are free (and the host vectors above too) when this returns
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
-    if (filtered) eng->filter = use_filter(*h_density, (double) n_vars * n_words);
-    if (n_vars != eng->n_vars || n_words != eng->n_words) eng->filter_pause.end();
+    if (may_filter) {
+        eng->filter = use_filter(*h_density, (double) density_samples(n_pairs));
+        eng->table_ok = fill;
+        eng->dense_before = !eng->filter;
+    }
     eng->n_vars = n_vars;
     eng->n_words = n_words;
     eng->n_blocks = n_blocks;
@@ -806,7 +847,9 @@ int gss_check_launch(gss_engine *eng) {
     if (!eng) return set_error(GSS_ERR_INVALID, "engine is NULL");
     GSS_TRY(ensure_device(eng));
     GSS_TRY(ensure_queues(eng));
-    GSS_TRY(launch_pass_into(eng, eng->state.ptr, eng->agg.ptr, eng->reports, eng->counts, eng->h_counts, kEngineInline));
+    GSS_TRY(ensure_table(eng));
+    GSS_TRY(launch_pass_into(eng, eng->state.ptr, eng->table_ok ? eng->agg.ptr : nullptr, eng->reports, eng->counts,
+                             eng->h_counts, kEngineInline));
     eng->launches++;
     eng->pass_pending = true;
     eng->inline_ok = true;
@@ -957,10 +1000,9 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
     bool filtered = false;
     eng->pass_filtered = false;
     auto choose_filter = [&]() {
-        const bool may = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && agg != nullptr &&
-                         filter_tasks(a) < kMaxFilterTasks;
-        filtered = may && eng->filter_pause.left == 0;
-        if (may && !filtered) eng->filter_pause.left--;
+        const bool may = persistent && eng->kind == GSS_KERNEL_AUTO && eng->filter && filter_tasks(a) < kMaxFilterTasks;
+        filtered = may && agg != nullptr && eng->filter_pause.left == 0;
+        if (may && eng->filter_pause.left > 0) eng->filter_pause.left--;
         eng->pass_filtered = filtered;
         eng->filtered_passes += filtered;
     };
@@ -1227,12 +1269,18 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
         return GSS_OK;
     };
     GSS_TRY(reserve_packed());
-    // The first state decides for all of them: a later one whose table keeps
-    // more costs time, not reports.
-    if (eng->filter) {
+    // The first state decides for all of them whether a table is filled while
+    // the filter does not pause: a later one whose table keeps more costs
+    // time, not reports. (slot 0 is the engine's own)
+    const bool tables = eng->filter && filter_gain(eng->n_clauses, n_words) >=
+                                           table_cost(n_vars, eng->n_blocks, eng->state_bw, direct);
+    if (tables) {
         const size_t abytes = (size_t) eng->n_blocks * n_vars * 2 * sizeof(uint2);
-        if (eng->agg2.reserve(abytes) != GSS_OK || eng->agg3.reserve(abytes) != GSS_OK) eng->filter = false;
+        for (DevBuf *t : {&eng->agg, &eng->agg2, &eng->agg3})
+            if (t->reserve(abytes) != GSS_OK) eng->filter = eng->table_ok = false;
+        GSS_TRY(ensure_table(eng));
     }
+    bool slot_table[NB] = {eng->table_ok, false, false};
     // packs pass b's reports (after its check, on the engine stream)
     auto pack = [&](int b, const DevBuf &rep, const DevBuf &cnt) -> int {
         if (!packed) return GSS_OK;
@@ -1252,6 +1300,12 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
 
     int launched = 0;
     bool slot_filtered[NB] = {false, false, false};
+    auto launch_slot = [&](int b) -> int {
+        GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, slot_table[b] ? agg_buf[b]->ptr : nullptr, *rep_buf[b],
+                                 *cnt_buf[b], *hcnt_buf[b], 0));
+        slot_filtered[b] = eng->pass_filtered;
+        return GSS_OK;
+    };
     // copies the reports of pass j back (the host waits for its kernel)
     auto finish = [&](int j) -> int {
         const int b = j % NB;
@@ -1276,13 +1330,13 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
             GSS_TRY(ensure_queues(eng));
             GSS_TRY(reserve_reports());
             GSS_TRY(reserve_packed());
-            GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, agg_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
+            GSS_TRY(launch_slot(b));
             GSS_TRY(pack(b, *rep_buf[b], *cnt_buf[b]));
             eng->launches++;
             GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[b], eng->stream));
             if (j + 1 < launched) {
                 const int nb = (j + 1) % NB;
-                GSS_TRY(launch_pass_into(eng, state_buf[nb]->ptr, agg_buf[nb]->ptr, *rep_buf[nb], *cnt_buf[nb], *hcnt_buf[nb], 0));
+                GSS_TRY(launch_slot(nb));
                 GSS_TRY(pack(nb, *rep_buf[nb], *cnt_buf[nb]));
                 eng->launches++;
                 GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[nb], eng->stream));
@@ -1325,18 +1379,19 @@ int passes_host(gss_engine *eng, int n_passes, const uint32_t *const *states, in
             GSS_CUDA_TRY(cudaMemcpyAsync(dst, states[i], sbytes, cudaMemcpyHostToDevice, eng->h2d));
             GSS_CUDA_TRY(cudaEventRecord(eng->ev_h2d[b], eng->h2d));
             GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_h2d[b], 0));
-            if (!direct || eng->filter)
+            slot_table[b] = tables && eng->filter && eng->filter_pause.left == 0;
+            if (b == 0) eng->table_ok = slot_table[0];
+            if (!direct || slot_table[b])
                 GSS_TRY(launch_load_state((const uint2 *) dst, (uint2 *) state_buf[b]->ptr,
-                                          eng->filter ? (uint2 *) agg_buf[b]->ptr : nullptr, nullptr,
-                                          (uint32_t) n_vars, (uint32_t) n_words, (uint32_t) eng->state_bw,
-                                          (uint32_t) eng->n_blocks, direct, eng->stream, eng->sm_count));
+                                          slot_table[b] ? (uint2 *) agg_buf[b]->ptr : nullptr, (uint32_t) n_vars,
+                                          (uint32_t) n_words, (uint32_t) eng->state_bw, (uint32_t) eng->n_blocks,
+                                          direct, eng->stream, eng->sm_count));
         }
         // report set b is free once pass i-3's reports are back
         if (i >= NB) GSS_CUDA_TRY(cudaStreamWaitEvent(eng->stream, eng->ev_d2h[b], 0));
-        GSS_TRY(launch_pass_into(eng, state_buf[b]->ptr, agg_buf[b]->ptr, *rep_buf[b], *cnt_buf[b], *hcnt_buf[b], 0));
+        GSS_TRY(launch_slot(b));
         GSS_TRY(pack(b, *rep_buf[b], *cnt_buf[b]));
         eng->launches++;
-        slot_filtered[b] = eng->pass_filtered;
         launched = i + 1;
         GSS_CUDA_TRY(cudaEventRecord(eng->ev_kernel[b], eng->stream));
         if (i > 0) GSS_TRY(finish(i - 1));

@@ -51,10 +51,13 @@ struct gss_engine {
 
     // assignment state, block-major [n_blocks][n_vars][state_bw words]
     DevBuf state, state_raw, start, solver_of_word;
-    // the filter's table of the state (and the count of its bits), and whether
-    // passes run behind it (use_filter)
+    // the filter's table of the state; whether the state is one whose passes
+    // may run behind it (use_filter) and it is filled (table_pays)
     DevBuf agg;
     bool filter = false;
+    bool table_ok = false;
+    double table_owed = 0;      // us that the passes of this state would have saved behind it
+    bool dense_before = false;  // the state before was none to filter: the next one is taken for its like
     bool pass_filtered = false;  // the pass launched last
     gss::FilterPause filter_pause;  // passes to run without it: it kept too much
     cudaEvent_t ev_caller = nullptr;  // the caller's work on the default stream (gss_state_set, on_device)

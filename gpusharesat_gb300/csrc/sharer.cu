@@ -520,8 +520,8 @@ int Sharer::rebuild_agg() {
     // without room for the table the passes run without it
     agg_ok_ = d_agg_.reserve((size_t) n_blocks_ * dev_vars_ * 2 * sizeof(uint2)) == GSS_OK;
     if (!agg_ok_) return GSS_OK;
-    return launch_load_state((const uint2 *) d_state_.ptr, nullptr, (uint2 *) d_agg_.ptr, nullptr,
-                             (uint32_t) dev_vars_, (uint32_t) dev_words_, (uint32_t) bw_, (uint32_t) n_blocks_, true,
+    return launch_load_state((const uint2 *) d_state_.ptr, nullptr, (uint2 *) d_agg_.ptr, (uint32_t) dev_vars_,
+                             (uint32_t) dev_words_, (uint32_t) bw_, (uint32_t) n_blocks_, true,
                              stream_, sm_count_);
 }
 

@@ -24,8 +24,8 @@ std::map<const void *, std::string> &kernels() {
 int streams = 0, events = 0;
 std::string fail_fn;
 int fail_after = 0;  // calls of fail_fn to let through first
-unsigned long long false_bits = 0;  // what the filter's tables hold
-unsigned kept_pairs = 0;            // what filtered passes keep
+unsigned false_bits = 0;   // what a sample of the state finds
+unsigned kept_pairs = 0;   // what filtered passes keep
 uintptr_t far_begin = 0, far_end = 0;  // memory of device 1
 dim3 cfg_grid, cfg_block;
 
@@ -59,7 +59,7 @@ void fake_fail(const char *fn, int after) {
     fail_fn = fn;
     fail_after = after;
 }
-void fake_filter(unsigned long long n_false, unsigned kept) {
+void fake_filter(unsigned n_false, unsigned kept) {
     false_bits = n_false;
     kept_pairs = kept;
 }
@@ -92,13 +92,12 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3, void **args, siz
     const std::string &name = kernels()[(const void *) k];
     log_text += "launch " + name;
     // the buffers these read
-    const int n = name.find("load_") != std::string::npos ? 2 : 0;
-    for (int i = 0; i < n; i++) note(" %llx", *(unsigned long long *) args[i], 0, 0);
+    const bool masks = name.find("load_masks_kernel") != std::string::npos;
+    if (masks || name.find("load_state_kernel") != std::string::npos)
+        for (int i : {0, masks ? 1 : 0, masks ? 6 : 0}) note(" %llx", *(unsigned long long *) args[i], 0, 0);
+    if (!masks && name.find("load_state_kernel") != std::string::npos && *(void **) args[2]) log_text += " table";
     note(" grid %llu\n", grid.x, 0, 0);
-    if (name.find("load_state_kernel") != std::string::npos) {  // (src, dst, table, count of its bits, ...)
-        unsigned long long *const count = *(unsigned long long **) args[3];
-        if (count) *count = false_bits;
-    }
+    if (masks && *(void **) args[6]) **(unsigned **) args[9] = false_bits;  // (.., state, pairs, samples, count)
     if (name.find("deliver_kernel") != std::string::npos)  // (.., n_parts, cap, host: counters, error flag, kept)
         (*(unsigned **) args[5])[*(unsigned *) args[3] + 1] = kept_pairs;
     return cudaSuccess;

@@ -72,8 +72,8 @@ def test_noalloc_refuses_what_the_kernel_cannot_read(fake):
 
 
 def _read_by_kernels(fake):
-    """The first two addresses given to the kernels that load states and masks."""
-    return {int(a, 16) for l in fake.log() if l.startswith("launch") and "load_" in l for a in l.split()[2:4]}
+    """The buffers given to the kernels that load states and masks."""
+    return {int(a, 16) for l in fake.log() if l.startswith("launch") and "load_" in l for a in l.split()[2:5]}
 
 
 @pytest.mark.parametrize("n_words", [1, 3, 8, 32, 33, 64])
@@ -199,7 +199,7 @@ def test_order_takes_the_table_before_the_pass_reads_it(fake):
 def _passes(fake, eng, n, kept=0, n_false=0):
     """n passes; how many of them ran behind the filter."""
     before = fake.lib.gss_engine_filtered_passes(eng)
-    fake.lib.fake_filter(ctypes.c_ulonglong(n_false), kept)
+    fake.lib.fake_filter(n_false, kept)
     for _ in range(n):
         assert fake.lib.gss_check_launch(eng) == 0, fake.error()
         assert fake.lib.gss_check_wait(eng, None) == 0, fake.error()
@@ -240,6 +240,98 @@ def test_pause_of_the_filter_grows_while_it_keeps_too_much(fake):
     # one success, and the next failure pauses for as long as the first
     assert [_passes(fake, eng, 1) for _ in range(65)] == [0] * 64 + [1]
     assert [_passes(fake, eng, 1, kept=90) for _ in range(6)] == [1, 0, 0, 0, 0, 1]
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def _tables(fake):
+    return sum("load_state_kernel" in l and " table" in l for l in fake.log())
+
+
+def _device_state(fake, eng, n_words, n_vars, n_false):
+    """A state and masks in (the fake's) device memory; what its sample finds."""
+    room = ctypes.create_string_buffer(8 * n_vars * n_words + 8 * n_words + 512)
+    base = (ctypes.addressof(room) + 255) // 256 * 256
+    fake.lib.fake_filter(n_false, 0)
+    assert fake.lib.gss_state_set(eng, vp(base), i64(n_vars), n_words, vp(base + 8 * n_vars * n_words), None,
+                                  1) == 0, fake.error()
+
+
+@pytest.mark.parametrize("n_words", [8, 20, 32, 40])
+def test_no_table_for_states_that_do_not_run_behind_it(fake, n_words):
+    """A dense state (fair-coin slots set nearly every bit) after a dense one
+    gets no table, and is a plain copy where the layouts are the same; the
+    first sparse one after them runs behind one."""
+    n_vars = 50
+    dense = min(4096, n_vars * n_words) * 2
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    _device_state(fake, eng, n_words, n_vars, dense)
+    for _ in range(3):
+        fake.reset()
+        _device_state(fake, eng, n_words, n_vars, dense)
+        assert _tables(fake) == 0
+        assert any(l.startswith("copy") and int(l.split()[3]) == 8 * n_vars * n_words for l in fake.log()) == \
+            (n_words in (8, 32))
+        assert _passes(fake, eng, 2, n_false=dense) == 0 and _tables(fake) == 0
+    _device_state(fake, eng, n_words, n_vars, dense // 10)
+    assert _passes(fake, eng, 4) >= 3
+    fake.reset()
+    _device_state(fake, eng, n_words, n_vars, dense // 10)
+    assert _tables(fake) == 1 and _passes(fake, eng, 1) == 1 and _tables(fake) == 1
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def test_no_table_during_a_pause(fake):
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    _device_state(fake, eng, 20, 50, 0)
+    assert _passes(fake, eng, 1, kept=90) == 1
+    fake.reset()
+    for k in range(4):
+        _device_state(fake, eng, 20, 50, 0)
+        assert _passes(fake, eng, 1) == 0 and _tables(fake) == 0
+    _device_state(fake, eng, 20, 50, 0)
+    assert _passes(fake, eng, 1) == 1 and _tables(fake) == 1
+    # a pause that ends over a state that was set during it
+    assert _passes(fake, eng, 1, kept=90) == 1
+    _device_state(fake, eng, 20, 50, 0)
+    fake.reset()
+    assert [_passes(fake, eng, 1) for _ in range(6)] == [0, 0, 0, 0, 1, 1] and _tables(fake) == 1
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def test_no_table_that_costs_more_than_it_saves(fake):
+    """A hundred clauses against 2^19 variables: gss_state_set fills no table;
+    passes over the same state fill it once they would have saved as much."""
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    fake.reset()
+    _device_state(fake, eng, 8, 1 << 19, 0)
+    assert _tables(fake) == 0
+    ran = [_passes(fake, eng, 1) for _ in range(12)]
+    assert ran[0] == 0 and ran[-1] == 1 and ran == sorted(ran) and _tables(fake) == 1
+    _device_state(fake, eng, 8, 1 << 19, 0)
+    assert _passes(fake, eng, 1) == 0 and _tables(fake) == 1
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def test_host_passes_without_tables(fake):
+    """Dense states through gss_check_passes_host: no pass gets a table."""
+    n_vars, n_words = 50, 20
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    states = [(ctypes.c_uint32 * (2 * n_vars * n_words))() for _ in range(7)]
+    start = (ctypes.c_uint32 * n_words)(*[0xFFFFFFFF] * n_words)
+    outs = [(ctypes.c_uint32 * 64)() for _ in states]
+    call = lambda: fake.lib.gss_check_passes_host(
+        eng, len(states), (vp * 7)(*[ctypes.addressof(s) for s in states]), i64(n_vars), n_words, start, None,
+        (vp * 7)(*[ctypes.addressof(o) for o in outs]), (i64 * 7)(*[16] * 7), (i64 * 7)())
+    for n_false, kept, tables, filtered in ((0, 0, 7, 7), (2000, 0, 1, 0), (2000, 0, 0, 0), (0, 0, 7, 7)):
+        fake.reset()
+        fake.lib.fake_filter(n_false, kept)
+        before = fake.lib.gss_engine_filtered_passes(eng)
+        assert call() == 0, fake.error()
+        assert (_tables(fake), fake.lib.gss_engine_filtered_passes(eng) - before) == (tables, filtered)
     assert fake.lib.gss_engine_destroy(eng) == 0
 
 
