@@ -992,6 +992,13 @@ int Sharer::collect(Pass &p) {
         GSS_TRY(run_check(p));
         GSS_CUDA_TRY(cudaEventSynchronize(p.counted));
     }
+    // a filter that keeps most clauses costs more than it saves: leave it out
+    // for some passes, then look again
+    if (filter_pause_.left > 0) filter_pause_.left--;
+    if (p.filtered)
+        filter_pause_.note(filter_keeps_too_much(((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1], p.n_clauses,
+                                                 n_blocks_));
+    if (filter_pause_.left > 0) agg_ok_ = false;  // no upkeep meanwhile
     // the pass's variables take their last slot's value in all 32 slots
     // (stream-ordered: the next pass's updates are scattered after this)
     if (p.n_updates > 0) {
@@ -1001,12 +1008,6 @@ int Sharer::collect(Pass &p) {
         GSS_CUDA_TRY(cudaGetLastError());
         if (agg_ok_) GSS_TRY(refresh_agg(p.n_updates));
     }
-    // a filter that keeps most clauses costs more than it saves: leave it out
-    // for some passes, then look again
-    if (filter_pause_.left > 0) filter_pause_.left--;
-    if (p.filtered)
-        filter_pause_.note(filter_keeps_too_much(((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1], p.n_clauses,
-                                                 n_blocks_));
     if (p.copying) GSS_CUDA_TRY(cudaEventRecord(p.copied, stream_));
     p.pending = false;
     p.collected = true;
@@ -1172,7 +1173,8 @@ int Sharer::launch_pass() {
             GSS_CUDA_TRY(cudaGetLastError());
         }
         // the filter's table follows while the database is large enough for it
-        if (!agg_possible_ || (int64_t) dev_clauses_ * n_blocks_ < filter_from_)
+        // and passes run behind it; after that it is filled anew
+        if (!agg_possible_ || filter_pause_.left > 0 || (int64_t) dev_clauses_ * n_blocks_ < filter_from_)
             agg_ok_ = false;
         else if (!agg_ok_)
             GSS_TRY(rebuild_agg());

@@ -398,6 +398,28 @@ def test_sharer_drops_the_table_before_clauses(fake, make_sharer, grow):
     assert sharer.getGlobalStat("gpuReduceDbs") == before
 
 
+def test_sharer_keeps_no_table_up_during_a_pause(fake, make_sharer):
+    """One pass of which the filter keeps too much, then passes without it: no
+    launch fills or refreshes the table until it is used again."""
+    sharer = make_sharer(0)
+    upkeep = lambda: [l.split()[1] for l in fake.log() if "refresh_agg" in l or " table" in l]
+
+    def one(kept):
+        fake.reset()
+        fake.lib.fake_filter(0, kept)
+        before = sharer.filteredPasses()
+        assert sharer.trySetSolverValues(1, [2, 5])
+        sharer.trySendAssignment(1)
+        sharer.unsetSolverValues(1, [2, 5])
+        sharer.gpuRun()
+        return sharer.filteredPasses() - before, len(upkeep())
+
+    assert one(0)[0] == 1
+    assert one(90) == (1, 2)  # refreshed after the pass before, and for its own updates
+    assert [one(0) for _ in range(4)] == [(0, 0)] * 4
+    assert one(0) == (1, 1) and one(0) == (1, 2)  # filled anew, then kept up
+
+
 @pytest.mark.parametrize("after", [0, 1, 2])
 def test_sharer_layout_that_ran_out_of_memory_is_made_again(fake, make_sharer, after):
     """The solvers' numbers of a new layout, 35 blocks of 32 words, reach the

@@ -152,6 +152,37 @@ def test_filter_switched_on_and_off(lib):
         plain.close()
 
 
+def test_table_after_a_pause(lib):
+    """Most clauses are false under some solver's trail for a while: the filter
+    keeps them and pauses, the state moves on without its table, and the passes
+    behind the table filled anew report what the plain ones do."""
+    n_vars, n_solvers = 60, 9
+    rng = np.random.default_rng(5)
+    s, plain = _pair(n_vars, n_solvers)
+    try:
+        ses = _Session(rng, [s, plain], n_vars, n_solvers)
+        filtered = []
+        for step in range(60):
+            if step in (0, 30):
+                for x in ses.every:  # short clauses, half of them reporting in each of many words
+                    for k in range(300):
+                        x.addClause(-1, [lit(k % n_vars, k % 3 == 0), lit((k + 7) % n_vars, k % 2 == 0)])
+            if step in (12, 42):  # and many more that do not
+                ses.add(3000, planted=20)
+            for solver in range(n_solvers):
+                ses.move(solver, 40 if step % 10 == 0 else 5)
+            ses.run()
+            filtered.append(s.filteredPasses())
+            ses.compare(step)
+        ses.run()
+        ses.compare("end")
+        assert filtered[0] == 1 and filtered[4] == 1  # it pauses after the first
+        assert filtered[-1] > 20
+    finally:
+        s.close()
+        plain.close()
+
+
 def test_variant_changed_between_passes(lib):
     """The state that the solvers sent goes over to the layout of another
     kernel, and back behind the filter."""
