@@ -289,8 +289,7 @@ int gss_engine_destroy(gss_engine *eng) {
     cudaSetDevice(eng->device);
     if (eng->stream) cudaStreamSynchronize(eng->stream);
     if (eng->own_stream) cudaStreamDestroy(eng->own_stream);
-    if (eng->graph_exec) cudaGraphExecDestroy(eng->graph_exec);
-    if (eng->graph) cudaGraphDestroy(eng->graph);
+    for (auto &g : eng->graphs) g.clear();
     if (eng->ev_caller) cudaEventDestroy(eng->ev_caller);
     if (eng->h2d) cudaStreamDestroy(eng->h2d);
     if (eng->d2h) cudaStreamDestroy(eng->d2h);
@@ -1048,24 +1047,22 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
                 (uintptr_t) a.counts, (uintptr_t) h_counts.ptr, (uintptr_t) max_inline,
                 (uintptr_t) eng->d_args.ptr, (uintptr_t) eng->state_kind, (uintptr_t) eng->state_lpc,
                 (uintptr_t) eng->state_g, (uintptr_t) eng->n_parts, (uintptr_t) (a.n_clauses > 0 && a.n_blocks > 0),
-                (uintptr_t) bucketed, (uintptr_t) filtered, (uintptr_t) eng->d_plan.ptr, (uintptr_t) (eng->plan_ranges > 0)};
-            if (key != eng->graph_key || !eng->graph_exec) {
-                if (eng->graph_exec) cudaGraphExecDestroy(eng->graph_exec);
-                if (eng->graph) cudaGraphDestroy(eng->graph);
-                eng->graph_exec = nullptr;
-                eng->graph = nullptr;
+                (uintptr_t) bucketed, (uintptr_t) eng->d_plan.ptr, (uintptr_t) (eng->plan_ranges > 0)};
+            gss_engine::PassGraph &pg = eng->graphs[filtered ? 1 : 0];
+            if (key != pg.key || !pg.exec) {
+                pg.clear();
                 GSS_CUDA_TRY(cudaStreamBeginCapture(eng->stream, cudaStreamCaptureModeThreadLocal));
                 const int rc = body();
                 cudaGraph_t g = nullptr;
                 const cudaError_t e = cudaStreamEndCapture(eng->stream, &g);
                 GSS_TRY(rc);
                 if (e != cudaSuccess) return set_error(GSS_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-                eng->graph = g;
-                GSS_CUDA_TRY(cudaGraphInstantiate(&eng->graph_exec, g, 0));
-                eng->graph_key = key;
+                pg.graph = g;
+                GSS_CUDA_TRY(cudaGraphInstantiate(&pg.exec, g, 0));
+                pg.key = key;
                 eng->graph_captures++;
             }
-            GSS_CUDA_TRY(cudaGraphLaunch(eng->graph_exec, eng->stream));
+            GSS_CUDA_TRY(cudaGraphLaunch(pg.exec, eng->stream));
         } else {
             GSS_TRY(body());
         }

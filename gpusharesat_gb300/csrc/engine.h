@@ -107,9 +107,19 @@ struct gss_engine {
     uint64_t plan_built = ~0ull;
     uint32_t plan_ranges = 0;
     bool use_graph = false;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
-    std::vector<uintptr_t> graph_key;
+    // one for plain passes and one for those behind the filter: a database or
+    // a state that makes passes change between them does not capture again
+    struct PassGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        std::vector<uintptr_t> key;
+        void clear() {
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+            exec = nullptr;
+            graph = nullptr;
+        }
+    } graphs[2];
     int64_t graph_captures = 0;
     int64_t filtered_passes = 0;
 

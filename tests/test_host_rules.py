@@ -256,6 +256,17 @@ def _device_state(fake, eng, n_words, n_vars, n_false):
                                   1) == 0, fake.error()
 
 
+def test_one_capture_for_plain_and_one_for_filtered_passes(fake):
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    assert fake.lib.gss_engine_set_graph(eng, 1) == 0
+    _state(fake, eng, 20)
+    ran = [_passes(fake, eng, 1, kept=90) for _ in range(40)]
+    assert 0 < sum(ran) < 40 and fake.lib.gss_engine_graph_captures(eng) == 2
+    assert fake.log().count("graph") == 40
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
 @pytest.mark.parametrize("n_words", [8, 20, 32, 40])
 def test_no_table_for_states_that_do_not_run_behind_it(fake, n_words):
     """A dense state (fair-coin slots set nearly every bit) after a dense one
