@@ -284,13 +284,19 @@ bool valid_narrow_variant(int words);
 int launch_check_filtered(const CheckArgs *d_args, const CheckArgs &h_args, int wpl, int lpc, uint32_t *work,
                           cudaStream_t stream, int sm_count);
 bool valid_filtered_variant(int wpl, int lpc);
-// A filtered pass that keeps more than this share of its (clause, block) pairs
-// costs more than the plain one (500k clauses x 1024 slots: 0.29 kept 51
-// against 62 us, 0.34 to 0.37 even, 0.40 73 against 67); the passes after it run
-// without before the next try.
-constexpr double kFilterKeepMost = 1.0 / 3;
-inline bool filter_keeps_too_much(uint32_t kept, int64_t n_clauses, int64_t n_blocks) {
-    return (double) kept > kFilterKeepMost * (double) n_clauses * (double) n_blocks;
+// The share of its (clause, block) pairs that a filtered pass may keep: past it
+// the pass costs more than the plain one, and the passes after it run without
+// before the next try. The plain scan of a narrow block is cheap, so the line
+// lies lower there. Break-even measured over states of rising mixture, clauses
+// of 3, 2 to 30, 2 to 100, 20 to 60 and Zipf lengths, 5e5 and 1e6 of them, 2^13 /
+// 2^16 / 2^18 / 2^20 variables: 8 words 0.20, 0.20, 0.05, 0.20; 16 words 0.30,
+// 0.30, 0.25, 0.33; 32 words 0.6, 0.6, 0.33, 0.5; two blocks of 32 over 2^18
+// 0.38. Under these lines no measured pass of 16 or 32 words lost to the plain
+// one (32 words: 0.96 of it at most), six of 136 of 8 words lost 5 to 14%, and
+// three of 90 of 14 words 6 to 19%; with 1/3 for all, 8 words had lost up to 48%.
+inline double filter_keep_most(int bw) { return bw <= 8 ? 0.10 : bw <= 16 ? 0.20 : 1.0 / 3; }
+inline bool filter_keeps_too_much(uint32_t kept, int64_t n_clauses, int64_t n_blocks, int bw) {
+    return (double) kept > filter_keep_most(bw) * (double) n_clauses * (double) n_blocks;
 }
 // How long: a state that comes and goes should not cost the ones after it the
 // filter, and one that stays should not be tried often. The pause doubles

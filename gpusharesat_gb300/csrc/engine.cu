@@ -160,12 +160,16 @@ int words_per_lane(int kind) { return kind == GSS_KERNEL_WIDE4 ? 4 : kind == GSS
 // Whether the word-level filter pays for a state whose table has so many
 // bits set, of `pairs` (variable, word) pairs: F is the share of (literal,
 // word) pairs where some slot makes the literal false; a word outlives k
-// literals with a probability near F^k + k F^(k-1). Measured on 500k clauses x
-// 1024 slots over states of rising mixture, filtered against plain: F = 0.25
-// 28 to 49 against 58 to 67 us, 0.33 43 to 62 against 69 to 72; past 0.6 the
-// filter alone costs what it saves. In between it depends on how many clauses
-// report, which the pass itself tells (kFilterKeepMost).
-bool use_filter(uint64_t n_false, double pairs) { return pairs > 0 && (double) n_false < 0.55 * 2.0 * pairs; }
+// literals with a probability near F^k + k F^(k-1). Past the line the reading
+// of the table alone costs what it saves, whatever it keeps: states of rising
+// mixture, filtered against plain, 2 to 100 literals a clause and 32 words:
+// F = 0.25 22 against 54 us, 0.40 52 against 68, 0.55 75 against 76, 0.61 87
+// against 83 (2^18 variables); 0.48 122 against 167, 0.61 177 against 208, 0.68
+// 218 against 218 (2^20). The crossover is 0.54 to 0.67 at 8 to 64 words; with
+// 20 to 60 literals 0.67 to over 0.75. Short clauses cross earlier (2 to 30
+// literals 0.35 to 0.50, 3 literals 0.29), by what the filter keeps of them,
+// which the pass itself tells (filter_keep_most).
+bool use_filter(uint64_t n_false, double pairs) { return pairs > 0 && (double) n_false < 0.60 * 2.0 * pairs; }
 
 // What a pass saves behind a table that pays, and what filling the table adds
 // to gss_state_set (in place: the state is read once more for it), in us. A
@@ -1128,7 +1132,8 @@ int launch_pass_into(gss_engine *eng, const void *state, const void *agg, DevBuf
 namespace {
 // After a pass: what its filter kept (hc: the counters on the host).
 void note_kept(gss_engine *eng, const uint32_t *hc, bool filtered) {
-    if (filtered) eng->filter_pause.note(filter_keeps_too_much(hc[eng->n_parts + 1], eng->n_clauses, eng->n_blocks));
+    if (filtered) eng->filter_pause.note(filter_keeps_too_much(hc[eng->n_parts + 1], eng->n_clauses, eng->n_blocks,
+                                                         eng->state_bw));
 }
 }  // namespace
 

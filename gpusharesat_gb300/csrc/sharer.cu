@@ -997,7 +997,7 @@ int Sharer::collect(Pass &p) {
     if (filter_pause_.left > 0) filter_pause_.left--;
     if (p.filtered)
         filter_pause_.note(filter_keeps_too_much(((const uint32_t *) p.h_counts.ptr)[n_parts_ + 1], p.n_clauses,
-                                                 n_blocks_));
+                                                 n_blocks_, bw_));
     if (filter_pause_.left > 0) agg_ok_ = false;  // no upkeep meanwhile
     // the pass's variables take their last slot's value in all 32 slots
     // (stream-ordered: the next pass's updates are scattered after this)

@@ -256,6 +256,29 @@ def _device_state(fake, eng, n_words, n_vars, n_false):
                                   1) == 0, fake.error()
 
 
+@pytest.mark.parametrize("n_words,most", [(5, 10), (8, 10), (9, 20), (16, 20), (17, 33), (32, 33), (40, 66)])
+def test_share_the_filter_may_keep(fake, n_words, most):
+    """Of 100 clauses, a block each: narrow blocks pause earlier, whose plain
+    scan is cheap."""
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    _state(fake, eng, n_words)
+    _passes(fake, eng, 2)
+    assert _passes(fake, eng, 3, kept=most) == 3
+    assert _passes(fake, eng, 2, kept=most + 1) == 1
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+@pytest.mark.parametrize("share,behind", [(0.59, True), (0.61, False)])
+def test_density_up_to_which_passes_are_filtered(fake, share, behind):
+    rc, eng = fake.engine()
+    _database(fake, eng)
+    fake.lib.fake_filter(int(share * 2 * 50 * 20), 0)
+    _state(fake, eng, 20)
+    assert _passes(fake, eng, 1, n_false=int(share * 2 * 50 * 20)) == behind
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
 def test_one_capture_for_plain_and_one_for_filtered_passes(fake):
     rc, eng = fake.engine()
     _database(fake, eng)
