@@ -171,18 +171,11 @@ int words_per_lane(int kind) { return kind == GSS_KERNEL_WIDE4 ? 4 : kind == GSS
 // which the pass itself tells (filter_keep_most).
 bool use_filter(uint64_t n_false, double pairs) { return pairs > 0 && (double) n_false < 0.60 * 2.0 * pairs; }
 
-// What a pass saves behind a table that pays, and what filling the table adds
-// to gss_state_set (in place: the state is read once more for it), in us. A
-// table is filled for the pass after it where it costs no more than that pass
-// saves. Measured on model and trail states, 2 to 100 literals a clause, pass
-// behind the table against plain, 5e3 / 2e5 / 4e5 clauses over 2^18 variables:
-// 8 words 21/23, 27/30, 32/37 us; 13 words 21/25, 27/31, 32/42; 32 words
-// 21/29, 27/42, 31/60; 64 words 21/28, 31/65, 39/96. gss_state_set with the
-// table against without, 2^18 / 2^20 variables: 8 words 25/22, 47/41; 13 words
-// 31/26, 70/61; 32 words 44/41, 114/99; 64 words 80/72, 240/224.
-double filter_gain(int64_t n_clauses, int n_words) {
-    return 0.25 * std::min(n_words, 32) + 2.0e-6 * (double) n_clauses * n_words;
-}
+// What filling the table adds to gss_state_set (in place: the state is read
+// once more for it), in us. A table is filled for the pass after it where it
+// costs no more than that pass saves (filter_gain). Measured, gss_state_set
+// with the table against without, 2^18 / 2^20 variables: 8 words 25/22, 47/41;
+// 13 words 31/26, 70/61; 32 words 44/41, 114/99; 64 words 80/72, 240/224.
 double table_cost(int64_t n_vars, int n_blocks, int bw, bool in_place) {
     const double rows = (double) n_vars * n_blocks, block_bytes = (double) n_vars * bw * sizeof(uint2);
     return in_place ? 3.0 + 4.0e-6 * rows + block_bytes * n_blocks / 6.0e6 : 1.2 + 4.0e-6 * rows + block_bytes / 25.0e6;

@@ -505,7 +505,7 @@ int Sharer::ensure_state() {
 
 int Sharer::set_filter_from(int64_t pairs) {
     if (pairs < -1) return set_error(GSS_ERR_INVALID, "pairs must be 0 or more, or -1 for the default");
-    filter_from_ = pairs < 0 ? kFilterMinPairs : pairs;
+    filter_from_ = pairs;
     return GSS_OK;
 }
 
@@ -1174,7 +1174,9 @@ int Sharer::launch_pass() {
         }
         // the filter's table follows while the database is large enough for it
         // and passes run behind it; after that it is filled anew
-        if (!agg_possible_ || filter_pause_.left > 0 || (int64_t) dev_clauses_ * n_blocks_ < filter_from_)
+        const bool pays = filter_from_ < 0 ? filter_gain(dev_clauses_, dev_words_) >= kTableUpkeep
+                                           : (int64_t) dev_clauses_ * n_blocks_ >= filter_from_;
+        if (!agg_possible_ || filter_pause_.left > 0 || !pays)
             agg_ok_ = false;
         else if (!agg_ok_)
             GSS_TRY(rebuild_agg());

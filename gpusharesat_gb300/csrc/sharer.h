@@ -21,10 +21,15 @@ namespace gss {
 constexpr uint8_t kTrue = 0, kFalse = 1, kUndef = 2;
 // records that come back with a pass's counters (256 KB of pinned memory)
 constexpr uint32_t kSharerInline = 16384 - kInlineOffset / sizeof(gss_report);
-// (clauses x slot blocks) from which the filter pays for its table's upkeep,
-// two launches a pass (7 solvers, 50k clauses: 120 us a pass without, 126
-// with; 64 solvers, 1.2e6 clauses: 220 us of check without, 85 with).
-constexpr int64_t kFilterMinPairs = 150000;
+// What the filter's table costs a pass in upkeep, in us: two launches over the
+// rows that changed, before the check and after it (filter_gain is what it
+// saves). Measured, two gpuRun calls with 8 updates a solver, filtered against
+// plain, 1e5 / 2e5 / 4e5 clauses of 2 to 100 literals over 2^18 variables: 5
+// solvers 35/32, 39/35, 43/42 us; 8 solvers 36/33, 41/36, 45/43; 16 solvers
+// 40/37, 44/41, 49/52; 32 solvers 41/45, 48/56, 53/74; 64 solvers 54/67, 57/85,
+// 67/115, and at 3e4 clauses 32 solvers 42/43, 64 solvers 47/50. 400 updates a
+// solver, 2^15 variables and 2 to 30 literals move the line little.
+constexpr double kTableUpkeep = 11.0;
 constexpr int kSlots = 32;  // assignments per solver per pass (Assigs.cuh:37-39)
 
 // Statistics, in the reference's order and with its names
@@ -315,7 +320,7 @@ private:
     bool agg_possible_ = false; // the layout has a filtered kernel
     bool agg_ok_ = false;       // d_agg_ follows the state
     FilterPause filter_pause_;  // passes to run without the filter (it kept too much)
-    int64_t filter_from_ = kFilterMinPairs;  // (clauses x slot blocks) from which passes run behind it
+    int64_t filter_from_ = -1;  // (clauses x slot blocks) from which passes run behind it; -1: where it pays
     int64_t filtered_passes_ = 0;
     PinnedBuf h_updates_;
     PinnedBuf h_append_;             // staging of appended clauses (literals, offsets, ids)

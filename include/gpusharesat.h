@@ -501,7 +501,8 @@ int gss_sharer_set_variant(gss_sharer *s, int kind, int lanes_per_clause, int de
  * appended from then on and to reduceDb. No counterpart in the reference. */
 int gss_sharer_set_locality(gss_sharer *s, int range_log2);
 /* (clauses x slot blocks) from which a pass of the automatic variant runs
- * behind the word-level filter (0 or more; -1 = the measured default), and how
+ * behind the word-level filter (0 or more; -1, the default, = where the pass
+ * saves more than the filter's table costs, by clauses and solvers), and how
  * many passes did (for tests and tuning). The reports do not depend on it. */
 int gss_sharer_set_filter_from(gss_sharer *s, int64_t pairs);
 int64_t gss_sharer_filtered_passes(gss_sharer *s);

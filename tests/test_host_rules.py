@@ -432,6 +432,26 @@ def test_sharer_drops_the_table_before_clauses(fake, make_sharer, grow):
     assert sharer.getGlobalStat("gpuReduceDbs") == before
 
 
+@pytest.mark.parametrize("n_solvers,below,above", [(8, 200_000, 600_000), (40, 30_000, 45_000)])
+def test_sharer_filters_where_it_pays(fake, make_sharer, n_solvers, below, above):
+    """The default line, by clauses and solvers: a database of so many clauses
+    is checked by the plain kernel, one of so many behind the filter."""
+    sharer = make_sharer(1 << 60)
+    sharer.setFilterFrom(-1)
+    sharer.setCpuSolverCount(n_solvers)
+    add, clause = sharer.lib.gss_sharer_add_clause, (ctypes.c_int * 3)(2, 5, 8)
+
+    def grow_to(n):
+        for _ in range(n - sharer.getAddedClauseCount()):
+            add(sharer.h, -1, clause, 3)
+        before = sharer.filteredPasses()
+        _some_passes(sharer)
+        return sharer.filteredPasses() - before
+
+    assert grow_to(below) == 0
+    assert grow_to(above) == 2
+
+
 def test_sharer_keeps_no_table_up_during_a_pause(fake, make_sharer):
     """One pass of which the filter keeps too much, then passes without it: no
     launch fills or refreshes the table until it is used again."""
