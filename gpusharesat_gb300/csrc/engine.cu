@@ -709,10 +709,11 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
     if (n_vars != eng->n_vars || n_words != eng->n_words) eng->filter_pause.end();
     eng->filter = eng->table_ok = false;
     eng->table_owed = 0;
-    const bool fill = may_filter && !eng->dense_before && eng->filter_pause.left == 0 &&
-                      filter_gain(eng->n_clauses, n_words) >=
-                          table_cost(n_vars, n_blocks, bw, laid_out && !read_state) &&
+    // (its room is had here in any case: later it would be a pass that waits)
+    const bool room = may_filter && !eng->dense_before && eng->filter_pause.left == 0 &&
                       eng->agg.reserve((size_t) n_blocks * n_vars * 2 * sizeof(uint2)) == GSS_OK;
+    const bool fill = room && filter_gain(eng->n_clauses, n_words) >=
+                                  table_cost(n_vars, n_blocks, bw, laid_out && !read_state);
     // the density's sample, in a corner of the counters' pinned buffer
     uint32_t *const h_density = (uint32_t *) ((char *) eng->h_counts.ptr + kDensityOffset);
     const uint64_t n_pairs = (uint64_t) n_vars * n_words;
