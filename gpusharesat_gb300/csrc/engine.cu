@@ -697,6 +697,9 @@ int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_
             (k == 0 ? read_state : read_masks) = false;
     }
     if (eng->pass_pending) GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
+    // a larger buffer takes the place of the state's: without it there is no
+    // state, and no pass of one
+    if (std::max<size_t>(bbytes, 8) > eng->state.bytes) eng->n_vars = eng->n_words = eng->n_blocks = 0;
     GSS_TRY(reserve_over_table(eng, eng->state, std::max<size_t>(bbytes, 8)));
     GSS_TRY(eng->start.reserve(std::max<size_t>(padded * sizeof(uint32_t), 4)));
     GSS_TRY(eng->solver_of_word.reserve(std::max<size_t>(padded * sizeof(int32_t), 4)));

@@ -136,6 +136,26 @@ def test_launcher_reports_the_runtime_error_and_asks_again(tmp_path, n_words):
     assert fake.lib.gss_engine_destroy(eng) == 0
 
 
+@pytest.mark.parametrize("n_words", [3, 20])
+def test_no_pass_of_a_state_that_found_no_room(fake, n_words):
+    """gss_state_set gives the old state's buffer up for a larger one; when that
+    cannot be had, the next pass is refused instead of reading nothing."""
+    rc, eng = fake.engine()
+    fake.lib.gss_engine_set_variant(eng, 0, 0, 2, 0)  # (the direct kernel: no table that could make room)
+    _database(fake, eng)
+    _state(fake, eng, n_words)
+    assert _passes(fake, eng, 1) == 0
+    state = (ctypes.c_uint32 * (2 * 5000 * n_words))()
+    start = (ctypes.c_uint32 * n_words)()
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 1)
+    assert fake.lib.gss_state_set(eng, state, i64(5000), n_words, start, None, 0) == -3
+    fake.reset()
+    assert fake.lib.gss_check_launch(eng) < 0 and not any("check" in l for l in fake.log())
+    _state(fake, eng, n_words)
+    assert fake.lib.gss_check_launch(eng) == 0, fake.error()
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
 def _append(fake, eng):
     n = 3000
     lits = (ctypes.c_int32 * (2 * n))(*[2 * (k % 50) for k in range(2 * n)])
