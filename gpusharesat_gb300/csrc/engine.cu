@@ -406,8 +406,8 @@ int upload_tiles(gss_engine *eng) {
     return GSS_OK;
 }
 
-// Copies the whole host mirror to the device (after a set or a compaction).
-int upload_all(gss_engine *eng) {
+// Copies the whole host mirror to the device.
+int upload_mirror(gss_engine *eng) {
     const int64_t n = (int64_t) eng->h_ids.size();
     const int64_t n_lits = eng->h_off.back();
     GSS_TRY(ensure_device(eng));
@@ -428,6 +428,24 @@ int upload_all(gss_engine *eng) {
     eng->alive_dirty = false;
     eng->tiles_stale = true;
     return GSS_OK;
+}
+
+// The same after a set or a compaction, which gave the old buffers up: where
+// that fails the database is empty, not half there.
+int upload_all(gss_engine *eng) {
+    const int rc = upload_mirror(eng);
+    if (rc == GSS_OK) return GSS_OK;
+    eng->h_lits.clear();
+    eng->h_off.assign(1, 0);
+    eng->h_ids.clear();
+    eng->index_of.clear();
+    eng->h_alive.clear();
+    eng->n_clauses = eng->n_lits = eng->n_dead = 0;
+    eng->max_var = -1;
+    eng->alive_dirty = false;
+    eng->tiles_stale = true;
+    eng->db_version++;
+    return rc;
 }
 
 // Variable-range order of a batch. The variables are cut into ranges of
@@ -540,14 +558,14 @@ int gss_db_append(gss_engine *eng, const int32_t *lits, const int64_t *offsets, 
     }
     const int64_t base = eng->h_off.empty() ? 0 : eng->h_off.back();
     if (base + offsets[n_clauses] > 0x7FFFFF00LL) return set_error(GSS_ERR_INVALID, "too many literals");
-    mirror_append(eng, lits, offsets, n_clauses, ids, std::max(eng->max_var, max_var));
-    const int64_t n = (int64_t) eng->h_ids.size();
-    const int64_t n_lits = eng->h_off.back();
+    const int64_t n = first + n_clauses, n_lits = base + offsets[n_clauses];
     GSS_TRY(ensure_device(eng));
     GSS_CUDA_TRY(cudaStreamSynchronize(eng->stream));
     GSS_TRY(grow_over_table(eng, eng->lits, (n_lits + 8) * sizeof(int32_t), base * sizeof(int32_t)));
     GSS_TRY(grow_over_table(eng, eng->offsets, (n + 1) * sizeof(int64_t), (first + 1) * sizeof(int64_t)));
     GSS_TRY(grow_over_table(eng, eng->orig, n * sizeof(uint32_t), first * sizeof(uint32_t)));
+    // (with the room for it: a batch that finds none leaves the database as it is)
+    mirror_append(eng, lits, offsets, n_clauses, ids, std::max(eng->max_var, max_var));
     // new literals, then zero padding past the end
     std::vector<int32_t> tail(eng->h_lits.begin() + base, eng->h_lits.end());
     tail.resize(tail.size() + 8, 0);

@@ -156,6 +156,53 @@ def test_no_pass_of_a_state_that_found_no_room(fake, n_words):
     assert fake.lib.gss_engine_destroy(eng) == 0
 
 
+def test_database_that_found_no_room_is_empty(fake):
+    """gss_db_set gives the old buffers up for larger ones; when those cannot be
+    had the database is empty, and later batches start from there."""
+    rc, eng = fake.engine()
+    fake.lib.gss_engine_set_variant(eng, 0, 0, 2, 0)  # (the direct kernel: no table that could make room)
+    fake.lib.gss_db_clause_count.restype = fake.lib.gss_db_live_count.restype = i64
+    _database(fake, eng)
+    _state(fake, eng, 3)
+    n = 3000
+    lits, offsets = (ctypes.c_int32 * (2 * n))(), (i64 * (n + 1))(*range(0, 2 * n + 1, 2))
+    for after in range(3):
+        fake.reset()
+        fake.fail("malloc", after)
+        assert fake.lib.gss_db_set(eng, lits, offsets, i64(n)) == -3
+        assert fake.lib.gss_db_clause_count(eng) == 0 and fake.lib.gss_db_live_count(eng) == 0
+        fake.reset()
+        assert fake.lib.gss_check_launch(eng) == 0 and fake.lib.gss_check_wait(eng, None) == 0
+        assert not any("check_kernel" in l for l in fake.log())
+        assert fake.lib.gss_db_append(eng, lits, offsets, i64(10), None) == 0, fake.error()
+        assert fake.lib.gss_db_clause_count(eng) == 10
+        assert fake.lib.gss_engine_destroy(eng) == 0  # (small buffers again)
+        rc, eng = fake.engine()
+        fake.lib.gss_engine_set_variant(eng, 0, 0, 2, 0)
+        _database(fake, eng)
+        _state(fake, eng, 3)
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
+def test_batch_that_found_no_room_changes_nothing(fake):
+    rc, eng = fake.engine()
+    fake.lib.gss_engine_set_variant(eng, 0, 0, 2, 0)
+    fake.lib.gss_db_clause_count.restype = fake.lib.gss_db_live_count.restype = i64
+    _database(fake, eng)
+    n = 3000
+    lits, offsets = (ctypes.c_int32 * (2 * n))(), (i64 * (n + 1))(*range(0, 2 * n + 1, 2))
+    ids = (ctypes.c_uint32 * n)(*range(200, 200 + n))
+    for after in (0, 1, 1):  # literals, offsets, ids: what was had stays
+        fake.fail("malloc", after)
+        assert fake.lib.gss_db_append(eng, lits, offsets, i64(n), ids) == -3
+        assert fake.lib.gss_db_clause_count(eng) == 100
+        assert fake.lib.gss_db_delete(eng, ids, i64(1)) == -6
+    fake.reset()
+    assert fake.lib.gss_db_append(eng, lits, offsets, i64(n), ids) == 0, fake.error()
+    assert fake.lib.gss_db_delete(eng, ids, i64(1)) == 0 and fake.lib.gss_db_live_count(eng) == 99 + n
+    assert fake.lib.gss_engine_destroy(eng) == 0
+
+
 def _append(fake, eng):
     n = 3000
     lits = (ctypes.c_int32 * (2 * n))(*[2 * (k % 50) for k in range(2 * n)])
