@@ -549,6 +549,12 @@ int Sharer::upload_db() {
     for (uint32_t i = 0; i < n; i++) meta_[i].lit_off = (uint32_t) offsets[i];
     std::vector<uint32_t> orig(std::max<uint32_t>(n, 1));
     for (uint32_t i = 0; i < n; i++) orig[i] = i;
+    // the old buffers are given up for larger ones: nothing is on the device
+    // until all of it is (launch_pass tries again)
+    dev_clauses_ = 0;
+    dev_lits_ = 0;
+    h_dev_meta_.clear();
+    upload_failed_ = true;
     GSS_TRY(reserve(d_lits_, lits.size() * sizeof(int32_t)));
     GSS_TRY(reserve(d_offsets_, (n + 1) * sizeof(int64_t)));
     GSS_TRY(reserve(d_orig_, orig.size() * sizeof(uint32_t)));
@@ -559,6 +565,7 @@ int Sharer::upload_db() {
     GSS_CUDA_TRY(cudaMemcpyAsync(d_orig_.ptr, orig.data(), orig.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                  stream_));
     GSS_CUDA_TRY(cudaStreamSynchronize(stream_));
+    upload_failed_ = false;
     dev_clauses_ = n;
     dev_lits_ = offsets[n];
     h_dev_meta_.resize(n);
@@ -1085,6 +1092,7 @@ int Sharer::launch_pass() {
     Pass &prev = pass_[cur_];
     Pass &p = pass_[cur_ ^ 1];
     GSS_TRY(deliver(p));  // delivered by the previous call already; kept for safety
+    if (upload_failed_) GSS_TRY(upload_db());
     std::vector<int64_t> ids;
     std::vector<int32_t> lits;
     std::vector<uint32_t> lens;

@@ -307,6 +307,7 @@ private:
     bool alive_synced_ = false;      // d_alive_ holds h_alive_ except [alive_lo_, alive_hi_)
     size_t alive_lo_ = SIZE_MAX, alive_hi_ = 0;
     int64_t device_compactions_ = 0;
+    bool upload_failed_ = false;  // the device has nothing of the database (upload_db)
 
     // assignments
     int n_vars_ = 0;

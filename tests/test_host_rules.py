@@ -553,6 +553,28 @@ def test_sharer_layout_that_ran_out_of_memory_is_made_again(fake, make_sharer, a
     assert any(l.startswith("copy") and l.split()[3] == str(4 * 32 * 35) for l in fake.log())
 
 
+def test_sharer_uploads_again_what_found_no_room(fake, make_sharer):
+    """The database does not fit twice over: gpuRun fails, no kernel runs over
+    buffers that are gone, and the next gpuRun brings all clauses back."""
+    import gpusharesat_gb300 as g
+    sharer = make_sharer(1 << 60)
+    for k in range(4000):  # clauses that a reduction keeps
+        assert sharer.addClause(-1, [2 * (k % 20), 2 * (20 + k % 20)]) >= 0
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 50)
+    for _ in range(2):
+        fake.reset()
+        with pytest.raises(g.GssError):
+            sharer.gpuRun()
+        assert not any("check_" in l and "kernel" in l for l in fake.log() if l.startswith("launch"))
+    fake.lib.gss_debug_fail_device_alloc(i64(0), 0)
+    fake.reset()
+    _some_passes(sharer)
+    clauses = sharer.getGlobalStat("gpuClauses")
+    assert clauses >= 4000
+    assert any(l.startswith("copy") and l.split()[3] == str(8 * (clauses + 1)) for l in fake.log())  # the offsets
+    assert sum("check_" in l for l in fake.log() if l.startswith("launch")) == 2
+
+
 def test_sharer_keeps_its_state_when_the_variant_changes(fake, make_sharer):
     """The values that the solvers sent go over to the new layout, which runs
     the kernel that was asked for."""
