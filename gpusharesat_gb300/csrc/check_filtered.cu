@@ -213,7 +213,7 @@ __device__ __forceinline__ uint32_t check_survivors(const CheckArgs &a, StagedRe
 // exact check.
 //
 // Bound by the L2's rate of random requests, a table entry each (ncu on 2e6
-// clauses x 1024 slots: 13.3M requests in 60 us, 220 G/s; the plain kernel
+// clauses x 1024 slots: 11.2M requests in 59 us, 189 G/s; the plain kernel
 // takes 245 us there). Hence: table entries keep their place in L2
 // (L1::no_allocate alone marks them evict-first there: half of them missed,
 // 86 us), nothing scattered is allocated in L1 (its 128-byte lines bound the

@@ -193,9 +193,9 @@ int gss_max_clause_len(void);
 /* Sets the assignment bit planes: state[n_vars][n_words][2] and
  * start[n_words] (slots to check in each word), and solver_of_word[n_words]
  * (may be NULL: word w belongs to solver w). `on_device` = 1 when the three
- * pointers are device pointers (copied device-to-device), 0 for host
- * pointers (copied host-to-device; pinned memory makes this asynchronous).
- * The copy is ordered on the engine's stream. */
+ * pointers are device pointers (read behind what the caller queued on the
+ * default stream; what lies on another GPU or between words is copied first),
+ * 0 for host pointers. The buffers are free when the call returns. */
 int gss_state_set(gss_engine *eng, const uint32_t *state, int64_t n_vars, int n_words,
                   const uint32_t *start, const int32_t *solver_of_word, int on_device);
 
